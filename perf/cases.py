@@ -15,7 +15,6 @@ Five kinds of work, each at the sizes its users run, the smallest included:
               32 KiB, the zero-copy form above.
 """
 import ctypes
-import gc
 import math
 import os
 
@@ -141,21 +140,36 @@ class _Collective:
         self.lib.call("flagcxEmuDestroy", self.handle)
 
 
+class _Training:
+    """A trainer that goes when the program drops it: its parameters' gradient hooks refer back to it, a cycle through
+    autograd that the garbage collector does not see, and it holds several GB."""
+
+    def __init__(self, model):
+        torch.cuda.empty_cache()  # what an earlier trainer's graph and side streams have left in the allocator
+        self.trainer = DataParallelTrainer(model)
+
+    def __del__(self):
+        for p in self.trainer.model.parameters():
+            if p._post_accumulate_grad_hooks is not None:
+                p._post_accumulate_grad_hooks.clear()
+            p.grad = None
+            p.data = p.data.new_empty(0)
+        self.trainer.__dict__.clear()
+
+
 def prepare(case, seed):
     kind = case["kind"]
     g = torch.Generator(device="cuda").manual_seed(seed)
     s = {"kind": kind}
     if kind == "train":
-        gc.collect()  # an earlier trainer's hooks refer to it in a cycle; its activations fill a good part of the GPU
-        torch.cuda.empty_cache()
         torch.manual_seed(seed)
         cfg = GPT2Config.medium() if case["model"] == "medium" else GPT2Config.tiny()
         with torch.device("cuda"):
             model = GPT2(cfg)
-        s["trainer"] = DataParallelTrainer(model)
+        s["training"] = _Training(model)
         s["tokens"], s["targets"] = (torch.randint(0, cfg.vocab, (case["batch"], case["seq"]), generator=g, device="cuda") for _ in range(2))
         for _ in range(3):  # a loop in its steady state: the third step has captured the graph
-            s["trainer"].step(s["tokens"], s["targets"])
+            s["training"].trainer.step(s["tokens"], s["targets"])
     elif kind == "linear":
         t, i, o = case["tokens"], case["n_in"], case["n_out"]
         s["x"], s["dy"] = _randn(g, t, i), _randn(g, t, o)
@@ -196,8 +210,9 @@ def prepare(case, seed):
 def run(s):
     kind = s["kind"]
     if kind == "train":
-        loss = s["trainer"].step(s["tokens"], s["targets"])
-        return {"loss": loss, "master": s["trainer"].master}
+        trainer = s["training"].trainer
+        loss = trainer.step(s["tokens"], s["targets"])
+        return {"loss": loss, "master": trainer.master}
     if kind == "linear":
         y = linear(s["x"], s["w"], s["bias"])
         dx, dw, db = torch.autograd.grad(y, (s["x"], s["w"], s["bias"]), s["dy"])
