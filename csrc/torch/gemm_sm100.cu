@@ -316,10 +316,6 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
             uint4 o = stg[rr * 8 + ((lane & 7) ^ (rr & 7))];
             if (row0 + rr < Mrows) {
               __nv_bfloat16 *d = dst0 + (size_t)rr * ldd + col;
-              if (MODE == FCX_GEMM_ROWMAP) {
-                const int4 info = p.rowInfo[row0 + rr];
-                d = (__nv_bfloat16 *)(dc.heap[info.x] + p.combineOff) + ((size_t)info.y * p.topk + info.z) * p.N + col;
-              }
               if (MODE == FCX_GEMM_PLAIN && (splitK > 1 || p.accumulate)) {
                 // one K piece of several, or a contribution to a gradient that is being accumulated: added into C
                 const uint32_t *w = (const uint32_t *)&o;
@@ -358,16 +354,6 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
   __syncthreads();
   fenceAfter();
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(512) : "memory");
-
-  if (MODE == FCX_GEMM_ROWMAP) {
-    // every row this CTA produced has been stored (possibly on peers): tell every rank that this CTA is done
-    __threadfence_system();
-    __syncthreads();
-    if ((int)threadIdx.x < dc.nranks) {
-      uint64_t *cnt = (uint64_t *)(dc.heap[threadIdx.x] + p.doneOff);
-      asm volatile("red.release.sys.global.add.u64 [%0], %1;" ::"l"(cnt), "l"((uint64_t)1) : "memory");
-    }
-  }
 
   // ------------------------------------------------------------ RS: reduce the tiles this rank owns
   if (MODE == FCX_GEMM_RS) {
@@ -570,23 +556,6 @@ extern "C" cudaError_t fcxGemmBf16DynM(const void *a, const void *b, void *c, in
   FcxDevComm dc{};
   int tiles = ((Mmax + BM - 1) / BM) * ((N + bn - 1) / bn);
   return launch<FCX_GEMM_PLAIN>(ma, mb, p, dc, std::min(tiles, smCount()), s);
-}
-
-extern "C" cudaError_t fcxGemmRowMapBf16(const FcxDevComm *dc, const void *a, const void *b, int Mmax, const int *mPtr, int N, int K, int lda,
-                                         int ldb, const void *rowInfo, size_t combineOff, size_t doneOff, int topk, int *errFlag,
-                                         int *gridOut, cudaStream_t s) {
-  if (K % 8 || lda % 8 || ldb % 8 || N % 8 || Mmax <= 0) return cudaErrorInvalidValue;
-  CUtensorMap ma, mb;
-  const int bn = pickBn(Mmax, N, smCount());
-  if (!makeMap(&ma, a, Mmax, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, bn)) return cudaErrorNotSupported;
-  FcxGemmParams p{};
-  p.M = Mmax; p.N = N; p.K = K; p.c = nullptr; p.ldc = N; p.errFlag = errFlag; p.mPtr = mPtr;
-  p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
-  p.rowInfo = (const int4 *)rowInfo; p.combineOff = combineOff; p.doneOff = doneOff; p.topk = topk;
-  // a fixed grid: the receivers count one arrival per CTA of every rank
-  int grid = smCount();
-  if (gridOut) *gridOut = grid;
-  return launch<FCX_GEMM_ROWMAP>(ma, mb, p, *dc, grid, s);
 }
 
 extern "C" cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, const void *gathered, size_t gatherOff, size_t flagOff,

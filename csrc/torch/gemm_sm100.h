@@ -7,7 +7,6 @@
 #define FCX_GEMM_PLAIN 0
 #define FCX_GEMM_AG 1
 #define FCX_GEMM_RS 2
-#define FCX_GEMM_ROWMAP 3
 
 struct FcxGemmParams {
   int M, N, K;          // C[M,N] = A[M,K] * B[N,K]^T, bf16 in, fp32 accumulate, bf16 out
@@ -15,7 +14,7 @@ struct FcxGemmParams {
   int ldc;
   int rotate;           // first row block (of 128 rows) this rank works on
   int bn;               // columns per tile: 256 or 128 (RS: 256)
-  int group;            // PLAIN/ROWMAP: row blocks per band of the tile order (0: row-major)
+  int group;            // PLAIN: row blocks per band of the tile order (0: row-major)
   int rowsPerRank;      // M / nranks (AG, RS)
   int gemmCtas;         // AG: CTAs [0, gemmCtas) compute, the rest move data
   const void *aLocal;   // AG: this rank's [rowsPerRank, K] block
@@ -25,12 +24,6 @@ struct FcxGemmParams {
   uint64_t epoch;       // 1-based use count of the flag/counter array that flagOff points to
   int *errFlag;         // device int, set to 1 when a bounded wait gave up
   const int *mPtr;      // optional device-resident row count (<= M); rows beyond it are neither computed nor stored
-  // ROWMAP (mixture-of-experts combine): output row r goes to rank rowInfo[r].x, token rowInfo[r].y, choice rowInfo[r].z:
-  // heap[rank] + combineOff + ((token * topk + choice) * N) bf16 elements; afterwards every CTA adds 1 to the u64 counter
-  // at doneOff on every rank.
-  const int4 *rowInfo;
-  size_t combineOff, doneOff;
-  int topk;
   // PLAIN only.  Operand storage: 0 = K-major (A is [M,K], B is [N,K], rows contiguous along K, the default);
   // 1 = MN-major (A is stored [K,M], B is stored [K,N]: the transposed operands of the backward GEMMs, read
   // where they lie instead of being transposed first).
@@ -74,9 +67,6 @@ const char *fcxGemmLastDetail();  // what the calling thread's last failed fcxGe
 // c[Mmax,N] = a[*mPtr rows, K] @ b^T with the row count read on the device.
 cudaError_t fcxGemmBf16DynM(const void *a, const void *b, void *c, int Mmax, const int *mPtr, int N, int K, int lda, int ldb, int ldc,
                             int *errFlag, cudaStream_t s);
-// Expert output GEMM with the combine all-to-all fused into its epilogue (see FcxGemmParams::rowInfo).
-cudaError_t fcxGemmRowMapBf16(const FcxDevComm *dc, const void *a, const void *b, int Mmax, const int *mPtr, int N, int K, int lda, int ldb,
-                              const void *rowInfo, size_t combineOff, size_t doneOff, int topk, int *errFlag, int *gridOut, cudaStream_t s);
 #ifdef __cplusplus
 }
 #endif

@@ -6,6 +6,7 @@
 #include "flagcx.h"
 #include "flagcx_ext.h"
 #include "gemm_sm100.h"
+#include "moe_gemm_sm100.h"
 #include "moe_sm100.h"
 
 namespace fcxt {
@@ -77,21 +78,53 @@ static void gemmDynM(const at::Tensor &a, const at::Tensor &b, at::Tensor &c, co
   TORCH_CHECK(e == cudaSuccess, "tcgen05 GEMM launch failed: ", cudaGetErrorString(e));
 }
 
-// Expert output projection whose epilogue returns every row to the rank the token came from.  Returns the grid size:
-// each of its CTAs adds 1 to done_counter on every rank.
-static int64_t gemmRowMap(uint64_t comm, const at::Tensor &a, const at::Tensor &b, const at::Tensor &mPtr, const at::Tensor &info,
-                          at::Tensor &combine, at::Tensor &doneCounter, int64_t topk, at::Tensor &err) {
-  checkBf16Mat(a, "a");
-  checkBf16Mat(b, "b");
-  TORCH_CHECK(a.size(1) == b.size(1), "inner dimensions differ");
-  TORCH_CHECK(info.scalar_type() == at::kInt && info.numel() >= a.size(0) * 4, "info must be int32 [rows, 4]");
-  c10::cuda::CUDAGuard g(a.device());
+// The weights of this rank's experts as the launchers take them: pointers and row strides.
+static void expertWeights(const std::vector<at::Tensor> &w, int64_t rows, int64_t cols, std::vector<const void *> &ptrs, std::vector<int> &ld) {
+  TORCH_CHECK(!w.empty() && w.size() <= FCX_MOE_MAX_EXPERTS, "between 1 and ", FCX_MOE_MAX_EXPERTS, " expert weights");
+  for (const at::Tensor &t : w) {
+    checkBf16Mat(t, "expert weight");
+    TORCH_CHECK(t.size(0) == rows && t.size(1) == cols, "expert weights must be [", rows, ", ", cols, "]");
+    ptrs.push_back(t.data_ptr());
+    ld.push_back((int)t.stride(0));
+  }
+}
+
+// h = silu(x wg^T) * (x wu^T) for every local expert in one launch.  x [L * capL, H], h [L * capL, F], w: L x [2F, H], rows int32 [L].
+static void moeUp(const at::Tensor &x, const std::vector<at::Tensor> &w, at::Tensor &h, const at::Tensor &rows, at::Tensor &err) {
+  checkBf16Mat(x, "x");
+  checkBf16Mat(h, "h");
+  const int64_t L = (int64_t)w.size();
+  TORCH_CHECK(x.is_contiguous() && h.is_contiguous() && h.size(0) == x.size(0) && L > 0 && x.size(0) % (L * 128) == 0,
+              "x and h must be contiguous, with a multiple of 128 rows per expert");
+  TORCH_CHECK(rows.is_cuda() && rows.scalar_type() == at::kInt && rows.numel() >= L, "rows must be int32 [L]");
+  std::vector<const void *> ptrs;
+  std::vector<int> ld;
+  expertWeights(w, 2 * h.size(1), x.size(1), ptrs, ld);
+  c10::cuda::CUDAGuard g(x.device());
+  auto e = fcxMoeUpGrouped(x.data_ptr(), ptrs.data(), h.data_ptr(), rows.data_ptr<int>(), (int)L, (int)(x.size(0) / L), (int)x.size(1),
+                           (int)h.size(1), ld.data(), err.data_ptr<int>(), cur());
+  TORCH_CHECK(e == cudaSuccess, "grouped expert GEMM launch failed: ", cudaGetErrorString(e));
+}
+
+// Expert output projections, all experts in one launch, whose epilogue returns every row to the rank the token came from.
+// Returns the grid size: each of its CTAs adds 1 to done_counter on every rank.
+static int64_t moeDown(uint64_t comm, const at::Tensor &h, const std::vector<at::Tensor> &w, const at::Tensor &rows, const at::Tensor &info,
+                       at::Tensor &combine, at::Tensor &doneCounter, int64_t topk, at::Tensor &err) {
+  checkBf16Mat(h, "h");
+  const int64_t L = (int64_t)w.size();
+  TORCH_CHECK(h.is_contiguous() && L > 0 && h.size(0) % (L * 128) == 0, "h must be contiguous, with a multiple of 128 rows per expert");
+  TORCH_CHECK(rows.is_cuda() && rows.scalar_type() == at::kInt && rows.numel() >= L, "rows must be int32 [L]");
+  TORCH_CHECK(info.scalar_type() == at::kInt && info.numel() >= h.size(0) * 4, "info must be int32 [rows, 4]");
+  std::vector<const void *> ptrs;
+  std::vector<int> ld;
+  expertWeights(w, w[0].size(0), h.size(1), ptrs, ld);
+  c10::cuda::CUDAGuard g(h.device());
   FcxDevComm dc = devComm(comm);
   int grid = 0;
-  auto e = fcxGemmRowMapBf16(&dc, a.data_ptr(), b.data_ptr(), (int)a.size(0), mPtr.data_ptr<int>(), (int)b.size(0), (int)a.size(1),
-                             (int)a.stride(0), (int)b.stride(0), info.data_ptr(), heapOffset(comm, combine), heapOffset(comm, doneCounter),
-                             (int)topk, err.data_ptr<int>(), &grid, cur());
-  TORCH_CHECK(e == cudaSuccess, "fused GEMM combine launch failed: ", cudaGetErrorString(e));
+  auto e = fcxMoeDownGrouped(&dc, h.data_ptr(), ptrs.data(), rows.data_ptr<int>(), (int)L, (int)(h.size(0) / L), (int)w[0].size(0),
+                             (int)h.size(1), ld.data(), info.data_ptr(), heapOffset(comm, combine), heapOffset(comm, doneCounter), (int)topk,
+                             err.data_ptr<int>(), &grid, cur());
+  TORCH_CHECK(e == cudaSuccess, "grouped expert GEMM + combine launch failed: ", cudaGetErrorString(e));
   return grid;
 }
 
@@ -114,7 +147,8 @@ void bindMoe(py::module &m) {
         py::arg("err"), py::arg("ctas"), py::arg("experts_per_rank") = 1);
   m.def("silu_mul", &siluMul, py::arg("gu"), py::arg("h"), py::arg("rows") = py::none());
   m.def("gemm_dyn_m", &gemmDynM);
-  m.def("gemm_rowmap", &gemmRowMap);
+  m.def("moe_up", &moeUp);
+  m.def("moe_down", &moeDown);
   m.def("moe_combine", &moeCombine);
 }
 

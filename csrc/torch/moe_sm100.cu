@@ -9,10 +9,10 @@
 //                   with a (source rank, token, choice) record, and returns
 //                   once every source has finished writing into this rank.
 //                   The number of rows received stays on the device.
-//   (expert MLP)    tcgen05 GEMMs with a device-resident row count
-//                   (gemm_sm100.cu); the down projection runs in ROWMAP mode:
-//                   its epilogue stores every output row directly into the
-//                   combine buffer of the rank the token came from.
+//   (expert MLP)    grouped tcgen05 GEMMs with device-resident row counts
+//                   (moe_gemm_sm100.cu); the down projection's epilogue
+//                   stores every output row directly into the combine buffer
+//                   of the rank the token came from.
 //   fcxMoeCombine   waits for every CTA of every expert to report, then
 //                   out[t] = sum_k w[t,k] * returned[t,k].
 //
@@ -40,33 +40,37 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
   const int n = dc.nranks, me = dc.rank, L = p.L, E = n * L, capL = p.cap / L;
   const int entries = p.T * p.K;
   __shared__ int warpTotals[THREADS / 32];
-  __shared__ int running;
   volatile int *err = p.errFlag;
 
-  // ---- phase 1: CTA e numbers, in token order, the entries routed to expert e
+  // ---- phase 1: CTA e numbers, in token order, the entries routed to expert e.  Every warp counts a contiguous stretch
+  // of the entries, one barrier shares the counts, and a second look (in L1 by then) hands out the numbers.  In steps of
+  // a whole CTA, four barriers each, 16384 entries took 32 dependent steps.
   if ((int)blockIdx.x < E) {
-    const int e = blockIdx.x;
-    if (threadIdx.x == 0) running = 0;
+    const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int WARPS = THREADS / 32;
+    const int per = ((entries + WARPS - 1) / WARPS + 31) / 32 * 32;
+    const int lo = min(entries, warp * per), hi = min(entries, lo + per);
+    int mine = 0;
+#pragma unroll 8
+    for (int i = lo + lane; i < hi; i += 32) mine += p.topkIdx[i] == e ? 1 : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if (lane == 0) warpTotals[warp] = mine;
     __syncthreads();
-    for (int base = 0; base < entries; base += THREADS) {
-      const int i = base + threadIdx.x;
-      const int hit = (i < entries && p.topkIdx[i] == e) ? 1 : 0;
-      const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      const int before = __popc(ballot & ((1u << lane) - 1));
-      if (lane == 0) warpTotals[warp] = __popc(ballot);
-      __syncthreads();
-      int warpBase = 0, total = 0;
-      for (int w = 0; w < THREADS / 32; w++) {
-        if (w < warp) warpBase += warpTotals[w];
-        total += warpTotals[w];
-      }
-      if (hit) p.slot[i] = running + warpBase + before;
-      __syncthreads();
-      if (threadIdx.x == 0) running += total;
-      __syncthreads();
+    int running = 0, total = 0;
+    for (int w = 0; w < WARPS; w++) {
+      if (w < warp) running += warpTotals[w];
+      total += warpTotals[w];
     }
-    if (threadIdx.x == 0) p.localCounts[e] = running;
+#pragma unroll 4
+    for (int base = lo; base < hi; base += 32) {
+      const int i = base + lane;
+      const bool hit = i < hi && p.topkIdx[i] == e;
+      const unsigned ballot = __ballot_sync(0xffffffffu, hit);
+      if (hit) p.slot[i] = running + __popc(ballot & ((1u << lane) - 1));
+      running += __popc(ballot);
+    }
+    if (threadIdx.x == 0) p.localCounts[e] = total;
   }
   __threadfence();
   grid.sync();
@@ -115,6 +119,13 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
       const uint4 *src = (const uint4 *)((const __nv_bfloat16 *)p.x + (size_t)t * p.H);
       uint4 *dst = (uint4 *)(dc.heap[dstRank] + p.recvOff + (size_t)pos * p.H * 2);
       int v = lane;
+      for (; v + 224 < vecs; v += 256) {  // eight 16-byte loads in flight per lane
+        uint4 r[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = src[v + 32 * j];
+#pragma unroll
+        for (int j = 0; j < 8; j++) dst[v + 32 * j] = r[j];
+      }
       for (; v + 96 < vecs; v += 128) {
         uint4 a = src[v], b = src[v + 32], c = src[v + 64], d = src[v + 96];
         dst[v] = a; dst[v + 32] = b; dst[v + 64] = c; dst[v + 96] = d;
@@ -163,7 +174,11 @@ __global__ void __launch_bounds__(256) siluMulKernel(const __nv_bfloat16 *__rest
   }
 }
 
-// out[t] = sum_k w[t,k] * ret[t,k], after every CTA of every expert's output GEMM has reported
+// out[t] = sum_k w[t,k] * ret[t,k], after every CTA of every expert's output GEMM has reported.
+// KC > 0: K is KC (1, 2, 4), 8 / KC output vectors per thread and step with every choice's row loaded before the first is
+// used, eight 16-byte loads in flight; positions in 32 bits (their 64-bit divisions cost more than the loads).
+// KC = 0: any K and any size, one vector at a time.
+template <int KC>
 __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, const __nv_bfloat16 *__restrict__ ret, const float *__restrict__ w,
                                                         __nv_bfloat16 *__restrict__ out, int T, int H, int K, size_t doneOff, uint64_t want,
                                                         int *errFlag) {
@@ -174,34 +189,36 @@ __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, con
   }
   if (!__syncthreads_and(ok)) return;
   const size_t vecPerRow = H / 8, total = (size_t)T * vecPerRow, stride = (size_t)gridDim.x * blockDim.x;
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (K <= 4) {
-    // two output vectors per thread and step, every choice's row loaded before the first is used: up to eight
-    // 16-byte loads in flight per thread (the kernel is bound by load latency, not by bytes)
-    for (; i < total; i += 2 * stride) {
-      const size_t pos[2] = {i, i + stride};
-      uint4 v[2][4];
-      float wk[2][4];
+  if constexpr (KC > 0) {
+    constexpr int U = 8 / KC;
+    const uint32_t tot = (uint32_t)total, per = (uint32_t)vecPerRow, step = (uint32_t)stride;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < tot; i += U * step) {
+      uint4 v[U][KC];
+      float wk[U][KC];
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const bool live = pos[u] < total;
-        const size_t t = live ? pos[u] / vecPerRow : 0, c = live ? pos[u] % vecPerRow : 0;
+      for (int u = 0; u < U; u++) {
+        const uint32_t pos = min(i + u * step, tot - 1), t = pos / per, c = pos - t * per;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          wk[u][k] = (live && k < K) ? w[t * K + k] : 0.f;
-          // a choice that was not dispatched (expert id out of range, capacity overflow) has weight 0 and no row
-          v[u][k] = wk[u][k] != 0.f ? *(const uint4 *)(ret + ((t * K + k) * H) + c * 8) : make_uint4(0, 0, 0, 0);
+        for (int k = 0; k < KC; k++) {
+          wk[u][k] = w[t * KC + k];
+          // volatile: the compiler would move each load behind the test of its weight, one at a time
+          asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(v[u][k].x), "=r"(v[u][k].y), "=r"(v[u][k].z), "=r"(v[u][k].w)
+                       : "l"(ret + ((size_t)t * KC + k) * H + c * 8) : "memory");
         }
       }
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
+      for (int u = 0; u < U; u++) {
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < KC; k++) {
+          // a choice that was not dispatched (expert id out of range, capacity overflow) has weight 0 and whatever the
+          // buffer holds in the place of a row
+          if (wk[u][k] == 0.f) v[u][k] = make_uint4(0, 0, 0, 0);
           const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&v[u][k];
 #pragma unroll
           for (int j = 0; j < 4; j++) {
-            float2 f = __bfloat1622float2(h2[j]);
+            const float2 f = __bfloat1622float2(h2[j]);
             acc[2 * j] += wk[u][k] * f.x;
             acc[2 * j + 1] += wk[u][k] * f.y;
           }
@@ -210,34 +227,32 @@ __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, con
         __nv_bfloat162 *o2 = (__nv_bfloat162 *)&o;
 #pragma unroll
         for (int j = 0; j < 4; j++) o2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-        if (pos[u] < total) {
-          const size_t t = pos[u] / vecPerRow, c = pos[u] % vecPerRow;
-          *(uint4 *)(out + t * H + c * 8) = o;
+        const uint32_t pos = i + u * step;
+        if (pos < tot) *(uint4 *)(out + (size_t)pos * 8) = o;  // out is contiguous
+      }
+    }
+  } else {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+      const size_t t = i / vecPerRow, c = i % vecPerRow;
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int k = 0; k < K; k++) {
+        const float wk = w[t * K + k];
+        if (wk == 0.f) continue;  // a choice that was not dispatched (expert id out of range, capacity overflow) has no row
+        uint4 v = *(const uint4 *)(ret + ((t * K + k) * H) + c * 8);
+        const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&v;
+  #pragma unroll
+        for (int j = 0; j < 4; j++) {
+          float2 f = __bfloat1622float2(h2[j]);
+          acc[2 * j] += wk * f.x;
+          acc[2 * j + 1] += wk * f.y;
         }
       }
+      uint4 o;
+      __nv_bfloat162 *o2 = (__nv_bfloat162 *)&o;
+  #pragma unroll
+      for (int j = 0; j < 4; j++) o2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+      *(uint4 *)(out + t * H + c * 8) = o;
     }
-    return;
-  }
-  for (; i < total; i += stride) {
-    const size_t t = i / vecPerRow, c = i % vecPerRow;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < K; k++) {
-      const float wk = w[t * K + k];
-      if (wk == 0.f) continue;  // a choice that was not dispatched (expert id out of range, capacity overflow) has no row
-      uint4 v = *(const uint4 *)(ret + ((t * K + k) * H) + c * 8);
-      const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&v;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        float2 f = __bfloat1622float2(h2[j]);
-        acc[2 * j] += wk * f.x;
-        acc[2 * j + 1] += wk * f.y;
-      }
-    }
-    uint4 o;
-    __nv_bfloat162 *o2 = (__nv_bfloat162 *)&o;
-#pragma unroll
-    for (int j = 0; j < 4; j++) o2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-    *(uint4 *)(out + t * H + c * 8) = o;
   }
 }
 
@@ -262,6 +277,10 @@ extern "C" cudaError_t fcxSiluMul(const void *gu, void *h, const int *rows, int 
 extern "C" cudaError_t fcxMoeCombine(const FcxDevComm *dc, const void *ret, const float *w, void *out, int T, int H, int K, size_t doneOff,
                                      uint64_t want, int *errFlag, cudaStream_t s) {
   if (H % 8) return cudaErrorInvalidValue;
-  moeCombineKernel<<<296, 256, 0, s>>>(*dc, (const __nv_bfloat16 *)ret, w, (__nv_bfloat16 *)out, T, H, K, doneOff, want, errFlag);
+  // positions may run past the total by up to eight grid strides
+  const bool small = (uint64_t)T * (H / 8) + 16ull * 592 * 256 < (1ull << 32);
+  auto kernel = !small ? moeCombineKernel<0> : K == 1 ? moeCombineKernel<1> : K == 2 ? moeCombineKernel<2> : K == 4 ? moeCombineKernel<4>
+                                                                                                                 : moeCombineKernel<0>;
+  kernel<<<592, 256, 0, s>>>(*dc, (const __nv_bfloat16 *)ret, w, (__nv_bfloat16 *)out, T, H, K, doneOff, want, errFlag);
   return cudaGetLastError();
 }

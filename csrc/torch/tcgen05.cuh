@@ -108,6 +108,44 @@ __device__ __forceinline__ void mmaF8(uint32_t dTmem, uint64_t aDesc, uint64_t b
       ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// ------------------------------------------------------------------ CTA pairs (cta_group::2)
+
+__device__ __forceinline__ uint32_t ctaRankInCluster() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Address of the same shared-memory location in CTA `rank` of this cluster.
+__device__ __forceinline__ uint32_t mapToCta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void clusterSync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// TMA tile load into this CTA's shared memory whose bytes are counted on a barrier of the pair's leader CTA.
+__device__ __forceinline__ void tmaLoad2dPair(void *smemDst, const CUtensorMap *map, int x, int y, uint32_t barClusterAddr) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(smemAddr(smemDst)), "l"(map), "r"(x), "r"(y), "r"(barClusterAddr) : "memory");
+}
+__device__ __forceinline__ void mmaF16Pair(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrive on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are done.
+__device__ __forceinline__ void mmaCommitPair(uint64_t *bar) {
+  const uint16_t both = 3;
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smemAddr(bar)), "h"(both) : "memory");
+}
+__device__ __forceinline__ void mbarArriveRemote(uint32_t barClusterAddr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(barClusterAddr) : "memory");
+}
+
 // ------------------------------------------------------------------ host side
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

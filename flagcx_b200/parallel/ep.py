@@ -1,19 +1,18 @@
 """Expert-parallel mixture-of-experts layer (one or several experts per rank, top-k routing).
 
-Fused path (``ExpertParallelContext.forward``), five launches and no host
+Fused path (``ExpertParallelContext.forward``), four launches and no host
 round trip:
 
 1. ``moe_dispatch``  one cooperative kernel: per-expert counts, count-matrix
    exchange through the symmetric heap, token push over NVLink into the
    expert's segment of its rank's input buffer; the received row counts
-   (one per local expert) stay on the device.  Steps 2-4 run once per
-   local expert.
-2. up/gate GEMM      tcgen05 GEMM whose row count is read on the device.
-3. ``silu_mul``
-4. down GEMM         tcgen05 GEMM in ROWMAP mode: the epilogue stores every
-   output row straight into the combine buffer of the token's home rank
-   (the combine all-to-all never exists as a separate step).
-5. ``moe_combine``   waits for every expert's GEMM CTAs, then the weighted
+   (one per local expert) stay on the device.
+2. ``moe_up``        gate and up projections of all local experts as one
+   grouped tcgen05 GEMM, with silu(gate) * up in its epilogue.
+3. ``moe_down``      down projections, grouped likewise: the epilogue stores
+   every output row straight into the combine buffer of the token's home
+   rank (the combine all-to-all never exists as a separate step).
+4. ``moe_combine``   waits for every rank's GEMM CTAs, then the weighted
    sum over the k choices.
 
 Unfused path (``unfused_forward``): what a FlagCX user writes today:
@@ -82,7 +81,6 @@ class ExpertParallelContext:
         self.local_counts = torch.zeros(nranks * self.L, dtype=i32, device=dev)
         self.recv_total = torch.zeros(self.L, dtype=i32, device=dev)  # rows received per local expert
         self.err = torch.zeros(1, dtype=i32, device=dev)
-        self.gu = torch.empty(self.cap, 2 * ffn, dtype=bf, device=dev)
         self.h = torch.empty(self.cap, ffn, dtype=bf, device=dev)
         self.calls = 0
         self.comb_want = [0, 0]
@@ -107,14 +105,11 @@ class ExpertParallelContext:
         nat.moe_dispatch(self.comm, x, topk_idx, self.count_mat[par], self.count_flags[par], self.recv[par], self.info[par],
                          self.disp_done[par], epoch, self.slot, self.local_counts, self.recv_total, self.err, self.dispatch_ctas,
                          self.L)
-        for l in range(self.L):  # every local expert works on its own segment, sized on the device by its row count
-            seg = slice(l * self.cap_l, (l + 1) * self.cap_l)
-            rows = self.recv_total[l:l + 1]
-            nat.gemm_dyn_m(self.recv[par][seg], w_gate_up[l], self.gu[seg], rows, self.err)
-            nat.silu_mul(self.gu[seg], self.h[seg], rows)
-            grid = nat.gemm_rowmap(self.comm, self.h[seg], w_down[l], rows, self.info[par][seg], self.combine[par], self.comb_done[par],
-                                   self.K, self.err)
-            self.comb_want[par] += grid * self.n  # every rank launches the same grids
+        # every local expert works on its own segment, sized on the device by its row count; all of them share a launch
+        nat.moe_up(self.recv[par], [w_gate_up[l] for l in range(self.L)], self.h, self.recv_total, self.err)
+        grid = nat.moe_down(self.comm, self.h, [w_down[l] for l in range(self.L)], self.recv_total, self.info[par], self.combine[par],
+                            self.comb_done[par], self.K, self.err)
+        self.comb_want[par] += grid * self.n  # every rank launches the same grid
         nat.moe_combine(self.comm, self.combine[par], topk_w, out, self.comb_done[par], self.comb_want[par], self.err)
         return out
 

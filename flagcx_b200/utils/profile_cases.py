@@ -208,7 +208,7 @@ def main():
         return
     elif args.case in ("moe_dispatch", "moe_layer"):
         # one-rank communicator: the dispatch kernel (count, exchange, push), the device-row-count GEMMs,
-        # the ROWMAP epilogue and the combine kernel all run, with this GPU as its own peer
+        # the row-scattering epilogue and the combine kernel all run, with this GPU as its own peer
         import os
         os.environ.setdefault("FLAGCX_HEAP_USER_BYTES", "1G")
         from flagcx_b200.parallel.ep import ExpertParallelContext
