@@ -558,11 +558,22 @@ extern "C" cudaError_t fcxGemmBf16DynM(const void *a, const void *b, void *c, in
   return launch<FCX_GEMM_PLAIN>(ma, mb, p, dc, std::min(tiles, smCount()), s);
 }
 
+// All-gather -> GEMM and GEMM -> reduce-scatter of one rank: there is nothing to exchange, so the plain GEMM writes the
+// result itself (as CTA pairs where the shape suits) in place of a copy of the partial tiles in the staging area that is
+// then read back.  K is not cut: the sums stay fp32 until the one rounding, as in the fused kernels.
+static cudaError_t oneRank(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int *errFlag, cudaStream_t s) {
+  FcxGemmOpts o{};
+  o.splitK = 1;
+  o.pair = -1;
+  return fcxGemmBf16Opts(a, b, c, M, N, K, lda, ldb, ldc, &o, errFlag, s);
+}
+
 extern "C" cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, const void *gathered, size_t gatherOff, size_t flagOff,
                                      const void *b, void *c, int M, int N, int K, int ldb, int ldc, uint64_t epoch, int commCtas,
                                      int *errFlag, cudaStream_t s) {
   const int n = dc->nranks;
   if (K % 8 || ldb % 8 || ldc % 8 || M % (n * BM) || commCtas < 1) return cudaErrorInvalidValue;
+  if (n == 1) return oneRank(aLocal, b, c, M, N, K, K, ldb, ldc, errFlag, s);
   CUtensorMap ma, mb;
   const int bn = pickBn(M, N, std::max(1, smCount() - commCtas));
   CUtensorMap mal;
@@ -583,6 +594,7 @@ extern "C" cudaError_t fcxGemmRsBf16(const FcxDevComm *dc, const void *a, const 
                                      int N, int K, int lda, int ldb, int ldc, uint64_t epoch, int *errFlag, cudaStream_t s) {
   const int n = dc->nranks;
   if (K % 8 || lda % 8 || ldb % 8 || ldc % 8 || N % 8 || M % (n * BM)) return cudaErrorInvalidValue;
+  if (n == 1) return oneRank(a, b, out, M, N, K, lda, ldb, ldc, errFlag, s);
   CUtensorMap ma, mb;
   if (!makeMap(&ma, a, M, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, BN)) return cudaErrorNotSupported;
   FcxGemmParams p{};

@@ -100,6 +100,11 @@ class TensorParallelContext:
         stage = self.rs_stage[par].view(-1)[: rows * n_out]
         return self.nat.gemm_rs(self.comm, a, w, stage, self.rs_counters[par], epoch, self.err)
 
+    def plain_gemm_nn(self, a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+        """``a @ w`` for the backward pass of a single rank: nothing is exchanged, so the plain GEMM reads the weight
+        transposed where it lies (no transposed copy of it, no gathered copy of ``a``).  The sum over K is not cut."""
+        return self.nat.gemm(a, w, False, True, None, 1, self.err)
+
     def check(self):
         """Raise if a kernel of this context gave up on a wait (call after a synchronize)."""
         if int(self.err.item()) != 0:
@@ -152,7 +157,10 @@ class _ColumnParallel(torch.autograd.Function):
         # peers will push into again a few calls from now, and they cannot get there before this rank has
         # contributed to the reduce-scatter below.
         dw = gemm(dy, full, True, True)              # [N, rows] @ [rows, K]
-        dx_local = tp.gemm_rs(dy, tp.transposed(w))  # [rows, N] @ [N, K] -> rows/n x K
+        if tp.n == 1:
+            dx_local = tp.plain_gemm_nn(dy, w)
+        else:
+            dx_local = tp.gemm_rs(dy, tp.transposed(w))  # [rows, N] @ [N, K] -> rows/n x K
         return dx_local, dw, None
 
 
@@ -176,8 +184,11 @@ class _RowParallel(torch.autograd.Function):
         a, w = ctx.saved_tensors
         tp = ctx.tp
         dz_local = dz_local.contiguous()
-        da = tp.ag_gemm(dz_local, tp.transposed(w))  # [rows, N] @ [N, K_local]
-        full = tp.last_gathered(dz_local)
+        if tp.n == 1:
+            da, full = tp.plain_gemm_nn(dz_local, w), dz_local
+        else:
+            da = tp.ag_gemm(dz_local, tp.transposed(w))  # [rows, N] @ [N, K_local]
+            full = tp.last_gathered(dz_local)
         dw = gemm(full, a, True, True)               # [N, rows] @ [rows, K_local]
         return da, dw, None
 
