@@ -4,21 +4,21 @@
 // layers: activations carry one fp32 scale per row and 128 columns of K
 // (sa[K/128][M]), weights one per 128x128 block (sb[ceil(N/128)][K/128]).
 // The tensor cores cannot apply such scales themselves, so every 128-deep
-// slice of K is multiplied into its own TMEM accumulator (tcgen05.mma
+// slice of K is multiplied into a TMEM accumulator of its own (tcgen05.mma
 // kind::f8f6f4, fp32 accumulate) and the epilogue warps fold it into
 // registers as acc += sa[row,kb] * sb[nb,kb] * partial while the next slices
-// are already being multiplied: four TMEM accumulators of 128 columns rotate
-// between the MMA issuer and the epilogue.
+// are already being multiplied.
 //
 // The reference has no GEMM; its users would pair flagcx collectives with a
 // vendor scaled matmul.
 //
-// One CTA per SM, 384 threads, persistent over 128x128 tiles:
-//   warp 0     TMA producer (A and B slices of 128x128 bytes, 128-byte swizzle, 6 stages, no multicast)
-//   warp 1     MMA issuer (4 x K32 instructions per slice)
-//   warp 2     TMEM allocation
-//   warps 4-11 promotion + epilogue: warp w reads TMEM lanes 32*(w%4).. (one output row per thread) and the
-//              column half (w-4)/4 of the tile, 64 fp32 accumulators per thread, two TMEM loads in flight
+// Two kernels, persistent over their tiles:
+//   gemmFp8PairKernel  256 x 256 tiles on CTA pairs (cta_group::2), two 256-column accumulators.  A CTA fetches 32 KB per
+//                      slice for 128 x 256 results; the 128 x 128 tiles of the one-CTA kernel fetch the same for half of
+//                      them, and L2 cannot deliver that to 148 SMs at the fp8 rate.
+//   gemmFp8Kernel<BN>  128 x BN tiles on single CTAs (BN 128 or 64), four accumulators: for outputs with too few tiles.
+// Roles: warps 0-7 promotion + epilogue (warp w reads TMEM lanes 32*(w%4).., one output row per thread, and half of the
+// tile's columns), warp 8 TMA producer (128-byte swizzle, no multicast), warp 9 MMA issuer and TMEM allocation.
 // Every wait is bounded; a wait that gives up sets the error flag and the kernel drains and returns.
 #include <algorithm>
 #include <cstdlib>
@@ -35,24 +35,22 @@ namespace {
 
 using namespace fcxmma;
 
-constexpr int BM = 128, BN = 128, BK = 128, STAGES = 6, ACC_BUFS = 4;
-constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int EPI_WARPS = 8;
-constexpr int EPI_BYTES = EPI_WARPS * 32 * 128;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
-constexpr int THREADS = 384;
+constexpr int BM = 128, BK = 128;
+constexpr int A_BYTES = BM * BK;
+constexpr int EPI_WARPS = 8, THREADS = 320;
+constexpr int STG_BYTES = 32 * 64;  // a block of 32 rows x 32 bf16 columns on its way to the TMA unit; two per epilogue warp
+constexpr int EPI_BYTES = EPI_WARPS * 2 * STG_BYTES;
 
 struct Params {
   int M, N, K;
   const float *sa;  // [K/128][M]
   const float *sb;  // [ceil(N/128)][K/128]
-  __nv_bfloat16 *c;
-  int ldc, group;
+  int group;
   int *errFlag;
 };
 
-// D fp32, A and B e4m3 (format 0), both K-major, M = 128, N = 128
-__device__ __forceinline__ constexpr uint32_t instrDescF8() { return (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); }
+// D fp32, A and B e4m3 (format 0), both K-major
+__device__ __forceinline__ constexpr uint32_t instrDescF8(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
 
 __device__ __forceinline__ void tileCoord(const Params &p, int nM, int nN, int t, int *mb, int *nb) {
   const int perBand = p.group * nN, band = t / perBand, first = band * p.group;
@@ -61,8 +59,69 @@ __device__ __forceinline__ void tileCoord(const Params &p, int nM, int nN, int t
   *nb = within / rowsHere;
 }
 
+// The scales of one output row, GROUP slices at a time.  The loads of the next group are issued together when a group
+// begins and used when it ends: a load per slice, even one issued eight slices ahead, made every slice wait for the
+// youngest outstanding load (about 800 clocks a slice in place of the 256 its multiplication takes).
+template <int GROUP>
+struct Scales {
+  const float *a, *b;
+  int M, nK;
+  float cur[GROUP], na[GROUP], nb[GROUP];
+  __device__ __forceinline__ void fetch(int kb0) {
+#pragma unroll
+    for (int j = 0; j < GROUP; j++) {
+      na[j] = kb0 + j < nK ? a[(size_t)(kb0 + j) * M] : 0.f;
+      nb[j] = kb0 + j < nK ? b[kb0 + j] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void turn() {
+#pragma unroll
+    for (int j = 0; j < GROUP; j++) cur[j] = na[j] * nb[j];
+  }
+};
+
+// COLS fp32 values per lane (one row) -> bf16 -> C, 32 columns at a time through this warp's two staging blocks (laid out
+// as the TMA unit's 64-byte swizzle wants them); the unit clips what lies beyond M and N.
+template <int COLS>
+__device__ __forceinline__ void storeRows(const float (&acc)[COLS], const CUtensorMap *tmC, uint8_t *stg, int row0, int col0, int M, int N, int lane,
+                                          uint32_t *blockNo) {
+#pragma unroll
+  for (int c0 = 0; c0 < COLS; c0 += 32) {
+    if (row0 < M && col0 + c0 < N) {
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+      __syncwarp();
+      uint4 *blk = (uint4 *)(stg + (*blockNo & 1) * STG_BYTES);  // the one whose store is the older
+      ++*blockNo;
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        uint4 o;
+        o.x = pack2(acc[c0 + 8 * v + 0], acc[c0 + 8 * v + 1]);
+        o.y = pack2(acc[c0 + 8 * v + 2], acc[c0 + 8 * v + 3]);
+        o.z = pack2(acc[c0 + 8 * v + 4], acc[c0 + 8 * v + 5]);
+        o.w = pack2(acc[c0 + 8 * v + 6], acc[c0 + 8 * v + 7]);
+        blk[lane * 4 + (v ^ ((lane >> 1) & 3))] = o;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                     ::"l"(tmC), "r"(col0 + c0), "r"(row0), "r"(smemAddr(blk)) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ one CTA per tile
+
+constexpr int stageBytes(int bn) { return A_BYTES + bn * BK; }
+constexpr int stages(int bn) { return bn == 128 ? 5 : 7; }
+constexpr int smemBytes(int bn) { return stages(bn) * stageBytes(bn) + EPI_BYTES + 1024 + 256; }
+
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                                                            const Params p) {
+                                                            const __grid_constant__ CUtensorMap tmC, const Params p) {
+  constexpr int STAGES = stages(BN), STAGE_BYTES = stageBytes(BN), ACC_BUFS = 4, COLS = BN / 2;
   extern __shared__ uint8_t smemRaw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int *err = p.errFlag;
@@ -79,8 +138,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
     for (int b = 0; b < ACC_BUFS; b++) { mbarInit(&tmemFull[b], 1); mbarInit(&tmemEmpty[b], EPI_WARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(tmemBaseSlot)), "r"(512) : "memory");
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(tmemBaseSlot)), "r"(ACC_BUFS * BN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   fenceBefore();
@@ -88,7 +147,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
 
-  if (warp == 0) {
+  if (warp == 8) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
@@ -106,12 +165,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 9) {
     if (lane == 0) {
       int stage = 0, buf = 0;
       uint32_t phase = 0, accPhase = 0;
       bool ok = true;
-      const uint32_t idesc = instrDescF8();
+      const uint32_t idesc = instrDescF8(BM, BN);
       for (int t = blockIdx.x; t < nTiles && ok; t += gridDim.x) {
         for (int kb = 0; kb < nK; kb++) {
           if (!mbarWait(&tmemEmpty[buf], accPhase ^ 1, err)) { ok = false; break; }
@@ -129,120 +188,271 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
         }
       }
     }
-  } else if (warp >= 4) {
-    const int q = warp & 3, half = (warp - 4) >> 2;  // TMEM lane quarter (fixed by warp index % 4) and column half
-    constexpr int COLS = BN / 2;
+  } else {
+    const int q = warp & 3, half = warp >> 2;  // TMEM lane quarter (fixed by warp index % 4) and column half
+    constexpr int GROUP = 8;
     int buf = 0;
-    uint32_t accPhase = 0;
+    uint32_t accPhase = 0, blockNo = 0;
     bool live = true;
+    uint8_t *stg = epiStage + (size_t)warp * 2 * STG_BYTES;
     for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
       int mb, nb;
       tileCoord(p, nM, nN, t, &mb, &nb);
-      const int row = mb * BM + q * 32 + lane;
-      const float *saRow = p.sa + min(row, p.M - 1);
-      const float *sbRow = p.sb + (size_t)nb * nK;
+      const int row0 = mb * BM + q * 32;
+      Scales<GROUP> sc{p.sa + min(row0 + lane, p.M - 1), p.sb + (size_t)(nb * BN / 128) * nK, p.M, nK};
+      sc.fetch(0);
       float acc[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; j++) acc[j] = 0.f;
-      // The scales of the next eight slices are always in flight (a global load takes several slice times).
-      constexpr int AHEAD = 8;
-      float ringA[AHEAD], ringB[AHEAD];
+      sc.turn();
+      for (int kb0 = 0; kb0 < nK; kb0 += GROUP) {
+        sc.fetch(kb0 + GROUP);
 #pragma unroll
-      for (int j = 0; j < AHEAD; j++) {
-        ringA[j] = j < nK ? saRow[(size_t)j * p.M] : 0.f;
-        ringB[j] = j < nK ? sbRow[j] : 0.f;
-      }
-      for (int kb0 = 0; kb0 < nK; kb0 += AHEAD) {
-#pragma unroll
-        for (int j = 0; j < AHEAD; j++) {
-          const int kb = kb0 + j;
-          if (kb < nK) {
-            const float scale = ringA[j] * ringB[j];
-            if (kb + AHEAD < nK) {
-              ringA[j] = saRow[(size_t)(kb + AHEAD) * p.M];
-              ringB[j] = sbRow[kb + AHEAD];
-            }
+        for (int j = 0; j < GROUP; j++) {
+          if (kb0 + j < nK) {
             if (live) live = __all_sync(0xffffffffu, mbarWait(&tmemFull[buf], accPhase, err));
             if (live) {
               fenceAfter();
-              uint32_t r0[32], r1[32];
+              uint32_t r[COLS];
               const uint32_t taddr = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * COLS);
-              tmemLd32(taddr, r0);
-              tmemLd32(taddr + 32, r1);
+#pragma unroll
+              for (int c = 0; c < COLS; c += 32) tmemLd32(taddr + c, r + c);
               tmemLdWait();
               fenceBefore();
               __syncwarp();
               if (lane == 0) mbarArrive(&tmemEmpty[buf]);  // the values are in registers: the accumulator may be overwritten
 #pragma unroll
-              for (int i = 0; i < 32; i++) acc[i] = fmaf(scale, __uint_as_float(r0[i]), acc[i]);
-#pragma unroll
-              for (int i = 0; i < 32; i++) acc[32 + i] = fmaf(scale, __uint_as_float(r1[i]), acc[32 + i]);
+              for (int i = 0; i < COLS; i++) acc[i] = fmaf(sc.cur[j], __uint_as_float(r[i]), acc[i]);
             }
             if (++buf == ACC_BUFS) { buf = 0; accPhase ^= 1; }
           }
         }
+        sc.turn();
       }
-      if (!live) continue;
-      // one row per lane -> transposed through shared memory so that 8 lanes store one 128-byte line of a row
-      const int row0 = mb * BM + q * 32;
-      uint4 *stg = (uint4 *)(epiStage + (size_t)(warp - 4) * 32 * 128);
-#pragma unroll
-      for (int v = 0; v < 8; v++) {
-        uint4 o;
-        o.x = pack2(acc[8 * v + 0], acc[8 * v + 1]);
-        o.y = pack2(acc[8 * v + 2], acc[8 * v + 3]);
-        o.z = pack2(acc[8 * v + 4], acc[8 * v + 5]);
-        o.w = pack2(acc[8 * v + 6], acc[8 * v + 7]);
-        stg[lane * 8 + (v ^ (lane & 7))] = o;
-      }
-      __syncwarp();
-      const int col = nb * BN + half * COLS + (lane & 7) * 8;
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int rr = i * 4 + (lane >> 3);
-        uint4 o = stg[rr * 8 + ((lane & 7) ^ (rr & 7))];
-        if (row0 + rr < p.M) {
-          __nv_bfloat16 *d = p.c + (size_t)(row0 + rr) * p.ldc + col;
-          if (col + 8 <= p.N) *(uint4 *)d = o;
-          else {
-            const __nv_bfloat16 *e = (const __nv_bfloat16 *)&o;
-            for (int j = 0; j < 8 && col + j < p.N; j++) d[j] = e[j];
-          }
-        }
-      }
-      __syncwarp();
+      if (live) storeRows<COLS>(acc, &tmC, stg, row0, nb * BN + half * COLS, p.M, p.N, lane, &blockNo);
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   fenceBefore();
   __syncthreads();
   fenceAfter();
-  if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(512) : "memory");
+  if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(ACC_BUFS * BN) : "memory");
+}
+
+// ------------------------------------------------------------------ CTA pairs, 256 x 256 tiles
+
+constexpr int PN = 256, PNH = 128, PSTAGES = 6, PSTAGE_BYTES = A_BYTES + PNH * BK;
+constexpr int PTHREADS = 384;  // three warp groups: two of epilogue warps, one for the producer and the issuer
+// 128 sums per thread need more than the 168 registers that 384 threads get each: the third group gives some of its own.
+// 216 x 256 + 72 x 128 = 168 x 384.
+constexpr int EPI_REGS = 216, ROLE_REGS = 72;
+constexpr int PSMEM_BYTES = PSTAGES * PSTAGE_BYTES + EPI_BYTES + 1024 + 256;
+
+__device__ __forceinline__ void mmaF8Pair(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
+    gemmFp8PairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+                      const Params p) {
+  extern __shared__ uint8_t smemRaw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int *err = p.errFlag;
+  const uint32_t cr = ctaRankInCluster();  // 0 = leader
+  const int pair = blockIdx.x >> 1, nPairs = gridDim.x >> 1;
+  uint8_t *tiles = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
+  uint8_t *epiStage = tiles + PSTAGES * PSTAGE_BYTES;
+  uint64_t *bars = (uint64_t *)(epiStage + EPI_BYTES);
+  uint64_t *fullBar = bars, *emptyBar = bars + PSTAGES, *accFull = bars + 2 * PSTAGES, *accEmpty = bars + 2 * PSTAGES + 2;
+  uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * PSTAGES + 4);
+
+  const int nN = (p.N + PN - 1) / PN, nM = (p.M + 2 * BM - 1) / (2 * BM), nTiles = nN * nM, nK = p.K / BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PSTAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&emptyBar[s], 1); }
+    for (int b = 0; b < 2; b++) { mbarInit(&accFull[b], 1); mbarInit(&accEmpty[b], 2 * EPI_WARPS); }  // the warps of both CTAs
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(tmemBaseSlot)), "r"(2 * PN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  fenceBefore();
+  __syncthreads();
+  clusterSync();  // the peer's barriers exist before anything arrives on them
+  fenceAfter();
+  const uint32_t tmemBase = *tmemBaseSlot;
+
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGS));
+    if (warp == 8) {
+      // ---- TMA producer (both CTAs): own 128 rows of A, own 128 of the 256 weight rows; bytes counted on the leader's barrier
+      if (lane == 0) {
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int t = pair; t < nTiles && ok; t += nPairs) {
+          int mb, nb;
+          tileCoord(p, nM, nN, t, &mb, &nb);
+          for (int kb = 0; kb < nK; kb++) {
+            if (!mbarWait(&emptyBar[stage], phase ^ 1, err)) { ok = false; break; }
+            if (cr == 0) mbarExpectTx(&fullBar[stage], 2 * PSTAGE_BYTES);
+            const uint32_t bar = mapToCta(smemAddr(&fullBar[stage]), 0);
+            uint8_t *sa = tiles + stage * PSTAGE_BYTES, *sb = sa + A_BYTES;
+            tmaLoad2dPair(sa, &tmA, kb * BK, mb * 2 * BM + (int)cr * BM, bar);
+            tmaLoad2dPair(sb, &tmB, kb * BK, nb * PN + (int)cr * PNH, bar);
+            if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
+          }
+        }
+      }
+    } else if (warp == 9) {
+      // ---- MMA issuer: one thread of the leader CTA
+      if (lane == 0 && cr == 0) {
+        int stage = 0, buf = 0;
+        uint32_t phase = 0, accPhase = 0;
+        bool ok = true;
+        const uint32_t idesc = instrDescF8(2 * BM, PN);
+        for (int t = pair; t < nTiles && ok; t += nPairs) {
+          for (int kb = 0; kb < nK; kb++) {
+            if (!mbarWait(&accEmpty[buf], accPhase ^ 1, err)) { ok = false; break; }
+            if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
+            fenceAfter();
+            const uint32_t sa = smemAddr(tiles + stage * PSTAGE_BYTES), sb = sa + A_BYTES;
+  #pragma unroll
+            for (int k = 0; k < BK / 32; k++)
+              mmaF8Pair(tmemBase + (uint32_t)buf * PN, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, k > 0 ? 1u : 0u);
+            mmaCommitPair(&emptyBar[stage]);
+            mmaCommitPair(&accFull[buf]);
+            if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
+            if (++buf == 2) { buf = 0; accPhase ^= 1; }
+          }
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPI_REGS));
+    // ---- promotion + epilogue (both CTAs): 128 fp32 sums per thread.  A warp's 128 columns are one scale block of the weight.
+    const int q = warp & 3, half = warp >> 2;
+    constexpr int GROUP = 4, COLS = 128;
+    int buf = 0;
+    uint32_t accPhase = 0, blockNo = 0;
+    bool live = true;
+    uint8_t *stg = epiStage + (size_t)warp * 2 * STG_BYTES;
+    const uint32_t emptyAddr = mapToCta(smemAddr(accEmpty), 0);
+    const int lastBlock = (p.N - 1) / 128;
+    for (int t = pair; t < nTiles; t += nPairs) {
+      int mb, nb;
+      tileCoord(p, nM, nN, t, &mb, &nb);
+      const int row0 = mb * 2 * BM + (int)cr * BM + q * 32;
+      Scales<GROUP> sc{p.sa + min(row0 + lane, p.M - 1), p.sb + (size_t)min(nb * 2 + half, lastBlock) * nK, p.M, nK};
+      sc.fetch(0);
+      float acc[COLS];
+#pragma unroll
+      for (int j = 0; j < COLS; j++) acc[j] = 0.f;
+      sc.turn();
+      for (int kb0 = 0; kb0 < nK; kb0 += GROUP) {
+        sc.fetch(kb0 + GROUP);
+#pragma unroll
+        for (int j = 0; j < GROUP; j++) {
+          if (kb0 + j < nK) {
+            if (live) live = __all_sync(0xffffffffu, mbarWait(&accFull[buf], accPhase, err));
+            if (live) {
+              fenceAfter();
+              const uint32_t taddr = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * PN + half * COLS);
+#pragma unroll
+              for (int c = 0; c < COLS; c += 32) {
+                uint32_t r[32];
+                tmemLd32(taddr + c, r);
+                tmemLdWait();
+                if (c + 32 == COLS) {
+                  fenceBefore();
+                  __syncwarp();
+                  if (lane == 0) mbarArriveRemote(emptyAddr + buf * 8);  // all of it is in registers
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i++) acc[c + i] = fmaf(sc.cur[j], __uint_as_float(r[i]), acc[c + i]);
+              }
+            }
+            if (++buf == 2) { buf = 0; accPhase ^= 1; }
+          }
+        }
+        sc.turn();
+      }
+      if (live) storeRows<COLS>(acc, &tmC, stg, row0, nb * PN + half * COLS, p.M, p.N, lane, &blockNo);
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+
+  // ---- tear-down: nobody leaves, and no TMEM is freed, while the peer may still use this CTA's memory or barriers
+  fenceBefore();
+  __syncthreads();
+  clusterSync();
+  fenceAfter();
+  if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(2 * PN) : "memory");
 }
 
 // ------------------------------------------------------------------ quantisation
 
-// One warp per (row, 128-column block): scale = amax / 448, q = x / scale.
+// Four fp32 values -> four e4m3 bytes.
+__device__ __forceinline__ uint32_t pack4Fp8(float a, float b, float c, float d) {
+  return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3) |
+         (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3) << 16;
+}
+
+// scale = amax / 448 over a (row, 128-column block), q = x / scale.  A lane holds VEC consecutive values (8: half a warp
+// per block, 16-byte loads; 4: a warp per block, for rows that are only 8-byte aligned) of UNROLL blocks whose loads are
+// all issued before the first is used: one 8-byte load in flight per lane left the kernel waiting (2.1 TB/s).
+template <int VEC, int UNROLL>
 __global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *__restrict__ x, __nv_fp8_storage_t *__restrict__ q,
                                                       float *__restrict__ sa, int M, int K, int ldx) {
+  constexpr int LANES = 128 / VEC, PER_CTA = 256 / LANES;  // lanes per block, blocks per CTA and step
   const int nKb = K / 128;
-  const size_t warpId = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5), total = (size_t)M * nKb;
-  if (warpId >= total) return;
-  const int lane = threadIdx.x & 31;
-  const int row = (int)(warpId / nKb), kb = (int)(warpId % nKb);
-  const uint2 raw = *(const uint2 *)(x + (size_t)row * ldx + kb * 128 + lane * 4);
-  const __nv_bfloat162 *h = (const __nv_bfloat162 *)&raw;
-  float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-  float amax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y)));
+  const size_t total = (size_t)M * nKb;
+  const int sub = threadIdx.x / LANES, l = threadIdx.x % LANES;
+  const size_t first = (size_t)blockIdx.x * PER_CTA * UNROLL + sub;
+  uint32_t raw[UNROLL][VEC / 2];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  const float scale = amax > 0.f ? amax / 448.f : 1.f, inv = 1.f / scale;
-  uint32_t out = (uint32_t)__nv_cvt_float_to_fp8(a.x * inv, __NV_SATFINITE, __NV_E4M3) |
-                 (uint32_t)__nv_cvt_float_to_fp8(a.y * inv, __NV_SATFINITE, __NV_E4M3) << 8 |
-                 (uint32_t)__nv_cvt_float_to_fp8(b.x * inv, __NV_SATFINITE, __NV_E4M3) << 16 |
-                 (uint32_t)__nv_cvt_float_to_fp8(b.y * inv, __NV_SATFINITE, __NV_E4M3) << 24;
-  *(uint32_t *)(q + (size_t)row * K + kb * 128 + lane * 4) = out;
-  if (lane == 0) sa[(size_t)kb * M + row] = scale;
+  for (int u = 0; u < UNROLL; u++) {
+    const size_t b = first + (size_t)u * PER_CTA;
+    if (b < total) {
+      const size_t row = b / nKb, kb = b % nKb;
+      const __nv_bfloat16 *src = x + row * ldx + kb * 128 + l * VEC;
+      if (VEC == 8) *(uint4 *)raw[u] = *(const uint4 *)src;
+      else *(uint2 *)raw[u] = *(const uint2 *)src;
+    } else {
+#pragma unroll
+      for (int j = 0; j < VEC / 2; j++) raw[u][j] = 0;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UNROLL; u++) {
+    const size_t b = first + (size_t)u * PER_CTA;
+    float v[VEC], amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < VEC / 2; j++) {
+      const float2 f = __bfloat1622float2(*(const __nv_bfloat162 *)&raw[u][j]);
+      v[2 * j] = f.x;
+      v[2 * j + 1] = f.y;
+      amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (b >= total) continue;
+    const size_t row = b / nKb, kb = b % nKb;
+    const float scale = amax > 0.f ? amax / 448.f : 1.f, inv = 1.f / scale;
+    uint32_t out[VEC / 4];
+#pragma unroll
+    for (int j = 0; j < VEC / 4; j++) out[j] = pack4Fp8(v[4 * j] * inv, v[4 * j + 1] * inv, v[4 * j + 2] * inv, v[4 * j + 3] * inv);
+    __nv_fp8_storage_t *dst = q + row * K + kb * 128 + l * VEC;
+    if (VEC == 8) *(uint2 *)dst = make_uint2(out[0], out[VEC / 4 - 1]);
+    else *(uint32_t *)dst = out[0];
+    if (l == 0) sa[kb * M + row] = scale;
+  }
 }
 
 // One CTA per 128x128 block of the weight.
@@ -303,31 +513,76 @@ int smCount() {
 
 }  // namespace
 
+namespace {
+
+template <int BN>
+cudaError_t launchOne(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
+  CUtensorMap mb;
+  if (!makeTileMap(&mb, bq, p.N, p.K, p.K, BN, 1)) return cudaErrorNotSupported;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(gemmFp8Kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(BN));
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  gemmFp8Kernel<BN><<<std::min(tiles, smCount()), THREADS, smemBytes(BN), s>>>(ma, mb, mc, p);
+  return cudaGetLastError();
+}
+
+cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
+  CUtensorMap mb;
+  if (!makeTileMap(&mb, bq, p.N, p.K, p.K, PNH, 1)) return cudaErrorNotSupported;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(gemmFp8PairKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + PN - 1) / PN);
+  gemmFp8PairKernel<<<2 * std::min(tiles, smCount() / 2), PTHREADS, PSMEM_BYTES, s>>>(ma, mb, mc, p);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+// Which tile: 0 = 256 x 256 on CTA pairs, 128 or 64 = 128 x that many columns on single CTAs.  The time is about the
+// number of waves times the time of one 128-deep slice of a tile.
+extern "C" int fcxGemmFp8Tile(int M, int N, int sms) {
+  const int m1 = (M + 127) / 128, m2 = (M + 255) / 256;
+  auto waves = [](long long tiles, int slots) { return (double)((tiles + slots - 1) / slots); };
+  const double pair = waves((long long)m2 * ((N + 255) / 256), sms / 2) * 600;
+  const double one = waves((long long)m1 * ((N + 127) / 128), sms) * 400;
+  const double half = waves((long long)m1 * ((N + 63) / 64), sms) * 300;
+  if (pair <= one && pair <= half) return 0;
+  return one <= half ? 128 : 64;
+}
+
 extern "C" cudaError_t fcxGemmFp8Blockwise(const void *aq, const float *sa, const void *bq, const float *sb, void *c, int M, int N, int K,
                                            int ldc, int *errFlag, cudaStream_t s) {
   if (K % 128 || ldc % 8 || M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
   if (((uintptr_t)aq | (uintptr_t)bq | (uintptr_t)c) & 15) return cudaErrorInvalidValue;
-  CUtensorMap ma, mb;
-  if (!makeTileMap(&ma, aq, M, K, K, BM, 1) || !makeTileMap(&mb, bq, N, K, K, BN, 1)) return cudaErrorNotSupported;
+  CUtensorMap ma, mc;
+  if (!makeTileMap(&ma, aq, M, K, K, BM, 1) || !makeStoreMap(&mc, c, M, N, ldc)) return cudaErrorNotSupported;
   Params p{};
-  p.M = M; p.N = N; p.K = K; p.sa = sa; p.sb = sb; p.c = (__nv_bfloat16 *)c; p.ldc = ldc; p.errFlag = errFlag;
-  const int nN = (N + BN - 1) / BN;
-  p.group = nN >= 48 ? 16 : 8;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(gemmFp8Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  const int tiles = ((M + BM - 1) / BM) * nN;
-  gemmFp8Kernel<<<std::min(tiles, smCount()), THREADS, SMEM_BYTES, s>>>(ma, mb, p);
-  return cudaGetLastError();
+  p.M = M; p.N = N; p.K = K; p.sa = sa; p.sb = sb; p.errFlag = errFlag;
+  static const int forced = [] { const char *e = getenv("FLAGCX_FP8_TILE"); return e ? atoi(e) : -1; }();
+  const int tile = forced >= 0 ? forced : fcxGemmFp8Tile(M, N, smCount());
+  p.group = tile == 0 ? 8 : (N + 127) / 128 >= 48 ? 16 : 8;
+  return tile == 0 ? launchPair(ma, bq, mc, p, s) : tile == 128 ? launchOne<128>(ma, bq, mc, p, s) : launchOne<64>(ma, bq, mc, p, s);
 }
 
 extern "C" cudaError_t fcxQuantFp8Act(const void *x, void *q, float *sa, int M, int K, int ldx, cudaStream_t s) {
   if (K % 128 || ldx % 4) return cudaErrorInvalidValue;
-  const size_t warps = (size_t)M * (K / 128);
-  quantActKernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>((const __nv_bfloat16 *)x, (__nv_fp8_storage_t *)q, sa, M, K, ldx);
+  const size_t blocks = (size_t)M * (K / 128);
+  if (blocks == 0) return cudaSuccess;
+  const bool wide = ldx % 8 == 0 && ((uintptr_t)x & 15) == 0;
+  const __nv_bfloat16 *src = (const __nv_bfloat16 *)x;
+  __nv_fp8_storage_t *dst = (__nv_fp8_storage_t *)q;
+  // four blocks per lane group once that still leaves two CTAs for every SM, else one: a small batch wants many CTAs
+  if (wide && blocks >= 16 * 4 * 2 * (size_t)smCount()) quantActKernel<8, 4><<<(unsigned)((blocks + 63) / 64), 256, 0, s>>>(src, dst, sa, M, K, ldx);
+  else if (wide) quantActKernel<8, 1><<<(unsigned)((blocks + 15) / 16), 256, 0, s>>>(src, dst, sa, M, K, ldx);
+  else quantActKernel<4, 1><<<(unsigned)((blocks + 7) / 8), 256, 0, s>>>(src, dst, sa, M, K, ldx);
   return cudaGetLastError();
 }
 
