@@ -341,14 +341,13 @@ extern "C" int fcxGemmPairMode() {
   return mode;
 }
 
-// Whether the pair kernel is the better choice for this shape: whole 256-row blocks (or so many rows that the
-// half-empty last block does not matter) and at least most of one 256-column block.
+// Whether the pair kernel is the better choice for this shape: by the waves of tiles that either kernel needs, times what
+// a K block of its tile costs; the pair kernel has to win clearly, since half-empty pair tiles waste both SMs.
 extern "C" int fcxGemmPairSuits(int M, int N, int K) {
   const int mode = fcxGemmPairMode();
   if (mode == 0 || M < 129 || K < 8) return 0;
   if (mode == 2) return 1;
-  const int padded = (M + 255) / 256 * 256;
-  return (double)padded <= 1.07 * M && N >= 192;
+  return fcxGemmPairCost(M, N, K, smCount2() / 2) <= 0.85 * fcxGemmTileCost(M, N, K, smCount2(), nullptr);
 }
 
 extern "C" cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,

@@ -427,15 +427,17 @@ int tileGroup(int nN) {
   return g >= 0 ? g : (nN >= 24 ? 16 : 8);  // wide outputs: taller bands keep more of B in L2 per wave
 }
 
-// Columns per tile.  128-column tiles cost almost as much as 256-column ones (the A tile is re-read for half the
-// math, and shared-memory bandwidth is what bounds the MMA), so they do not pay even when they fill the last
-// wave better; FLAGCX_GEMM_BN=128 selects them for experiments.
-int pickBn(int, int, int) {
-  static int bn = 0;
-  if (!bn) {
+// Columns per tile of the one-CTA kernel: the choice of fcxGemmTileCost, or FLAGCX_GEMM_BN (64, 128, 256) for experiments.
+int pickBn(int M, int N, int K, int sms) {
+  static int forced = -1;
+  if (forced < 0) {
     const char *e = getenv("FLAGCX_GEMM_BN");
-    bn = e && atoi(e) == 128 ? 128 : 256;
+    const int v = e ? atoi(e) : 0;
+    forced = v == 64 || v == 128 || v == 256 ? v : 0;
   }
+  if (forced) return forced;
+  int bn = 256;
+  fcxGemmTileCost(M, N, K, sms, &bn);
   return bn;
 }
 
@@ -457,7 +459,7 @@ extern "C" cudaError_t fcxGemmBf16(const void *a, const void *b, void *c, int M,
   if (K % 8 || lda % 8 || ldb % 8 || ldc % 8 || M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
   if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, smCount());
+  const int bn = pickBn(M, N, K, smCount());
   if (!makeMap(&ma, a, M, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, bn)) return cudaErrorNotSupported;
   FcxGemmParams p{};
   p.M = M; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.rotate = 0; p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
@@ -494,6 +496,36 @@ extern "C" int fcxGemmPickSplitK(int requested, int units, int slots, int nK, in
   return (nK + kPer - 1) / kPer;
 }
 
+static double waveCost(int units, int slots, int nK, int N, double blockCost) {
+  const int sk = fcxGemmPickSplitK(0, units, slots, nK, N);
+  const int waves = (units * sk + slots - 1) / slots;
+  return waves * ((nK + sk - 1) / sk) * blockCost * (1.0 + 0.03 * (sk - 1));
+}
+
+// Estimated clocks of the one-CTA kernel with its best tile width, and that width.  A 64-deep K block of a 128 x bn tile is
+// bound by what one SM can fetch (16 KB of A and bn x 128 bytes of B at about 64 bytes a clock): 768, 512 and 384 clocks
+// for 256, 128 and 64 columns.  Narrow tiles re-read A and never pay once 256-column tiles fill the SMs, but with few
+// tiles they put more SMs to work on the same K steps.
+extern "C" double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut) {
+  const int nK = (K + BK - 1) / BK, nM = (M + BM - 1) / BM;
+  const int widths[3] = {256, 128, 64};
+  const double clocks[3] = {768, 512, 384};
+  double best = 0;
+  for (int i = 0; i < 3; i++) {
+    const double c = waveCost(nM * ((N + widths[i] - 1) / widths[i]), sms, nK, N, clocks[i]);
+    if (i == 0 || c < 0.9 * best) {
+      best = c;
+      if (bnOut) *bnOut = widths[i];
+    }
+  }
+  return best;
+}
+
+// The same for the CTA-pair kernel: 32 KB per CTA and K block of a 256 x 256 tile.
+extern "C" double fcxGemmPairCost(int M, int N, int K, int pairs) {
+  return waveCost(((M + 255) / 256) * ((N + 255) / 256), pairs, (K + BK - 1) / BK, N, 512);
+}
+
 // What went wrong in the last fcxGemmBf16Ex call of this thread that did not return cudaSuccess.
 static thread_local char gGemmDetail[256];
 extern "C" const char *fcxGemmLastDetail() { return gGemmDetail; }
@@ -512,7 +544,7 @@ extern "C" cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, in
     return fcxGemmPairBf16(a, b, c, M, N, K, lda, ldb, ldc, aMN, bMN, bias, splitK, accumulate, o->geluOut, tileGroup((N + 255) / 256) / 2,
                            errFlag, s, gGemmDetail, sizeof gGemmDetail);
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, smCount());
+  const int bn = pickBn(M, N, K, smCount());
   // K-major operand: rows = M (or N), box of 128 (bn) rows x 64 K; MN-major operand: rows = K, box of 64 lines x 64 columns
   const bool okA = aMN ? makeMap(&ma, a, K, M, lda, BK) : makeMap(&ma, a, M, K, lda, BM);
   const bool okB = bMN ? makeMap(&mb, b, K, N, ldb, BK) : makeMap(&mb, b, N, K, ldb, bn);
@@ -549,7 +581,7 @@ extern "C" cudaError_t fcxGemmBf16DynM(const void *a, const void *b, void *c, in
                                        int *errFlag, cudaStream_t s) {
   if (K % 8 || lda % 8 || ldb % 8 || ldc % 8 || Mmax <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
-  const int bn = pickBn(Mmax, N, smCount());
+  const int bn = pickBn(Mmax, N, K, smCount());
   if (!makeMap(&ma, a, Mmax, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, bn)) return cudaErrorNotSupported;
   FcxGemmParams p{};
   p.M = Mmax; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.mPtr = mPtr; p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
@@ -575,7 +607,7 @@ extern "C" cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, c
   if (K % 8 || ldb % 8 || ldc % 8 || M % (n * BM) || commCtas < 1) return cudaErrorInvalidValue;
   if (n == 1) return oneRank(aLocal, b, c, M, N, K, K, ldb, ldc, errFlag, s);
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, std::max(1, smCount() - commCtas));
+  const int bn = pickBn(M, N, K, std::max(1, smCount() - commCtas));
   CUtensorMap mal;
   if (!makeMap(&ma, gathered, M, K, K, BM) || !makeMap(&mb, b, N, K, ldb, bn) || !makeMap(&mal, aLocal, M / n, K, K, BM))
     return cudaErrorNotSupported;

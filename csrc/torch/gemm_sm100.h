@@ -13,7 +13,7 @@ struct FcxGemmParams {
   void *c;              // PLAIN/AG: C; RS: this rank's [M/n, N] result
   int ldc;
   int rotate;           // first row block (of 128 rows) this rank works on
-  int bn;               // columns per tile: 256 or 128 (RS: 256)
+  int bn;               // columns per tile: 256, 128 or 64 (RS: 256)
   int group;            // PLAIN: row blocks per band of the tile order (0: row-major)
   int rowsPerRank;      // M / nranks (AG, RS)
   int gemmCtas;         // AG: CTAs [0, gemmCtas) compute, the rest move data
@@ -58,6 +58,8 @@ typedef struct FcxGemmOpts {
 cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, const FcxGemmOpts *o,
                             int *errFlag, cudaStream_t s);
 int fcxGemmPickSplitK(int requested, int units, int slots, int nK, int N);
+double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut);
+double fcxGemmPairCost(int M, int N, int K, int pairs);
 int fcxGemmPairMode();
 int fcxGemmPairSuits(int M, int N, int K);
 cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,
