@@ -20,7 +20,6 @@ struct flagcxEmu {
   char *heaps[FCX_MAX_RANKS] = {};
   FcxDevComm host[FCX_MAX_RANKS];
   FcxDevComm *dcsDev = nullptr;
-  FcxCollArgs *argsDev = nullptr;
   FcxP2pArgs *p2pDev = nullptr;
   FcxDevError *errHost = nullptr;
   uint64_t seq = 0;
@@ -64,7 +63,6 @@ flagcxResult_t flagcxEmuCreate(flagcxEmu_t *out, int nranks, size_t stageBytes) 
     d.segs = nullptr;
   }
   FCX_CHECK(cudaToResult(cudaMalloc((void **)&e->dcsDev, sizeof(FcxDevComm) * FCX_MAX_RANKS), "emu alloc"));
-  FCX_CHECK(cudaToResult(cudaMalloc((void **)&e->argsDev, sizeof(FcxCollArgs) * FCX_MAX_RANKS), "emu alloc"));
   FCX_CHECK(cudaToResult(cudaMalloc((void **)&e->p2pDev, sizeof(FcxP2pArgs) * FCX_MAX_RANKS), "emu alloc"));
   FCX_CHECK(cudaToResult(cudaMemcpy(e->dcsDev, e->host, sizeof(FcxDevComm) * FCX_MAX_RANKS, cudaMemcpyHostToDevice), "emu copy"));
   *out = e;
@@ -76,7 +74,6 @@ flagcxResult_t flagcxEmuDestroy(flagcxEmu_t e) {
   cudaDeviceSynchronize();
   for (int r = 0; r < e->n; r++) cudaFree(e->heaps[r]);
   cudaFree(e->dcsDev);
-  cudaFree(e->argsDev);
   cudaFree(e->p2pDev);
   cudaFreeHost(e->errHost);
   cudaGetLastError();
@@ -100,8 +97,10 @@ flagcxResult_t flagcxEmuCollective(flagcxEmu_t e, flagcxCommOp_t op, const char 
   }
   const int n = e->n;
   const size_t es = dtypeSize(dt);
-  FcxCollArgs as[FCX_MAX_RANKS];
-  memset(as, 0, sizeof as);
+  FcxEmuRanks l;
+  memset(&l, 0, sizeof l);
+  memcpy(l.dc, e->host, sizeof(FcxDevComm) * n);
+  FcxCollArgs *as = l.args;
   uint64_t seq = ++e->seq;
   for (int r = 0; r < n; r++) {
     FcxCollArgs &a = as[r];
@@ -143,9 +142,7 @@ flagcxResult_t flagcxEmuCollective(flagcxEmu_t e, flagcxCommOp_t op, const char 
       default: break;
     }
   }
-  cudaStream_t st = (cudaStream_t)cudaStream;
-  FCX_CHECK(cudaToResult(cudaMemcpyAsync(e->argsDev, as, sizeof(FcxCollArgs) * n, cudaMemcpyHostToDevice, st), "emu args"));
-  return cudaToResult(fcxLaunchCollEmu(e->dcsDev, e->argsDev, &as[0], n, nctas, st), "emu launch");
+  return cudaToResult(fcxLaunchCollEmu(&l, n, nctas, (cudaStream_t)cudaStream), "emu launch");
 }
 
 flagcxResult_t flagcxEmuSendRecv(flagcxEmu_t e, int nops, const int *srcRank, const int *dstRank, void *const *sendbuf,

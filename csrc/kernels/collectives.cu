@@ -142,76 +142,80 @@ __device__ void arLL(const FcxDevComm &dc, const FcxCollArgs &a, uint64_t seq, i
   const bool reduces = mode != 2 || me == a.root;
   const bool alS = aligned16(send), alR = aligned16(a.recv);
   const size_t llOff = FCX_OFF_LL + (size_t)(seq & 1) * FCX_MAX_RANKS * FCX_LL_SLOT_BYTES;
-  bool ok = true;
+  // All lines go out before any is waited for, and every peer's line of a unit is asked for before the first is used: a
+  // line at a time, the kernel spent a trip to L2 per peer and unit one after the other (7 x 0.5 us with eight ranks).
   for (size_t u = gtid; u < nunits; u += gstride) {
-    int nv = (int)min((size_t)G, a.count - u * G);
+    const int nv = (int)min((size_t)G, a.count - u * G);
     Acc mine[G];
-    loadUnit<T, G>(send + u * 16, alS, nv, mine);
+    uint4 raw;
+    if (mode != 1) {
+      loadUnit<T, G>(send + u * 16, alS, nv, mine);
+      packUnit<T, G>(mine, &raw);
+    }
     for (int k = 1; k < n; k++) {
       int p = (me + k) % n;
       if (mode == 2 && p != a.root) continue;
-      uint4 raw;
       if (mode == 1) {
         const char *src = (const char *)a.send + (size_t)p * pieceBytes + u * 16;
-        Acc theirs[G];
-        loadUnit<T, G>(src, aligned16(src), nv, theirs);
-        packUnit<T, G>(theirs, &raw);
-      } else {
+        loadUnit<T, G>(src, aligned16(src), nv, mine);
         packUnit<T, G>(mine, &raw);
       }
       char *line = dc.heap[p] + llOff + (size_t)me * FCX_LL_SLOT_BYTES + u * 32;
       llStore(line, raw.x, raw.y, tag);
       llStore(line + 16, raw.z, raw.w, tag);
     }
-    if (!reduces) continue;
-    Acc acc[G];
-    bool first = true;
-    for (int p = 0; p < n; p++) {
-      Acc in[G];
-      if (p == me) {
+  }
+  if (!reduces) return;
+  const char *lines = dc.heap[me] + llOff;
+  for (size_t u = gtid; u < nunits; u += gstride) {
+    const int nv = (int)min((size_t)G, a.count - u * G);
+    Acc mine[G];
+    loadUnit<T, G>(send + u * 16, alS, nv, mine);
+    uint4 lo[FCX_MAX_RANKS], hi[FCX_MAX_RANKS];
+    unsigned pending = ((1u << n) - 1u) & ~(1u << me), spins = 0;
+    uint64_t t0 = 0;
+    for (;;) {
 #pragma unroll
-        for (int i = 0; i < G; i++) in[i] = mine[i];
-      } else {
-        const char *line = dc.heap[me] + llOff + (size_t)p * FCX_LL_SLOT_BYTES + u * 32;
-        uint4 lo = llLoad(line), hi = llLoad(line + 16);
-        if (!(lo.y == tag && lo.w == tag && hi.y == tag && hi.w == tag)) {
-          uint64_t t0 = globalTimerNs();
-          unsigned spins = 0;
-          for (;;) {
-            lo = llLoad(line);
-            hi = llLoad(line + 16);
-            if (lo.y == tag && lo.w == tag && hi.y == tag && hi.w == tag) break;
-            if ((++spins & 63u) == 0u) {
-              if (*(volatile unsigned int *)&localOf(dc)->abortSeen) { ok = false; break; }
-              if (globalTimerNs() - t0 > dc.timeoutNs) {
-                giveUp(dc, FCX_ERR_TIMEOUT, p, FCX_WAIT_LL, cta, tag, lo.y, seq);
-                ok = false;
-                break;
-              }
-              if ((spins & 1023u) == 0u && *dc.abortWord) {
-                giveUp(dc, FCX_ERR_ABORT, p, FCX_WAIT_LL, cta, tag, lo.y, seq);
-                ok = false;
-                break;
-              }
-            }
-          }
-          if (!ok) break;
+      for (int p = 0; p < FCX_MAX_RANKS; p++)
+        if (pending >> p & 1u) {
+          lo[p] = llLoad(lines + (size_t)p * FCX_LL_SLOT_BYTES + u * 32);
+          hi[p] = llLoad(lines + (size_t)p * FCX_LL_SLOT_BYTES + u * 32 + 16);
         }
-        union { uint4 v; T t[G]; } w;
-        w.v = make_uint4(lo.x, lo.z, hi.x, hi.z);
 #pragma unroll
-        for (int i = 0; i < G; i++) in[i] = Elem<T>::up(w.t[i]);
-      }
-      if (first) {
-#pragma unroll
-        for (int i = 0; i < G; i++) acc[i] = in[i];
-        first = false;
-      } else {
-#pragma unroll
-        for (int i = 0; i < G; i++) acc[i] = applyOp<Acc>(acc[i], in[i], a.redop);
+      for (int p = 0; p < FCX_MAX_RANKS; p++)
+        if ((pending >> p & 1u) && lo[p].y == tag && lo[p].w == tag && hi[p].y == tag && hi[p].w == tag) pending &= ~(1u << p);
+      if (!pending) break;
+      if (spins == 0) t0 = globalTimerNs();
+      if ((++spins & 63u) == 0u) {
+        const int late = __ffs(pending) - 1;
+        if (*(volatile unsigned int *)&localOf(dc)->abortSeen) return;
+        if (globalTimerNs() - t0 > dc.timeoutNs) {
+          giveUp(dc, FCX_ERR_TIMEOUT, late, FCX_WAIT_LL, cta, tag, 0, seq);
+          return;
+        }
+        if ((spins & 1023u) == 0u && *dc.abortWord) {
+          giveUp(dc, FCX_ERR_ABORT, late, FCX_WAIT_LL, cta, tag, 0, seq);
+          return;
+        }
       }
     }
-    if (!ok) break;
+    Acc acc[G];
+#pragma unroll
+    for (int p = 0; p < FCX_MAX_RANKS; p++)  // in rank order on every rank
+      if (p < n) {
+        Acc in[G];
+        if (p == me) {
+#pragma unroll
+          for (int i = 0; i < G; i++) in[i] = mine[i];
+        } else {
+          union { uint4 v; T t[G]; } w;
+          w.v = make_uint4(lo[p].x, lo[p].z, hi[p].x, hi[p].z);
+#pragma unroll
+          for (int i = 0; i < G; i++) in[i] = Elem<T>::up(w.t[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < G; i++) acc[i] = p == 0 ? in[i] : applyOp<Acc>(acc[i], in[i], a.redop);
+      }
 #pragma unroll
     for (int i = 0; i < G; i++) acc[i] = finish<Acc>(acc[i], a.redop, n, a.scale);
     uint4 outv;
@@ -768,13 +772,18 @@ __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
       bool ok = true;
       for (size_t w = gtid; w < nwords && ok; w += gstride) {
         const size_t valid = min((size_t)8, bytes - w * 8);
-        for (int k = 1; k < n && ok; k++) {
-          int p = (me + k) % n;
-          if (!inSrc[p]) continue;
-          uint4 v;
-          ok = llWaitLine(dc, dc.heap[me] + llOff + (size_t)p * FCX_LL_SLOT_BYTES + w * 16, tag, p, cta, seq, &v);
-          if (ok) st8(inDst[p] + w * 8, valid, v.x, v.z);
-        }
+        // every peer's line is asked for before the first is waited for
+        uint4 v[FCX_MAX_RANKS];
+#pragma unroll
+        for (int p = 0; p < FCX_MAX_RANKS; p++)
+          if (p < n && inSrc[p]) v[p] = llLoad(dc.heap[me] + llOff + (size_t)p * FCX_LL_SLOT_BYTES + w * 16);
+#pragma unroll
+        for (int p = 0; p < FCX_MAX_RANKS; p++)
+          if (p < n && inSrc[p] && ok) {
+            if (v[p].y != tag || v[p].w != tag)
+              ok = llWaitLine(dc, dc.heap[me] + llOff + (size_t)p * FCX_LL_SLOT_BYTES + w * 16, tag, p, cta, seq, &v[p]);
+            if (ok) st8(inDst[p] + w * 8, valid, v[p].x, v[p].z);
+          }
       }
       epilogue(dc, seq, nctas);
       return;
@@ -1057,13 +1066,17 @@ __global__ void __launch_bounds__(FCX_THREADS, 1) fcxP2pKernel(FcxDevComm dc, Fc
 // Emulation: rank = blockIdx.x / ctasPerRank.  Launched cooperatively so that
 // all emulated ranks are resident at once and may wait on one another.
 template <typename TIn, typename TOut>
-__global__ void __launch_bounds__(FCX_THREADS, 1) fcxCollEmuKernel(const FcxDevComm *dcs, const FcxCollArgs *as, int ctasPerRank) {
-  int r = blockIdx.x / ctasPerRank;
-  fcxCollBody<TIn, TOut>(dcs[r], as[r], blockIdx.x % ctasPerRank, ctasPerRank);
+__global__ void __launch_bounds__(FCX_THREADS, 1) fcxCollEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
+  __shared__ FcxDevComm dc;
+  __shared__ FcxCollArgs a;
+  emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
+  fcxCollBody<TIn, TOut>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
-__global__ void __launch_bounds__(FCX_THREADS, 1) fcxMoveEmuKernel(const FcxDevComm *dcs, const FcxCollArgs *as, int ctasPerRank) {
-  int r = blockIdx.x / ctasPerRank;
-  fcxMoveBody(dcs[r], as[r], blockIdx.x % ctasPerRank, ctasPerRank);
+__global__ void __launch_bounds__(FCX_THREADS, 1) fcxMoveEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
+  __shared__ FcxDevComm dc;
+  __shared__ FcxCollArgs a;
+  emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
+  fcxMoveBody(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxP2pEmuKernel(const FcxDevComm *dcs, const FcxP2pArgs *gs, int ctasPerRank) {
   int r = blockIdx.x / ctasPerRank;
@@ -1094,8 +1107,8 @@ cudaError_t launchTyped(const FcxDevComm &dc, const FcxCollArgs &a, int nctas, c
 }
 
 template <typename TIn, typename TOut>
-cudaError_t launchTypedEmu(const FcxDevComm *dcs, const FcxCollArgs *as, int nranks, int nctas, cudaStream_t s) {
-  void *params[] = {(void *)&dcs, (void *)&as, (void *)&nctas};
+cudaError_t launchTypedEmu(const FcxEmuRanks &l, int nranks, int nctas, cudaStream_t s) {
+  void *params[] = {(void *)&l, (void *)&nctas};
   return cudaLaunchCooperativeKernel((const void *)fcxCollEmuKernel<TIn, TOut>, dim3(nranks * nctas), dim3(FCX_THREADS),
                                      params, 0, s);
 }
@@ -1147,21 +1160,20 @@ extern "C" cudaError_t fcxLaunchWaitTest(const FcxDevComm *dc, uint64_t want, cu
   return cudaGetLastError();
 }
 
-// dcs/as/gs are device arrays with one entry per emulated rank.
-extern "C" cudaError_t fcxLaunchCollEmu(const FcxDevComm *dcs, const FcxCollArgs *as, const FcxCollArgs *hostArgs0,
-                                        int nranks, int nctas, cudaStream_t s) {
-  const FcxCollArgs *a = hostArgs0;
+extern "C" cudaError_t fcxLaunchCollEmu(const FcxEmuRanks *l, int nranks, int nctas, cudaStream_t s) {
+  const FcxCollArgs *a = &l->args[0];
   if (a->kind < 0 || a->kind >= FCX_K_NUM || !kindServes(a)) return cudaErrorInvalidValue;
-  void *params[] = {(void *)&dcs, (void *)&as, (void *)&nctas};
-  if (a->kind == FCX_K_MOVE_ZC || isZcReduceKind(a->kind)) return fcxLaunchZcEmu(dcs, as, hostArgs0, nranks, nctas, s);
+  void *params[] = {(void *)l, (void *)&nctas};
+  if (a->kind == FCX_K_MOVE_ZC || isZcReduceKind(a->kind)) return fcxLaunchZcEmu(l, nranks, nctas, s);
   if (isMoveKind(a->kind))
     return cudaLaunchCooperativeKernel((const void *)fcxMoveEmuKernel, dim3(nranks * nctas), dim3(FCX_THREADS), params, 0, s);
-  if (a->kind == FCX_K_BARRIER) return launchTypedEmu<uint8_t, uint8_t>(dcs, as, nranks, nctas, s);
-#define CALL(TI, TO) launchTypedEmu<TI, TO>(dcs, as, nranks, nctas, s)
+  if (a->kind == FCX_K_BARRIER) return launchTypedEmu<uint8_t, uint8_t>(*l, nranks, nctas, s);
+#define CALL(TI, TO) launchTypedEmu<TI, TO>(*l, nranks, nctas, s)
   FCX_DISPATCH_ALL(a, CALL);
 #undef CALL
 }
 
+// dcs/gs are device arrays with one entry per emulated rank.
 extern "C" cudaError_t fcxLaunchP2pEmu(const FcxDevComm *dcs, const FcxP2pArgs *gs, int nranks, int ctasPerRank,
                                        cudaStream_t s) {
   void *params[] = {(void *)&dcs, (void *)&gs, (void *)&ctasPerRank};

@@ -421,4 +421,15 @@ __device__ __forceinline__ uint4 mmFinish(uint4 r, int op, int nranks, float sca
 }
 
 
+// An emulated rank's descriptor and arguments, fetched into shared memory by the whole CTA: the bodies look at them all
+// the time, and field by field each first look would be a trip to memory of its own.
+template <typename Ranks>
+__device__ __forceinline__ void emuRank(const Ranks &l, int r, FcxDevComm *dc, FcxCollArgs *a) {
+  static_assert(sizeof(FcxDevComm) % 4 == 0 && sizeof(FcxCollArgs) % 4 == 0, "copied in words");
+  const uint32_t *sd = (const uint32_t *)&l.dc[r], *sa = (const uint32_t *)&l.args[r];
+  for (int i = threadIdx.x; i < (int)(sizeof(FcxDevComm) / 4); i += blockDim.x) ((uint32_t *)dc)[i] = sd[i];
+  for (int i = threadIdx.x; i < (int)(sizeof(FcxCollArgs) / 4); i += blockDim.x) ((uint32_t *)a)[i] = sa[i];
+  __syncthreads();
+}
+
 }  // namespace fcxdev

@@ -15,13 +15,17 @@ __global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcMoveKernel(FcxDevComm dc,
   fcxZcMoveBody(dc, a, blockIdx.x, gridDim.x);
 }
 template <typename TIn, typename TOut>
-__global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcReduceEmuKernel(const FcxDevComm *dcs, const FcxCollArgs *as, int ctasPerRank) {
-  int r = blockIdx.x / ctasPerRank;
-  fcxZcReduceBody<TIn, TOut>(dcs[r], as[r], blockIdx.x % ctasPerRank, ctasPerRank);
+__global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcReduceEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
+  __shared__ FcxDevComm dc;
+  __shared__ FcxCollArgs a;
+  emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
+  fcxZcReduceBody<TIn, TOut>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
-__global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcMoveEmuKernel(const FcxDevComm *dcs, const FcxCollArgs *as, int ctasPerRank) {
-  int r = blockIdx.x / ctasPerRank;
-  fcxZcMoveBody(dcs[r], as[r], blockIdx.x % ctasPerRank, ctasPerRank);
+__global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcMoveEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
+  __shared__ FcxDevComm dc;
+  __shared__ FcxCollArgs a;
+  emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
+  fcxZcMoveBody(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
 
 }  // namespace fcxdev
@@ -36,8 +40,8 @@ cudaError_t launchZc(const FcxDevComm &dc, const FcxCollArgs &a, int nctas, cuda
   return cudaGetLastError();
 }
 template <typename TIn, typename TOut>
-cudaError_t launchZcEmu(const FcxDevComm *dcs, const FcxCollArgs *as, int nranks, int nctas, cudaStream_t s) {
-  void *params[] = {(void *)&dcs, (void *)&as, (void *)&nctas};
+cudaError_t launchZcEmu(const FcxEmuRanks &l, int nranks, int nctas, cudaStream_t s) {
+  void *params[] = {(void *)&l, (void *)&nctas};
   return cudaLaunchCooperativeKernel((const void *)fcxZcReduceEmuKernel<TIn, TOut>, dim3(nranks * nctas), dim3(FCX_THREADS),
                                      params, 0, s);
 }
@@ -54,13 +58,13 @@ extern "C" cudaError_t fcxLaunchZc(const FcxDevComm *dc, const FcxCollArgs *a, i
 #undef CALL
 }
 
-extern "C" cudaError_t fcxLaunchZcEmu(const FcxDevComm *dcs, const FcxCollArgs *as, const FcxCollArgs *a, int nranks, int nctas,
-                                      cudaStream_t s) {
+extern "C" cudaError_t fcxLaunchZcEmu(const FcxEmuRanks *l, int nranks, int nctas, cudaStream_t s) {
+  const FcxCollArgs *a = &l->args[0];
   if (a->kind == FCX_K_MOVE_ZC) {
-    void *params[] = {(void *)&dcs, (void *)&as, (void *)&nctas};
+    void *params[] = {(void *)l, (void *)&nctas};
     return cudaLaunchCooperativeKernel((const void *)fcxZcMoveEmuKernel, dim3(nranks * nctas), dim3(FCX_THREADS), params, 0, s);
   }
-#define CALL(TI, TO) launchZcEmu<TI, TO>(dcs, as, nranks, nctas, s)
+#define CALL(TI, TO) launchZcEmu<TI, TO>(*l, nranks, nctas, s)
   FCX_DISPATCH_ALL(a, CALL);
 #undef CALL
 }
