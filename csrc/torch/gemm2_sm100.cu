@@ -28,6 +28,7 @@
 #include <stdint.h>
 
 #include "gemm_sm100.h"
+#include "pdl.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -115,6 +116,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   clusterSync();  // the peer's barriers exist before anything arrives on them
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();  // everything above touches only this CTA's own memories
 
   if (warp == 0) {
     // ---- TMA producer (both CTAs): own half of A and of B; bytes counted on the leader's barrier
@@ -388,9 +391,7 @@ extern "C" cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, in
     if (e != cudaSuccess) return e;
   }
   const int grid = 2 * std::min(units * p.splitK, pairs);
-  if (geluOut) fcxGemmPairKernel<true><<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, mc, mc2, p);
-  else fcxGemmPairKernel<false><<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, mc, mc2, p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = fcxpdl::launchPdl(geluOut ? fcxGemmPairKernel<true> : fcxGemmPairKernel<false>, grid, THREADS, SMEM_BYTES, s, ma, mb, mc, mc2, p);
   if (e != cudaSuccess && detail)
     snprintf(detail, detailLen, "pair kernel launch: %s (M %d N %d K %d splitK %d grid %d)", cudaGetErrorString(e), M, N, K, p.splitK, grid);
   return e;

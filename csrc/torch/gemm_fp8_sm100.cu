@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include "gemm_fp8_sm100.h"
+#include "pdl.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -146,6 +147,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
   __syncthreads();
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();  // everything above touches only this CTA's own memories
 
   if (warp == 8) {
     if (lane == 0) {
@@ -287,6 +290,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
   clusterSync();  // the peer's barriers exist before anything arrives on them
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();  // everything above touches only this CTA's own memories
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGS));
@@ -415,6 +420,8 @@ __global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *__res
   const size_t total = (size_t)M * nKb;
   const int sub = threadIdx.x / LANES, l = threadIdx.x % LANES;
   const size_t first = (size_t)blockIdx.x * PER_CTA * UNROLL + sub;
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
   uint32_t raw[UNROLL][VEC / 2];
 #pragma unroll
   for (int u = 0; u < UNROLL; u++) {
@@ -526,8 +533,7 @@ cudaError_t launchOne(const CUtensorMap &ma, const void *bq, const CUtensorMap &
     attr = true;
   }
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  gemmFp8Kernel<BN><<<std::min(tiles, smCount()), THREADS, smemBytes(BN), s>>>(ma, mb, mc, p);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(gemmFp8Kernel<BN>, std::min(tiles, smCount()), THREADS, smemBytes(BN), s, ma, mb, mc, p);
 }
 
 cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
@@ -540,8 +546,7 @@ cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap 
     attr = true;
   }
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + PN - 1) / PN);
-  gemmFp8PairKernel<<<2 * std::min(tiles, smCount() / 2), PTHREADS, PSMEM_BYTES, s>>>(ma, mb, mc, p);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(gemmFp8PairKernel, 2 * std::min(tiles, smCount() / 2), PTHREADS, PSMEM_BYTES, s, ma, mb, mc, p);
 }
 
 }  // namespace
@@ -566,8 +571,7 @@ extern "C" cudaError_t fcxGemmFp8Blockwise(const void *aq, const float *sa, cons
   if (!makeTileMap(&ma, aq, M, K, K, BM, 1) || !makeStoreMap(&mc, c, M, N, ldc)) return cudaErrorNotSupported;
   Params p{};
   p.M = M; p.N = N; p.K = K; p.sa = sa; p.sb = sb; p.errFlag = errFlag;
-  static const int forced = [] { const char *e = getenv("FLAGCX_FP8_TILE"); return e ? atoi(e) : -1; }();
-  const int tile = forced >= 0 ? forced : fcxGemmFp8Tile(M, N, smCount());
+  const int tile = fcxGemmFp8Tile(M, N, smCount());
   p.group = tile == 0 ? 8 : (N + 127) / 128 >= 48 ? 16 : 8;
   return tile == 0 ? launchPair(ma, bq, mc, p, s) : tile == 128 ? launchOne<128>(ma, bq, mc, p, s) : launchOne<64>(ma, bq, mc, p, s);
 }
@@ -580,10 +584,9 @@ extern "C" cudaError_t fcxQuantFp8Act(const void *x, void *q, float *sa, int M, 
   const __nv_bfloat16 *src = (const __nv_bfloat16 *)x;
   __nv_fp8_storage_t *dst = (__nv_fp8_storage_t *)q;
   // four blocks per lane group once that still leaves two CTAs for every SM, else one: a small batch wants many CTAs
-  if (wide && blocks >= 16 * 4 * 2 * (size_t)smCount()) quantActKernel<8, 4><<<(unsigned)((blocks + 63) / 64), 256, 0, s>>>(src, dst, sa, M, K, ldx);
-  else if (wide) quantActKernel<8, 1><<<(unsigned)((blocks + 15) / 16), 256, 0, s>>>(src, dst, sa, M, K, ldx);
-  else quantActKernel<4, 1><<<(unsigned)((blocks + 7) / 8), 256, 0, s>>>(src, dst, sa, M, K, ldx);
-  return cudaGetLastError();
+  if (wide && blocks >= 16 * 4 * 2 * (size_t)smCount()) return fcxpdl::launchPdl(quantActKernel<8, 4>, (unsigned)((blocks + 63) / 64), 256, 0, s, src, dst, sa, M, K, ldx);
+  if (wide) return fcxpdl::launchPdl(quantActKernel<8, 1>, (unsigned)((blocks + 15) / 16), 256, 0, s, src, dst, sa, M, K, ldx);
+  return fcxpdl::launchPdl(quantActKernel<4, 1>, (unsigned)((blocks + 7) / 8), 256, 0, s, src, dst, sa, M, K, ldx);
 }
 
 extern "C" cudaError_t fcxQuantFp8Weight(const void *w, void *q, float *sb, int N, int K, int ldw, cudaStream_t s) {

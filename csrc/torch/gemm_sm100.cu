@@ -44,6 +44,7 @@
 #include <stdint.h>
 
 #include "gemm_sm100.h"
+#include "pdl.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
   uint64_t *fullBar = bars, *emptyBar = bars + STAGES, *tmemFull = bars + 2 * STAGES, *tmemEmpty = bars + 2 * STAGES + 2;
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 4);
 
+  if (MODE == FCX_GEMM_PLAIN && p.mPtr) fcxpdl::pdlWait();  // the row count comes from the kernel before
   const int Mrows = p.mPtr ? min(*p.mPtr, p.M) : p.M;  // the row count may live on the device
   const int bn = p.bn;  // columns per tile: 256, or 128 when that fills the SMs better
   const int nN = (p.N + bn - 1) / bn, nM = (Mrows + BM - 1) / BM;
@@ -157,6 +159,10 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
   __syncthreads();
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
+  if (MODE == FCX_GEMM_PLAIN) {
+    fcxpdl::pdlRelease();
+    fcxpdl::pdlWait();  // everything above touches only this CTA's own memories
+  }
 
   if (warp == 0) {
     // ---- TMA producer
@@ -413,6 +419,8 @@ cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, const FcxGemmPara
     if (e != cudaSuccess) return e;
     attr = true;
   }
+  // the kernels that exchange with peers are launched plainly: their first accesses are flags and peers' memory
+  if (MODE == FCX_GEMM_PLAIN) return fcxpdl::launchPdl(fcxGemmKernel<MODE>, grid, THREADS, SMEM_BYTES, s, a, b, aLocal ? *aLocal : a, p, dc);
   fcxGemmKernel<MODE><<<grid, THREADS, SMEM_BYTES, s>>>(a, b, aLocal ? *aLocal : a, p, dc);
   return cudaGetLastError();
 }

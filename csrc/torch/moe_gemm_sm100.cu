@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "moe_gemm_sm100.h"
+#include "pdl.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -73,6 +74,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 4);
 
   const int nN = (p.N + COLS - 1) / COLS, nK = (p.K + BK - 1) / BK;
+  fcxpdl::pdlRelease();
+  if (threadIdx.x < 64) fcxpdl::pdlWait();  // the row counts come from the kernel before
   if ((int)threadIdx.x < p.L) rowsOf[threadIdx.x] = max(0, min(p.rows[threadIdx.x], p.capL));
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&emptyBar[s], 1); }
@@ -97,6 +100,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   clusterSync();  // the peer's barriers exist before anything arrives on them
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
+  fcxpdl::pdlWait();
   const int nTiles = tileStart[p.L];
 
   // Tile t -> (expert, 256-row block of its segment, column block).  `e` only moves forward: a role's tiles ascend.
@@ -299,8 +303,7 @@ cudaError_t launchGroup(const CUtensorMap &a, const CUtensorMap &h, const Weight
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  moeGroupKernel<UP, BN><<<2 * pairCount(), THREADS, smemBytes(BN), s>>>(a, h, wm, p, dc);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(moeGroupKernel<UP, BN>, 2 * pairCount(), THREADS, smemBytes(BN), s, a, h, wm, p, dc);
 }
 
 }  // namespace

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "moe_sm100.h"
+#include "pdl.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -183,6 +184,7 @@ __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, con
                                                         __nv_bfloat16 *__restrict__ out, int T, int H, int K, size_t doneOff, uint64_t want,
                                                         int *errFlag) {
   bool ok = true;
+  fcxpdl::pdlWait();
   if (threadIdx.x == 0) {
     ok = fcxdev::waitGe(dc, (const uint64_t *)(dc.heap[dc.rank] + doneOff), want, -1, FCX_WAIT_DEVAPI, blockIdx.x, want);
     if (!ok) *errFlag = 1;
@@ -281,6 +283,5 @@ extern "C" cudaError_t fcxMoeCombine(const FcxDevComm *dc, const void *ret, cons
   const bool small = (uint64_t)T * (H / 8) + 16ull * 592 * 256 < (1ull << 32);
   auto kernel = !small ? moeCombineKernel<0> : K == 1 ? moeCombineKernel<1> : K == 2 ? moeCombineKernel<2> : K == 4 ? moeCombineKernel<4>
                                                                                                                  : moeCombineKernel<0>;
-  kernel<<<592, 256, 0, s>>>(*dc, (const __nv_bfloat16 *)ret, w, (__nv_bfloat16 *)out, T, H, K, doneOff, want, errFlag);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(kernel, 592, 256, 0, s, *dc, (const __nv_bfloat16 *)ret, w, (__nv_bfloat16 *)out, T, H, K, doneOff, want, errFlag);
 }

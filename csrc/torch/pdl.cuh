@@ -1,0 +1,29 @@
+// Programmatic dependent launch for kernels that follow one another on a stream: the next kernel's CTAs come up (barriers,
+// TMEM, shared memory) while the last CTAs of the one before still run, and pdlWait() holds every thread until that kernel
+// has finished and its writes are visible.  A kernel launched with launchPdl calls pdlWait() before its first access to
+// global memory, reads and writes alike; behind anything but a kernel that calls pdlRelease() the wait is an ordinary
+// stream dependency.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace fcxpdl {
+
+__device__ __forceinline__ void pdlRelease() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launchPdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+}  // namespace fcxpdl
