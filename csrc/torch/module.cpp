@@ -89,20 +89,22 @@ static std::tuple<at::Tensor, at::Tensor> biasGeluBwd(const at::Tensor &dy, cons
   checkBf16(x, "x");
   c10::cuda::CUDAGuard g(x.device());
   const int C = (int)x.size(-1), M = (int)(x.numel() / C);
+  checkBf16(bias, "bias");
+  TORCH_CHECK(dy.numel() == x.numel() && bias.numel() == C, "dy must have x's shape and bias one element per column");
   auto dx = at::empty_like(x);
-  CUDA_OK(fcxBiasGeluBwd(dy.data_ptr(), x.data_ptr(), bias.data_ptr(), dx.data_ptr(), M, C, cur()));
   const bool into = dbiasInto.has_value() && dbiasInto->defined();
   if (into) {
     checkBf16(*dbiasInto, "dbias_into");
     TORCH_CHECK(dbiasInto->numel() == C, "dbias_into must have one element per column");
   }
   auto dbias = into ? *dbiasInto : at::empty_like(bias);
-  auto partial = at::empty({fcxColSumPartials(M), C}, x.options().dtype(at::kFloat));
-  CUDA_OK(fcxColSum(dx.data_ptr(), dbias.data_ptr(), partial.data_ptr<float>(), M, C, into ? 1 : 0, cur()));
+  auto partial = at::empty({fcxBiasGeluBwdPartials(M, C), C}, x.options().dtype(at::kFloat));
+  CUDA_OK(fcxBiasGeluBwd(dy.data_ptr(), x.data_ptr(), bias.data_ptr(), dx.data_ptr(), dbias.data_ptr(), partial.data_ptr<float>(), M, C,
+                         into ? 1 : 0, cur()));
   return {dx, dbias};
 }
 
-static at::Tensor colSum(const at::Tensor &a, const c10::optional<at::Tensor> &intoT) {
+at::Tensor colSum(const at::Tensor &a, const c10::optional<at::Tensor> &intoT) {
   checkBf16(a, "a");
   c10::cuda::CUDAGuard g(a.device());
   const int C = (int)a.size(-1), M = (int)(a.numel() / C);

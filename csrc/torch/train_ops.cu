@@ -13,6 +13,7 @@
 
 #include "train_ops.h"
 #include "train_ops_noalloc.h"
+#include "pdl.cuh"
 
 #include <mutex>
 
@@ -98,6 +99,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnFwdKernel(const bf16 *__re
     }
     cpAsyncCommit();  // an empty group past the last row keeps the group count uniform
   };
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
 #pragma unroll
   for (int st = 0; st < STAGES - 1; st++) issue(warp + st * nwarps, st);
   int k = 0;
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnFwdKernel(const bf16 *__re
   cpAsyncWait<0>();
 }
 
-// Backward, part 1: dx = rstd * (g*dy - mean(g*dy) - xhat * mean(g*dy*xhat)) [+ dres].
+// Backward, part 1, for rows wider than 1024: dx = rstd * (g*dy - mean(g*dy) - xhat * mean(g*dy*xhat)) [+ dres].
 // Same streaming scheme for dy and x; the residual gradient, needed only for the last step of a row, is loaded into
 // registers when the row's turn begins.
 template <int MAXV, int STAGES, int LN_WARPS>
@@ -177,6 +180,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdDxKernel(const bf16 *__
     }
     cpAsyncCommit();
   };
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
 #pragma unroll
   for (int st = 0; st < STAGES - 1; st++) issue(warp + st * nwarps, st);
   float muN = warp < M ? mean[warp] : 0.f, rsN = warp < M ? rstd[warp] : 0.f;  // statistics one row ahead
@@ -229,7 +234,136 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdDxKernel(const bf16 *__
   cpAsyncWait<0>();
 }
 
-// Backward, part 2: dgamma[c] = sum_r dy[r,c] * xhat[r,c], dbeta[c] = sum_r dy[r,c].
+// Backward in one pass over dy, x and dres for rows up to 1024 wide: dx as below, and the parameter gradients
+// dgamma[c] = sum_r dy[r,c] * xhat[r,c], dbeta[c] = sum_r dy[r,c] from the values that are on chip anyway (a second kernel
+// read dy and x again: 33 MB at 8192 x 1024).  The three rows of a warp stream through a ring in shared memory.  A thread
+// holds 32 columns' dgamma and dbeta sums, which leaves no room for the row: it is looked at twice in shared memory, once
+// for the two means and once for the results, so that sixteen warps fit on an SM (with eight that keep the row in
+// registers the arithmetic set the pace: 19 us at 8192 x 1024).  At the end the warps fold their sums in shared memory and
+// a CTA leaves [2][C] of them in `partial` for lnParamFoldKernel.
+template <int MAXV, int STAGES, int LN_WARPS>
+__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdFusedKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
+                                                                     const bf16 *__restrict__ gamma, const float *__restrict__ mean,
+                                                                     const float *__restrict__ rstd, const bf16 *__restrict__ dres,
+                                                                     bf16 *__restrict__ dx, float *__restrict__ partial, int M, int C) {
+  extern __shared__ __align__(16) uint8_t lnSmem[];
+  const int warpInCta = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = blockIdx.x * LN_WARPS + warpInCta, nwarps = gridDim.x * LN_WARPS;
+  const int nv = C / 256;
+  const size_t rowBytes = (size_t)C * 2;
+  uint8_t *ring = lnSmem + (size_t)warpInCta * STAGES * 3 * rowBytes;
+  auto issue = [&](int row, int st) {
+    if (row < M) {
+      uint8_t *dst = ring + (size_t)st * 3 * rowBytes;
+#pragma unroll
+      for (int i = 0; i < MAXV; i++)
+        if (i < nv) {
+          const size_t off = (size_t)(i * 32 + lane) * 16;
+          cpAsync16(dst + off, (const uint8_t *)(dy + (size_t)row * C) + off);
+          cpAsync16(dst + rowBytes + off, (const uint8_t *)(x + (size_t)row * C) + off);
+          if (dres) cpAsync16(dst + 2 * rowBytes + off, (const uint8_t *)(dres + (size_t)row * C) + off);
+        }
+    }
+    cpAsyncCommit();
+  };
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
+#pragma unroll
+  for (int st = 0; st < STAGES - 1; st++) issue(warp + st * nwarps, st);
+  float dg[MAXV][8], db[MAXV][8];
+#pragma unroll
+  for (int i = 0; i < MAXV; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) dg[i][j] = db[i][j] = 0.f;
+  float muN = warp < M ? mean[warp] : 0.f, rsN = warp < M ? rstd[warp] : 0.f;  // statistics one row ahead
+  int k = 0;
+  for (int row = warp; row < M; row += nwarps, k++) {
+    issue(row + (STAGES - 1) * nwarps, (k + STAGES - 1) % STAGES);
+    const float mu = muN, rs = rsN;
+    if (row + nwarps < M) { muN = mean[row + nwarps]; rsN = rstd[row + nwarps]; }
+    cpAsyncWait<STAGES - 1>();
+    const uint8_t *base = ring + (size_t)(k % STAGES) * 3 * rowBytes;
+    const Bf8 *dyr = (const Bf8 *)base, *xr = (const Bf8 *)(base + rowBytes), *rr = (const Bf8 *)(base + 2 * rowBytes);
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < MAXV; i++)
+      if (i < nv) {
+        float d[8], xv[8], g[8];
+        unpack8(dyr[i * 32 + lane], d);
+        unpack8(xr[i * 32 + lane], xv);
+        unpack8(((const Bf8 *)gamma)[i * 32 + lane], g);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float xh = (xv[j] - mu) * rs, gy = g[j] * d[j];
+          s1 += gy;
+          s2 += gy * xh;
+          dg[i][j] += d[j] * xh;
+          db[i][j] += d[j];
+        }
+      }
+    s1 = warpSum(s1) / C;
+    s2 = warpSum(s2) / C;
+#pragma unroll
+    for (int i = 0; i < MAXV; i++)
+      if (i < nv) {
+        float d[8], xv[8], g[8], o[8];
+        unpack8(dyr[i * 32 + lane], d);
+        unpack8(xr[i * 32 + lane], xv);
+        unpack8(((const Bf8 *)gamma)[i * 32 + lane], g);
+        if (dres) unpack8(rr[i * 32 + lane], o);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float t = rs * (g[j] * d[j] - s1 - (xv[j] - mu) * rs * s2);
+          o[j] = dres ? o[j] + t : t;
+        }
+        ((Bf8 *)(dx + (size_t)row * C))[i * 32 + lane] = pack8(o);
+      }
+  }
+  cpAsyncWait<0>();
+  __syncthreads();  // the ring becomes the warps' sums: [warp][2][C]
+  float *sums = (float *)lnSmem + (size_t)warpInCta * 2 * C;
+#pragma unroll
+  for (int i = 0; i < MAXV; i++)
+    if (i < nv) {
+      float4 *g4 = (float4 *)(sums + (i * 32 + lane) * 8), *b4 = (float4 *)(sums + C + (i * 32 + lane) * 8);
+      g4[0] = make_float4(dg[i][0], dg[i][1], dg[i][2], dg[i][3]);
+      g4[1] = make_float4(dg[i][4], dg[i][5], dg[i][6], dg[i][7]);
+      b4[0] = make_float4(db[i][0], db[i][1], db[i][2], db[i][3]);
+      b4[1] = make_float4(db[i][4], db[i][5], db[i][6], db[i][7]);
+    }
+  __syncthreads();
+  for (int c = threadIdx.x; c < 2 * C; c += LN_WARPS * 32) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < LN_WARPS; w++) t += ((const float *)lnSmem)[(size_t)w * 2 * C + c];
+    partial[(size_t)blockIdx.x * 2 * C + c] = t;
+  }
+}
+
+// dgamma / dbeta from the `parts` partial sums of lnBwdFusedKernel: a CTA folds 32 of the 2 C columns, eight groups of
+// lanes an eighth of the parts each.
+__global__ void __launch_bounds__(256) lnParamFoldKernel(const float *__restrict__ partial, int parts, int C, bf16 *__restrict__ dgamma,
+                                                         bf16 *__restrict__ dbeta, int accumulate) {
+  __shared__ float red[8][33];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // 2 C is a multiple of 32
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
+  float t = 0.f;
+#pragma unroll 4
+  for (int p = grp; p < parts; p += 8) t += partial[(size_t)p * 2 * C + c];
+  red[grp][lane] = t;
+  __syncthreads();
+  if (grp == 0) {
+    t = 0.f;
+#pragma unroll
+    for (int g = 0; g < 8; g++) t += red[g][lane];
+    bf16 *dst = c < C ? dgamma + c : dbeta + (c - C);
+    if (accumulate) t += __bfloat162float(*dst);
+    *dst = __float2bfloat16_rn(t);
+  }
+}
+
+// Backward, part 2, for rows wider than 1024: dgamma[c] = sum_r dy[r,c] * xhat[r,c], dbeta[c] = sum_r dy[r,c].
 // A CTA owns 64 columns and one slice of the rows; partial sums go to
 // `partial` ([gridDim.y][2][C], fp32 scratch); the CTA that finishes a column block last folds them into dgamma / dbeta.
 __global__ void __launch_bounds__(256) lnBwdParamKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
@@ -237,6 +371,8 @@ __global__ void __launch_bounds__(256) lnBwdParamKernel(const bf16 *__restrict__
                                                         float *__restrict__ partial, int M, int C, bf16 *__restrict__ dgamma,
                                                         bf16 *__restrict__ dbeta, int accumulate) {
   __shared__ float redG[32][64 + 1], redB[32][64 + 1];
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
   const int col0 = blockIdx.x * 64;
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   float dg[8] = {0, 0, 0, 0, 0, 0, 0, 0}, db[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -335,6 +471,8 @@ __device__ __forceinline__ float geluGrad(float x) {
 // y = gelu(x + bias); x is [M, C].  Each thread keeps four 16-byte loads in flight.
 __global__ void __launch_bounds__(256) biasGeluFwdKernel(const bf16 *__restrict__ x, const bf16 *__restrict__ bias,
                                                          bf16 *__restrict__ y, size_t nvec, int C) {
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
   const int cv = C / 8;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -362,35 +500,78 @@ __global__ void __launch_bounds__(256) biasGeluFwdKernel(const bf16 *__restrict_
   }
 }
 
-// dx = dy * gelu'(x + bias)
+// dx = dy * gelu'(x + bias) and, from the same values, the partial column sums of the bias gradient ([gridDim.y][C], fp32,
+// folded by colSumFoldKernel).  A CTA owns VX * 8 columns (all 256 threads side by side on wide rows) and every gridDim.y-th
+// group of 256 / VX rows, four rows (eight 16-byte loads) in flight per thread; a thread keeps its eight columns throughout.
+// Bound by memory (dy, x, dx: 201 MB and 30 us at 8192 x 4096) with the arithmetic close behind.  Blocks of 64 columns with a
+// fold in the last CTA, as in the plain column sum, took 55 us: their CTAs lived for eight rows per thread.
 __global__ void __launch_bounds__(256) biasGeluBwdKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
-                                                         const bf16 *__restrict__ bias, bf16 *__restrict__ dx, size_t nvec, int C) {
-  const int cv = C / 8;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + stride < nvec; i += 2 * stride) {
-    Bf8 xv[2], dv[2];
-#pragma unroll
-    for (int j = 0; j < 2; j++) { xv[j] = ((const Bf8 *)x)[i + j * stride]; dv[j] = ((const Bf8 *)dy)[i + j * stride]; }
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-      float a[8], b[8], d[8];
-      unpack8(xv[j], a);
-      unpack8(dv[j], d);
-      unpack8(((const Bf8 *)bias)[(i + j * stride) % cv], b);
-#pragma unroll
-      for (int k = 0; k < 8; k++) d[k] *= geluGrad(a[k] + b[k]);
-      ((Bf8 *)dx)[i + j * stride] = pack8(d);
-    }
-  }
-  for (; i < nvec; i += stride) {
-    float a[8], b[8], d[8];
-    unpack8(((const Bf8 *)x)[i], a);
-    unpack8(((const Bf8 *)bias)[i % cv], b);
-    unpack8(((const Bf8 *)dy)[i], d);
+                                                         const bf16 *__restrict__ bias, bf16 *__restrict__ dx, float *__restrict__ partial,
+                                                         int M, int C, int VX) {
+  __shared__ float red[2048];
+  const int tx = threadIdx.x % VX, ty = threadIdx.x / VX, RY = 256 / VX;
+  const int col = (blockIdx.x * VX + tx) * 8;
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, b[8];
+  unpack8(*(const Bf8 *)(bias + col), b);
+  auto one = [&](const Bf8 &xv, const Bf8 &dv, size_t off) {
+    float a[8], d[8];
+    unpack8(xv, a);
+    unpack8(dv, d);
 #pragma unroll
     for (int k = 0; k < 8; k++) d[k] *= geluGrad(a[k] + b[k]);
-    ((Bf8 *)dx)[i] = pack8(d);
+    const Bf8 o = pack8(d);
+    *(Bf8 *)(dx + off) = o;
+    unpack8(o, d);  // the sum is that of the stored gradient
+#pragma unroll
+    for (int k = 0; k < 8; k++) acc[k] += d[k];
+  };
+  const int step = gridDim.y * RY;
+  int r = blockIdx.y * RY + ty;
+  for (; r + 3 * step < M; r += 4 * step) {
+    Bf8 xv[4], dv[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const size_t off = (size_t)(r + u * step) * C + col;
+      xv[u] = *(const Bf8 *)(x + off);
+      dv[u] = *(const Bf8 *)(dy + off);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) one(xv[u], dv[u], (size_t)(r + u * step) * C + col);
+  }
+  for (; r < M; r += step) {
+    const size_t off = (size_t)r * C + col;
+    one(*(const Bf8 *)(x + off), *(const Bf8 *)(dy + off), off);
+  }
+  // fold the row lanes of the CTA, then one sum per column
+#pragma unroll
+  for (int k = 0; k < 8; k++) red[(ty * VX + tx) * 8 + k] = acc[k];
+  __syncthreads();
+  for (int c = threadIdx.x; c < VX * 8; c += 256) {
+    float t = 0.f;
+    for (int y = 0; y < RY; y++) t += red[y * VX * 8 + c];
+    partial[(size_t)blockIdx.y * C + blockIdx.x * VX * 8 + c] = t;
+  }
+}
+
+// out[c] (+)= the sum of `parts` partial column sums; a CTA folds 32 columns, eight groups of lanes an eighth of the parts each.
+__global__ void __launch_bounds__(256) colSumFoldKernel(const float *__restrict__ partial, int parts, int C, bf16 *__restrict__ out, int accumulate) {
+  __shared__ float red[8][33];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // C is a multiple of 64
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
+  float t = 0.f;
+#pragma unroll 4
+  for (int p = grp; p < parts; p += 8) t += partial[(size_t)p * C + c];
+  red[grp][lane] = t;
+  __syncthreads();
+  if (grp == 0) {
+    t = 0.f;
+#pragma unroll
+    for (int g = 0; g < 8; g++) t += red[g][lane];
+    if (accumulate) t += __bfloat162float(out[c]);
+    out[c] = __float2bfloat16_rn(t);
   }
 }
 
@@ -449,6 +630,8 @@ __global__ void colSumReduceKernel(const float *__restrict__ partial, int nparts
 // stream-ordered (they are: the backward pass runs on one stream).
 __global__ void __launch_bounds__(256) colSumFusedKernel(const bf16 *__restrict__ a, float *__restrict__ partial, bf16 *__restrict__ out,
                                                          int M, int C, int accumulate) {
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
   const int col0 = blockIdx.x * 64;
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -596,6 +779,8 @@ __global__ void __launch_bounds__(1024, 1) ceFwdBwdStreamKernel(bf16 *__restrict
     }
     cpAsyncCommit();
   };
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
   issue(blockIdx.x, 0);
   int k = 0;
   for (int row = blockIdx.x; row < M; row += gridDim.x, k++) {
@@ -696,6 +881,8 @@ __global__ void __launch_bounds__(256) adamwKernel(float *__restrict__ master, b
                                                    float *__restrict__ m, float *__restrict__ v, size_t n, float lr, float b1,
                                                    float b2, float eps, float wd, float bc1, float bc2, float gradScale,
                                                    int zeroGrad, const int *__restrict__ stepDev) {
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
   if (stepDev) {
     // step counter kept on the device so that a captured graph stays exact
     float st = (float)(*stepDev);
@@ -765,7 +952,10 @@ int smCount() {
 
 extern "C" {
 
-int fcxLnPartials(int M) { return max(1, min(32, M / 128)); }
+static int lnParts(int M) { return max(1, min(32, M / 128)); }
+constexpr int LN_BWD_WARPS = 16;
+static int lnFusedGrid(int M) { return std::max(1, std::min(smCount(), (M + LN_BWD_WARPS - 1) / LN_BWD_WARPS)); }
+int fcxLnPartials(int M) { return std::max(lnParts(M), lnFusedGrid(M)); }
 
 cudaError_t fcxLayerNormFwd(const void *x, const void *delta, const void *gamma, const void *beta, void *resOut, void *y,
                             float *mean, float *rstd, int M, int C, float eps, cudaStream_t s) {
@@ -784,9 +974,8 @@ cudaError_t fcxLayerNormFwd(const void *x, const void *delta, const void *gamma,
       if (e != cudaSuccess) return e;
       configured[configured[0] ? 1 : 0] = id;
     }
-    kernel<<<grid, warps * 32, smem, s>>>((const bf16 *)x, (const bf16 *)delta, (const bf16 *)gamma, (const bf16 *)beta, (bf16 *)resOut,
-                                          (bf16 *)y, mean, rstd, M, C, eps);
-    return cudaGetLastError();
+    return fcxpdl::launchPdl(kernel, grid, warps * 32, smem, s, (const bf16 *)x, (const bf16 *)delta, (const bf16 *)gamma, (const bf16 *)beta,
+                             (bf16 *)resOut, (bf16 *)y, mean, rstd, M, C, eps);
   };
   return C <= 1024 ? run(lnFwdKernel<4, 3, 16>) : run(lnFwdKernel<8, 3, 8>);
 }
@@ -796,56 +985,81 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
                             const void *dres, void *dx, void *dgamma, void *dbeta, float *partial, int M, int C, int accumulate,
                             cudaStream_t s) {
   if (C % 256 != 0 || C > 256 * 8) return cudaErrorInvalidValue;
-  const int warps = C <= 1024 ? 16 : 8;
-  const int grid = std::max(1, std::min(smCount(), (M + warps - 1) / warps));
-  const size_t smem = (size_t)warps * 3 * 2 * C * 2;  // warps x 3-deep ring x (dy, x) x row bytes <= 192 KB
-  auto run = [&](auto kernel) {
-    // both instantiations have the same pointer type, so this lambda exists once: remember the kernels by address
-    static thread_local const void *configured[2] = {nullptr, nullptr};
-    const void *id = (const void *)kernel;
-    if (configured[0] != id && configured[1] != id) {
+  if (C <= 1024) {
+    constexpr int STAGES = 2, WARPS = LN_BWD_WARPS;
+    const size_t smem = (size_t)WARPS * STAGES * 3 * C * 2;  // at most 192 KB; the warps' sums (WARPS x 2 x C fp32) fit in it
+    auto kernel = lnBwdFusedKernel<4, STAGES, WARPS>;
+    static thread_local bool attr = false;
+    if (!attr) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       if (e != cudaSuccess) return e;
-      configured[configured[0] ? 1 : 0] = id;
+      attr = true;
     }
-    kernel<<<grid, warps * 32, smem, s>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)gamma, mean, rstd, (const bf16 *)dres, (bf16 *)dx,
-                                          M, C);
-    return cudaGetLastError();
-  };
-  cudaError_t e = C <= 1024 ? run(lnBwdDxKernel<4, 3, 16>) : run(lnBwdDxKernel<8, 3, 8>);
+    const int grid = lnFusedGrid(M);
+    cudaError_t e = fcxpdl::launchPdl(kernel, grid, WARPS * 32, smem, s, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)gamma, mean, rstd,
+                                      (const bf16 *)dres, (bf16 *)dx, partial, M, C);
+    if (e != cudaSuccess) return e;
+    return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, 256, 0, s, (const float *)partial, grid, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
+  }
+  constexpr int WARPS = 8;
+  const size_t smem = (size_t)WARPS * 3 * 2 * C * 2;  // warps x 3-deep ring x (dy, x) x row bytes <= 192 KB
+  auto kernel = lnBwdDxKernel<8, 3, WARPS>;
+  static thread_local bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  cudaError_t e = fcxpdl::launchPdl(kernel, std::max(1, std::min(smCount(), (M + WARPS - 1) / WARPS)), WARPS * 32, smem, s, (const bf16 *)dy,
+                                    (const bf16 *)x, (const bf16 *)gamma, mean, rstd, (const bf16 *)dres, (bf16 *)dx, M, C);
   if (e != cudaSuccess) return e;
-  int parts = fcxLnPartials(M);
   // C <= 2048 here, so the 64-column blocks fit the ticket array: parameter partials and their reduction in one launch
-  lnBwdParamKernel<<<dim3(C / 64, parts), 256, 0, s>>>((const bf16 *)dy, (const bf16 *)x, mean, rstd, partial, M, C, (bf16 *)dgamma,
-                                                       (bf16 *)dbeta, accumulate);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(lnBwdParamKernel, dim3(C / 64, lnParts(M)), 256, 0, s, (const bf16 *)dy, (const bf16 *)x, mean, rstd, partial, M, C,
+                           (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
 }
 
 cudaError_t fcxBiasGeluFwd(const void *x, const void *bias, void *y, size_t M, int C, cudaStream_t s) {
   if (C % 8 != 0) return cudaErrorInvalidValue;
   size_t nvec = M * C / 8;
   int grid = (int)std::min<size_t>((nvec + 255) / 256, (size_t)smCount() * 8);
-  biasGeluFwdKernel<<<grid, 256, 0, s>>>((const bf16 *)x, (const bf16 *)bias, (bf16 *)y, nvec, C);
-  return cudaGetLastError();
-}
-
-cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void *dx, size_t M, int C, cudaStream_t s) {
-  if (C % 8 != 0) return cudaErrorInvalidValue;
-  size_t nvec = M * C / 8;
-  int grid = (int)std::min<size_t>((nvec + 255) / 256, (size_t)smCount() * 8);
-  biasGeluBwdKernel<<<grid, 256, 0, s>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)bias, (bf16 *)dx, nvec, C);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(biasGeluFwdKernel, grid, 256, 0, s, (const bf16 *)x, (const bf16 *)bias, (bf16 *)y, nvec, C);
 }
 
 int fcxColSumPartials(int M) { return max(1, min(32, M / 256)); }
+
+// Eight-column vectors that a CTA of biasGeluBwdKernel covers side by side, and its number of row groups.
+static void biasGeluBwdShape(int M, int C, int *vx, int *parts) {
+  const int cv = C / 8;
+  *vx = 256;
+  while (cv % *vx) *vx /= 2;  // C is a multiple of 64: 8 at least
+  const int rows = 256 / *vx, blocks = cv / *vx;
+  *parts = std::max(1, std::min((M + 4 * rows - 1) / (4 * rows), (4 * smCount() + blocks - 1) / blocks));
+}
+
+int fcxBiasGeluBwdPartials(int M, int C) {
+  int vx = 0, parts = 0;
+  if (C % 64 != 0 || C <= 0) return 1;
+  biasGeluBwdShape(M, C, &vx, &parts);
+  return parts;
+}
+
+cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void *dx, void *dbias, float *partial, int M, int C,
+                           int accumulate, cudaStream_t s) {
+  if (C % 64 != 0) return cudaErrorInvalidValue;
+  int vx = 0, parts = 0;
+  biasGeluBwdShape(M, C, &vx, &parts);
+  cudaError_t e = fcxpdl::launchPdl(biasGeluBwdKernel, dim3(C / 8 / vx, parts), 256, 0, s, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)bias,
+                                    (bf16 *)dx, partial, M, C, vx);
+  if (e != cudaSuccess) return e;
+  return fcxpdl::launchPdl(colSumFoldKernel, C / 32, 256, 0, s, (const float *)partial, parts, C, (bf16 *)dbias, accumulate);
+}
 
 // `partial` must hold fcxColSumPartials(M) * C floats.
 cudaError_t fcxColSum(const void *a, void *out, float *partial, int M, int C, int accumulate, cudaStream_t s) {
   if (C % 64 != 0) return cudaErrorInvalidValue;
   int parts = fcxColSumPartials(M);
   if (C / 64 <= 1024) {
-    colSumFusedKernel<<<dim3(C / 64, parts), 256, 0, s>>>((const bf16 *)a, partial, (bf16 *)out, M, C, accumulate);
-    return cudaGetLastError();
+    return fcxpdl::launchPdl(colSumFusedKernel, dim3(C / 64, parts), 256, 0, s, (const bf16 *)a, partial, (bf16 *)out, M, C, accumulate);
   }
   colSumKernel<<<dim3(C / 64, parts), 256, 0, s>>>((const bf16 *)a, partial, M, C);
   colSumReduceKernel<<<(C + 255) / 256, 256, 0, s>>>(partial, parts, C, (bf16 *)out, accumulate);
@@ -863,7 +1077,7 @@ cudaError_t fcxCrossEntropyFwdBwd(void *logits, const int64_t *targets, float *l
       if (e != cudaSuccess) return e;
       attr = true;
     }
-    ceFwdBwdStreamKernel<<<std::min(M, smCount()), 1024, ring, s>>>((bf16 *)logits, targets, losses, M, V, Vpad, gradScale);
+    return fcxpdl::launchPdl(ceFwdBwdStreamKernel, std::min(M, smCount()), 1024, ring, s, (bf16 *)logits, targets, losses, M, V, Vpad, gradScale);
   } else {
     ceFwdBwdKernel<<<M, 1024, 0, s>>>((bf16 *)logits, targets, losses, V, Vpad, gradScale);
   }
@@ -874,8 +1088,8 @@ cudaError_t fcxAdamW(float *master, void *param, void *grad, float *m, float *v,
                      float wd, int step, float gradScale, int zeroGrad, const int *stepDev, cudaStream_t s) {
   float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
   int grid = (int)std::min<size_t>((n / 8 + 255) / 256 + 1, (size_t)smCount() * 8);
-  adamwKernel<<<grid, 256, 0, s>>>(master, (bf16 *)param, (bf16 *)grad, m, v, n, lr, b1, b2, eps, wd, bc1, bc2, gradScale, zeroGrad, stepDev);
-  return cudaGetLastError();
+  return fcxpdl::launchPdl(adamwKernel, grid, 256, 0, s, master, (bf16 *)param, (bf16 *)grad, m, v, n, lr, b1, b2, eps, wd, bc1, bc2, gradScale,
+                           zeroGrad, stepDev);
 }
 
 }  // extern "C"

@@ -15,7 +15,10 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
                             const void *dres, void *dx, void *dgamma, void *dbeta, float *partial, int M, int C, int accumulate,
                             cudaStream_t s);
 cudaError_t fcxBiasGeluFwd(const void *x, const void *bias, void *y, size_t M, int C, cudaStream_t s);
-cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void *dx, size_t M, int C, cudaStream_t s);
+int fcxBiasGeluBwdPartials(int M, int C);
+// dx and the bias gradient (its column sums); `partial` must hold fcxBiasGeluBwdPartials(M, C) * C floats.
+cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void *dx, void *dbias, float *partial, int M, int C,
+                           int accumulate, cudaStream_t s);
 int fcxColSumPartials(int M);
 cudaError_t fcxColSum(const void *a, void *out, float *partial, int M, int C, int accumulate, cudaStream_t s);
 cudaError_t fcxCrossEntropyFwdBwd(void *logits, const int64_t *targets, float *losses, int M, int V, int Vpad, float gradScale,
