@@ -26,8 +26,10 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <vector>
 
 #include "gemm_sm100.h"
+#include "gemm_units.h"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
 
@@ -78,14 +80,29 @@ __device__ __forceinline__ float geluTanh(float x) {
   return 0.5f * x * (1.f + t);
 }
 
-// GELU = true: two outputs per tile: C = A B^T (kept for the backward pass) and C2 = gelu(A B^T + bias).
-template <bool GELU>
+// What the kernel needs of one product; `units` counts its tiles times its K pieces.
+struct PairProb {
+  CUtensorMap a, b, c;
+  int M, N, K, aMN, bMN, splitK, accumulate, group, units;
+};
+struct PairArgs {
+  PairProb prob[2];
+  CUtensorMap c2;  // GELU: the second output
+  const void *bias;
+  int extra;
+  int *errFlag;
+};
+
+// MODE_PLAIN: one product.  MODE_GELU: two outputs per tile: C = A B^T (kept for the backward pass) and
+// C2 = gelu(A B^T + bias).  MODE_DUAL: two independent products in one launch (the input and weight gradients of a linear
+// layer), so that the units of one fill the last wave of the other.
+enum { MODE_PLAIN, MODE_GELU, MODE_DUAL };
+template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-    fcxGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-                      const __grid_constant__ CUtensorMap tmC2, const FcxGemmParams p) {
+    fcxGemmPairKernel(const __grid_constant__ PairArgs args) {
   extern __shared__ uint8_t smemRaw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  volatile int *err = p.errFlag;
+  volatile int *err = args.errFlag;
   const uint32_t cr = ctaRankInCluster();  // 0 = leader
   const int pair = blockIdx.x >> 1, nPairs = gridDim.x >> 1;
 
@@ -96,11 +113,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   uint64_t *fullBar = bars, *emptyBar = bars + STAGES, *accFull = bars + 2 * STAGES, *accEmpty = bars + 2 * STAGES + 2;
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 4);
 
-  const int nN = (p.N + BN - 1) / BN, nM = (p.M + 2 * BM - 1) / (2 * BM);
-  const int nK = (p.K + BK - 1) / BK;
-  const int splitK = p.splitK > 1 ? p.splitK : 1;
-  const int kPer = (nK + splitK - 1) / splitK;
-  const int nTiles = nN * nM * splitK;
+  // Unit u of a product -> its tile and K range.
+  struct Where {
+    int mb, nb, kLo, kHi;
+    bool first;
+  };
+  auto locate = [](const PairProb &p, int u) {
+    Where w;
+    const int nN = (p.N + BN - 1) / BN, nM = (p.M + 2 * BM - 1) / (2 * BM), nK = (p.K + BK - 1) / BK;
+    const int kPer = (nK + p.splitK - 1) / p.splitK, piece = u % p.splitK;
+    tileCoord2(p.group, nM, nN, u / p.splitK, &w.mb, &w.nb);
+    w.kLo = piece * kPer;
+    w.kHi = min(nK, w.kLo + kPer);
+    w.first = piece == 0;
+    return w;
+  };
+  UnitIter it(pair, nPairs, args.prob[0].units, MODE == MODE_DUAL ? args.prob[1].units : 0, args.extra);
+  int which, unit;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&emptyBar[s], 1); }
@@ -125,25 +154,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = pair; t < nTiles && ok; t += nPairs) {
-        int mb, nb;
-        tileCoord2(p.group, nM, nN, t / splitK, &mb, &nb);
-        const int kLo = (t % splitK) * kPer, kHi = min(nK, kLo + kPer);
-        const int rowA = mb * 2 * BM + (int)cr * BM, colB = nb * BN + (int)cr * BNH;
-        for (int kb = kLo; kb < kHi; kb++) {
+      while (ok && it.next(&which, &unit)) {
+        const PairProb &p = args.prob[MODE == MODE_DUAL ? which : 0];
+        const Where w = locate(p, unit);
+        const int rowA = w.mb * 2 * BM + (int)cr * BM, colB = w.nb * BN + (int)cr * BNH;
+        for (int kb = w.kLo; kb < w.kHi; kb++) {
           if (!mbarWait(&emptyBar[stage], phase ^ 1, err)) { ok = false; break; }
           if (cr == 0) mbarExpectTx(&fullBar[stage], 2 * STAGE_BYTES);
           const uint32_t bar = mapToCta(smemAddr(&fullBar[stage]), 0);
           uint8_t *sa = tiles + stage * STAGE_BYTES, *sb = sa + A_BYTES;
           if (p.aMN) {
-            for (int j = 0; j < BM / 64; j++) tmaLoad2dPair(sa + j * MN_BLOCK_BYTES, &tmA, rowA + j * 64, kb * BK, bar);
+            for (int j = 0; j < BM / 64; j++) tmaLoad2dPair(sa + j * MN_BLOCK_BYTES, &p.a, rowA + j * 64, kb * BK, bar);
           } else {
-            tmaLoad2dPair(sa, &tmA, kb * BK, rowA, bar);
+            tmaLoad2dPair(sa, &p.a, kb * BK, rowA, bar);
           }
           if (p.bMN) {
-            for (int j = 0; j < BNH / 64; j++) tmaLoad2dPair(sb + j * MN_BLOCK_BYTES, &tmB, colB + j * 64, kb * BK, bar);
+            for (int j = 0; j < BNH / 64; j++) tmaLoad2dPair(sb + j * MN_BLOCK_BYTES, &p.b, colB + j * 64, kb * BK, bar);
           } else {
-            tmaLoad2dPair(sb, &tmB, kb * BK, colB, bar);
+            tmaLoad2dPair(sb, &p.b, kb * BK, colB, bar);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -155,21 +183,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       int stage = 0, buf = 0;
       uint32_t phase = 0, accPhase = 0;
       bool ok = true;
-      const uint32_t idesc = instrDescPair(p.aMN, p.bMN);
-      for (int t = pair; t < nTiles && ok; t += nPairs) {
+      while (ok && it.next(&which, &unit)) {
+        const PairProb &p = args.prob[MODE == MODE_DUAL ? which : 0];
+        const Where w = locate(p, unit);
+        const bool aMN = p.aMN, bMN = p.bMN;
+        const uint32_t idesc = instrDescPair(aMN, bMN);
         if (!mbarWait(&accEmpty[buf], accPhase ^ 1, err)) break;
         fenceAfter();
         const uint32_t dTmem = tmemBase + (uint32_t)buf * BN;
-        const int kLo = (t % splitK) * kPer, kHi = min(nK, kLo + kPer);
-        for (int kb = kLo; kb < kHi; kb++) {
+        for (int kb = w.kLo; kb < w.kHi; kb++) {
           if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
           fenceAfter();
           const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / 16; k++) {
-            const uint64_t da = p.aMN ? smemDescMN(sa + k * 2048, MN_BLOCK_BYTES) : smemDesc(sa + k * 32);
-            const uint64_t db = p.bMN ? smemDescMN(sb + k * 2048, MN_BLOCK_BYTES) : smemDesc(sb + k * 32);
-            mmaF16Pair(dTmem, da, db, idesc, (kb > kLo || k > 0) ? 1u : 0u);
+            const uint64_t da = aMN ? smemDescMN(sa + k * 2048, MN_BLOCK_BYTES) : smemDesc(sa + k * 32);
+            const uint64_t db = bMN ? smemDescMN(sb + k * 2048, MN_BLOCK_BYTES) : smemDesc(sb + k * 32);
+            mmaF16Pair(dTmem, da, db, idesc, (kb > w.kLo || k > 0) ? 1u : 0u);
           }
           mmaCommitPair(&emptyBar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -192,18 +222,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     bool live = true;
     uint8_t *stgBase = epiStage + (size_t)ew * STG_DEPTH * STG_BYTES;
     float *biasW = biasStage + ew * 128;
-    const bool reduce = splitK > 1 || p.accumulate;
-    for (int t = pair; t < nTiles; t += nPairs) {
-      int mb, nb;
-      tileCoord2(p.group, nM, nN, t / splitK, &mb, &nb);
-      const bool firstSplit = (t % splitK) == 0;
+    while (it.next(&which, &unit)) {
+      const PairProb &p = args.prob[MODE == MODE_DUAL ? which : 0];
+      const Where w = locate(p, unit);
+      const bool reduce = p.splitK > 1 || p.accumulate;
       if (live) live = __all_sync(0xffffffffu, mbarWait(&accFull[buf], accPhase, err));
       if (live) {
         fenceAfter();
-        const int row0 = mb * 2 * BM + (int)cr * BM + q * 32, colBase = nb * BN + half * 128;
-        const bool addBias = p.bias != nullptr && firstSplit;
+        const int row0 = w.mb * 2 * BM + (int)cr * BM + q * 32, colBase = w.nb * BN + half * 128;
+        const bool addBias = MODE != MODE_DUAL && args.bias != nullptr && w.first;
         if (addBias) {  // this warp's 128 bias values, once per tile, as fp32 in shared memory (columns past N read as 0)
-          const __nv_bfloat16 *bias = (const __nv_bfloat16 *)p.bias;
+          const __nv_bfloat16 *bias = (const __nv_bfloat16 *)args.bias;
 #pragma unroll
           for (int j = 0; j < 4; j++) {
             const int cidx = colBase + j * 32 + lane;
@@ -216,7 +245,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           if (colBase + c0 >= p.N || row0 >= p.M) break;
           uint32_t r[32];
           tmemLd32(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * 128 + c0), r);
-          if (GELU) {
+          if (MODE == MODE_GELU) {
             // both staging blocks of this warp are used per step: the product goes into the first, the activation
             // into the second, and one thread hands both to the TMA unit
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -254,9 +283,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             __syncwarp();
             if (lane == 0) {
               asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(&tmC), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stgPre)) : "memory");
+                           ::"l"(&p.c), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stgPre)) : "memory");
               asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(&tmC2), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stgAct)) : "memory");
+                           ::"l"(&args.c2), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stgAct)) : "memory");
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
             chunkNo++;
@@ -295,10 +324,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           if (lane == 0) {
             if (reduce)
               asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(&tmC), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stg)) : "memory");
+                           ::"l"(&p.c), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stg)) : "memory");
             else
               asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                           ::"l"(&tmC), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stg)) : "memory");
+                           ::"l"(&p.c), "r"(colBase + c0), "r"(row0), "r"(smemAddr(stg)) : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
           chunkNo++;
@@ -353,46 +382,143 @@ extern "C" int fcxGemmPairSuits(int M, int N, int K) {
   return fcxGemmPairCost(M, N, K, smCount2() / 2) <= 0.85 * fcxGemmTileCost(M, N, K, smCount2(), nullptr);
 }
 
-extern "C" cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,
-                                       const void *bias, int splitK, int accumulate, void *geluOut, int group, int *errFlag, cudaStream_t s,
-                                       char *detail, size_t detailLen) {
-  CUtensorMap ma, mb;
-  const bool okA = aMN ? makeTileMap(&ma, a, K, M, lda, BK, 2) : makeTileMap(&ma, a, M, K, lda, BM, 2);
-  const bool okB = bMN ? makeTileMap(&mb, b, K, N, ldb, BK, 2) : makeTileMap(&mb, b, N, K, ldb, BNH, 2);
-  CUtensorMap mc, mc2;
-  bool okC = makeStoreMap(&mc, c, M, N, ldc);
-  if (geluOut) {
-    if (accumulate || ((uintptr_t)geluOut & 15)) return cudaErrorInvalidValue;
-    okC = okC && makeStoreMap(&mc2, geluOut, M, N, ldc);
-    splitK = 1;  // the activation needs the whole sum
-  } else {
-    mc2 = mc;
-  }
+static bool fillProb(PairProb *p, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN, int group,
+                     char *detail, size_t detailLen) {
+  const bool okA = aMN ? makeTileMap(&p->a, a, K, M, lda, BK, 2) : makeTileMap(&p->a, a, M, K, lda, BM, 2);
+  const bool okB = bMN ? makeTileMap(&p->b, b, K, N, ldb, BK, 2) : makeTileMap(&p->b, b, N, K, ldb, BNH, 2);
+  const bool okC = makeStoreMap(&p->c, c, M, N, ldc);
   if (!okA || !okB || !okC) {
     if (detail)
       snprintf(detail, detailLen, "tensor map of %s refused (pair kernel, M %d N %d K %d)", !okA ? "operand A" : !okB ? "operand B" : "C", M, N, K);
-    return cudaErrorNotSupported;
+    return false;
   }
+  p->M = M; p->N = N; p->K = K; p->aMN = aMN; p->bMN = bMN; p->group = group;
+  p->units = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+  p->splitK = 1;
+  return true;
+}
+
+template <int MODE>
+static cudaError_t launchPair(const PairArgs &args, int pairs, cudaStream_t s) {
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(fcxGemmPairKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fcxGemmPairKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(fcxGemmPairKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  FcxGemmParams p{};
-  p.M = M; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.bn = BN; p.group = group;
-  p.aMN = aMN; p.bMN = bMN; p.bias = bias;
-  const int units = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN), nK = (K + BK - 1) / BK, pairs = smCount2() / 2;
-  p.splitK = fcxGemmPickSplitK(splitK, units, pairs, nK, N);
+  return fcxpdl::launchPdl(fcxGemmPairKernel<MODE>, 2 * pairs, THREADS, SMEM_BYTES, s, args);
+}
+
+extern "C" cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,
+                                       const void *bias, int splitK, int accumulate, void *geluOut, int group, int *errFlag, cudaStream_t s,
+                                       char *detail, size_t detailLen) {
+  PairArgs args{};
+  if (geluOut && (accumulate || ((uintptr_t)geluOut & 15))) return cudaErrorInvalidValue;
+  const bool ok = fillProb(&args.prob[0], a, b, c, M, N, K, lda, ldb, ldc, aMN, bMN, group, detail, detailLen);
+  if (!ok) return cudaErrorNotSupported;
+  if (geluOut) {
+    if (!makeStoreMap(&args.c2, geluOut, M, N, ldc)) return cudaErrorNotSupported;
+    splitK = 1;  // the activation needs the whole sum
+  }
+  PairProb &p = args.prob[0];
+  const int nK = (K + BK - 1) / BK, pairs = smCount2() / 2;
+  p.splitK = fcxGemmPickSplitK(splitK, p.units, pairs, nK, N);
+  p.units *= p.splitK;
   p.accumulate = accumulate;
+  args.bias = bias;
+  args.errFlag = errFlag;
   if (p.splitK > 1 && !accumulate) {
     cudaError_t e = cudaMemsetAsync(c, 0, ((size_t)(M - 1) * ldc + N) * 2, s);
     if (e != cudaSuccess) return e;
   }
-  const int grid = 2 * std::min(units * p.splitK, pairs);
-  cudaError_t e = fcxpdl::launchPdl(geluOut ? fcxGemmPairKernel<true> : fcxGemmPairKernel<false>, grid, THREADS, SMEM_BYTES, s, ma, mb, mc, mc2, p);
+  const cudaError_t e = geluOut ? launchPair<MODE_GELU>(args, std::min(p.units, pairs), s) : launchPair<MODE_PLAIN>(args, std::min(p.units, pairs), s);
   if (e != cudaSuccess && detail)
-    snprintf(detail, detailLen, "pair kernel launch: %s (M %d N %d K %d splitK %d grid %d)", cudaGetErrorString(e), M, N, K, p.splitK, grid);
+    snprintf(detail, detailLen, "pair kernel launch: %s (M %d N %d K %d splitK %d units %d)", cudaGetErrorString(e), M, N, K, p.splitK, p.units);
   return e;
+}
+
+// How two products of units0 / units1 tiles with nK0 / nK1 K blocks each share one launch of `workers` workers: the K pieces
+// of both (never more than either is cut into in a launch of its own), which one goes first (the one with the longer units;
+// swap = the second product) and how many short units make up for a long one.  Every choice is tried; the time of a choice is
+// that of its busiest worker, in K blocks.  Returns 0 when two launches would be done sooner.
+extern "C" int fcxGemmDualPlan(int units0, int nK0, int alone0, int units1, int nK1, int alone1, int workers, int *split0, int *split1, int *swap,
+                               int *extra) {
+  auto pieces = [](int nK, int s) { const int per = (nK + s - 1) / s; return (nK + per - 1) / per; };
+  double best = 0;
+  int bestTime = 0;
+  for (int a = 1; a <= alone0; a++)
+    for (int b = 1; b <= alone1; b++) {
+      if (pieces(nK0, a) != a || pieces(nK1, b) != b) continue;
+      int len[2] = {(nK0 + a - 1) / a, (nK1 + b - 1) / b}, n[2] = {units0 * a, units1 * b};
+      const int sw = len[1] > len[0], P = std::min(workers, n[0] + n[1]);
+      if (sw) { std::swap(len[0], len[1]); std::swap(n[0], n[1]); }
+      const int rem = n[0] % P;
+      for (int ex = rem ? len[0] / len[1] : 0; ex <= (rem ? len[0] / len[1] + 1 : 0); ex++) {
+        const int uniform = std::max(0, n[1] - ex * (P - rem));  // short units that go round all workers
+        // the busiest workers are the first of those with one long unit more and the first of the others
+        auto shorts = [&](int me) { return uniform > me ? (uniform - me + P - 1) / P : 0; };
+        int time = (n[0] / P) * len[0] + (std::min(ex, (n[1] + P - rem - 1) / (P - rem)) + shorts(rem)) * len[1];
+        if (rem) time = std::max(time, (n[0] / P + 1) * len[0] + shorts(0) * len[1]);
+        const double cost = time * (1.0 + 0.02 * (a - 1 + b - 1));  // pieces are added in memory
+        if (best == 0 || cost < best) {
+          best = cost;
+          bestTime = time;
+          *split0 = a; *split1 = b; *swap = sw; *extra = ex;
+        }
+      }
+    }
+  const int apart = (units0 * alone0 + workers - 1) / workers * ((nK0 + alone0 - 1) / alone0) +
+                    (units1 * alone1 + workers - 1) / workers * ((nK1 + alone1 - 1) / alone1);
+  return bestTime <= apart;
+}
+
+// Whether `workers` workers visit every unit of a launch exactly once; the longest worker's time in `longest` (a unit of the
+// first product takes len0, of the second len1).
+extern "C" int fcxGemmUnitsCovered(int workers, int n0, int n1, int extra, int len0, int len1, int *longest) {
+  std::vector<int> seen0(n0, 0), seen1(n1, 0);
+  *longest = 0;
+  for (int w = 0; w < workers; w++) {
+    UnitIter it(w, workers, n0, n1, extra);
+    int prob, unit, time = 0;
+    while (it.next(&prob, &unit)) {
+      if (unit < 0 || unit >= (prob ? n1 : n0)) return 0;
+      (prob ? seen1 : seen0)[unit]++;
+      time += prob ? len1 : len0;
+    }
+    *longest = std::max(*longest, time);
+  }
+  for (int c : seen0)
+    if (c != 1) return 0;
+  for (int c : seen1)
+    if (c != 1) return 0;
+  return 1;
+}
+
+// dx[T,I] = dy[T,O] w[O,I] and dw[O,I] (+)= dy^T x in one launch.  Returns cudaErrorNotSupported when the pair kernel is not
+// the better one for both products: the caller then launches them one by one.
+extern "C" cudaError_t fcxGemmBackwardPair(const void *dy, const void *w, const void *x, void *dx, void *dw, int T, int I, int O, int lddy, int ldw,
+                                           int ldx, int accumulate, int groupX, int groupW, int *errFlag, cudaStream_t s) {
+  if (!fcxGemmPairSuits(T, I, O) || !fcxGemmPairSuits(O, I, T)) return cudaErrorNotSupported;
+  PairArgs args{};
+  PairProb px{}, pw{};
+  if (!fillProb(&px, dy, w, dx, T, I, O, lddy, ldw, I, 0, 1, groupX, nullptr, 0) ||
+      !fillProb(&pw, dy, x, dw, O, I, T, lddy, ldx, I, 1, 1, groupW, nullptr, 0))
+    return cudaErrorNotSupported;
+  const int nKx = (O + BK - 1) / BK, nKw = (T + BK - 1) / BK, pairs = smCount2() / 2;
+  int swap = 0;
+  if (!fcxGemmDualPlan(pw.units, nKw, fcxGemmPickSplitK(0, pw.units, pairs, nKw, I), px.units, nKx, fcxGemmPickSplitK(0, px.units, pairs, nKx, I),
+                       pairs, &pw.splitK, &px.splitK, &swap, &args.extra))
+    return cudaErrorNotSupported;
+  pw.accumulate = accumulate;
+  for (PairProb *p : {&px, &pw}) {
+    p->units *= p->splitK;
+    if (p->splitK > 1 && !p->accumulate) {
+      cudaError_t e = cudaMemsetAsync(p == &px ? dx : dw, 0, (size_t)p->M * p->N * 2, s);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  args.prob[0] = swap ? px : pw;
+  args.prob[1] = swap ? pw : px;
+  args.errFlag = errFlag;
+  return launchPair<MODE_DUAL>(args, std::min(px.units + pw.units, pairs), s);
 }

@@ -12,6 +12,7 @@ namespace fcxt {
 
 FcxDevComm devComm(uint64_t comm);                       // fused_ops.cpp
 size_t heapOffset(uint64_t comm, const at::Tensor &t);   // fused_ops.cpp
+at::Tensor colSum(const at::Tensor &a, const c10::optional<at::Tensor> &into);  // module.cpp
 
 static void checkMat(const at::Tensor &t, const char *name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.stride(1) == 1, name, " must be a 2-D bf16 CUDA tensor with contiguous rows");
@@ -64,6 +65,90 @@ static at::Tensor gemmEx(const at::Tensor &a, const at::Tensor &b, bool aMN, boo
                            (int)c.stride(0), &o, err.data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(e == cudaSuccess, "tcgen05 GEMM failed: ", cudaGetErrorString(e), ": ", fcxGemmLastDetail());
   return c;
+}
+
+// Forward of a linear layer in one call: (y [..., O], x as a contiguous [T, I] matrix, kept for the backward pass).
+static std::tuple<at::Tensor, at::Tensor> linearFwd(const at::Tensor &x, const at::Tensor &w, const c10::optional<at::Tensor> &bias,
+                                                    at::Tensor &err) {
+  const at::Tensor x2 = (x.dim() == 2 ? x : x.reshape({-1, x.size(-1)})).contiguous();
+  at::Tensor y = gemmEx(x2, w, false, false, bias, 0, err, -1, c10::nullopt, false);
+  if (x.dim() != 2) {
+    auto shape = x.sizes().vec();
+    shape.back() = w.size(0);
+    y = y.view(shape);
+  }
+  return {y, x2};
+}
+
+// Its backward in one call: dx = dy w, dw = dy^T x, db = column sums of dy, each as asked (undefined otherwise).  With dw_into
+// / db_into the weight or bias gradient is added to that tensor (the parameter's .grad) and not returned.
+static std::tuple<c10::optional<at::Tensor>, c10::optional<at::Tensor>, c10::optional<at::Tensor>> linearBwd(
+    const at::Tensor &dy, const at::Tensor &x2, const at::Tensor &w, bool needX, bool needW, bool needB, at::Tensor &err,
+    const c10::optional<at::Tensor> &dwInto, const c10::optional<at::Tensor> &dbInto) {
+  const at::Tensor dy2 = (dy.dim() == 2 ? dy : dy.reshape({-1, dy.size(-1)})).contiguous();
+  c10::optional<at::Tensor> dx, dw, db;
+  const bool intoW = dwInto.has_value() && dwInto->defined(), intoB = dbInto.has_value() && dbInto->defined();
+  bool done = false;
+  if (needX && needW) {
+    checkMat(dy2, "dy");
+    checkMat(x2, "x");
+    checkMat(w, "w");
+    const int64_t T = dy2.size(0), O = dy2.size(1), I = w.size(1);
+    TORCH_CHECK(w.size(0) == O && x2.size(0) == T && x2.size(1) == I, "dy, x and w disagree on a dimension");
+    TORCH_CHECK(!intoW || (dwInto->is_cuda() && dwInto->scalar_type() == at::kBFloat16 && dwInto->is_contiguous() && dwInto->dim() == 2 &&
+                           dwInto->size(0) == O && dwInto->size(1) == I),
+                "dw_into must be a contiguous bf16 [O, I] CUDA matrix");
+    c10::cuda::CUDAGuard g(dy2.device());
+    at::Tensor outX = at::empty({T, I}, dy2.options()), outW = intoW ? *dwInto : at::empty({O, I}, dy2.options());
+    auto e = fcxGemmBackwardBf16(dy2.data_ptr(), w.data_ptr(), x2.data_ptr(), outX.data_ptr(), outW.data_ptr(), (int)T, (int)I, (int)O,
+                                 (int)dy2.stride(0), (int)w.stride(0), (int)x2.stride(0), intoW ? 1 : 0, err.data_ptr<int>(),
+                                 at::cuda::getCurrentCUDAStream().stream());
+    done = e == cudaSuccess;
+    TORCH_CHECK(done || e == cudaErrorNotSupported, "tcgen05 GEMM launch failed: ", cudaGetErrorString(e));
+    if (done) {
+      dx = outX;
+      if (!intoW) dw = outW;
+    }
+  }
+  if (!done && needX) dx = gemmEx(dy2, w, false, true, c10::nullopt, 0, err, -1, c10::nullopt, false);
+  if (!done && needW) {
+    at::Tensor r = gemmEx(dy2, x2, true, true, c10::nullopt, 0, err, -1, dwInto, intoW);
+    if (!intoW) dw = r;
+  }
+  if (needB) {
+    at::Tensor r = colSum(dy2, dbInto);
+    if (!intoB) db = r;
+  }
+  return {dx, dw, db};
+}
+
+// The linear layer as an autograd function of its own: forward and backward stay in native code, so that on small layers
+// the interpreter is not what their time goes into.
+class LinearFunction : public torch::autograd::Function<LinearFunction> {
+ public:
+  static at::Tensor forward(torch::autograd::AutogradContext *ctx, const at::Tensor &x, const at::Tensor &w, const c10::optional<at::Tensor> &bias,
+                            at::Tensor err) {
+    auto [y, x2] = linearFwd(x, w, bias, err);
+    ctx->save_for_backward({x2, w});
+    ctx->saved_data["err"] = err;
+    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["bias"] = bias.has_value() && bias->defined();
+    return y;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    at::Tensor err = ctx->saved_data["err"].toTensor();
+    const auto shape = ctx->saved_data["shape"].toIntVector();
+    const bool bias = ctx->saved_data["bias"].toBool();
+    auto [dx, dw, db] = linearBwd(grads[0], saved[0], saved[1], ctx->needs_input_grad(0), ctx->needs_input_grad(1),
+                                  bias && ctx->needs_input_grad(2), err, c10::nullopt, c10::nullopt);
+    if (dx.has_value() && shape.size() != 2) dx = dx->view(shape);
+    return {dx.value_or(at::Tensor()), dw.value_or(at::Tensor()), db.value_or(at::Tensor()), at::Tensor()};
+  }
+};
+
+static at::Tensor linearApply(const at::Tensor &x, const at::Tensor &w, const c10::optional<at::Tensor> &bias, const at::Tensor &err) {
+  return LinearFunction::apply(x, w, bias, err);
 }
 
 // (pre, act) = (a w^T, gelu_tanh(a w^T + bias)) in one kernel: the CTA-pair GEMM writes both from its epilogue.  pre is what
@@ -180,6 +265,10 @@ void bindGemm(py::module &m) {
         "out: write the result there; accumulate: add it to what out holds (a gradient that collects contributions). "
         "bf16 GEMM on tcgen05 with either operand read K-major or MN-major, optional bias row; pair: -1 kernel chosen by shape, "
         "0 one-CTA kernel (128 x 256 tiles), 1 CTA-pair kernel (cta_group::2, 256 x 256 tiles)");
+  m.def("linear", &linearApply, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("err"), "differentiable x w^T + bias on tcgen05");
+  m.def("linear_fwd", &linearFwd, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("err"));
+  m.def("linear_bwd", &linearBwd, py::arg("dy"), py::arg("x2"), py::arg("w"), py::arg("need_x"), py::arg("need_w"), py::arg("need_b"),
+        py::arg("err"), py::arg("dw_into") = py::none(), py::arg("db_into") = py::none());
   m.def("gemm_bias_gelu", &gemmBiasGelu, py::arg("a"), py::arg("w"), py::arg("bias"), py::arg("err"),
         "(a w^T, gelu_tanh(a w^T + bias)) from one CTA-pair GEMM launch");
   m.def("ag_gemm", &agGemm);

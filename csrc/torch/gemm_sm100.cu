@@ -44,6 +44,7 @@
 #include <stdint.h>
 
 #include "gemm_sm100.h"
+#include "gemm_units.h"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
 
@@ -85,22 +86,30 @@ __device__ __forceinline__ void tileCoord(const FcxGemmParams &p, int nM, int t,
   *mb = (g + p.rotate) % nM;  // AG: the local rows first; RS: the rows this rank owns last
 }
 
+// The second of two independent products in one launch (DUAL: the input and weight gradients of a linear layer).
+struct SecondProduct {
+  CUtensorMap a, b;
+  FcxGemmParams p;
+  int extra;
+};
+
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                                                            const __grid_constant__ CUtensorMap tmALocal, const FcxGemmParams p,
-                                                            const FcxDevComm dc) {
+                                                            const __grid_constant__ CUtensorMap tmALocal, const __grid_constant__ FcxGemmParams p0,
+                                                            const FcxDevComm dc, const __grid_constant__ SecondProduct second) {
+  constexpr bool PLAIN = MODE == FCX_GEMM_PLAIN || MODE == FCX_GEMM_DUAL;
   extern __shared__ uint8_t smemRaw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  volatile int *err = p.errFlag;
+  volatile int *err = p0.errFlag;
 
   // ------------------------------------------------------------ communication CTAs (AG mode only)
-  if (MODE == FCX_GEMM_AG && (int)blockIdx.x >= p.gemmCtas) {
+  if (MODE == FCX_GEMM_AG && (int)blockIdx.x >= p0.gemmCtas) {
     // This rank's [rowsPerRank, K] block goes, 128 rows at a time, to every rank's gathered buffer
     // (this rank's own copy included); one flag per destination and 128-row block.
-    const int commCta = blockIdx.x - p.gemmCtas, nComm = gridDim.x - p.gemmCtas;
+    const int commCta = blockIdx.x - p0.gemmCtas, nComm = gridDim.x - p0.gemmCtas;
     const int n = dc.nranks, me = dc.rank;
-    const int blocksPerRank = p.rowsPerRank / BM;
-    const size_t blockBytes = (size_t)BM * p.K * 2;
+    const int blocksPerRank = p0.rowsPerRank / BM;
+    const size_t blockBytes = (size_t)BM * p0.K * 2;
     const int work = blocksPerRank * (n - 1);  // (remote destination, block) pairs; the local block is read where it lies
     for (int w = commCta; w < work; w += nComm) {
       // destinations rotate so that the ranks do not all write to the same GPU at once:
@@ -108,8 +117,8 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
       // order in which its GEMM CTAs consume the remote blocks
       const int k = 1 + w / blocksPerRank, b = w % blocksPerRank;
       const int dst = (me - k + n) % n;
-      const char *src = (const char *)p.aLocal + (size_t)b * blockBytes;
-      char *d = dc.heap[dst] + p.gatherOff + ((size_t)me * blocksPerRank + b) * blockBytes;
+      const char *src = (const char *)p0.aLocal + (size_t)b * blockBytes;
+      char *d = dc.heap[dst] + p0.gatherOff + ((size_t)me * blocksPerRank + b) * blockBytes;
       const uint4 *s4 = (const uint4 *)src;
       uint4 *d4 = (uint4 *)d;
       const size_t nvec = blockBytes / 16;
@@ -121,8 +130,8 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
       for (; i < nvec; i += THREADS) d4[i] = s4[i];
       __syncthreads();
       if (threadIdx.x == 0) {
-        uint64_t *flag = (uint64_t *)(dc.heap[dst] + p.flagOff) + (size_t)me * blocksPerRank + b;
-        fcxdev::stRelease(flag, p.epoch);
+        uint64_t *flag = (uint64_t *)(dc.heap[dst] + p0.flagOff) + (size_t)me * blocksPerRank + b;
+        fcxdev::stRelease(flag, p0.epoch);
       }
     }
     return;
@@ -136,15 +145,28 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
   uint64_t *fullBar = bars, *emptyBar = bars + STAGES, *tmemFull = bars + 2 * STAGES, *tmemEmpty = bars + 2 * STAGES + 2;
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 4);
 
-  if (MODE == FCX_GEMM_PLAIN && p.mPtr) fcxpdl::pdlWait();  // the row count comes from the kernel before
-  const int Mrows = p.mPtr ? min(*p.mPtr, p.M) : p.M;  // the row count may live on the device
-  const int bn = p.bn;  // columns per tile: 256, or 128 when that fills the SMs better
-  const int nN = (p.N + bn - 1) / bn, nM = (Mrows + BM - 1) / BM;
-  const int nK = (p.K + BK - 1) / BK;
-  const int splitK = (MODE == FCX_GEMM_PLAIN && p.splitK > 1) ? p.splitK : 1;
-  const int kPer = (nK + splitK - 1) / splitK;  // K blocks per split
-  const int nTiles = nN * nM * splitK;
-  const int gemmCtas = (MODE == FCX_GEMM_AG) ? p.gemmCtas : gridDim.x;
+  if (MODE == FCX_GEMM_PLAIN && p0.mPtr) fcxpdl::pdlWait();  // the row count comes from the kernel before
+  const int rows0 = p0.mPtr ? min(*p0.mPtr, p0.M) : p0.M;  // the row count may live on the device
+  const int gemmCtas = (MODE == FCX_GEMM_AG) ? p0.gemmCtas : gridDim.x;
+  // Unit of a product (tile, and piece of K when it is cut) -> where it lies.
+  struct Where {
+    int mb, nb, kLo, kHi;
+    bool first;
+  };
+  auto splitOf = [](const FcxGemmParams &p) { return PLAIN && p.splitK > 1 ? p.splitK : 1; };
+  auto locate = [&](const FcxGemmParams &p, int rows, int u) {
+    Where w;
+    const int nM = (rows + BM - 1) / BM, nK = (p.K + BK - 1) / BK, sk = splitOf(p), kPer = (nK + sk - 1) / sk, piece = u % sk;
+    tileCoord(p, nM, u / sk, &w.mb, &w.nb);
+    w.kLo = piece * kPer;
+    w.kHi = min(nK, w.kLo + kPer);
+    w.first = piece == 0;
+    return w;
+  };
+  auto unitsOf = [&](const FcxGemmParams &p, int rows) { return ((rows + BM - 1) / BM) * ((p.N + p.bn - 1) / p.bn) * splitOf(p); };
+  UnitIter it(blockIdx.x, gemmCtas, unitsOf(p0, rows0), MODE == FCX_GEMM_DUAL ? unitsOf(second.p, second.p.M) : 0,
+              MODE == FCX_GEMM_DUAL ? second.extra : 0);
+  int which = 0, unit = 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&emptyBar[s], 1); }
@@ -159,7 +181,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
   __syncthreads();
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
-  if (MODE == FCX_GEMM_PLAIN) {
+  if (PLAIN) {
     fcxpdl::pdlRelease();
     fcxpdl::pdlWait();  // everything above touches only this CTA's own memories
   }
@@ -170,11 +192,12 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < nTiles && ok; t += gemmCtas) {
-        int mb, nb;
-        tileCoord(p, nM, t / splitK, &mb, &nb);
-        const int kLo = (t % splitK) * kPer, kHi = min(nK, kLo + kPer);
-        const CUtensorMap *mapA = &tmA;
+      while (ok && it.next(&which, &unit)) {
+        const FcxGemmParams &p = MODE == FCX_GEMM_DUAL && which ? second.p : p0;
+        const Where w = locate(p, MODE == FCX_GEMM_DUAL ? p.M : rows0, unit);
+        const int bn = p.bn;
+        const int mb = w.mb, nb = w.nb;
+        const CUtensorMap *mapA = MODE == FCX_GEMM_DUAL && which ? &second.a : &tmA, *mapB = MODE == FCX_GEMM_DUAL && which ? &second.b : &tmB;
         int rowA = mb * BM;
         if (MODE == FCX_GEMM_AG) {
           const int blocksPerRank = p.rowsPerRank / BM, owner = mb / blocksPerRank;
@@ -190,20 +213,20 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
             asm volatile("fence.proxy.async;" ::: "memory");  // remote generic-proxy writes -> this CTA's TMA reads
           }
         }
-        for (int kb = kLo; kb < kHi; kb++) {
+        for (int kb = w.kLo; kb < w.kHi; kb++) {
           if (!mbarWait(&emptyBar[stage], phase ^ 1, err)) { ok = false; break; }
           mbarExpectTx(&fullBar[stage], A_BYTES + bn * BK * 2);
           uint8_t *sa = tiles + stage * STAGE_BYTES, *sb = sa + A_BYTES;
-          if (MODE == FCX_GEMM_PLAIN && p.aMN) {
+          if (PLAIN && p.aMN) {
             // stored [K, M]: two blocks of 64 columns (M) x BK lines (K)
             for (int j = 0; j < BM / 64; j++) tmaLoad2d(sa + j * MN_BLOCK_BYTES, mapA, rowA + j * 64, kb * BK, &fullBar[stage]);
           } else {
             tmaLoad2d(sa, mapA, kb * BK, rowA, &fullBar[stage]);
           }
-          if (MODE == FCX_GEMM_PLAIN && p.bMN) {
-            for (int j = 0; j < bn / 64; j++) tmaLoad2d(sb + j * MN_BLOCK_BYTES, &tmB, nb * bn + j * 64, kb * BK, &fullBar[stage]);
+          if (PLAIN && p.bMN) {
+            for (int j = 0; j < bn / 64; j++) tmaLoad2d(sb + j * MN_BLOCK_BYTES, mapB, nb * bn + j * 64, kb * BK, &fullBar[stage]);
           } else {
-            tmaLoad2d(sb, &tmB, kb * BK, nb * bn, &fullBar[stage]);
+            tmaLoad2d(sb, mapB, kb * BK, nb * bn, &fullBar[stage]);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -215,14 +238,16 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
       int stage = 0, buf = 0;
       uint32_t phase = 0, accPhase = 0;
       bool ok = true;
-      const bool aMN = MODE == FCX_GEMM_PLAIN && p.aMN, bMN = MODE == FCX_GEMM_PLAIN && p.bMN;
-      const uint32_t idesc = instrDesc(bn, aMN, bMN);
-      for (int t = blockIdx.x; t < nTiles && ok; t += gemmCtas) {
+      while (ok && it.next(&which, &unit)) {
+        const FcxGemmParams &p = MODE == FCX_GEMM_DUAL && which ? second.p : p0;
+        const Where w = locate(p, MODE == FCX_GEMM_DUAL ? p.M : rows0, unit);
+        const int bn = p.bn;
+        const bool aMN = PLAIN && p.aMN, bMN = PLAIN && p.bMN;
+        const uint32_t idesc = instrDesc(bn, aMN, bMN);
         if (!mbarWait(&tmemEmpty[buf], accPhase ^ 1, err)) break;
         fenceAfter();
-        const uint32_t dTmem = tmemBase + (uint32_t)buf * bn;
-        const int kLo = (t % splitK) * kPer, kHi = min(nK, kLo + kPer);
-        for (int kb = kLo; kb < kHi; kb++) {
+        const uint32_t dTmem = tmemBase + (uint32_t)buf * 256;
+        for (int kb = w.kLo; kb < w.kHi; kb++) {
           if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
           fenceAfter();
           const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
@@ -232,7 +257,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
             // MN-major: 16 K indices = two eight-line groups = 2048 bytes further
             const uint64_t da = aMN ? smemDescMN(sa + k * 2048, MN_BLOCK_BYTES) : smemDesc(sa + k * 32);
             const uint64_t db = bMN ? smemDescMN(sb + k * 2048, MN_BLOCK_BYTES) : smemDesc(sb + k * 32);
-            mmaF16(dTmem, da, db, idesc, (kb > kLo || k > 0) ? 1u : 0u);
+            mmaF16(dTmem, da, db, idesc, (kb > w.kLo || k > 0) ? 1u : 0u);
           }
           mmaCommit(&emptyBar[stage]);  // the stage may be refilled once these MMAs have read it
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -250,10 +275,11 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
     int buf = 0;
     uint32_t accPhase = 0;
     bool live = true;
-    for (int t = blockIdx.x; t < nTiles; t += gemmCtas) {
-      int mb, nb;
-      tileCoord(p, nM, t / splitK, &mb, &nb);
-      const bool firstSplit = (t % splitK) == 0;
+    while (it.next(&which, &unit)) {
+      const FcxGemmParams &p = MODE == FCX_GEMM_DUAL && which ? second.p : p0;
+      const Where w = locate(p, MODE == FCX_GEMM_DUAL ? p.M : rows0, unit);
+      const int bn = p.bn;
+      const int mb = w.mb, nb = w.nb, Mrows = MODE == FCX_GEMM_DUAL ? p.M : rows0, nN = (p.N + bn - 1) / bn;
       if (live) live = __all_sync(0xffffffffu, mbarWait(&tmemFull[buf], accPhase, err));
       if (live) {
         fenceAfter();
@@ -274,7 +300,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
         // turns that into stores where 8 lanes write one full 128-byte line of a row.
         uint4 *stg = (uint4 *)(epiStage + (size_t)q * 32 * 128);
         // the tile's bias values, once per tile and warp, as fp32 in shared memory (columns past N read as 0)
-        const bool addBias = MODE == FCX_GEMM_PLAIN && p.bias != nullptr && firstSplit;
+        const bool addBias = PLAIN && p.bias != nullptr && w.first;
         float *biasW = biasStage + q * 256;
         if (addBias) {
           const __nv_bfloat16 *bias = (const __nv_bfloat16 *)p.bias;
@@ -290,7 +316,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
           uint32_t r[32];
 #pragma unroll
           for (int h = 0; h < 2; h++) {
-            tmemLd32(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * bn + c0 + 32 * h), r);
+            tmemLd32(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256 + c0 + 32 * h), r);
             tmemLdWait();
             if (addBias) {
               // every lane holds one row and the same 32 columns: broadcast reads of the staged bias values
@@ -322,7 +348,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
             uint4 o = stg[rr * 8 + ((lane & 7) ^ (rr & 7))];
             if (row0 + rr < Mrows) {
               __nv_bfloat16 *d = dst0 + (size_t)rr * ldd + col;
-              if (MODE == FCX_GEMM_PLAIN && (splitK > 1 || p.accumulate)) {
+              if (PLAIN && (p.splitK > 1 || p.accumulate)) {
                 // one K piece of several, or a contribution to a gradient that is being accumulated: added into C
                 const uint32_t *w = (const uint32_t *)&o;
                 for (int j = 0; j < 4; j++)
@@ -363,6 +389,8 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
 
   // ------------------------------------------------------------ RS: reduce the tiles this rank owns
   if (MODE == FCX_GEMM_RS) {
+    const FcxGemmParams &p = p0;
+    const int nN = (p.N + BN - 1) / BN;
     const int n = dc.nranks, lBlocks = p.rowsPerRank / BM;
     const int items = lBlocks * nN;
     const uint64_t want = p.epoch * (uint64_t)n;
@@ -412,16 +440,19 @@ bool makeMap(CUtensorMap *m, const void *base, uint64_t rows, uint64_t cols, uin
 
 template <int MODE>
 cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, const FcxGemmParams &p, const FcxDevComm &dc, int grid, cudaStream_t s,
-                   const CUtensorMap *aLocal = nullptr) {
+                   const CUtensorMap *aLocal = nullptr, const SecondProduct *second = nullptr) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(fcxGemmKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return e;
     attr = true;
   }
+  SecondProduct none{};
+  const CUtensorMap &al = aLocal ? *aLocal : a;
+  const SecondProduct &q = second ? *second : none;
   // the kernels that exchange with peers are launched plainly: their first accesses are flags and peers' memory
-  if (MODE == FCX_GEMM_PLAIN) return fcxpdl::launchPdl(fcxGemmKernel<MODE>, grid, THREADS, SMEM_BYTES, s, a, b, aLocal ? *aLocal : a, p, dc);
-  fcxGemmKernel<MODE><<<grid, THREADS, SMEM_BYTES, s>>>(a, b, aLocal ? *aLocal : a, p, dc);
+  if (MODE == FCX_GEMM_PLAIN || MODE == FCX_GEMM_DUAL) return fcxpdl::launchPdl(fcxGemmKernel<MODE>, grid, THREADS, SMEM_BYTES, s, a, b, al, p, dc, q);
+  fcxGemmKernel<MODE><<<grid, THREADS, SMEM_BYTES, s>>>(a, b, al, p, dc, q);
   return cudaGetLastError();
 }
 
@@ -645,4 +676,58 @@ extern "C" cudaError_t fcxGemmRsBf16(const FcxDevComm *dc, const void *a, const 
   p.stageOff = stageOff; p.flagOff = flagOff; p.epoch = epoch;
   int tiles = (M / BM) * ((N + BN - 1) / BN);
   return launch<FCX_GEMM_RS>(ma, mb, p, *dc, std::min(tiles, smCount()), s);
+}
+
+// The input and weight gradients of a linear layer in one launch: dx[T,I] = dy[T,O] w[O,I], dw[O,I] = dy^T x (added to dw
+// with `accumulate`).  Returns cudaErrorNotSupported for sizes that are better off as two launches (one product on CTA
+// pairs and the other not).
+extern "C" cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const void *x, void *dx, void *dw, int T, int I, int O, int lddy, int ldw,
+                                           int ldx, int accumulate, int *errFlag, cudaStream_t s) {
+  if (T % 8 || I % 8 || O % 8 || lddy % 8 || ldw % 8 || ldx % 8 || T <= 0 || I <= 0 || O <= 0) return cudaErrorNotSupported;
+  if (((uintptr_t)dy | (uintptr_t)w | (uintptr_t)x | (uintptr_t)dx | (uintptr_t)dw) & 15) return cudaErrorNotSupported;
+  cudaGetLastError();
+  const bool pairX = fcxGemmPairSuits(T, I, O) != 0, pairW = fcxGemmPairSuits(O, I, T) != 0;
+  if (pairX != pairW) return cudaErrorNotSupported;
+  if (pairX) {
+    const int g = tileGroup((I + 255) / 256) / 2;
+    return fcxGemmBackwardPair(dy, w, x, dx, dw, T, I, O, lddy, ldw, ldx, accumulate, g, g, errFlag, s);
+  }
+  struct Product {
+    CUtensorMap a, b;
+    FcxGemmParams p;
+    int units, nK;
+  };
+  const int sms = smCount();
+  auto fill = [&](Product *q, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int aMN) {
+    const int bn = pickBn(M, N, K, sms);
+    if (!(aMN ? makeMap(&q->a, a, K, M, lda, BK) : makeMap(&q->a, a, M, K, lda, BM)) || !makeMap(&q->b, b, K, N, ldb, BK)) return false;
+    q->p = FcxGemmParams{};
+    q->p.M = M; q->p.N = N; q->p.K = K; q->p.c = c; q->p.ldc = N; q->p.errFlag = errFlag; q->p.bn = bn; q->p.group = tileGroup((N + bn - 1) / bn);
+    q->p.aMN = aMN; q->p.bMN = 1;
+    q->units = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
+    q->nK = (K + BK - 1) / BK;
+    return true;
+  };
+  Product px, pw;
+  if (!fill(&px, dy, w, dx, T, I, O, lddy, ldw, 0) || !fill(&pw, dy, x, dw, O, I, T, lddy, ldx, 1)) return cudaErrorNotSupported;
+  int swap = 0;
+  SecondProduct second{};
+  if (!fcxGemmDualPlan(pw.units, pw.nK, fcxGemmPickSplitK(0, pw.units, sms, pw.nK, I), px.units, px.nK,
+                       fcxGemmPickSplitK(0, px.units, sms, px.nK, I), sms, &pw.p.splitK, &px.p.splitK, &swap, &second.extra))
+    return cudaErrorNotSupported;
+  pw.p.accumulate = accumulate;
+  int total = 0;
+  for (Product *q : {&px, &pw}) {
+    total += q->units * q->p.splitK;
+    if (q->p.splitK > 1 && !q->p.accumulate) {
+      cudaError_t e = cudaMemsetAsync(q->p.c, 0, (size_t)q->p.M * q->p.N * 2, s);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  const Product &first = swap ? px : pw, &other = swap ? pw : px;
+  second.a = other.a;
+  second.b = other.b;
+  second.p = other.p;
+  FcxDevComm dc{};
+  return launch<FCX_GEMM_DUAL>(first.a, first.b, first.p, dc, std::min(total, sms), s, nullptr, &second);
 }

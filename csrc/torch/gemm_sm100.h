@@ -7,6 +7,7 @@
 #define FCX_GEMM_PLAIN 0
 #define FCX_GEMM_AG 1
 #define FCX_GEMM_RS 2
+#define FCX_GEMM_DUAL 3  // two plain products in one launch
 
 struct FcxGemmParams {
   int M, N, K;          // C[M,N] = A[M,K] * B[N,K]^T, bf16 in, fp32 accumulate, bf16 out
@@ -57,6 +58,11 @@ typedef struct FcxGemmOpts {
 } FcxGemmOpts;
 cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, const FcxGemmOpts *o,
                             int *errFlag, cudaStream_t s);
+cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const void *x, void *dx, void *dw, int T, int I, int O, int lddy, int ldw, int ldx,
+                                int accumulate, int *errFlag, cudaStream_t s);
+cudaError_t fcxGemmBackwardPair(const void *dy, const void *w, const void *x, void *dx, void *dw, int T, int I, int O, int lddy, int ldw, int ldx,
+                                int accumulate, int groupX, int groupW, int *errFlag, cudaStream_t s);
+int fcxGemmDualPlan(int units0, int nK0, int alone0, int units1, int nK1, int alone1, int workers, int *split0, int *split1, int *swap, int *extra);
 int fcxGemmPickSplitK(int requested, int units, int slots, int nK, int N);
 double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut);
 double fcxGemmPairCost(int M, int N, int K, int pairs);

@@ -31,6 +31,12 @@ def _direct(param):
     return g
 
 
+def _direct_weight(param):
+    """The same for a weight matrix: pieces of its gradient are added two columns at a time."""
+    g = _direct(param)
+    return g if g is not None and g.shape[1] % 2 == 0 else None
+
+
 def _done(param):
     cb = getattr(param, "_fcx_grad_ready", None)
     if cb is not None:
@@ -148,48 +154,32 @@ def gemm(a, b, a_mn: bool = False, b_mn: bool = False, bias=None, split_k: int =
 
 
 class _Linear(torch.autograd.Function):
-    """y = x w^T (+ bias) with all three GEMMs (forward, input gradient, weight gradient) on the library's own
+    """For parameters whose gradients are added in place; the others take the same path in native code.  y = x w^T (+ bias) with all three GEMMs (forward, input gradient, weight gradient) on the library's own
     tcgen05 kernel: the backward operands are read transposed in place, the weight gradient splits its long
     reduction over the tokens across CTAs, the bias gradient is the library's column-sum kernel."""
 
     @staticmethod
     def forward(ctx, x, w, bias):
-        x2 = x.reshape(-1, x.shape[-1])
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
+        y, x2 = _n().linear_fwd(x, w, bias, _err_flag(x.device))
         ctx.save_for_backward(x2, w)
-        ctx.has_bias = bias is not None
         ctx.in_shape = x.shape
         ctx.params = (w, bias)
-        y = gemm(x2, w, False, False, bias)
-        return y.view(*x.shape[:-1], w.shape[0])
+        return y
 
     @staticmethod
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        dx = dw = db = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, w, False, True).view(ctx.in_shape)      # [T,O] x [O,I]: w read as the [K=O, N=I] operand
         pw, pb = ctx.params
-        if ctx.needs_input_grad[1]:
-            gw = _direct(pw)
-            if gw is not None and gw.shape[1] % 2 == 0:
-                # [O,T] x [T,I]: both read transposed, K = tokens; added into the parameter's gradient in place
-                _n().gemm(dy2, x2, True, True, None, 0, _err_flag(dy2.device), -1, gw, True)
-                _done(pw)
-            else:
-                dw = gemm(dy2, x2, True, True)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            gb = _direct(pb)
-            if gb is not None:
-                _n().col_sum(dy2, gb)
-                _done(pb)
-            else:
-                db = _n().col_sum(dy2)
-        return dx, dw, db
+        need_x, need_w, need_b = ctx.needs_input_grad
+        need_b = need_b and pb is not None
+        gw, gb = _direct_weight(pw) if need_w else None, _direct(pb) if need_b else None
+        # all gradients in one call; the input and weight gradients share a launch where their sizes suit each other
+        dx, dw, db = _n().linear_bwd(dy, x2, w, need_x, need_w, need_b, _err_flag(dy.device), gw, gb)
+        if gw is not None:
+            _done(pw)
+        if gb is not None:
+            _done(pb)
+        return (dx.view(ctx.in_shape) if need_x and len(ctx.in_shape) != 2 else dx), dw, db
 
 
 class _LinearBiasGelu(torch.autograd.Function):
@@ -222,17 +212,12 @@ class _LinearBiasGelu(torch.autograd.Function):
             _done(pb)
         else:
             dpre, db = _n().bias_gelu_bwd(dy2, pre, bias)
-        dx = dw = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dpre, w, False, True).view(ctx.in_shape)
-        if ctx.needs_input_grad[1]:
-            gw = _direct(pw)
-            if gw is not None and gw.shape[1] % 2 == 0:
-                _n().gemm(dpre, x2, True, True, None, 0, _err_flag(dpre.device), -1, gw, True)
-                _done(pw)
-            else:
-                dw = gemm(dpre, x2, True, True)
-        return dx, dw, db
+        need_x, need_w = ctx.needs_input_grad[:2]
+        gw = _direct_weight(pw) if need_w else None
+        dx, dw, _ = _n().linear_bwd(dpre, x2, w, need_x, need_w, False, _err_flag(dpre.device), gw)
+        if gw is not None:
+            _done(pw)
+        return (dx.view(ctx.in_shape) if need_x else None), dw, db
 
 
 def linear_bias_gelu(x, w, bias):
@@ -244,4 +229,6 @@ def linear_bias_gelu(x, w, bias):
 def linear(x, w, bias=None):
     """``torch.nn.functional.linear`` for bf16 CUDA tensors on the library's tcgen05 GEMM (forward and backward).
     Shapes the kernel cannot take (inner sizes that are not multiples of 8) raise; there is no silent fallback."""
-    return _Linear.apply(x, w, bias)
+    if getattr(w, "_fcx_direct_grad", False) or getattr(bias, "_fcx_direct_grad", False):
+        return _Linear.apply(x, w, bias)  # gradients that are added in place (enable_direct_grad)
+    return _n().linear(x, w, bias, _err_flag(x.device))

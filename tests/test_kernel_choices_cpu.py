@@ -1,0 +1,73 @@
+"""Host-side rules that pick a kernel or a tile, checked without a GPU: every rule gives a legal answer over its whole
+range, and picks the variant that each side of its line was measured for."""
+import ctypes
+
+import pytest
+
+
+@pytest.fixture(scope="module")
+def ext():
+    import flagcx_b200
+    lib = ctypes.CDLL(flagcx_b200.native().__file__)
+    lib.fcxGemmTileCost.restype = ctypes.c_double
+    lib.fcxGemmTileCost.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)]
+    lib.fcxGemmPairCost.restype = ctypes.c_double
+    lib.fcxGemmFp8Tile.restype = ctypes.c_int
+    lib.fcxMoeTileColumns.restype = ctypes.c_int
+    lib.fcxGemmDualPlan.restype = lib.fcxGemmUnitsCovered.restype = ctypes.c_int
+    return lib
+
+
+def _width(ext, m, n, k):
+    bn = ctypes.c_int(0)
+    cost = ext.fcxGemmTileCost(m, n, k, 148, ctypes.byref(bn))
+    assert cost > 0
+    return bn.value
+
+
+def test_gemm_tile_width(ext):
+    for m in (1, 64, 128, 129, 1000, 8192):
+        for n in (8, 64, 72, 256, 1000, 4096):
+            for k in (8, 64, 1000, 8192):
+                assert _width(ext, m, n, k) in (64, 128, 256)
+    assert _width(ext, 8192, 4096, 4096) == 256  # enough tiles for every SM
+    assert _width(ext, 64, 3072, 1024) == 64     # 12 tiles of 256 columns: 12 of 148 SMs
+
+
+def test_fp8_tile(ext):
+    for m in (1, 128, 129, 333, 8192):
+        for n in (8, 64, 136, 1792, 4096):
+            assert ext.fcxGemmFp8Tile(m, n, 148) in (0, 64, 128)
+    assert ext.fcxGemmFp8Tile(8192, 4096, 148) == 0
+    assert ext.fcxGemmFp8Tile(333, 1792, 148) == 64
+
+
+def test_moe_tile(ext):
+    for blocks in (0, 1, 5, 74, 500):
+        for cols in (8, 128, 1024, 28672):
+            assert ext.fcxMoeTileColumns(blocks, cols, 74) in (128, 256)
+    assert ext.fcxMoeTileColumns(68, 28672, 74) == 256
+    assert ext.fcxMoeTileColumns(6, 1024, 74) == 128  # 24 wide tiles on 74 pairs
+
+
+def test_two_products_in_one_launch_cover_every_unit_once(ext):
+    longest, s0, s1, swap, extra = (ctypes.c_int(0) for _ in range(5))
+    for n in (1, 2, 73, 74, 148):
+        for n0 in (1, 5, 48, 74, 75, 200):
+            for n1 in (0, 1, 16, 74, 128, 500):
+                for ex in (0, 1, 3, 8, 200):
+                    workers = min(n, n0 + n1)
+                    assert ext.fcxGemmUnitsCovered(workers, n0, n1, ex, 1, 1, ctypes.byref(longest)) == 1, (n, n0, n1, ex)
+    # GPT-2-medium's backward GEMMs at 8192 tokens, (I, O): the launch ends within a short unit or so of a perfect split
+    for i, o in ((1024, 3072), (1024, 1024), (1024, 4096), (4096, 1024)):
+        uw, ux, kw, kx = (o // 256) * (i // 256), 32 * (i // 256), 128, o // 64
+        alone = [ext.fcxGemmPickSplitK(0, u, 74, k, i) for u, k in ((uw, kw), (ux, kx))]
+        ext.fcxGemmDualPlan(uw, kw, alone[0], ux, kx, alone[1], 74, *(ctypes.byref(v) for v in (s0, s1, swap, extra)))
+        assert 1 <= s0.value <= alone[0] and 1 <= s1.value <= alone[1]
+        units, lens = [uw * s0.value, ux * s1.value], [-(-kw // s0.value), -(-kx // s1.value)]
+        if swap.value:
+            units, lens = units[::-1], lens[::-1]
+        assert ext.fcxGemmUnitsCovered(74, units[0], units[1], extra.value, lens[0], lens[1], ctypes.byref(longest)) == 1
+        share = (uw * kw + ux * kx) / 74
+        print(i, o, s0.value, s1.value, units, lens, extra.value, longest.value, share)
+        assert longest.value <= share + 1.5 * lens[1], (i, o, longest.value, share)
