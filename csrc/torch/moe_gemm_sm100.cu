@@ -10,8 +10,9 @@
 // A tile is 256 rows (128 per CTA of the pair) x 256 accumulator columns.  UP: the leader CTA loads 128 gate rows of
 // the weight and its peer the matching 128 up rows, so both operands of the product lie in the same TMEM lanes, 128
 // columns apart, and an epilogue thread needs nobody else's values; the [rows, 2F] intermediate never reaches memory
-// (at 16384 rows and F = 14336 that is 0.94 GB written and read again).  With few tiles (fcxMoeNarrowTiles) the tile
-// is 256 x 128: twice the tiles, so that a small layer's chain of K steps is spread over more SMs.
+// (at 16384 rows and F = 14336 that is 0.94 GB written and read again).  Where the tiles are few, a tile is 256 x 128
+// columns instead, so that the chain of K steps of a small layer is spread over more SMs; which of the two takes fewer
+// waves times the time of a K step (moeTileColumns) depends on the row counts and is decided by every CTA for itself.
 //
 // Pipeline, barriers and bounded waits are those of the pair kernel in gemm2_sm100.cu.
 #include "../kernels/prims.cuh"
@@ -35,8 +36,9 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int EPI_WARPS = 8, STG_BYTES = 32 * 128;  // staging per epilogue warp: 32 rows x 128 bytes
 constexpr int THREADS = 384;
 
-constexpr int stageBytes(int bn) { return A_BYTES + bn / 2 * BK * 2; }
-constexpr int smemBytes(int bn) { return STAGES * stageBytes(bn) + EPI_WARPS * STG_BYTES + 1024 + 512; }
+constexpr int BN_MAX = 256, BOX = 64;  // accumulator columns of the wide tile; weight rows per TMA box
+constexpr int BOX_BYTES = BOX * BK * 2, STAGE_BYTES = A_BYTES + BN_MAX / 2 * BK * 2;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STG_BYTES + 1024 + 512;
 
 struct WeightMaps {
   CUtensorMap m[FCX_MOE_MAX_EXPERTS];
@@ -53,15 +55,22 @@ struct GroupParams {
   int topk;
 };
 
-template <bool UP, int BN>
+// 256 or 128 accumulator columns per tile for `rowBlocks` 256-row blocks and `cols` columns.  A K block of the narrow tile
+// takes a little over half of the wide one's time: at 512 tokens, H 1024, F 2048 and 4 experts the gate / up product took
+// 23 us in three waves of narrow tiles and about 36 us in two waves of wide ones.
+__host__ __device__ inline int moeTileColumns(long long rowBlocks, int cols, int pairs) {
+  const long long wide = (rowBlocks * ((cols + 255) / 256) + pairs - 1) / pairs, narrow = (rowBlocks * ((cols + 127) / 128) + pairs - 1) / pairs;
+  return narrow * 10 < wide * 18 ? 128 : 256;
+}
+
+template <bool UP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     moeGroupKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmH, const __grid_constant__ WeightMaps wm,
                    const GroupParams p, const FcxDevComm dc) {
-  constexpr int BNH = BN / 2, STAGE_BYTES = stageBytes(BN);
-  constexpr int COLS = UP ? BNH : BN;  // result columns per tile
   extern __shared__ uint8_t smemRaw[];
   __shared__ int tileStart[FCX_MOE_MAX_EXPERTS + 1];
   __shared__ int rowsOf[FCX_MOE_MAX_EXPERTS];
+  __shared__ int tileCols;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int *err = p.errFlag;
   const uint32_t cr = ctaRankInCluster();
@@ -73,7 +82,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   uint64_t *fullBar = bars, *emptyBar = bars + STAGES, *accFull = bars + 2 * STAGES, *accEmpty = bars + 2 * STAGES + 2;
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 4);
 
-  const int nN = (p.N + COLS - 1) / COLS, nK = (p.K + BK - 1) / BK;
+  const int nK = (p.K + BK - 1) / BK;
   fcxpdl::pdlRelease();
   if (threadIdx.x < 64) fcxpdl::pdlWait();  // the row counts come from the kernel before
   if ((int)threadIdx.x < p.L) rowsOf[threadIdx.x] = max(0, min(p.rows[threadIdx.x], p.capL));
@@ -83,17 +92,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(tmemBaseSlot)), "r"(2 * BN) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(tmemBaseSlot)), "r"(2 * BN_MAX) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int sum = 0;
+    int blocks = 0, sum = 0;
+    for (int e = 0; e < p.L; e++) blocks += (rowsOf[e] + 2 * BM - 1) / (2 * BM);
+    const int bnHere = moeTileColumns(blocks, UP ? 2 * p.N : p.N, nPairs), cols = UP ? bnHere / 2 : bnHere;
     for (int e = 0; e < p.L; e++) {
       tileStart[e] = sum;
-      sum += (rowsOf[e] + 2 * BM - 1) / (2 * BM) * nN;
+      sum += (rowsOf[e] + 2 * BM - 1) / (2 * BM) * ((p.N + cols - 1) / cols);
     }
     tileStart[p.L] = sum;
+    tileCols = bnHere;
   }
   fenceBefore();
   __syncthreads();
@@ -102,6 +114,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   const uint32_t tmemBase = *tmemBaseSlot;
   fcxpdl::pdlWait();
   const int nTiles = tileStart[p.L];
+  const int bn = tileCols, bnh = bn / 2, COLS = UP ? bnh : bn;  // COLS: result columns per tile
+  const int nN = (p.N + COLS - 1) / COLS;
 
   // Tile t -> (expert, 256-row block of its segment, column block).  `e` only moves forward: a role's tiles ascend.
   // Inside an expert, bands of `group` row blocks with the row block fastest, as in the plain kernels.
@@ -124,14 +138,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         int mb, nb;
         coord(t, e, &mb, &nb);
         const int rowA = e * p.capL + mb * 2 * BM + (int)cr * BM;
-        const int rowB = UP ? (int)cr * p.N + nb * BNH : nb * BN + (int)cr * BNH;
+        const int rowB = UP ? (int)cr * p.N + nb * bnh : nb * bn + (int)cr * bnh;
         for (int kb = 0; kb < nK; kb++) {
           if (!mbarWait(&emptyBar[stage], phase ^ 1, err)) { ok = false; break; }
-          if (cr == 0) mbarExpectTx(&fullBar[stage], 2 * STAGE_BYTES);
+          if (cr == 0) mbarExpectTx(&fullBar[stage], 2 * (A_BYTES + bnh * BK * 2));
           const uint32_t bar = mapToCta(smemAddr(&fullBar[stage]), 0);
           uint8_t *sa = tiles + stage * STAGE_BYTES, *sb = sa + A_BYTES;
           tmaLoad2dPair(sa, &tmA, kb * BK, rowA, bar);
-          tmaLoad2dPair(sb, &wm.m[e], kb * BK, rowB, bar);
+          for (int j = 0; j < bnh / BOX; j++) tmaLoad2dPair(sb + j * BOX_BYTES, &wm.m[e], kb * BK, rowB + j * BOX, bar);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -142,12 +156,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       int stage = 0, buf = 0;
       uint32_t phase = 0, accPhase = 0;
       bool ok = true;
-      // D fp32, A and B bf16, both K-major, M = 256 over the pair, N = BN
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+      // D fp32, A and B bf16, both K-major, M = 256 over the pair, N = bn
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
       for (int t = pair; t < nTiles && ok; t += nPairs) {
         if (!mbarWait(&accEmpty[buf], accPhase ^ 1, err)) break;
         fenceAfter();
-        const uint32_t dTmem = tmemBase + (uint32_t)buf * BN;
+        const uint32_t dTmem = tmemBase + (uint32_t)buf * BN_MAX;
         for (int kb = 0; kb < nK; kb++) {
           if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
           fenceAfter();
@@ -167,7 +181,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     // ---- epilogue (both CTAs, 8 warps): warp w owns TMEM lanes [32*(w%4), +32) and the left (warps 4-7) or right
     // (warps 8-11) half of the result columns.  A wait that gives up turns the warp dead: it walks on but touches nothing.
     const int ew = warp - 4, q = ew & 3, half = ew >> 2;
-    constexpr int HALF_COLS = COLS / 2;
+    const int HALF_COLS = COLS / 2;
     int buf = 0, e = 0;
     uint32_t accPhase = 0, chunkNo = 0;
     bool live = true;
@@ -180,7 +194,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         fenceAfter();
         const int lrow0 = mb * 2 * BM + (int)cr * BM + q * 32, rows = rowsOf[e];  // row inside the expert's segment
         const int col0 = nb * COLS + half * HALF_COLS;
-        const uint32_t lanes = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * HALF_COLS);
+        const uint32_t lanes = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN_MAX + half * HALF_COLS);
         if (UP) {
           // 32 gate and 32 up columns at a time -> 32 result columns; the TMA unit stores the 32 x 32 block (64-byte
           // swizzle) and clips columns past F.  Rows past the count land in the padding of the expert's own segment
@@ -190,7 +204,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             if (col0 + c0 >= p.N || lrow0 >= rows) break;
             uint32_t g[32], u[32];
             tmemLd32(lanes + c0, g);
-            tmemLd32(lanes + BNH + c0, u);
+            tmemLd32(lanes + bnh + c0, u);
             // two staging blocks of 2 KB: the one about to be refilled must have been read out by the TMA unit
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
             __syncwarp();
@@ -271,7 +285,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   __syncthreads();
   clusterSync();
   fenceAfter();
-  if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(2 * BN) : "memory");
+  if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(2 * BN_MAX) : "memory");
   if (!UP) {
     // every row this CTA produced has been stored (possibly on peers): tell every rank that this CTA is done
     __threadfence_system();
@@ -294,39 +308,36 @@ int pairCount() {
   return n;
 }
 
-template <bool UP, int BN>
+template <bool UP>
 cudaError_t launchGroup(const CUtensorMap &a, const CUtensorMap &h, const WeightMaps &wm, const GroupParams &p, const FcxDevComm &dc,
                         cudaStream_t s) {
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(moeGroupKernel<UP, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(BN));
+    cudaError_t e = cudaFuncSetAttribute(moeGroupKernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  return fcxpdl::launchPdl(moeGroupKernel<UP, BN>, 2 * pairCount(), THREADS, smemBytes(BN), s, a, h, wm, p, dc);
+  return fcxpdl::launchPdl(moeGroupKernel<UP>, 2 * pairCount(), THREADS, SMEM_BYTES, s, a, h, wm, p, dc);
 }
 
 }  // namespace
 
-extern "C" int fcxMoeNarrowTiles(int L, int capL, int cols, int pairs) {
-  return (long long)L * ((capL + 255) / 256) * ((cols + 255) / 256) < 2ll * pairs;
-}
+extern "C" int fcxMoeTileColumns(int rowBlocks, int cols, int pairs) { return moeTileColumns(rowBlocks, cols, pairs); }
 
 extern "C" cudaError_t fcxMoeUpGrouped(const void *x, const void *const *w, void *h, const int *rows, int L, int capL, int H, int F,
                                        const int *ldw, int *errFlag, cudaStream_t s) {
   if (L < 1 || L > FCX_MOE_MAX_EXPERTS || capL <= 0 || capL % 128 || H % 8 || F % 8 || H <= 0 || F <= 0) return cudaErrorInvalidValue;
   if (((uintptr_t)x | (uintptr_t)h) & 15) return cudaErrorInvalidValue;
-  const bool narrow = fcxMoeNarrowTiles(L, capL, 2 * F, pairCount());
   CUtensorMap ma, mh;
   WeightMaps wm{};
   if (!makeTileMap(&ma, x, (uint64_t)L * capL, H, H, BM, 2) || !makeStoreMap(&mh, h, (uint64_t)L * capL, F, F)) return cudaErrorNotSupported;
   for (int e = 0; e < L; e++)
-    if (ldw[e] % 8 || ((uintptr_t)w[e] & 15) || !makeTileMap(&wm.m[e], w[e], 2 * (uint64_t)F, H, ldw[e], narrow ? 64 : 128, 2))
+    if (ldw[e] % 8 || ((uintptr_t)w[e] & 15) || !makeTileMap(&wm.m[e], w[e], 2 * (uint64_t)F, H, ldw[e], BOX, 2))
       return cudaErrorInvalidValue;
   GroupParams p{};
   p.L = L; p.capL = capL; p.N = F; p.K = H; p.rows = rows; p.group = 8; p.errFlag = errFlag;
   FcxDevComm dc{};
-  return narrow ? launchGroup<true, 128>(ma, mh, wm, p, dc, s) : launchGroup<true, 256>(ma, mh, wm, p, dc, s);
+  return launchGroup<true>(ma, mh, wm, p, dc, s);
 }
 
 extern "C" cudaError_t fcxMoeDownGrouped(const FcxDevComm *dc, const void *h, const void *const *w, const int *rows, int L, int capL, int H,
@@ -334,15 +345,14 @@ extern "C" cudaError_t fcxMoeDownGrouped(const FcxDevComm *dc, const void *h, co
                                          int *errFlag, int *gridOut, cudaStream_t s) {
   if (L < 1 || L > FCX_MOE_MAX_EXPERTS || capL <= 0 || capL % 128 || H % 8 || F % 8 || H <= 0 || F <= 0) return cudaErrorInvalidValue;
   if ((uintptr_t)h & 15) return cudaErrorInvalidValue;
-  const bool narrow = fcxMoeNarrowTiles(L, capL, H, pairCount());
   CUtensorMap ma;
   WeightMaps wm{};
   if (!makeTileMap(&ma, h, (uint64_t)L * capL, F, F, BM, 2)) return cudaErrorNotSupported;
   for (int e = 0; e < L; e++)
-    if (ldw[e] % 8 || ((uintptr_t)w[e] & 15) || !makeTileMap(&wm.m[e], w[e], H, F, ldw[e], narrow ? 64 : 128, 2)) return cudaErrorInvalidValue;
+    if (ldw[e] % 8 || ((uintptr_t)w[e] & 15) || !makeTileMap(&wm.m[e], w[e], H, F, ldw[e], BOX, 2)) return cudaErrorInvalidValue;
   GroupParams p{};
   p.L = L; p.capL = capL; p.N = H; p.K = F; p.rows = rows; p.group = 8; p.errFlag = errFlag;
   p.rowInfo = (const int4 *)rowInfo; p.combineOff = combineOff; p.doneOff = doneOff; p.topk = topk;
   if (gridOut) *gridOut = 2 * pairCount();  // the receivers count one arrival per CTA of every rank
-  return narrow ? launchGroup<false, 128>(ma, ma, wm, p, *dc, s) : launchGroup<false, 256>(ma, ma, wm, p, *dc, s);
+  return launchGroup<false>(ma, ma, wm, p, *dc, s);
 }
