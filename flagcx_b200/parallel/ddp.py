@@ -303,9 +303,10 @@ class DataParallelTrainer:
 
     def kernels_per_step(self) -> int:
         """Launches of this framework's own kernels in one step: per layer 2
-        fused LayerNorm forward, 2 x 2 backward (dx; parameter gradients with
-        their reduction), bias-GELU forward + 2 backward (dx; bias gradient);
-        the tcgen05 GEMMs of the projections and the LM head; the final
+        fused LayerNorm forward, 2 x 2 backward (dx; parameter gradients),
+        bias-GELU forward + 2 backward (dx; bias gradient); the tcgen05 GEMMs
+        of the projections and the LM head (input and weight gradients in one
+        launch, so this is a lower bound where they take two); the final
         LayerNorm (1 + 2), the loss kernel, and per bucket one all-reduce
         kernel (more than one rank) and one AdamW kernel (one AdamW kernel in
         all when the optimizer is not overlapped)."""
@@ -314,9 +315,9 @@ class DataParallelTrainer:
         if os.environ.get("FLAGCX_MODEL_GEMM", "own") != "library" and os.environ.get("FLAGCX_MODEL_FUSED_GELU", "1") != "0":
             own -= L  # the GELU of the forward pass runs in the epilogue of the up-projection GEMM
         if os.environ.get("FLAGCX_MODEL_GEMM", "own") != "library":
-            # tcgen05 GEMMs: four projections per layer and the LM head, each forward + input gradient + weight
-            # gradient; the three biased projections' bias gradients take one column-sum kernel each
-            own += L * (4 * 3 + 3) + 3
+            # tcgen05 GEMMs: four projections per layer and the LM head, each forward + both gradients; the three biased
+            # projections' bias gradients take one column-sum kernel each
+            own += L * (4 * 2 + 3) + 2
         nb = len(self.buckets)
         adamw = nb if self.overlap_optimizer else (2 if self.world > 1 and self.split_tail else 1)
         return own + (nb if self.world > 1 else 0) + adamw
