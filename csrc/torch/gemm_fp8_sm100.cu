@@ -19,6 +19,10 @@
 //   gemmFp8Kernel<BN>  128 x BN tiles on single CTAs (BN 128 or 64), four accumulators: for outputs with too few tiles.
 // Roles: warps 0-7 promotion + epilogue (warp w reads TMEM lanes 32*(w%4).., one output row per thread, and half of the
 // tile's columns), warp 8 TMA producer (128-byte swizzle, no multicast), warp 9 MMA issuer and TMEM allocation.
+// The single-CTA kernel commits ONCE per slice, on the barrier of the slice's stage: the producer and the epilogue both wait
+// for it (8192 x 4096 x 4096 in 128-column tiles 227 -> 212 us, 333 x 1792 x 4096 18.1 -> 17.4).  It has at least as many stages
+// as accumulators, so that neither can miss a phase: the stage is not refilled before the producer has seen it done, nor its
+// successor multiplied before the epilogue has freed the accumulator.  On CTA pairs one commit was no faster (177 -> 184 us).
 // Every wait is bounded; a wait that gives up sets the error flag and the kernel drains and returns.
 #include <algorithm>
 #include <cstdlib>
@@ -129,14 +133,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
   uint8_t *tiles = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
   uint8_t *epiStage = tiles + STAGES * STAGE_BYTES;
   uint64_t *bars = (uint64_t *)(epiStage + EPI_BYTES);
-  uint64_t *fullBar = bars, *emptyBar = bars + STAGES, *tmemFull = bars + 2 * STAGES, *tmemEmpty = bars + 2 * STAGES + ACC_BUFS;
-  uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 2 * ACC_BUFS);
+  uint64_t *fullBar = bars, *doneBar = bars + STAGES, *tmemEmpty = bars + 2 * STAGES;
+  uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + ACC_BUFS);
 
   const int nN = (p.N + BN - 1) / BN, nM = (p.M + BM - 1) / BM, nTiles = nN * nM, nK = p.K / BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&emptyBar[s], 1); }
-    for (int b = 0; b < ACC_BUFS; b++) { mbarInit(&tmemFull[b], 1); mbarInit(&tmemEmpty[b], EPI_WARPS); }
+    for (int s = 0; s < STAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&doneBar[s], 1); }
+    for (int b = 0; b < ACC_BUFS; b++) mbarInit(&tmemEmpty[b], EPI_WARPS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 9) {
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
         int mb, nb;
         tileCoord(p, nM, nN, t, &mb, &nb);
         for (int kb = 0; kb < nK; kb++) {
-          if (!mbarWait(&emptyBar[stage], phase ^ 1, err)) { ok = false; break; }
+          if (!mbarWait(&doneBar[stage], phase ^ 1, err)) { ok = false; break; }
           mbarExpectTx(&fullBar[stage], STAGE_BYTES);
           uint8_t *sa = tiles + stage * STAGE_BYTES, *sb = sa + A_BYTES;
           tmaLoad2d(sa, &tmA, kb * BK, mb * BM, &fullBar[stage]);
@@ -184,8 +188,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
 #pragma unroll
           for (int k = 0; k < BK / 32; k++)  // 32 fp8 = 32 bytes further along K inside the 128-byte swizzle row
             mmaF8(dTmem, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, k > 0 ? 1u : 0u);
-          mmaCommit(&emptyBar[stage]);
-          mmaCommit(&tmemFull[buf]);
+          mmaCommit(&doneBar[stage]);  // the stage may be refilled and the accumulator read
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
           if (++buf == ACC_BUFS) { buf = 0; accPhase ^= 1; }
         }
@@ -194,8 +197,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
   } else {
     const int q = warp & 3, half = warp >> 2;  // TMEM lane quarter (fixed by warp index % 4) and column half
     constexpr int GROUP = 8;
-    int buf = 0;
-    uint32_t accPhase = 0, blockNo = 0;
+    int buf = 0, stage = 0;
+    uint32_t phase = 0, blockNo = 0;
     bool live = true;
     uint8_t *stg = epiStage + (size_t)warp * 2 * STG_BYTES;
     for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
 #pragma unroll
         for (int j = 0; j < GROUP; j++) {
           if (kb0 + j < nK) {
-            if (live) live = __all_sync(0xffffffffu, mbarWait(&tmemFull[buf], accPhase, err));
+            if (live) live = __all_sync(0xffffffffu, mbarWait(&doneBar[stage], phase, err));
             if (live) {
               fenceAfter();
               uint32_t r[COLS];
@@ -227,7 +230,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
 #pragma unroll
               for (int i = 0; i < COLS; i++) acc[i] = fmaf(sc.cur[j], __uint_as_float(r[i]), acc[i]);
             }
-            if (++buf == ACC_BUFS) { buf = 0; accPhase ^= 1; }
+            if (++buf == ACC_BUFS) buf = 0;
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
           }
         }
         sc.turn();
@@ -416,19 +420,37 @@ template <int VEC, int UNROLL>
 __global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *__restrict__ x, __nv_fp8_storage_t *__restrict__ q,
                                                       float *__restrict__ sa, int M, int K, int ldx) {
   constexpr int LANES = 128 / VEC, PER_CTA = 256 / LANES;  // lanes per block, blocks per CTA and step
-  const int nKb = K / 128;
-  const size_t total = (size_t)M * nKb;
+  const uint32_t nKb = K / 128;
+  const uint64_t total = (uint64_t)M * nKb;
   const int sub = threadIdx.x / LANES, l = threadIdx.x % LANES;
-  const size_t first = (size_t)blockIdx.x * PER_CTA * UNROLL + sub;
+  const uint64_t first = (uint64_t)blockIdx.x * PER_CTA * UNROLL + sub;
+  // One division for the first block, additions for the others: a 64-bit division and remainder for every block, once to
+  // load and once to store it, took longer than the loads (39 us in place of 15 at 8192 x 4096).
+  uint32_t row0, kb0;
+  if (total <= 0xffffffffu) {
+    row0 = (uint32_t)first / nKb;
+    kb0 = (uint32_t)first - row0 * nKb;
+  } else {
+    row0 = (uint32_t)(first / nKb);
+    kb0 = (uint32_t)(first - (uint64_t)row0 * nKb);
+  }
+  const uint32_t rowStep = PER_CTA / nKb, kbStep = PER_CTA - rowStep * nKb;
+  uint32_t rows[UNROLL], kbs[UNROLL];
+#pragma unroll
+  for (int u = 0; u < UNROLL; u++) {
+    rows[u] = row0;
+    kbs[u] = kb0;
+    row0 += rowStep;
+    kb0 += kbStep;
+    if (kb0 >= nKb) { kb0 -= nKb; row0++; }
+  }
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
   uint32_t raw[UNROLL][VEC / 2];
 #pragma unroll
   for (int u = 0; u < UNROLL; u++) {
-    const size_t b = first + (size_t)u * PER_CTA;
-    if (b < total) {
-      const size_t row = b / nKb, kb = b % nKb;
-      const __nv_bfloat16 *src = x + row * ldx + kb * 128 + l * VEC;
+    if (first + (uint64_t)u * PER_CTA < total) {
+      const __nv_bfloat16 *src = x + (size_t)rows[u] * ldx + kbs[u] * 128 + l * VEC;
       if (VEC == 8) *(uint4 *)raw[u] = *(const uint4 *)src;
       else *(uint2 *)raw[u] = *(const uint2 *)src;
     } else {
@@ -438,7 +460,6 @@ __global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *__res
   }
 #pragma unroll
   for (int u = 0; u < UNROLL; u++) {
-    const size_t b = first + (size_t)u * PER_CTA;
     float v[VEC], amax = 0.f;
 #pragma unroll
     for (int j = 0; j < VEC / 2; j++) {
@@ -449,16 +470,15 @@ __global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *__res
     }
 #pragma unroll
     for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (b >= total) continue;
-    const size_t row = b / nKb, kb = b % nKb;
+    if (first + (uint64_t)u * PER_CTA >= total) continue;
     const float scale = amax > 0.f ? amax / 448.f : 1.f, inv = 1.f / scale;
     uint32_t out[VEC / 4];
 #pragma unroll
     for (int j = 0; j < VEC / 4; j++) out[j] = pack4Fp8(v[4 * j] * inv, v[4 * j + 1] * inv, v[4 * j + 2] * inv, v[4 * j + 3] * inv);
-    __nv_fp8_storage_t *dst = q + row * K + kb * 128 + l * VEC;
+    __nv_fp8_storage_t *dst = q + (size_t)rows[u] * K + kbs[u] * 128 + l * VEC;
     if (VEC == 8) *(uint2 *)dst = make_uint2(out[0], out[VEC / 4 - 1]);
     else *(uint32_t *)dst = out[0];
-    if (l == 0) sa[kb * M + row] = scale;
+    if (l == 0) sa[(size_t)kbs[u] * M + rows[u]] = scale;
   }
 }
 
@@ -552,13 +572,14 @@ cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap 
 }  // namespace
 
 // Which tile: 0 = 256 x 256 on CTA pairs, 128 or 64 = 128 x that many columns on single CTAs.  The time is about the
-// number of waves times the time of one 128-deep slice of a tile.
+// number of waves times the time of one 128-deep slice of a tile, in nanoseconds: 7, 14 and 28 waves of 32 slices took 177,
+// 212 and 396 us at 8192 x 4096 x 4096.
 extern "C" int fcxGemmFp8Tile(int M, int N, int sms) {
   const int m1 = (M + 127) / 128, m2 = (M + 255) / 256;
   auto waves = [](long long tiles, int slots) { return (double)((tiles + slots - 1) / slots); };
-  const double pair = waves((long long)m2 * ((N + 255) / 256), sms / 2) * 600;
-  const double one = waves((long long)m1 * ((N + 127) / 128), sms) * 400;
-  const double half = waves((long long)m1 * ((N + 63) / 64), sms) * 300;
+  const double pair = waves((long long)m2 * ((N + 255) / 256), sms / 2) * 770;
+  const double one = waves((long long)m1 * ((N + 127) / 128), sms) * 465;
+  const double half = waves((long long)m1 * ((N + 63) / 64), sms) * 437;
   if (pair <= one && pair <= half) return 0;
   return one <= half ? 128 : 64;
 }
