@@ -23,6 +23,7 @@ struct flagcxEmu {
   FcxP2pArgs *p2pDev = nullptr;
   FcxDevError *errHost = nullptr;
   uint64_t seq = 0;
+  unsigned int absent = 0;
   uint64_t sendChunks[FCX_MAX_RANKS][FCX_MAX_RANKS] = {}, recvChunks[FCX_MAX_RANKS][FCX_MAX_RANKS] = {};
 };
 
@@ -100,6 +101,7 @@ flagcxResult_t flagcxEmuCollective(flagcxEmu_t e, flagcxCommOp_t op, const char 
   FcxEmuRanks l;
   memset(&l, 0, sizeof l);
   memcpy(l.dc, e->host, sizeof(FcxDevComm) * n);
+  l.absent = e->absent;
   FcxCollArgs *as = l.args;
   uint64_t seq = ++e->seq;
   for (int r = 0; r < n; r++) {
@@ -204,6 +206,24 @@ flagcxResult_t flagcxEmuGetError(flagcxEmu_t e, int *code) {
     const volatile FcxDevError *er = (const volatile FcxDevError *)((char *)e->errHost + 4096 * r);
     if (er->code) *code = er->code;
   }
+  return flagcxSuccess;
+}
+
+flagcxResult_t flagcxEmuSetAbsent(flagcxEmu_t e, unsigned int ranks) {
+  if (!e || ranks >> e->n) return flagcxInvalidArgument;
+  e->absent = ranks;
+  return flagcxSuccess;
+}
+
+flagcxResult_t flagcxEmuGetDeviceError(flagcxEmu_t e, int rank, int *code, int *peer, int *where, unsigned long long *expected,
+                                       unsigned long long *seen) {
+  if (!e || rank < 0 || rank >= e->n) return flagcxInvalidArgument;
+  const volatile FcxDevError *er = (const volatile FcxDevError *)((char *)e->errHost + 4096 * rank);
+  if (code) *code = (int)er->code;
+  if (peer) *peer = (int)er->peer;
+  if (where) *where = (int)er->where;
+  if (expected) *expected = er->expected;
+  if (seen) *seen = er->seen;
   return flagcxSuccess;
 }
 

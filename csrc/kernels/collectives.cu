@@ -187,14 +187,14 @@ __device__ void arLL(const FcxDevComm &dc, const FcxCollArgs &a, uint64_t seq, i
       if (!pending) break;
       if (spins == 0) t0 = globalTimerNs();
       if ((++spins & 63u) == 0u) {
-        const int late = __ffs(pending) - 1;
         if (*(volatile unsigned int *)&localOf(dc)->abortSeen) return;
-        if (globalTimerNs() - t0 > dc.timeoutNs) {
-          giveUp(dc, FCX_ERR_TIMEOUT, late, FCX_WAIT_LL, cta, tag, 0, seq);
-          return;
-        }
-        if ((spins & 1023u) == 0u && *dc.abortWord) {
-          giveUp(dc, FCX_ERR_ABORT, late, FCX_WAIT_LL, cta, tag, 0, seq);
+        const bool late = globalTimerNs() - t0 > dc.timeoutNs;
+        if (late || ((spins & 1023u) == 0u && *dc.abortWord)) {
+          // looked at once more for the report: the tag of an earlier collective tells a peer that is behind from one that never wrote
+          const int p = __ffs(pending) - 1;
+          const char *line = lines + (size_t)p * FCX_LL_SLOT_BYTES + u * 32;
+          const uint32_t first = llLoad(line).y, second = llLoad(line + 16).y;
+          giveUp(dc, late ? FCX_ERR_TIMEOUT : FCX_ERR_ABORT, p, FCX_WAIT_LL, cta, tag, first != tag ? first : second, seq);
           return;
         }
       }
@@ -1067,12 +1067,14 @@ __global__ void __launch_bounds__(FCX_THREADS, 1) fcxP2pKernel(FcxDevComm dc, Fc
 // all emulated ranks are resident at once and may wait on one another.
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxCollEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
+  if (l.absent >> (blockIdx.x / ctasPerRank) & 1u) return;
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
   fcxCollBody<TIn, TOut>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxMoveEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
+  if (l.absent >> (blockIdx.x / ctasPerRank) & 1u) return;
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);

@@ -236,6 +236,10 @@ _SIGNATURES = {
     "flagcxEmuSendRecv": (_R, [_vp, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.POINTER(_vp),
                                ctypes.POINTER(_vp), _szp, ctypes.c_int, _vp]),
     "flagcxEmuGetError": (_R, [_vp, ctypes.POINTER(ctypes.c_int)]),
+    "flagcxEmuSetAbsent": (_R, [_vp, ctypes.c_uint]),
+    "flagcxEmuGetDeviceError": (_R, [_vp, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
+                                     ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_ulonglong),
+                                     ctypes.POINTER(ctypes.c_ulonglong)]),
 }
 
 

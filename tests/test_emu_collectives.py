@@ -384,3 +384,32 @@ def test_barrier_kernel(lib):
             emu.coll("allreduce", "barrier", 1, None, None, 0, torch.int8)
     finally:
         emu.close()
+
+
+@pytest.mark.parametrize("op", ["allreduce", "reducescatter", "reduce"])
+def test_low_latency_wait_that_runs_out_reports_the_tag_it_saw(lib, monkeypatch, op):
+    """Rank 2 of 4 misses the third collective: every rank that needs it gives up after the time-out and names rank 2, the
+    tag it wanted (3) and the one that lies there (1, of the last collective that used the slot)."""
+    monkeypatch.setenv("FLAGCX_KERNEL_TIMEOUT_MS", "300")
+    n, count = 4, 100
+    emu = Emu(lib, n)
+    try:
+        kind = {"allreduce": "ar_ll", "reducescatter": "rs_ll", "reduce": "reduce_ll"}[op]
+        send = [torch.ones(count * n, device="cuda") for _ in range(n)]
+        recv = [torch.zeros(count * n, device="cuda") for _ in range(n)]
+        for _ in range(2):
+            emu.coll(op, kind, 1, send, recv, count, torch.float32)
+        assert bool((recv[0][:count] == n).all())
+        lib.call("flagcxEmuSetAbsent", emu.h, 1 << 2)
+        with pytest.raises(AssertionError, match="gave up, code 1"):
+            emu.coll(op, kind, 1, send, recv, count, torch.float32)
+        for r in range(n):
+            code, peer, where = (ctypes.c_int() for _ in range(3))
+            want, seen = ctypes.c_ulonglong(), ctypes.c_ulonglong()
+            lib.call("flagcxEmuGetDeviceError", emu.h, r, *(ctypes.byref(v) for v in (code, peer, where, want, seen)))
+            if r == 2 or (op == "reduce" and r != 0):
+                assert code.value == 0, r
+            else:
+                assert (code.value, peer.value, where.value, want.value, seen.value) == (1, 2, 3, 3, 1), r
+    finally:
+        emu.close()
