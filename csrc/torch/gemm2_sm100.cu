@@ -375,12 +375,14 @@ extern "C" int fcxGemmPairMode() {
 
 // Whether the pair kernel is the better choice for this shape: by the waves of tiles that either kernel needs, times what
 // a K block of its tile costs; the pair kernel has to win clearly, since half-empty pair tiles waste both SMs.
-extern "C" int fcxGemmPairSuits(int M, int N, int K) {
+// `cut`: the pieces of K that the launch asks for (0: the launcher's own choice, 1: K stays whole).
+extern "C" int fcxGemmPairSuitsCut(int M, int N, int K, int cut) {
   const int mode = fcxGemmPairMode();
   if (mode == 0 || M < 129 || K < 8) return 0;
   if (mode == 2) return 1;
-  return fcxGemmPairCost(M, N, K, smCount2() / 2) <= 0.85 * fcxGemmTileCost(M, N, K, smCount2(), nullptr);
+  return fcxGemmPairCostCut(M, N, K, smCount2() / 2, cut) <= 0.85 * fcxGemmTileCostCut(M, N, K, smCount2(), cut, nullptr);
 }
+extern "C" int fcxGemmPairSuits(int M, int N, int K) { return fcxGemmPairSuitsCut(M, N, K, 0); }
 
 static bool fillProb(PairProb *p, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN, int group,
                      char *detail, size_t detailLen) {

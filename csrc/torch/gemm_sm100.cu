@@ -466,8 +466,9 @@ int tileGroup(int nN) {
   return g >= 0 ? g : (nN >= 24 ? 16 : 8);  // wide outputs: taller bands keep more of B in L2 per wave
 }
 
-// Columns per tile of the one-CTA kernel: the choice of fcxGemmTileCost, or FLAGCX_GEMM_BN (64, 128, 256) for experiments.
-int pickBn(int M, int N, int K, int sms) {
+// Columns per tile of the one-CTA kernel: the choice of fcxGemmTileCostCut, or FLAGCX_GEMM_BN (64, 128, 256) for experiments.
+// `cut`: the pieces that the caller will ask fcxGemmPickSplitK for (1: K stays whole).
+int pickBn(int M, int N, int K, int sms, int cut) {
   static int forced = -1;
   if (forced < 0) {
     const char *e = getenv("FLAGCX_GEMM_BN");
@@ -476,7 +477,7 @@ int pickBn(int M, int N, int K, int sms) {
   }
   if (forced) return forced;
   int bn = 256;
-  fcxGemmTileCost(M, N, K, sms, &bn);
+  fcxGemmTileCostCut(M, N, K, sms, cut, &bn);
   return bn;
 }
 
@@ -498,7 +499,7 @@ extern "C" cudaError_t fcxGemmBf16(const void *a, const void *b, void *c, int M,
   if (K % 8 || lda % 8 || ldb % 8 || ldc % 8 || M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
   if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, K, smCount());
+  const int bn = pickBn(M, N, K, smCount(), 1);
   if (!makeMap(&ma, a, M, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, bn)) return cudaErrorNotSupported;
   FcxGemmParams p{};
   p.M = M; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.rotate = 0; p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
@@ -535,8 +536,8 @@ extern "C" int fcxGemmPickSplitK(int requested, int units, int slots, int nK, in
   return (nK + kPer - 1) / kPer;
 }
 
-static double waveCost(int units, int slots, int nK, int N, double blockCost) {
-  const int sk = fcxGemmPickSplitK(0, units, slots, nK, N);
+static double waveCost(int units, int slots, int nK, int N, int cut, double blockCost) {
+  const int sk = fcxGemmPickSplitK(cut, units, slots, nK, N);
   const int waves = (units * sk + slots - 1) / slots;
   return waves * ((nK + sk - 1) / sk) * blockCost * (1.0 + 0.03 * (sk - 1));
 }
@@ -544,14 +545,17 @@ static double waveCost(int units, int slots, int nK, int N, double blockCost) {
 // Estimated clocks of the one-CTA kernel with its best tile width, and that width.  A 64-deep K block of a 128 x bn tile is
 // bound by what one SM can fetch (16 KB of A and bn x 128 bytes of B at about 64 bytes a clock): 768, 512 and 384 clocks
 // for 256, 128 and 64 columns.  Narrow tiles re-read A and never pay once 256-column tiles fill the SMs, but with few
-// tiles they put more SMs to work on the same K steps.
-extern "C" double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut) {
+// tiles they put more SMs to work on the same K steps.  `cut` is the launch's own: a sum that stays whole (1) keeps as many
+// SMs busy as it has tiles, one that may be cut (0) fills them whatever its tiles are.  Uncut, measured: 512 x 1024 x 4096
+// 25.4 / 26.0 / 28.6 us in 64 / 128 / 256 columns and 27.2 on CTA pairs; 640 x 3584 x 4096 46.7 / 27.1 / 29.3 and 29.0;
+// 4096 x 1024 x 1792 42.3 / 24.4 / 16.6 and 15.8.
+extern "C" double fcxGemmTileCostCut(int M, int N, int K, int sms, int cut, int *bnOut) {
   const int nK = (K + BK - 1) / BK, nM = (M + BM - 1) / BM;
   const int widths[3] = {256, 128, 64};
   const double clocks[3] = {768, 512, 384};
   double best = 0;
   for (int i = 0; i < 3; i++) {
-    const double c = waveCost(nM * ((N + widths[i] - 1) / widths[i]), sms, nK, N, clocks[i]);
+    const double c = waveCost(nM * ((N + widths[i] - 1) / widths[i]), sms, nK, N, cut, clocks[i]);
     if (i == 0 || c < 0.9 * best) {
       best = c;
       if (bnOut) *bnOut = widths[i];
@@ -560,10 +564,13 @@ extern "C" double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut) {
   return best;
 }
 
+extern "C" double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut) { return fcxGemmTileCostCut(M, N, K, sms, 0, bnOut); }
+
 // The same for the CTA-pair kernel: 32 KB per CTA and K block of a 256 x 256 tile.
-extern "C" double fcxGemmPairCost(int M, int N, int K, int pairs) {
-  return waveCost(((M + 255) / 256) * ((N + 255) / 256), pairs, (K + BK - 1) / BK, N, 512);
+extern "C" double fcxGemmPairCostCut(int M, int N, int K, int pairs, int cut) {
+  return waveCost(((M + 255) / 256) * ((N + 255) / 256), pairs, (K + BK - 1) / BK, N, cut, 512);
 }
+extern "C" double fcxGemmPairCost(int M, int N, int K, int pairs) { return fcxGemmPairCostCut(M, N, K, pairs, 0); }
 
 // What went wrong in the last fcxGemmBf16Ex call of this thread that did not return cudaSuccess.
 static thread_local char gGemmDetail[256];
@@ -579,11 +586,11 @@ extern "C" cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, in
   if ((aMN && M % 8) || (bMN && N % 8) || (bias && ((uintptr_t)bias & 1)) || (accumulate && N % 2)) return cudaErrorInvalidValue;
   gGemmDetail[0] = 0;
   cudaGetLastError();  // an error left behind by an earlier, unrelated call of this thread is not this launch's
-  if (o->geluOut || (o->pair >= 0 ? o->pair > 0 : fcxGemmPairSuits(M, N, K) != 0))  // CTA pairs on 256 x 256 tiles (gemm2_sm100.cu)
+  if (o->geluOut || (o->pair >= 0 ? o->pair > 0 : fcxGemmPairSuitsCut(M, N, K, splitK) != 0))  // CTA pairs on 256 x 256 tiles (gemm2_sm100.cu)
     return fcxGemmPairBf16(a, b, c, M, N, K, lda, ldb, ldc, aMN, bMN, bias, splitK, accumulate, o->geluOut, tileGroup((N + 255) / 256) / 2,
                            errFlag, s, gGemmDetail, sizeof gGemmDetail);
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, K, smCount());
+  const int bn = pickBn(M, N, K, smCount(), splitK);
   // K-major operand: rows = M (or N), box of 128 (bn) rows x 64 K; MN-major operand: rows = K, box of 64 lines x 64 columns
   const bool okA = aMN ? makeMap(&ma, a, K, M, lda, BK) : makeMap(&ma, a, M, K, lda, BM);
   const bool okB = bMN ? makeMap(&mb, b, K, N, ldb, BK) : makeMap(&mb, b, N, K, ldb, bn);
@@ -620,7 +627,7 @@ extern "C" cudaError_t fcxGemmBf16DynM(const void *a, const void *b, void *c, in
                                        int *errFlag, cudaStream_t s) {
   if (K % 8 || lda % 8 || ldb % 8 || ldc % 8 || Mmax <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
-  const int bn = pickBn(Mmax, N, K, smCount());
+  const int bn = pickBn(Mmax, N, K, smCount(), 1);
   if (!makeMap(&ma, a, Mmax, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, bn)) return cudaErrorNotSupported;
   FcxGemmParams p{};
   p.M = Mmax; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.mPtr = mPtr; p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
@@ -646,7 +653,7 @@ extern "C" cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, c
   if (K % 8 || ldb % 8 || ldc % 8 || M % (n * BM) || commCtas < 1) return cudaErrorInvalidValue;
   if (n == 1) return oneRank(aLocal, b, c, M, N, K, K, ldb, ldc, errFlag, s);
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, K, std::max(1, smCount() - commCtas));
+  const int bn = pickBn(M, N, K, std::max(1, smCount() - commCtas), 1);
   CUtensorMap mal;
   if (!makeMap(&ma, gathered, M, K, K, BM) || !makeMap(&mb, b, N, K, ldb, bn) || !makeMap(&mal, aLocal, M / n, K, K, BM))
     return cudaErrorNotSupported;
@@ -699,7 +706,7 @@ extern "C" cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const 
   };
   const int sms = smCount();
   auto fill = [&](Product *q, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int aMN) {
-    const int bn = pickBn(M, N, K, sms);
+    const int bn = pickBn(M, N, K, sms, 0);
     if (!(aMN ? makeMap(&q->a, a, K, M, lda, BK) : makeMap(&q->a, a, M, K, lda, BM)) || !makeMap(&q->b, b, K, N, ldb, BK)) return false;
     q->p = FcxGemmParams{};
     q->p.M = M; q->p.N = N; q->p.K = K; q->p.c = c; q->p.ldc = N; q->p.errFlag = errFlag; q->p.bn = bn; q->p.group = tileGroup((N + bn - 1) / bn);

@@ -65,9 +65,12 @@ cudaError_t fcxGemmBackwardPair(const void *dy, const void *w, const void *x, vo
 int fcxGemmDualPlan(int units0, int nK0, int alone0, int units1, int nK1, int alone1, int workers, int *split0, int *split1, int *swap, int *extra);
 int fcxGemmPickSplitK(int requested, int units, int slots, int nK, int N);
 double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut);
+double fcxGemmTileCostCut(int M, int N, int K, int sms, int cut, int *bnOut);
 double fcxGemmPairCost(int M, int N, int K, int pairs);
+double fcxGemmPairCostCut(int M, int N, int K, int pairs, int cut);
 int fcxGemmPairMode();
 int fcxGemmPairSuits(int M, int N, int K);
+int fcxGemmPairSuitsCut(int M, int N, int K, int cut);
 cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,
                             const void *bias, int splitK, int accumulate, void *geluOut, int group, int *errFlag, cudaStream_t s,
                             char *detail, size_t detailLen);

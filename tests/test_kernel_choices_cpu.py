@@ -34,6 +34,25 @@ def test_gemm_tile_width(ext):
     assert _width(ext, 64, 3072, 1024) == 64     # 12 tiles of 256 columns: 12 of 148 SMs
 
 
+def test_uncut_sums_get_the_kernel_that_is_fastest_uncut(ext):
+    """A launch that keeps K whole (one-rank tensor parallel, all-gather GEMM, the plain NT form) is priced without a cut: what
+    it gets is within the rule's own margin (the pair kernel has to win by 15 %) of the cheapest kernel and tile."""
+    ext.fcxGemmTileCostCut.restype = ctypes.c_double
+    ext.fcxGemmPairSuitsCut.restype = ctypes.c_int
+    few_rows = [(512, 1024, 4096), (256, 1024, 4096), (256, 2048, 2048), (256, 4096, 4096), (512, 2048, 4096), (1024, 1024, 4096), (384, 2048, 2048)]
+    rest = [(m, n, k) for m in (64, 128, 640, 2328, 8192) for n in (64, 200, 1792, 4096) for k in (64, 1000, 4096)]
+    for m, n, k in few_rows + rest:
+        def uncut(rows, cols, slots, clocks):
+            return -(-(-(-m // rows) * -(-n // cols)) // slots) * -(-k // 64) * clocks
+        costs = {64: uncut(128, 64, 148, 384), 128: uncut(128, 128, 148, 512), 256: uncut(128, 256, 148, 768), "pair": uncut(256, 256, 74, 512)}
+        bn = ctypes.c_int(0)
+        tile = ext.fcxGemmTileCostCut(m, n, k, 148, 1, ctypes.byref(bn))
+        assert tile == costs[bn.value]
+        chosen = "pair" if ext.fcxGemmPairSuitsCut(m, n, k, 1) else bn.value
+        least = min(costs.values()) if m >= 129 else min(v for c, v in costs.items() if c != "pair")
+        assert costs[chosen] <= least / 0.85 + 1e-6, ((m, n, k), chosen, costs)
+
+
 def test_fp8_tile(ext):
     for m in (1, 128, 129, 333, 8192):
         for n in (8, 64, 136, 1792, 4096):
