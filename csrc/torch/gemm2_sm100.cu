@@ -423,8 +423,8 @@ extern "C" cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, in
     splitK = 1;  // the activation needs the whole sum
   }
   PairProb &p = args.prob[0];
-  const int nK = (K + BK - 1) / BK, pairs = smCount2() / 2;
-  p.splitK = fcxGemmPickSplitK(splitK, p.units, pairs, nK, N);
+  const int pairs = smCount2() / 2;
+  p.splitK = fcxGemmPieces(splitK, M, N, K, p.units, pairs, smCount2());
   p.units *= p.splitK;
   p.accumulate = accumulate;
   args.bias = bias;
@@ -508,8 +508,8 @@ extern "C" cudaError_t fcxGemmBackwardPair(const void *dy, const void *w, const 
     return cudaErrorNotSupported;
   const int nKx = (O + BK - 1) / BK, nKw = (T + BK - 1) / BK, pairs = smCount2() / 2;
   int swap = 0;
-  if (!fcxGemmDualPlan(pw.units, nKw, fcxGemmPickSplitK(0, pw.units, pairs, nKw, I), px.units, nKx, fcxGemmPickSplitK(0, px.units, pairs, nKx, I),
-                       pairs, &pw.splitK, &px.splitK, &swap, &args.extra))
+  if (!fcxGemmDualPlan(pw.units, nKw, fcxGemmPieces(0, O, I, T, pw.units, pairs, smCount2()), px.units, nKx,
+                       fcxGemmPieces(0, T, I, O, px.units, pairs, smCount2()), pairs, &pw.splitK, &px.splitK, &swap, &args.extra))
     return cudaErrorNotSupported;
   pw.accumulate = accumulate;
   for (PairProb *p : {&px, &pw}) {

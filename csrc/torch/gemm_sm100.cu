@@ -536,8 +536,22 @@ extern "C" int fcxGemmPickSplitK(int requested, int units, int slots, int nK, in
   return (nK + kPer - 1) / kPer;
 }
 
-static double waveCost(int units, int slots, int nK, int N, int cut, double blockCost) {
-  const int sk = fcxGemmPickSplitK(cut, units, slots, nK, N);
+// The pieces of K of one launch: those asked for, else the launcher's choice for `units` tiles on `slots` workers.  Each piece
+// is rounded to bf16 once more where it is added in memory, so the choice of a kernel and tile must not cost exactness: K
+// is never cut finer than by CTA pairs where the rows fill their 256-row blocks to 7 %, and by single CTAs with 256-column
+// tiles elsewhere.  (The pair kernel counts half the slots and, with a half-empty last row block, less than half the tiles:
+// 288 x 3392 x 3832 would be cut in 5 in place of 3.)
+extern "C" int fcxGemmPieces(int requested, int M, int N, int K, int units, int slots, int sms) {
+  const int nK = (K + BK - 1) / BK, pieces = fcxGemmPickSplitK(requested, units, slots, nK, N);
+  if (requested > 0) return pieces;
+  const int nN = (N + BN - 1) / BN, pairRows = (M + 2 * BM - 1) / (2 * BM);
+  const bool fills = M > BM && N >= 192 && pairRows * 2 * BM <= 1.07 * M;
+  const int most = fills ? fcxGemmPickSplitK(0, pairRows * nN, sms / 2, nK, N) : fcxGemmPickSplitK(0, (M + BM - 1) / BM * nN, sms, nK, N);
+  return pieces <= most ? pieces : fcxGemmPickSplitK(most, units, slots, nK, N);
+}
+
+static double waveCost(int M, int N, int K, int units, int slots, int sms, int cut, double blockCost) {
+  const int nK = (K + BK - 1) / BK, sk = fcxGemmPieces(cut, M, N, K, units, slots, sms);
   const int waves = (units * sk + slots - 1) / slots;
   return waves * ((nK + sk - 1) / sk) * blockCost * (1.0 + 0.03 * (sk - 1));
 }
@@ -550,12 +564,12 @@ static double waveCost(int units, int slots, int nK, int N, int cut, double bloc
 // 25.4 / 26.0 / 28.6 us in 64 / 128 / 256 columns and 27.2 on CTA pairs; 640 x 3584 x 4096 46.7 / 27.1 / 29.3 and 29.0;
 // 4096 x 1024 x 1792 42.3 / 24.4 / 16.6 and 15.8.
 extern "C" double fcxGemmTileCostCut(int M, int N, int K, int sms, int cut, int *bnOut) {
-  const int nK = (K + BK - 1) / BK, nM = (M + BM - 1) / BM;
+  const int nM = (M + BM - 1) / BM;
   const int widths[3] = {256, 128, 64};
   const double clocks[3] = {768, 512, 384};
   double best = 0;
   for (int i = 0; i < 3; i++) {
-    const double c = waveCost(nM * ((N + widths[i] - 1) / widths[i]), sms, nK, N, cut, clocks[i]);
+    const double c = waveCost(M, N, K, nM * ((N + widths[i] - 1) / widths[i]), sms, sms, cut, clocks[i]);
     if (i == 0 || c < 0.9 * best) {
       best = c;
       if (bnOut) *bnOut = widths[i];
@@ -568,7 +582,7 @@ extern "C" double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut) { re
 
 // The same for the CTA-pair kernel: 32 KB per CTA and K block of a 256 x 256 tile.
 extern "C" double fcxGemmPairCostCut(int M, int N, int K, int pairs, int cut) {
-  return waveCost(((M + 255) / 256) * ((N + 255) / 256), pairs, (K + BK - 1) / BK, N, cut, 512);
+  return waveCost(M, N, K, ((M + 255) / 256) * ((N + 255) / 256), pairs, 2 * pairs, cut, 512);
 }
 extern "C" double fcxGemmPairCost(int M, int N, int K, int pairs) { return fcxGemmPairCostCut(M, N, K, pairs, 0); }
 
@@ -602,8 +616,8 @@ extern "C" cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, in
   FcxGemmParams p{};
   p.M = M; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.rotate = 0; p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
   p.aMN = aMN; p.bMN = bMN; p.bias = bias; p.accumulate = accumulate;
-  const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn), nK = (K + BK - 1) / BK;
-  p.splitK = fcxGemmPickSplitK(splitK, tiles, smCount(), nK, N);
+  const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
+  p.splitK = fcxGemmPieces(splitK, M, N, K, tiles, smCount(), smCount());
   if (p.splitK > 1 && !accumulate) {
     cudaError_t e = cudaMemsetAsync(c, 0, ((size_t)(M - 1) * ldc + N) * 2, s);
     if (e != cudaSuccess) return e;
@@ -719,8 +733,8 @@ extern "C" cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const 
   if (!fill(&px, dy, w, dx, T, I, O, lddy, ldw, 0) || !fill(&pw, dy, x, dw, O, I, T, lddy, ldx, 1)) return cudaErrorNotSupported;
   int swap = 0;
   SecondProduct second{};
-  if (!fcxGemmDualPlan(pw.units, pw.nK, fcxGemmPickSplitK(0, pw.units, sms, pw.nK, I), px.units, px.nK,
-                       fcxGemmPickSplitK(0, px.units, sms, px.nK, I), sms, &pw.p.splitK, &px.p.splitK, &swap, &second.extra))
+  if (!fcxGemmDualPlan(pw.units, pw.nK, fcxGemmPieces(0, O, I, T, pw.units, sms, sms), px.units, px.nK,
+                       fcxGemmPieces(0, T, I, O, px.units, sms, sms), sms, &pw.p.splitK, &px.p.splitK, &swap, &second.extra))
     return cudaErrorNotSupported;
   pw.p.accumulate = accumulate;
   int total = 0;

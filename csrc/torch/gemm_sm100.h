@@ -64,6 +64,7 @@ cudaError_t fcxGemmBackwardPair(const void *dy, const void *w, const void *x, vo
                                 int accumulate, int groupX, int groupW, int *errFlag, cudaStream_t s);
 int fcxGemmDualPlan(int units0, int nK0, int alone0, int units1, int nK1, int alone1, int workers, int *split0, int *split1, int *swap, int *extra);
 int fcxGemmPickSplitK(int requested, int units, int slots, int nK, int N);
+int fcxGemmPieces(int requested, int M, int N, int K, int units, int slots, int sms);
 double fcxGemmTileCost(int M, int N, int K, int sms, int *bnOut);
 double fcxGemmTileCostCut(int M, int N, int K, int sms, int cut, int *bnOut);
 double fcxGemmPairCost(int M, int N, int K, int pairs);

@@ -1,6 +1,8 @@
 """Host-side rules that pick a kernel or a tile, checked without a GPU: every rule gives a legal answer over its whole
 range, and picks the variant that each side of its line was measured for."""
 import ctypes
+import math
+import random
 
 import pytest
 
@@ -51,6 +53,29 @@ def test_uncut_sums_get_the_kernel_that_is_fastest_uncut(ext):
         chosen = "pair" if ext.fcxGemmPairSuitsCut(m, n, k, 1) else bn.value
         least = min(costs.values()) if m >= 129 else min(v for c, v in costs.items() if c != "pair")
         assert costs[chosen] <= least / 0.85 + 1e-6, ((m, n, k), chosen, costs)
+
+
+def test_no_choice_of_kernel_cuts_a_sum_finer(ext):
+    """Every piece of K is one more rounding to bf16.  Whatever kernel and tile a size gets, it is cut into no more pieces than
+    by the simple rule: CTA pairs for rows that fill their 256-row blocks to 7 %, else single CTAs of 256 columns."""
+    rng = random.Random(5)
+    sizes = [(288, 3392, 3832), (1072, 2368, 3592), (2376, 1280, 2960), (312, 3416, 3520), (640, 2112, 4048)]
+    def size(lo, hi):
+        return int(math.exp(rng.uniform(math.log(lo), math.log(hi)))) // 8 * 8
+    sizes += [(size(16, 8200), size(512, 4100), size(512, 8200)) for _ in range(20000)]
+    for m, n, k in sizes:
+        n_k, m1, m2 = -(-k // 64), -(-m // 128), -(-m // 256)
+        if m >= 129 and m2 * 256 <= 1.07 * m and n >= 192:
+            simple = ext.fcxGemmPickSplitK(0, m2 * -(-n // 256), 74, n_k, n)
+        else:
+            simple = ext.fcxGemmPickSplitK(0, m1 * -(-n // 256), 148, n_k, n)
+        if ext.fcxGemmPairSuits(m, n, k):
+            pieces = ext.fcxGemmPieces(0, m, n, k, m2 * -(-n // 256), 74, 148)
+        else:
+            pieces = ext.fcxGemmPieces(0, m, n, k, m1 * -(-n // _width(ext, m, n, k)), 148, 148)
+        assert 1 <= pieces <= simple, (m, n, k, pieces, simple)
+        assert (pieces - 1) * -(-n_k // pieces) < n_k  # the last piece is not empty
+    assert ext.fcxGemmPieces(5, 288, 3392, 3832, 28, 74, 148) == 5  # a caller's own count stands
 
 
 def test_fp8_tile(ext):
