@@ -177,7 +177,7 @@ static std::tuple<at::Tensor, at::Tensor> gemmBiasGelu(const at::Tensor &a, cons
 // y[M,N] = all_gather(x_local)[M,K] @ w[N,K]^T.  gathered: heap tensor [M,K]; flags: heap int64 tensor [M/128];
 // epoch: 1-based use count of this (gathered, flags) pair.
 static at::Tensor agGemm(uint64_t comm, const at::Tensor &xLocal, at::Tensor &gathered, at::Tensor &flags, const at::Tensor &w,
-                         int64_t epoch, int64_t commCtas, at::Tensor &err) {
+                         int64_t epoch, int64_t commCtas, at::Tensor &err, bool exchange) {
   checkMat(xLocal, "x_local");
   checkMat(w, "w");
   TORCH_CHECK(xLocal.is_contiguous() && gathered.is_contiguous(), "x_local and gathered must be contiguous");
@@ -187,7 +187,7 @@ static at::Tensor agGemm(uint64_t comm, const at::Tensor &xLocal, at::Tensor &ga
   TORCH_CHECK(gathered.numel() >= (int64_t)M * K && flags.numel() >= M / 128, "workspace too small");
   auto y = at::empty({M, N}, xLocal.options());
   auto e = fcxAgGemmBf16(&dc, xLocal.data_ptr(), gathered.data_ptr(), heapOffset(comm, gathered), heapOffset(comm, flags), w.data_ptr(),
-                         y.data_ptr(), M, N, K, (int)w.stride(0), (int)y.stride(0), (uint64_t)epoch, (int)commCtas, err.data_ptr<int>(),
+                         y.data_ptr(), M, N, K, (int)w.stride(0), (int)y.stride(0), (uint64_t)epoch, (int)commCtas, exchange, err.data_ptr<int>(),
                          at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(e == cudaSuccess, "fused all-gather GEMM launch failed: ", cudaGetErrorString(e));
   return y;
@@ -196,7 +196,7 @@ static at::Tensor agGemm(uint64_t comm, const at::Tensor &xLocal, at::Tensor &ga
 // out[M/n,N] = reduce_scatter(a[M,K] @ w[N,K]^T).  stage: heap bf16 tensor [n, M/n, N]; counters: heap int64 tensor
 // [M/n/128 * ceil(N/256)]; epoch: 1-based use count of this (stage, counters) pair.
 static at::Tensor gemmRs(uint64_t comm, const at::Tensor &a, const at::Tensor &w, at::Tensor &stage, at::Tensor &counters, int64_t epoch,
-                         at::Tensor &err) {
+                         at::Tensor &err, bool exchange) {
   checkMat(a, "a");
   checkMat(w, "w");
   c10::cuda::CUDAGuard g(a.device());
@@ -206,7 +206,7 @@ static at::Tensor gemmRs(uint64_t comm, const at::Tensor &a, const at::Tensor &w
   TORCH_CHECK(stage.numel() >= (int64_t)M * N && counters.numel() >= (M / dc.nranks / 128) * ((N + 255) / 256), "workspace too small");
   auto out = at::empty({M / dc.nranks, N}, a.options());
   auto e = fcxGemmRsBf16(&dc, a.data_ptr(), w.data_ptr(), out.data_ptr(), heapOffset(comm, stage), heapOffset(comm, counters), M, N, K,
-                         (int)a.stride(0), (int)w.stride(0), (int)out.stride(0), (uint64_t)epoch, err.data_ptr<int>(),
+                         (int)a.stride(0), (int)w.stride(0), (int)out.stride(0), (uint64_t)epoch, exchange, err.data_ptr<int>(),
                          at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(e == cudaSuccess, "fused GEMM reduce-scatter launch failed: ", cudaGetErrorString(e));
   return out;
@@ -271,8 +271,11 @@ void bindGemm(py::module &m) {
         py::arg("err"), py::arg("dw_into") = py::none(), py::arg("db_into") = py::none());
   m.def("gemm_bias_gelu", &gemmBiasGelu, py::arg("a"), py::arg("w"), py::arg("bias"), py::arg("err"),
         "(a w^T, gelu_tanh(a w^T + bias)) from one CTA-pair GEMM launch");
-  m.def("ag_gemm", &agGemm);
-  m.def("gemm_rs", &gemmRs);
+  m.def("ag_gemm", &agGemm, py::arg("comm"), py::arg("x_local"), py::arg("gathered"), py::arg("flags"), py::arg("w"), py::arg("epoch"),
+        py::arg("comm_ctas"), py::arg("err"), py::arg("exchange") = false,
+        "exchange: take the exchanging kernel on a communicator of one rank too (it gets the plain GEMM otherwise)");
+  m.def("gemm_rs", &gemmRs, py::arg("comm"), py::arg("a"), py::arg("w"), py::arg("stage"), py::arg("counters"), py::arg("epoch"), py::arg("err"),
+        py::arg("exchange") = false);
 }
 
 }  // namespace fcxt

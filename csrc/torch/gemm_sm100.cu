@@ -652,7 +652,8 @@ extern "C" cudaError_t fcxGemmBf16DynM(const void *a, const void *b, void *c, in
 
 // All-gather -> GEMM and GEMM -> reduce-scatter of one rank: there is nothing to exchange, so the plain GEMM writes the
 // result itself (as CTA pairs where the shape suits) in place of a copy of the partial tiles in the staging area that is
-// then read back.  K is not cut: the sums stay fp32 until the one rounding, as in the fused kernels.
+// then read back.  K is not cut: the sums stay fp32 until the one rounding, as in the fused kernels.  `exchange` of the two
+// entry points below takes the exchanging kernel all the same, with this GPU as its own peer: tests and profiles need it.
 static cudaError_t oneRank(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int *errFlag, cudaStream_t s) {
   FcxGemmOpts o{};
   o.splitK = 1;
@@ -662,10 +663,10 @@ static cudaError_t oneRank(const void *a, const void *b, void *c, int M, int N, 
 
 extern "C" cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, const void *gathered, size_t gatherOff, size_t flagOff,
                                      const void *b, void *c, int M, int N, int K, int ldb, int ldc, uint64_t epoch, int commCtas,
-                                     int *errFlag, cudaStream_t s) {
+                                     int exchange, int *errFlag, cudaStream_t s) {
   const int n = dc->nranks;
   if (K % 8 || ldb % 8 || ldc % 8 || M % (n * BM) || commCtas < 1) return cudaErrorInvalidValue;
-  if (n == 1) return oneRank(aLocal, b, c, M, N, K, K, ldb, ldc, errFlag, s);
+  if (n == 1 && !exchange) return oneRank(aLocal, b, c, M, N, K, K, ldb, ldc, errFlag, s);
   CUtensorMap ma, mb;
   const int bn = pickBn(M, N, K, std::max(1, smCount() - commCtas), 1);
   CUtensorMap mal;
@@ -683,10 +684,10 @@ extern "C" cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, c
 }
 
 extern "C" cudaError_t fcxGemmRsBf16(const FcxDevComm *dc, const void *a, const void *b, void *out, size_t stageOff, size_t flagOff, int M,
-                                     int N, int K, int lda, int ldb, int ldc, uint64_t epoch, int *errFlag, cudaStream_t s) {
+                                     int N, int K, int lda, int ldb, int ldc, uint64_t epoch, int exchange, int *errFlag, cudaStream_t s) {
   const int n = dc->nranks;
   if (K % 8 || lda % 8 || ldb % 8 || ldc % 8 || N % 8 || M % (n * BM)) return cudaErrorInvalidValue;
-  if (n == 1) return oneRank(a, b, out, M, N, K, lda, ldb, ldc, errFlag, s);
+  if (n == 1 && !exchange) return oneRank(a, b, out, M, N, K, lda, ldb, ldc, errFlag, s);
   CUtensorMap ma, mb;
   if (!makeMap(&ma, a, M, K, lda, BM) || !makeMap(&mb, b, N, K, ldb, BN)) return cudaErrorNotSupported;
   FcxGemmParams p{};

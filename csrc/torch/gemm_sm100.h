@@ -39,10 +39,11 @@ struct FcxGemmParams {
 extern "C" {
 #endif
 cudaError_t fcxGemmBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int *errFlag, cudaStream_t s);
+// One rank has nothing to exchange and takes the plain GEMM, unless `exchange` asks for the kernel of several ranks.
 cudaError_t fcxAgGemmBf16(const FcxDevComm *dc, const void *aLocal, const void *gathered, size_t gatherOff, size_t flagOff, const void *b,
-                          void *c, int M, int N, int K, int ldb, int ldc, uint64_t epoch, int commCtas, int *errFlag, cudaStream_t s);
+                          void *c, int M, int N, int K, int ldb, int ldc, uint64_t epoch, int commCtas, int exchange, int *errFlag, cudaStream_t s);
 cudaError_t fcxGemmRsBf16(const FcxDevComm *dc, const void *a, const void *b, void *out, size_t stageOff, size_t flagOff, int M, int N, int K,
-                          int lda, int ldb, int ldc, uint64_t epoch, int *errFlag, cudaStream_t s);
+                          int lda, int ldb, int ldc, uint64_t epoch, int exchange, int *errFlag, cudaStream_t s);
 // General form: operand storage per FcxGemmParams::aMN / bMN (lda / ldb = elements between the stored rows),
 // optional bias row, splitK = 0 lets the launcher pick (it splits K when the tiles would fill under half of the SMs).
 cudaError_t fcxGemmBf16Ex(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,

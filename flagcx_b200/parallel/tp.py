@@ -42,6 +42,7 @@ class TensorParallelContext:
         self.err = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.ag_calls = 0
         self.rs_calls = 0
+        self.exchange = nranks > 1  # one rank takes plain GEMMs; set it, and the exchanging kernels run with this GPU as its own peer
         torch.cuda.synchronize()
         # nobody may push into a workspace that its owner has not cleared yet
         if nranks > 1:
@@ -56,7 +57,8 @@ class TensorParallelContext:
         self.ag_calls += 1
         rows, k = x_local.shape[0] * self.n, x_local.shape[1]
         gathered = self.gathered[par].view(-1)[: rows * k].view(rows, k)
-        return self.nat.ag_gemm(self.comm, x_local, gathered, self.ag_flags[par], w, epoch, self._comm_ctas(rows, k, w.shape[0]), self.err)
+        return self.nat.ag_gemm(self.comm, x_local, gathered, self.ag_flags[par], w, epoch, self._comm_ctas(rows, k, w.shape[0]), self.err,
+                                self.exchange)
 
     def last_gathered(self, x_local: torch.Tensor) -> torch.Tensor:
         """The full [rows, K] matrix that the most recent ``ag_gemm`` call gathered: the remote rows are where the
@@ -98,7 +100,7 @@ class TensorParallelContext:
         self.rs_calls += 1
         rows, n_out = a.shape[0], w.shape[0]
         stage = self.rs_stage[par].view(-1)[: rows * n_out]
-        return self.nat.gemm_rs(self.comm, a, w, stage, self.rs_counters[par], epoch, self.err)
+        return self.nat.gemm_rs(self.comm, a, w, stage, self.rs_counters[par], epoch, self.err, self.exchange)
 
     def plain_gemm_nn(self, a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """``a @ w`` for the backward pass of a single rank: nothing is exchanged, so the plain GEMM reads the weight
@@ -157,10 +159,10 @@ class _ColumnParallel(torch.autograd.Function):
         # peers will push into again a few calls from now, and they cannot get there before this rank has
         # contributed to the reduce-scatter below.
         dw = gemm(dy, full, True, True)              # [N, rows] @ [rows, K]
-        if tp.n == 1:
-            dx_local = tp.plain_gemm_nn(dy, w)
-        else:
+        if tp.exchange:
             dx_local = tp.gemm_rs(dy, tp.transposed(w))  # [rows, N] @ [N, K] -> rows/n x K
+        else:
+            dx_local = tp.plain_gemm_nn(dy, w)
         return dx_local, dw, None
 
 
@@ -184,11 +186,11 @@ class _RowParallel(torch.autograd.Function):
         a, w = ctx.saved_tensors
         tp = ctx.tp
         dz_local = dz_local.contiguous()
-        if tp.n == 1:
-            da, full = tp.plain_gemm_nn(dz_local, w), dz_local
-        else:
+        if tp.exchange:
             da = tp.ag_gemm(dz_local, tp.transposed(w))  # [rows, N] @ [N, K_local]
             full = tp.last_gathered(dz_local)
+        else:
+            da, full = tp.plain_gemm_nn(dz_local, w), dz_local
         dw = gemm(full, a, True, True)               # [N, rows] @ [rows, K_local]
         return da, dw, None
 

@@ -144,8 +144,8 @@ def main():
         lib.call("flagcxEmuDestroy", emu)
     elif args.case in ("gemm_dgrad", "gemm_wgrad", "gemm_ag", "gemm_rs"):
         # the backward GEMMs of a linear layer (operands read transposed in place; the weight gradient splits K) and
-        # the fused all-gather / reduce-scatter forms on a one-rank communicator (comm CTAs, flags, staging and tail
-        # reduction all run, with this GPU as its own peer)
+        # the fused all-gather / reduce-scatter forms on a one-rank communicator: the kernels of several ranks, asked for
+        # explicitly (one rank takes the plain GEMM otherwise), with this GPU as its own peer (flags, staging, tail reduction)
         err = torch.zeros(1, dtype=torch.int32, device="cuda")
         pk = ROOT / "MEASURED_PEAKS.json"
         tf_peak = json.loads(pk.read_text())["bf16_tflops"] if pk.exists() else 1590.0
@@ -168,6 +168,7 @@ def main():
             comm = lib.flagcxCommInitRank(1, lib.flagcxGetUniqueId(), 0)
             M, N, K = 8192, 4096, 4096
             tp = TensorParallelContext(comm.value, 1, 0, max_rows=M, max_k=K, max_n=N, comm_ctas=4)
+            tp.exchange = True
             a = (torch.randn(M, K, device="cuda") * 0.1).bfloat16()
             b = (torch.randn(N, K, device="cuda") * 0.1).bfloat16()
             ms = timed((lambda: tp.ag_gemm(a, b)) if args.case == "gemm_ag" else (lambda: tp.gemm_rs(a, b)))

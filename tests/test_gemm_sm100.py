@@ -1,8 +1,11 @@
 """tcgen05 GEMM family against fp32 PyTorch references, on one GPU.
 
-The fused all-gather/reduce-scatter forms run here on a one-rank communicator:
-that still exercises the comm CTAs, the per-block flags, the proxy fence in
-front of the TMA loads, the staging/counter path and the reduction phase."""
+The fused all-gather/reduce-scatter forms run here on a one-rank communicator,
+both as a single rank takes them (plain GEMM) and as several ranks do
+(``exchange``): the tile order by owner, the loads from the local block, the
+staging and counter path and the reduction phase, with this GPU as its own peer.
+What only peers reach (the comm CTAs' pushes, the waits for their flags) needs
+several GPUs."""
 import ctypes
 
 import pytest
@@ -65,10 +68,12 @@ def comm1():
     lib.flagcxCommDestroy(comm)
 
 
-def test_fused_forms_on_one_rank(nat, comm1):
+@pytest.mark.parametrize("exchange", [False, True])
+def test_fused_forms_on_one_rank(nat, comm1, exchange):
     from flagcx_b200.parallel.tp import TensorParallelContext
     lib, comm = comm1
     tp = TensorParallelContext(comm.value, 1, 0, max_rows=1024, max_k=1024, max_n=1024, comm_ctas=4)
+    tp.exchange = exchange
     torch.manual_seed(2)
     for rep in range(3):  # both workspace parities and a reused one
         x = (torch.randn(1024, 512, device="cuda") * 0.5).bfloat16()
@@ -80,13 +85,48 @@ def test_fused_forms_on_one_rank(nat, comm1):
         ref = _ref(x, w)
         _close(y, ref, 512)
         _close(z, ref, 512)
+    # the exchanging reduce-scatter kernel counts its tiles, the plain GEMM touches no counter
+    assert bool((tp.rs_counters[0][:4] > 0).all()) == exchange
 
 
-def test_tensor_parallel_linears_forward_and_backward(nat, comm1):
+@pytest.mark.parametrize("M,N,K,width", [(1024, 1000, 512, 64), (2048, 1000, 264, 128), (4096, 1000, 264, 256), (128, 72, 64, 64)])
+def test_exchanging_forms_at_every_tile_width(nat, comm1, M, N, K, width):
+    """The all-gather GEMM in 64, 128 and 256 columns and the reduce-scatter GEMM over two epochs of both its workspaces, with N
+    that ends inside a tile."""
+    from flagcx_b200.parallel.tp import TensorParallelContext
+    lib, comm = comm1
+    ext = ctypes.CDLL(nat.__file__)
+    ext.fcxGemmTileCostCut.restype = ctypes.c_double
+    bn = ctypes.c_int(0)
+    ext.fcxGemmTileCostCut(M, N, K, torch.cuda.get_device_properties(0).multi_processor_count - 4, 1, ctypes.byref(bn))
+    assert bn.value == width
+    tp = TensorParallelContext(comm.value, 1, 0, max_rows=M, max_k=K, max_n=N, comm_ctas=4)
+    tp.exchange = True
+    torch.manual_seed(M)
+    for rep in range(4):
+        x = torch.randn(M, K, device="cuda").bfloat16()
+        w = torch.randn(N, K, device="cuda").bfloat16()
+        y, z = tp.ag_gemm(x, w), tp.gemm_rs(x, w)
+        torch.cuda.synchronize()
+        tp.check()
+        ref = x.double() @ w.double().t()
+        # fp32 sums of K products and one rounding to bf16 (the staged tile of one rank is rounded already)
+        bound = 2.0 ** -8 * ref.abs() + K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())
+        for got in (y, z):
+            assert float(((got.double() - ref).abs() / bound).max()) <= 1.0, rep
+        full = tp.last_gathered(x)
+        assert torch.equal(full, x)
+    tiles = -(-N // 256)
+    assert tp.rs_counters[0][: M // 128 * tiles].tolist() == [2] * (M // 128 * tiles)  # one arrival per tile, epoch and rank
+
+
+@pytest.mark.parametrize("exchange", [False, True])
+def test_tensor_parallel_linears_forward_and_backward(nat, comm1, exchange):
     """Autograd wrappers of the fused kernels against plain PyTorch autograd (one rank: gather and scatter are identities)."""
     from flagcx_b200.parallel.tp import TensorParallelContext, column_parallel_linear, row_parallel_linear
     lib, comm = comm1
     tp = TensorParallelContext(comm.value, 1, 0, max_rows=512, max_k=1024, max_n=1024)
+    tp.exchange = exchange
     torch.manual_seed(5)
     x = (torch.randn(512, 256, device="cuda") * 0.5).bfloat16().requires_grad_()
     w1 = (torch.randn(1024, 256, device="cuda") * 0.05).bfloat16().requires_grad_()
