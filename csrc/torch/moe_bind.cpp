@@ -24,7 +24,7 @@ static void checkBf16Mat(const at::Tensor &t, const char *name) {
 // Route this rank's tokens to their experts.  All heap tensors belong to one buffer set; epoch is that set's 1-based use count.
 static void moeDispatch(uint64_t comm, const at::Tensor &x, const at::Tensor &topkIdx, at::Tensor &countMat, at::Tensor &countFlags,
                         at::Tensor &recv, at::Tensor &info, at::Tensor &done, int64_t epoch, at::Tensor &slot, at::Tensor &localCounts,
-                        at::Tensor &recvTotal, at::Tensor &err, int64_t ctas, int64_t expertsPerRank) {
+                        at::Tensor &recvTotal, at::Tensor &err, int64_t ctas, int64_t expertsPerRank, bool exchange) {
   checkBf16Mat(x, "x");
   TORCH_CHECK(x.is_contiguous() && topkIdx.is_contiguous() && topkIdx.scalar_type() == at::kInt && topkIdx.dim() == 2, "topk_idx must be int32 [T, K]");
   TORCH_CHECK(topkIdx.size(0) == x.size(0), "topk_idx and x disagree on the token count");
@@ -49,6 +49,7 @@ static void moeDispatch(uint64_t comm, const at::Tensor &x, const at::Tensor &to
   p.infoOff = heapOffset(comm, info);
   p.doneOff = heapOffset(comm, done);
   p.epoch = (uint64_t)epoch;
+  p.exchange = exchange ? 1 : 0;
   p.slot = slot.data_ptr<int>();
   p.localCounts = localCounts.data_ptr<int>();
   p.recvTotal = recvTotal.data_ptr<int>();
@@ -144,7 +145,7 @@ static void moeCombine(uint64_t comm, const at::Tensor &combine, const at::Tenso
 void bindMoe(py::module &m) {
   m.def("moe_dispatch", &moeDispatch, py::arg("comm"), py::arg("x"), py::arg("topk_idx"), py::arg("count_mat"), py::arg("count_flags"),
         py::arg("recv"), py::arg("info"), py::arg("done"), py::arg("epoch"), py::arg("slot"), py::arg("local_counts"), py::arg("recv_total"),
-        py::arg("err"), py::arg("ctas"), py::arg("experts_per_rank") = 1);
+        py::arg("err"), py::arg("ctas"), py::arg("experts_per_rank") = 1, py::arg("exchange") = false);
   m.def("silu_mul", &siluMul, py::arg("gu"), py::arg("h"), py::arg("rows") = py::none());
   m.def("gemm_dyn_m", &gemmDynM);
   m.def("moe_up", &moeUp);

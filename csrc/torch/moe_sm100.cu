@@ -39,6 +39,7 @@ constexpr int THREADS = 512;
 __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm dc, const FcxMoeParams p) {
   cg::grid_group grid = cg::this_grid();
   const int n = dc.nranks, me = dc.rank, L = p.L, E = n * L, capL = p.cap / L;
+  const bool talk = n > 1 || p.exchange;
   const int entries = p.T * p.K;
   __shared__ int warpTotals[THREADS / 32];
   volatile int *err = p.errFlag;
@@ -78,8 +79,8 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
 
   // ---- phase 2: every rank learns the whole count matrix [source][expert].  One rank alone has it already: no message, no
   // flag to wait for, and at the end nobody to tell (each of them costs a trip to memory and back, and the last a barrier
-  // of the whole grid).
-  if (n > 1 && blockIdx.x == 0 && (int)threadIdx.x < n) {
+  // of the whole grid), unless the caller asks for it all the same.
+  if (talk && blockIdx.x == 0 && (int)threadIdx.x < n) {
     const int r = threadIdx.x;
     int *mat = (int *)(dc.heap[r] + p.countMatOff) + me * E;
     for (int e = 0; e < E; e++) mat[e] = p.localCounts[e];
@@ -89,11 +90,11 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
   __shared__ int baseOf[64];  // where this rank's tokens start in expert e's segment
   {
     bool ok = true;
-    if (n > 1 && (int)threadIdx.x < n)
+    if (talk && (int)threadIdx.x < n)
       ok = fcxdev::waitGe(dc, (const uint64_t *)(dc.heap[me] + p.countFlagOff) + threadIdx.x, p.epoch, threadIdx.x, FCX_WAIT_DEVAPI,
                           blockIdx.x, p.epoch);
     if (!__syncthreads_and(ok)) { if (threadIdx.x == 0) *err = 1; }
-    const int *mat = n > 1 ? (const int *)(dc.heap[me] + p.countMatOff) : p.localCounts;
+    const int *mat = talk ? (const int *)(dc.heap[me] + p.countMatOff) : p.localCounts;
     if ((int)threadIdx.x < E) {
       int b = 0, tot = 0;
       for (int r = 0; r < n; r++) {
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
       }
       baseOf[threadIdx.x] = b;
       if (tot > capL && blockIdx.x == 0) *err = 2;  // an expert's segment would overflow: tokens beyond the capacity are dropped
-      if (n == 1 && blockIdx.x == 0) p.recvTotal[threadIdx.x] = min(tot, capL);
+      if (!talk && blockIdx.x == 0) p.recvTotal[threadIdx.x] = min(tot, capL);
     }
     __syncthreads();
   }
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
       if (lane == 0) ((int4 *)(dc.heap[dstRank] + p.infoOff))[pos] = make_int4(me, t, k, 0);
     }
   }
-  if (n == 1) return;
+  if (!talk) return;
   __threadfence_system();
   grid.sync();
 

@@ -19,6 +19,7 @@ struct FcxMoeParams {
   size_t infoOff;       // int4 [cap]: (source rank, token, choice, 0) of every row
   size_t doneOff;       // u64 [nranks]: source s has finished pushing (value = epoch)
   uint64_t epoch;       // 1-based use count of this buffer set
+  int exchange;         // one rank: exchange counts and arrivals with itself all the same, as several ranks do
   int *slot;            // local scratch int32 [T*K]
   int *localCounts;     // local scratch int32 [nranks * L]
   int *recvTotal;       // out, device int32 [L]: rows received by each of this rank's experts

@@ -84,6 +84,7 @@ class ExpertParallelContext:
         self.h = torch.empty(self.cap, ffn, dtype=bf, device=dev)
         self.calls = 0
         self.comb_want = [0, 0]
+        self.exchange = nranks > 1  # one rank skips the exchange of counts and arrivals; set it, and it has them with itself
         torch.cuda.synchronize()
         if nranks > 1:  # nobody may write into a workspace that its owner has not cleared yet
             t = torch.zeros(1, device=dev)
@@ -104,7 +105,7 @@ class ExpertParallelContext:
         assert len(w_gate_up) == self.L and len(w_down) == self.L, "one weight pair per local expert"
         nat.moe_dispatch(self.comm, x, topk_idx, self.count_mat[par], self.count_flags[par], self.recv[par], self.info[par],
                          self.disp_done[par], epoch, self.slot, self.local_counts, self.recv_total, self.err, self.dispatch_ctas,
-                         self.L)
+                         self.L, self.exchange)
         # every local expert works on its own segment, sized on the device by its row count; all of them share a launch
         nat.moe_up(self.recv[par], [w_gate_up[l] for l in range(self.L)], self.h, self.recv_total, self.err)
         grid = nat.moe_down(self.comm, self.h, [w_down[l] for l in range(self.L)], self.recv_total, self.info[par], self.combine[par],

@@ -208,8 +208,8 @@ def main():
                           "fraction_of_gemm_peak": round(tf / tf_peak, 3), "peak": label, "err": int(err.item())}))
         return
     elif args.case in ("moe_dispatch", "moe_layer"):
-        # one-rank communicator: the dispatch kernel (count, exchange, push), the device-row-count GEMMs,
-        # the row-scattering epilogue and the combine kernel all run, with this GPU as its own peer
+        # one-rank communicator: dispatch, grouped expert GEMMs with the row-scattering epilogue, combine; the dispatch
+        # exchanges counts and arrivals as several ranks do (one rank skips that otherwise), with this GPU as its own peer
         import os
         os.environ.setdefault("FLAGCX_HEAP_USER_BYTES", "1G")
         from flagcx_b200.parallel.ep import ExpertParallelContext
@@ -218,6 +218,7 @@ def main():
         comm = lib.flagcxCommInitRank(1, lib.flagcxGetUniqueId(), 0)
         T, H, F, K = 8192, 4096, 2048, 2
         ep = ExpertParallelContext(comm.value, 1, 0, T, H, F, K)
+        ep.exchange = True
         x = torch.randn(T, H, device="cuda").bfloat16()
         idx = torch.zeros(T, K, dtype=torch.int32, device="cuda")
         wts = torch.rand(T, K, device="cuda")
@@ -230,7 +231,7 @@ def main():
                 par, epoch = state["calls"] & 1, (state["calls"] >> 1) + 1
                 state["calls"] += 1
                 nat.moe_dispatch(comm.value, x, idx, ep.count_mat[par], ep.count_flags[par], ep.recv[par], ep.info[par], ep.disp_done[par],
-                                 epoch, ep.slot, ep.local_counts, ep.recv_total, ep.err, ep.dispatch_ctas)
+                                 epoch, ep.slot, ep.local_counts, ep.recv_total, ep.err, ep.dispatch_ctas, 1, True)
             ms = timed(disp)
             nbytes = T * K * H * 2 * 2  # every (token, choice) row read once and written once
         else:

@@ -117,13 +117,16 @@ def test_grouped_expert_gemms(nat, comm1, L, cap, H, F):
 
 
 @pytest.mark.parametrize("entries,experts,H", [((1, 1), 2, 264), ((513, 2), 5, 1024), ((300, 4), 8, 2056), ((130, 3), 4, 128)])
-def test_dispatch_and_combine_edges(nat, comm1, entries, experts, H):
-    """Token counts that end inside a warp's stretch of the numbering, and 1, 2, 3 and 4 choices in the combine."""
+@pytest.mark.parametrize("exchange", [False, True])
+def test_dispatch_and_combine_edges(nat, comm1, entries, experts, H, exchange):
+    """Token counts that end inside a warp's stretch of the numbering, 1, 2, 3 and 4 choices in the combine, and the dispatch
+    both as one rank runs it and with the exchange of counts and arrivals of several ranks, this GPU being its own peer."""
     from flagcx_b200.parallel.ep import ExpertParallelContext, moe_reference
     T, K = entries
     F = 128
     torch.manual_seed(T)
     ep = ExpertParallelContext(comm1.value, 1, 0, T, H, F, K, dispatch_ctas=8, experts_per_rank=experts, capacity_factor=float(experts))
+    ep.exchange = exchange
     idx = torch.stack([torch.randperm(experts, device="cuda")[:K] for _ in range(T)]).int().contiguous()
     w = torch.rand(T, K, device="cuda")
     up = [_bf(2 * F, H, scale=0.05) for _ in range(experts)]
@@ -137,6 +140,10 @@ def test_dispatch_and_combine_edges(nat, comm1, entries, experts, H):
         ref = moe_reference(x, idx, w, up, down)
         # bf16 roundings of the gate / up products (reference), of h, of y and of the result: four of 2^-9 in quadrature
         assert float((out.float() - ref).norm() / ref.norm()) < 4 * 2.0 ** -9
+    # the calls alternate between two buffer sets: epochs 1 and 2 of the first, 1 of the second
+    assert [int(f[0].item()) for f in ep.count_flags + ep.disp_done] == ([2, 1, 2, 1] if exchange else [0] * 4)
+    if exchange:
+        assert ep.count_mat[0].tolist() == [int((idx == e).sum().item()) for e in range(experts)]
 
 
 @pytest.mark.parametrize("M,C", [(1, 256), (1185, 1024), (1184 * 4 + 3, 768), (9, 512)])
