@@ -417,8 +417,7 @@ __device__ __forceinline__ uint32_t pack4Fp8(float a, float b, float c, float d)
 // per block, 16-byte loads; 4: a warp per block, for rows that are only 8-byte aligned) of UNROLL blocks whose loads are
 // all issued before the first is used: one 8-byte load in flight per lane left the kernel waiting (2.1 TB/s).
 template <int VEC, int UNROLL>
-__global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *__restrict__ x, __nv_fp8_storage_t *__restrict__ q,
-                                                      float *__restrict__ sa, int M, int K, int ldx) {
+__global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *x, __nv_fp8_storage_t *q, float *sa, int M, int K, int ldx) {
   constexpr int LANES = 128 / VEC, PER_CTA = 256 / LANES;  // lanes per block, blocks per CTA and step
   const uint32_t nKb = K / 128;
   const uint64_t total = (uint64_t)M * nKb;

@@ -185,9 +185,8 @@ __global__ void __launch_bounds__(256) siluMulKernel(const __nv_bfloat16 *__rest
 // used, eight 16-byte loads in flight; positions in 32 bits (their 64-bit divisions cost more than the loads).
 // KC = 0: any K and any size, one vector at a time.
 template <int KC>
-__global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, const __nv_bfloat16 *__restrict__ ret, const float *__restrict__ w,
-                                                        __nv_bfloat16 *__restrict__ out, int T, int H, int K, size_t doneOff, uint64_t want,
-                                                        int *errFlag) {
+__global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, const __nv_bfloat16 *ret, const float *w, __nv_bfloat16 *out, int T,
+                                                        int H, int K, size_t doneOff, uint64_t want, int *errFlag) {
   bool ok = true;
   fcxpdl::pdlWait();
   if (threadIdx.x == 0) {

@@ -3,6 +3,10 @@
 // has finished and its writes are visible.  A kernel launched with launchPdl calls pdlWait() before its first access to
 // global memory, reads and writes alike; behind anything but a kernel that calls pdlRelease() the wait is an ordinary
 // stream dependency.
+//
+// The pointer parameters of such a kernel carry no __restrict__: what they point to may still be written, by the kernel
+// before, while this one is resident.  For a `const ... __restrict__` pointer the compiler may use the non-coherent load
+// path, which is for memory that nobody writes while the kernel lives, and may move a load across the wait.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -75,11 +75,8 @@ template <int N>
 __device__ __forceinline__ void cpAsyncWait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <int MAXV, int STAGES, int LN_WARPS>
-__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnFwdKernel(const bf16 *__restrict__ x, const bf16 *__restrict__ delta,
-                                                                const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
-                                                                bf16 *__restrict__ resOut, bf16 *__restrict__ y,
-                                                                float *__restrict__ mean, float *__restrict__ rstd, int M, int C,
-                                                                float eps) {
+__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnFwdKernel(const bf16 *x, const bf16 *delta, const bf16 *gamma, const bf16 *beta,
+                                                                bf16 *resOut, bf16 *y, float *mean, float *rstd, int M, int C, float eps) {
   extern __shared__ __align__(16) uint8_t lnSmem[];
   const int warpInCta = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warp = blockIdx.x * LN_WARPS + warpInCta, nwarps = gridDim.x * LN_WARPS;
@@ -157,10 +154,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnFwdKernel(const bf16 *__re
 // Same streaming scheme for dy and x; the residual gradient, needed only for the last step of a row, is loaded into
 // registers when the row's turn begins.
 template <int MAXV, int STAGES, int LN_WARPS>
-__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdDxKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
-                                                                  const bf16 *__restrict__ gamma, const float *__restrict__ mean,
-                                                                  const float *__restrict__ rstd, const bf16 *__restrict__ dres,
-                                                                  bf16 *__restrict__ dx, int M, int C) {
+__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdDxKernel(const bf16 *dy, const bf16 *x, const bf16 *gamma, const float *mean,
+                                                                  const float *rstd, const bf16 *dres, bf16 *dx, int M, int C) {
   extern __shared__ __align__(16) uint8_t lnSmem[];
   const int warpInCta = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warp = blockIdx.x * LN_WARPS + warpInCta, nwarps = gridDim.x * LN_WARPS;
@@ -242,10 +237,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdDxKernel(const bf16 *__
 // registers the arithmetic set the pace: 19 us at 8192 x 1024).  At the end the warps fold their sums in shared memory and
 // a CTA leaves [2][C] of them in `partial` for lnParamFoldKernel.
 template <int MAXV, int STAGES, int LN_WARPS>
-__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdFusedKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
-                                                                     const bf16 *__restrict__ gamma, const float *__restrict__ mean,
-                                                                     const float *__restrict__ rstd, const bf16 *__restrict__ dres,
-                                                                     bf16 *__restrict__ dx, float *__restrict__ partial, int M, int C) {
+__global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdFusedKernel(const bf16 *dy, const bf16 *x, const bf16 *gamma, const float *mean,
+                                                                     const float *rstd, const bf16 *dres, bf16 *dx, float *partial, int M, int C) {
   extern __shared__ __align__(16) uint8_t lnSmem[];
   const int warpInCta = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warp = blockIdx.x * LN_WARPS + warpInCta, nwarps = gridDim.x * LN_WARPS;
@@ -342,8 +335,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdFusedKernel(const bf16 
 
 // dgamma / dbeta from the `parts` partial sums of lnBwdFusedKernel: a CTA folds 32 of the 2 C columns, eight groups of
 // lanes an eighth of the parts each.
-__global__ void __launch_bounds__(256) lnParamFoldKernel(const float *__restrict__ partial, int parts, int C, bf16 *__restrict__ dgamma,
-                                                         bf16 *__restrict__ dbeta, int accumulate) {
+__global__ void __launch_bounds__(256) lnParamFoldKernel(const float *partial, int parts, int C, bf16 *dgamma, bf16 *dbeta, int accumulate) {
   __shared__ float red[8][33];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // 2 C is a multiple of 32
   fcxpdl::pdlRelease();
@@ -366,10 +358,8 @@ __global__ void __launch_bounds__(256) lnParamFoldKernel(const float *__restrict
 // Backward, part 2, for rows wider than 1024: dgamma[c] = sum_r dy[r,c] * xhat[r,c], dbeta[c] = sum_r dy[r,c].
 // A CTA owns 64 columns and one slice of the rows; partial sums go to
 // `partial` ([gridDim.y][2][C], fp32 scratch); the CTA that finishes a column block last folds them into dgamma / dbeta.
-__global__ void __launch_bounds__(256) lnBwdParamKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
-                                                        const float *__restrict__ mean, const float *__restrict__ rstd,
-                                                        float *__restrict__ partial, int M, int C, bf16 *__restrict__ dgamma,
-                                                        bf16 *__restrict__ dbeta, int accumulate) {
+__global__ void __launch_bounds__(256) lnBwdParamKernel(const bf16 *dy, const bf16 *x, const float *mean, const float *rstd, float *partial,
+                                                        int M, int C, bf16 *dgamma, bf16 *dbeta, int accumulate) {
   __shared__ float redG[32][64 + 1], redB[32][64 + 1];
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
@@ -469,8 +459,7 @@ __device__ __forceinline__ float geluGrad(float x) {
 }
 
 // y = gelu(x + bias); x is [M, C].  Each thread keeps four 16-byte loads in flight.
-__global__ void __launch_bounds__(256) biasGeluFwdKernel(const bf16 *__restrict__ x, const bf16 *__restrict__ bias,
-                                                         bf16 *__restrict__ y, size_t nvec, int C) {
+__global__ void __launch_bounds__(256) biasGeluFwdKernel(const bf16 *x, const bf16 *bias, bf16 *y, size_t nvec, int C) {
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
   const int cv = C / 8;
@@ -505,9 +494,8 @@ __global__ void __launch_bounds__(256) biasGeluFwdKernel(const bf16 *__restrict_
 // group of 256 / VX rows, four rows (eight 16-byte loads) in flight per thread; a thread keeps its eight columns throughout.
 // Bound by memory (dy, x, dx: 201 MB and 30 us at 8192 x 4096) with the arithmetic close behind.  Blocks of 64 columns with a
 // fold in the last CTA, as in the plain column sum, took 55 us: their CTAs lived for eight rows per thread.
-__global__ void __launch_bounds__(256) biasGeluBwdKernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x,
-                                                         const bf16 *__restrict__ bias, bf16 *__restrict__ dx, float *__restrict__ partial,
-                                                         int M, int C, int VX) {
+__global__ void __launch_bounds__(256) biasGeluBwdKernel(const bf16 *dy, const bf16 *x, const bf16 *bias, bf16 *dx, float *partial, int M, int C,
+                                                         int VX) {
   __shared__ float red[2048];
   const int tx = threadIdx.x % VX, ty = threadIdx.x / VX, RY = 256 / VX;
   const int col = (blockIdx.x * VX + tx) * 8;
@@ -556,7 +544,7 @@ __global__ void __launch_bounds__(256) biasGeluBwdKernel(const bf16 *__restrict_
 }
 
 // out[c] (+)= the sum of `parts` partial column sums; a CTA folds 32 columns, eight groups of lanes an eighth of the parts each.
-__global__ void __launch_bounds__(256) colSumFoldKernel(const float *__restrict__ partial, int parts, int C, bf16 *__restrict__ out, int accumulate) {
+__global__ void __launch_bounds__(256) colSumFoldKernel(const float *partial, int parts, int C, bf16 *out, int accumulate) {
   __shared__ float red[8][33];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // C is a multiple of 64
   fcxpdl::pdlRelease();
@@ -628,8 +616,7 @@ __global__ void colSumReduceKernel(const float *__restrict__ partial, int nparts
 // after the partial sums are visible) folds the block's partial sums and writes the result.  The tickets live in the
 // library image and return to zero by themselves; concurrent calls on one device would share them, so calls must be
 // stream-ordered (they are: the backward pass runs on one stream).
-__global__ void __launch_bounds__(256) colSumFusedKernel(const bf16 *__restrict__ a, float *__restrict__ partial, bf16 *__restrict__ out,
-                                                         int M, int C, int accumulate) {
+__global__ void __launch_bounds__(256) colSumFusedKernel(const bf16 *a, float *partial, bf16 *out, int M, int C, int accumulate) {
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
   const int col0 = blockIdx.x * 64;
@@ -762,8 +749,7 @@ __global__ void __launch_bounds__(1024) ceFwdBwdKernel(bf16 *__restrict__ logits
 // row a CTA works on lies in shared memory, and the next row streams in with cp.async during the three passes over the
 // current one, so the logits are read from DRAM exactly once and the reads never wait for the arithmetic.  A thread
 // copies exactly the vectors it reads itself, so the only synchronisation of the ring is cp.async.wait_group.
-__global__ void __launch_bounds__(1024, 1) ceFwdBwdStreamKernel(bf16 *__restrict__ logits, const int64_t *__restrict__ targets,
-                                                                float *__restrict__ losses, int M, int V, int Vpad,
+__global__ void __launch_bounds__(1024, 1) ceFwdBwdStreamKernel(bf16 *logits, const int64_t *targets, float *losses, int M, int V, int Vpad,
                                                                 float gradScale) {
   extern __shared__ __align__(16) uint8_t ceSmem[];
   __shared__ float red[2][32];
@@ -877,10 +863,9 @@ __global__ void __launch_bounds__(1024, 1) ceFwdBwdStreamKernel(bf16 *__restrict
 // ---------------------------------------------------------------- AdamW on flat buffers
 // master (fp32) is the truth; param (bf16) is refreshed from it.  The gradient
 // is read once and cleared, so no separate zero_grad pass is needed.
-__global__ void __launch_bounds__(256) adamwKernel(float *__restrict__ master, bf16 *__restrict__ param, bf16 *__restrict__ grad,
-                                                   float *__restrict__ m, float *__restrict__ v, size_t n, float lr, float b1,
-                                                   float b2, float eps, float wd, float bc1, float bc2, float gradScale,
-                                                   int zeroGrad, const int *__restrict__ stepDev) {
+__global__ void __launch_bounds__(256) adamwKernel(float *master, bf16 *param, bf16 *grad, float *m, float *v, size_t n, float lr, float b1,
+                                                   float b2, float eps, float wd, float bc1, float bc2, float gradScale, int zeroGrad,
+                                                   const int *stepDev) {
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
   if (stepDev) {
