@@ -28,6 +28,7 @@
 #include <stdint.h>
 #include <vector>
 
+#include "device_state.h"
 #include "gemm_sm100.h"
 #include "gemm_units.h"
 #include "pdl.cuh"
@@ -350,38 +351,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(512) : "memory");
 }
 
-int smCount2() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 }  // namespace
 
 // 0 = never, 1 = when the shape suits (default), 2 = whenever the kernel can take the shape.
 extern "C" int fcxGemmPairMode() {
-  static int mode = -1;
-  if (mode < 0) {
+  static const int mode = [] {
     const char *e = getenv("FLAGCX_GEMM_2SM");
-    mode = e ? std::max(0, std::min(2, atoi(e))) : 1;
-  }
+    return e ? std::max(0, std::min(2, atoi(e))) : 1;
+  }();
   return mode;
 }
 
 // Whether the pair kernel is the better choice for this shape: by the waves of tiles that either kernel needs, times what
 // a K block of its tile costs; the pair kernel has to win clearly, since half-empty pair tiles waste both SMs.
 // `cut`: the pieces of K that the launch asks for (0: the launcher's own choice, 1: K stays whole).
-extern "C" int fcxGemmPairSuitsCut(int M, int N, int K, int cut) {
+// `bn`: the tile width of the one-CTA kernel, for when it is that.
+extern "C" int fcxGemmChoose(int M, int N, int K, int sms, int cut, int *bn) {
+  const double tile = fcxGemmTileCostCut(M, N, K, sms, cut, bn);
   const int mode = fcxGemmPairMode();
   if (mode == 0 || M < 129 || K < 8) return 0;
-  if (mode == 2) return 1;
-  return fcxGemmPairCostCut(M, N, K, smCount2() / 2, cut) <= 0.85 * fcxGemmTileCostCut(M, N, K, smCount2(), cut, nullptr);
+  return mode == 2 || fcxGemmPairCostCut(M, N, K, sms / 2, cut) <= 0.85 * tile;
 }
+extern "C" int fcxGemmPairSuitsCut(int M, int N, int K, int cut) { return fcxGemmChoose(M, N, K, fcxhost::smCount(), cut, nullptr); }
 extern "C" int fcxGemmPairSuits(int M, int N, int K) { return fcxGemmPairSuitsCut(M, N, K, 0); }
 
 static bool fillProb(PairProb *p, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN, int group,
@@ -402,12 +393,9 @@ static bool fillProb(PairProb *p, const void *a, const void *b, void *c, int M, 
 
 template <int MODE>
 static cudaError_t launchPair(const PairArgs &args, int pairs, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(fcxGemmPairKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static fcxhost::OncePerDevice once;
+  const cudaError_t e = once([] { return cudaFuncSetAttribute(fcxGemmPairKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+  if (e != cudaSuccess) return e;
   return fcxpdl::launchPdl(fcxGemmPairKernel<MODE>, 2 * pairs, THREADS, SMEM_BYTES, s, args);
 }
 
@@ -423,8 +411,8 @@ extern "C" cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, in
     splitK = 1;  // the activation needs the whole sum
   }
   PairProb &p = args.prob[0];
-  const int pairs = smCount2() / 2;
-  p.splitK = fcxGemmPieces(splitK, M, N, K, p.units, pairs, smCount2());
+  const int sms = fcxhost::smCount(), pairs = sms / 2;
+  p.splitK = fcxGemmPieces(splitK, M, N, K, p.units, pairs, sms);
   p.units *= p.splitK;
   p.accumulate = accumulate;
   args.bias = bias;
@@ -496,20 +484,19 @@ extern "C" int fcxGemmUnitsCovered(int workers, int n0, int n1, int extra, int l
   return 1;
 }
 
-// dx[T,I] = dy[T,O] w[O,I] and dw[O,I] (+)= dy^T x in one launch.  Returns cudaErrorNotSupported when the pair kernel is not
-// the better one for both products: the caller then launches them one by one.
+// dx[T,I] = dy[T,O] w[O,I] and dw[O,I] (+)= dy^T x in one launch, for products that both suit the pair kernel.  Returns
+// cudaErrorNotSupported when two launches would be done sooner.
 extern "C" cudaError_t fcxGemmBackwardPair(const void *dy, const void *w, const void *x, void *dx, void *dw, int T, int I, int O, int lddy, int ldw,
                                            int ldx, int accumulate, int groupX, int groupW, int *errFlag, cudaStream_t s) {
-  if (!fcxGemmPairSuits(T, I, O) || !fcxGemmPairSuits(O, I, T)) return cudaErrorNotSupported;
   PairArgs args{};
   PairProb px{}, pw{};
   if (!fillProb(&px, dy, w, dx, T, I, O, lddy, ldw, I, 0, 1, groupX, nullptr, 0) ||
       !fillProb(&pw, dy, x, dw, O, I, T, lddy, ldx, I, 1, 1, groupW, nullptr, 0))
     return cudaErrorNotSupported;
-  const int nKx = (O + BK - 1) / BK, nKw = (T + BK - 1) / BK, pairs = smCount2() / 2;
+  const int nKx = (O + BK - 1) / BK, nKw = (T + BK - 1) / BK, sms = fcxhost::smCount(), pairs = sms / 2;
   int swap = 0;
-  if (!fcxGemmDualPlan(pw.units, nKw, fcxGemmPieces(0, O, I, T, pw.units, pairs, smCount2()), px.units, nKx,
-                       fcxGemmPieces(0, T, I, O, px.units, pairs, smCount2()), pairs, &pw.splitK, &px.splitK, &swap, &args.extra))
+  if (!fcxGemmDualPlan(pw.units, nKw, fcxGemmPieces(0, O, I, T, pw.units, pairs, sms), px.units, nKx,
+                       fcxGemmPieces(0, T, I, O, px.units, pairs, sms), pairs, &pw.splitK, &px.splitK, &swap, &args.extra))
     return cudaErrorNotSupported;
   pw.accumulate = accumulate;
   for (PairProb *p : {&px, &pw}) {

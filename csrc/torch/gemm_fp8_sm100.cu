@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_state.h"
 #include "gemm_fp8_sm100.h"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
@@ -526,16 +527,7 @@ __global__ void __launch_bounds__(256) quantWeightKernel(const __nv_bfloat16 *__
   }
 }
 
-int smCount() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
+using fcxhost::smCount;
 
 }  // namespace
 
@@ -545,12 +537,9 @@ template <int BN>
 cudaError_t launchOne(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
   CUtensorMap mb;
   if (!makeTileMap(&mb, bq, p.N, p.K, p.K, BN, 1)) return cudaErrorNotSupported;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(gemmFp8Kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(BN));
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static fcxhost::OncePerDevice once;
+  const cudaError_t e = once([] { return cudaFuncSetAttribute(gemmFp8Kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(BN)); });
+  if (e != cudaSuccess) return e;
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   return fcxpdl::launchPdl(gemmFp8Kernel<BN>, std::min(tiles, smCount()), THREADS, smemBytes(BN), s, ma, mb, mc, p);
 }
@@ -558,12 +547,9 @@ cudaError_t launchOne(const CUtensorMap &ma, const void *bq, const CUtensorMap &
 cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
   CUtensorMap mb;
   if (!makeTileMap(&mb, bq, p.N, p.K, p.K, PNH, 1)) return cudaErrorNotSupported;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(gemmFp8PairKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static fcxhost::OncePerDevice once;
+  const cudaError_t e = once([] { return cudaFuncSetAttribute(gemmFp8PairKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM_BYTES); });
+  if (e != cudaSuccess) return e;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + PN - 1) / PN);
   return fcxpdl::launchPdl(gemmFp8PairKernel, 2 * std::min(tiles, smCount() / 2), PTHREADS, PSMEM_BYTES, s, ma, mb, mc, p);
 }

@@ -43,6 +43,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_state.h"
 #include "gemm_sm100.h"
 #include "gemm_units.h"
 #include "pdl.cuh"
@@ -441,12 +442,9 @@ bool makeMap(CUtensorMap *m, const void *base, uint64_t rows, uint64_t cols, uin
 template <int MODE>
 cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, const FcxGemmParams &p, const FcxDevComm &dc, int grid, cudaStream_t s,
                    const CUtensorMap *aLocal = nullptr, const SecondProduct *second = nullptr) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(fcxGemmKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static fcxhost::OncePerDevice once;
+  const cudaError_t e = once([] { return cudaFuncSetAttribute(fcxGemmKernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+  if (e != cudaSuccess) return e;
   SecondProduct none{};
   const CUtensorMap &al = aLocal ? *aLocal : a;
   const SecondProduct &q = second ? *second : none;
@@ -458,39 +456,38 @@ cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, const FcxGemmPara
 
 // Row blocks per band of the tile order (FLAGCX_GEMM_TILE_GROUP; 0 = plain row-major order).
 int tileGroup(int nN) {
-  static int g = -2;
-  if (g == -2) {
+  static const int g = [] {
     const char *e = getenv("FLAGCX_GEMM_TILE_GROUP");
-    g = e ? std::max(0, atoi(e)) : -1;
-  }
+    return e ? std::max(0, atoi(e)) : -1;
+  }();
   return g >= 0 ? g : (nN >= 24 ? 16 : 8);  // wide outputs: taller bands keep more of B in L2 per wave
 }
 
-// Columns per tile of the one-CTA kernel: the choice of fcxGemmTileCostCut, or FLAGCX_GEMM_BN (64, 128, 256) for experiments.
-// `cut`: the pieces that the caller will ask fcxGemmPickSplitK for (1: K stays whole).
-int pickBn(int M, int N, int K, int sms, int cut) {
-  static int forced = -1;
-  if (forced < 0) {
+// FLAGCX_GEMM_BN (64, 128, 256): columns per tile of the one-CTA kernel, for experiments.
+int forcedBn() {
+  static const int forced = [] {
     const char *e = getenv("FLAGCX_GEMM_BN");
     const int v = e ? atoi(e) : 0;
-    forced = v == 64 || v == 128 || v == 256 ? v : 0;
-  }
-  if (forced) return forced;
-  int bn = 256;
-  fcxGemmTileCostCut(M, N, K, sms, cut, &bn);
-  return bn;
+    return v == 64 || v == 128 || v == 256 ? v : 0;
+  }();
+  return forced;
 }
 
-int smCount() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
+// Columns per tile of the one-CTA kernel.  `cut`: the pieces that the caller will ask fcxGemmPickSplitK for (1: K stays whole).
+int pickBn(int M, int N, int K, int sms, int cut) {
+  int bn = 256;
+  if (!forcedBn()) fcxGemmTileCostCut(M, N, K, sms, cut, &bn);
+  return forcedBn() ? forcedBn() : bn;
 }
+
+// The same choice together with that of the kernel: whether CTA pairs are the better one.
+bool choose(int M, int N, int K, int sms, int cut, int *bn) {
+  const bool pair = fcxGemmChoose(M, N, K, sms, cut, bn) != 0;
+  if (forcedBn()) *bn = forcedBn();
+  return pair;
+}
+
+using fcxhost::smCount;
 
 }  // namespace
 
@@ -543,7 +540,7 @@ extern "C" int fcxGemmPickSplitK(int requested, int units, int slots, int nK, in
 // 288 x 3392 x 3832 would be cut in 5 in place of 3.)
 extern "C" int fcxGemmPieces(int requested, int M, int N, int K, int units, int slots, int sms) {
   const int nK = (K + BK - 1) / BK, pieces = fcxGemmPickSplitK(requested, units, slots, nK, N);
-  if (requested > 0) return pieces;
+  if (requested > 0 || pieces == 1) return pieces;
   const int nN = (N + BN - 1) / BN, pairRows = (M + 2 * BM - 1) / (2 * BM);
   const bool fills = M > BM && N >= 192 && pairRows * 2 * BM <= 1.07 * M;
   const int most = fills ? fcxGemmPickSplitK(0, pairRows * nN, sms / 2, nK, N) : fcxGemmPickSplitK(0, (M + BM - 1) / BM * nN, sms, nK, N);
@@ -600,11 +597,13 @@ extern "C" cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, in
   if ((aMN && M % 8) || (bMN && N % 8) || (bias && ((uintptr_t)bias & 1)) || (accumulate && N % 2)) return cudaErrorInvalidValue;
   gGemmDetail[0] = 0;
   cudaGetLastError();  // an error left behind by an earlier, unrelated call of this thread is not this launch's
-  if (o->geluOut || (o->pair >= 0 ? o->pair > 0 : fcxGemmPairSuitsCut(M, N, K, splitK) != 0))  // CTA pairs on 256 x 256 tiles (gemm2_sm100.cu)
+  const int sms = smCount();
+  int bn = 256;
+  const bool pair = choose(M, N, K, sms, splitK, &bn);
+  if (o->geluOut || (o->pair >= 0 ? o->pair > 0 : pair))  // CTA pairs on 256 x 256 tiles (gemm2_sm100.cu)
     return fcxGemmPairBf16(a, b, c, M, N, K, lda, ldb, ldc, aMN, bMN, bias, splitK, accumulate, o->geluOut, tileGroup((N + 255) / 256) / 2,
                            errFlag, s, gGemmDetail, sizeof gGemmDetail);
   CUtensorMap ma, mb;
-  const int bn = pickBn(M, N, K, smCount(), splitK);
   // K-major operand: rows = M (or N), box of 128 (bn) rows x 64 K; MN-major operand: rows = K, box of 64 lines x 64 columns
   const bool okA = aMN ? makeMap(&ma, a, K, M, lda, BK) : makeMap(&ma, a, M, K, lda, BM);
   const bool okB = bMN ? makeMap(&mb, b, K, N, ldb, BK) : makeMap(&mb, b, N, K, ldb, bn);
@@ -617,16 +616,16 @@ extern "C" cudaError_t fcxGemmBf16Opts(const void *a, const void *b, void *c, in
   p.M = M; p.N = N; p.K = K; p.c = c; p.ldc = ldc; p.errFlag = errFlag; p.rotate = 0; p.bn = bn; p.group = tileGroup((N + bn - 1) / bn);
   p.aMN = aMN; p.bMN = bMN; p.bias = bias; p.accumulate = accumulate;
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-  p.splitK = fcxGemmPieces(splitK, M, N, K, tiles, smCount(), smCount());
+  p.splitK = fcxGemmPieces(splitK, M, N, K, tiles, sms, sms);
   if (p.splitK > 1 && !accumulate) {
     cudaError_t e = cudaMemsetAsync(c, 0, ((size_t)(M - 1) * ldc + N) * 2, s);
     if (e != cudaSuccess) return e;
   }
   FcxDevComm dc{};
-  cudaError_t e = launch<FCX_GEMM_PLAIN>(ma, mb, p, dc, std::min(tiles * p.splitK, smCount()), s);
+  cudaError_t e = launch<FCX_GEMM_PLAIN>(ma, mb, p, dc, std::min(tiles * p.splitK, sms), s);
   if (e != cudaSuccess)
     snprintf(gGemmDetail, sizeof gGemmDetail, "kernel launch: %s (M %d N %d K %d aMN %d bMN %d splitK %d grid %d)", cudaGetErrorString(e), M, N,
-             K, aMN, bMN, p.splitK, std::min(tiles * p.splitK, smCount()));
+             K, aMN, bMN, p.splitK, std::min(tiles * p.splitK, sms));
   return e;
 }
 
@@ -708,7 +707,9 @@ extern "C" cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const 
   if (T % 8 || I % 8 || O % 8 || lddy % 8 || ldw % 8 || ldx % 8 || T <= 0 || I <= 0 || O <= 0) return cudaErrorNotSupported;
   if (((uintptr_t)dy | (uintptr_t)w | (uintptr_t)x | (uintptr_t)dx | (uintptr_t)dw) & 15) return cudaErrorNotSupported;
   cudaGetLastError();
-  const bool pairX = fcxGemmPairSuits(T, I, O) != 0, pairW = fcxGemmPairSuits(O, I, T) != 0;
+  const int sms = smCount();
+  int bnX = 256, bnW = 256;
+  const bool pairX = choose(T, I, O, sms, 0, &bnX), pairW = choose(O, I, T, sms, 0, &bnW);
   if (pairX != pairW) return cudaErrorNotSupported;
   if (pairX) {
     const int g = tileGroup((I + 255) / 256) / 2;
@@ -719,9 +720,7 @@ extern "C" cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const 
     FcxGemmParams p;
     int units, nK;
   };
-  const int sms = smCount();
-  auto fill = [&](Product *q, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int aMN) {
-    const int bn = pickBn(M, N, K, sms, 0);
+  auto fill = [&](Product *q, const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int aMN, int bn) {
     if (!(aMN ? makeMap(&q->a, a, K, M, lda, BK) : makeMap(&q->a, a, M, K, lda, BM)) || !makeMap(&q->b, b, K, N, ldb, BK)) return false;
     q->p = FcxGemmParams{};
     q->p.M = M; q->p.N = N; q->p.K = K; q->p.c = c; q->p.ldc = N; q->p.errFlag = errFlag; q->p.bn = bn; q->p.group = tileGroup((N + bn - 1) / bn);
@@ -731,7 +730,7 @@ extern "C" cudaError_t fcxGemmBackwardBf16(const void *dy, const void *w, const 
     return true;
   };
   Product px, pw;
-  if (!fill(&px, dy, w, dx, T, I, O, lddy, ldw, 0) || !fill(&pw, dy, x, dw, O, I, T, lddy, ldx, 1)) return cudaErrorNotSupported;
+  if (!fill(&px, dy, w, dx, T, I, O, lddy, ldw, 0, bnX) || !fill(&pw, dy, x, dw, O, I, T, lddy, ldx, 1, bnW)) return cudaErrorNotSupported;
   int swap = 0;
   SecondProduct second{};
   if (!fcxGemmDualPlan(pw.units, pw.nK, fcxGemmPieces(0, O, I, T, pw.units, sms, sms), px.units, px.nK,

@@ -72,6 +72,7 @@ double fcxGemmPairCost(int M, int N, int K, int pairs);
 double fcxGemmPairCostCut(int M, int N, int K, int pairs, int cut);
 int fcxGemmPairMode();
 int fcxGemmPairSuits(int M, int N, int K);
+int fcxGemmChoose(int M, int N, int K, int sms, int cut, int *bn);
 int fcxGemmPairSuitsCut(int M, int N, int K, int cut);
 cudaError_t fcxGemmPairBf16(const void *a, const void *b, void *c, int M, int N, int K, int lda, int ldb, int ldc, int aMN, int bMN,
                             const void *bias, int splitK, int accumulate, void *geluOut, int group, int *errFlag, cudaStream_t s,

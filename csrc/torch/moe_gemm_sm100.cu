@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_state.h"
 #include "moe_gemm_sm100.h"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
@@ -297,26 +298,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   }
 }
 
-int pairCount() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    n = sms > 1 ? sms / 2 : 74;
-  }
-  return n;
-}
+int pairCount() { return fcxhost::smCount() / 2; }
 
 template <bool UP>
 cudaError_t launchGroup(const CUtensorMap &a, const CUtensorMap &h, const WeightMaps &wm, const GroupParams &p, const FcxDevComm &dc,
                         cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(moeGroupKernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static fcxhost::OncePerDevice once;
+  const cudaError_t e = once([] { return cudaFuncSetAttribute(moeGroupKernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+  if (e != cudaSuccess) return e;
   return fcxpdl::launchPdl(moeGroupKernel<UP>, 2 * pairCount(), THREADS, SMEM_BYTES, s, a, h, wm, p, dc);
 }
 

@@ -2,6 +2,7 @@
 // mbarriers with bounded waits, TMA tile loads (never multicast), shared-memory
 // matrix descriptors, tcgen05.mma / commit / ld, TMEM fences.
 #pragma once
+#include <atomic>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -153,13 +154,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 inline EncodeTiledFn encodeFn() {
-  static EncodeTiledFn fn = nullptr;
+  static std::atomic<EncodeTiledFn> known{nullptr};
+  EncodeTiledFn fn = known.load(std::memory_order_relaxed);
   if (!fn) {
     void *p = nullptr;
     cudaDriverEntryPointQueryResult st;
     if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &st) == cudaSuccess &&
         st == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
+      known.store(fn = (EncodeTiledFn)p, std::memory_order_relaxed);
   }
   return fn;
 }

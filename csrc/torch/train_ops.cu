@@ -13,6 +13,7 @@
 
 #include "train_ops.h"
 #include "train_ops_noalloc.h"
+#include "device_state.h"
 #include "pdl.cuh"
 
 #include <mutex>
@@ -920,16 +921,7 @@ __global__ void __launch_bounds__(256) adamwKernel(float *master, bf16 *param, b
   }
 }
 
-int smCount() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
+using fcxhost::smCount;
 
 }  // namespace
 
@@ -951,14 +943,10 @@ cudaError_t fcxLayerNormFwd(const void *x, const void *delta, const void *gamma,
   const int grid = std::max(1, std::min(smCount(), (M + warps - 1) / warps));
   const size_t smem = (size_t)warps * 3 * 2 * C * 2;
   auto run = [&](auto kernel) {
-    // both instantiations have the same pointer type, so this lambda exists once: remember the kernels by address
-    static thread_local const void *configured[2] = {nullptr, nullptr};
-    const void *id = (const void *)kernel;
-    if (configured[0] != id && configured[1] != id) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      if (e != cudaSuccess) return e;
-      configured[configured[0] ? 1 : 0] = id;
-    }
+    // both instantiations have the same pointer type, so this lambda exists once: one entry for each
+    static fcxhost::OncePerDevice once[2];
+    const cudaError_t e = once[warps == 8]([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
+    if (e != cudaSuccess) return e;
     return fcxpdl::launchPdl(kernel, grid, warps * 32, smem, s, (const bf16 *)x, (const bf16 *)delta, (const bf16 *)gamma, (const bf16 *)beta,
                              (bf16 *)resOut, (bf16 *)y, mean, rstd, M, C, eps);
   };
@@ -974,14 +962,11 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
     constexpr int STAGES = 2, WARPS = LN_BWD_WARPS;
     const size_t smem = (size_t)WARPS * STAGES * 3 * C * 2;  // at most 192 KB; the warps' sums (WARPS x 2 x C fp32) fit in it
     auto kernel = lnBwdFusedKernel<4, STAGES, WARPS>;
-    static thread_local bool attr = false;
-    if (!attr) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      if (e != cudaSuccess) return e;
-      attr = true;
-    }
+    static fcxhost::OncePerDevice once;
+    cudaError_t e = once([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
+    if (e != cudaSuccess) return e;
     const int grid = lnFusedGrid(M);
-    cudaError_t e = fcxpdl::launchPdl(kernel, grid, WARPS * 32, smem, s, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)gamma, mean, rstd,
+    e = fcxpdl::launchPdl(kernel, grid, WARPS * 32, smem, s, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)gamma, mean, rstd,
                                       (const bf16 *)dres, (bf16 *)dx, partial, M, C);
     if (e != cudaSuccess) return e;
     return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, 256, 0, s, (const float *)partial, grid, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
@@ -989,13 +974,10 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
   constexpr int WARPS = 8;
   const size_t smem = (size_t)WARPS * 3 * 2 * C * 2;  // warps x 3-deep ring x (dy, x) x row bytes <= 192 KB
   auto kernel = lnBwdDxKernel<8, 3, WARPS>;
-  static thread_local bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  cudaError_t e = fcxpdl::launchPdl(kernel, std::max(1, std::min(smCount(), (M + WARPS - 1) / WARPS)), WARPS * 32, smem, s, (const bf16 *)dy,
+  static fcxhost::OncePerDevice once;
+  cudaError_t e = once([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
+  if (e != cudaSuccess) return e;
+  e = fcxpdl::launchPdl(kernel, std::max(1, std::min(smCount(), (M + WARPS - 1) / WARPS)), WARPS * 32, smem, s, (const bf16 *)dy,
                                     (const bf16 *)x, (const bf16 *)gamma, mean, rstd, (const bf16 *)dres, (bf16 *)dx, M, C);
   if (e != cudaSuccess) return e;
   // C <= 2048 here, so the 64-column blocks fit the ticket array: parameter partials and their reduction in one launch
@@ -1056,12 +1038,9 @@ cudaError_t fcxCrossEntropyFwdBwd(void *logits, const int64_t *targets, float *l
   if (Vpad % 8 != 0 || V > Vpad) return cudaErrorInvalidValue;
   const size_t ring = (size_t)Vpad * 2 * 2;
   if (ring <= 224 * 1024 && ((uintptr_t)logits & 15) == 0) {
-    static thread_local bool attr = false;
-    if (!attr) {
-      cudaError_t e = cudaFuncSetAttribute(ceFwdBwdStreamKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-      if (e != cudaSuccess) return e;
-      attr = true;
-    }
+    static fcxhost::OncePerDevice once;
+    const cudaError_t e = once([] { return cudaFuncSetAttribute(ceFwdBwdStreamKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024); });
+    if (e != cudaSuccess) return e;
     return fcxpdl::launchPdl(ceFwdBwdStreamKernel, std::min(M, smCount()), 1024, ring, s, (bf16 *)logits, targets, losses, M, V, Vpad, gradScale);
   } else {
     ceFwdBwdKernel<<<M, 1024, 0, s>>>((bf16 *)logits, targets, losses, V, Vpad, gradScale);
