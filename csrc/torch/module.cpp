@@ -114,8 +114,7 @@ at::Tensor colSum(const at::Tensor &a, const c10::optional<at::Tensor> &intoT) {
     TORCH_CHECK(intoT->numel() == C, "into must have one element per column");
   }
   auto out = into ? *intoT : at::empty({C}, a.options());
-  auto partial = at::empty({fcxColSumPartials(M), C}, a.options().dtype(at::kFloat));
-  CUDA_OK(fcxColSum(a.data_ptr(), out.data_ptr(), partial.data_ptr<float>(), M, C, into ? 1 : 0, cur()));
+  CUDA_OK(fcxColSum(a.data_ptr(), out.data_ptr(), M, C, into ? 1 : 0, cur()));
   return out;
 }
 

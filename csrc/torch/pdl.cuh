@@ -15,19 +15,34 @@ namespace fcxpdl {
 __device__ __forceinline__ void pdlRelease() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// `cluster`: CTAs per cluster, or {0, 0, 0} for a kernel that has none or sets its own.
 template <typename... Params, typename... Args>
-inline cudaError_t launchPdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
+inline cudaError_t launchPdlAttr(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, dim3 cluster, cudaStream_t s, Args &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster.x;
+  attr[1].val.clusterDim.y = cluster.y;
+  attr[1].val.clusterDim.z = cluster.z;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster.x ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launchPdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
+  return launchPdlAttr(kernel, grid, block, smem, dim3(0, 0, 0), s, static_cast<Args &&>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launchPdlCluster(void (*kernel)(Params...), dim3 grid, dim3 block, dim3 cluster, cudaStream_t s, Args &&...args) {
+  return launchPdlAttr(kernel, grid, block, 0, cluster, s, static_cast<Args &&>(args)...);
 }
 
 }  // namespace fcxpdl

@@ -16,7 +16,10 @@
 #include "device_state.h"
 #include "pdl.cuh"
 
+#include <cooperative_groups.h>
 #include <mutex>
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -58,10 +61,6 @@ __device__ __forceinline__ Bf8 pack8(const float *f) {
   *reinterpret_cast<uint4 *>(&p) = u;
   return p;
 }
-
-// Tickets of the one-launch reductions (colSumFusedKernel, lnBwdParamKernel): one counter per 64-column block.
-__device__ unsigned int gColTickets[1024];
-__device__ unsigned int gLnTickets[1024];
 
 // ---------------------------------------------------------------- LayerNorm
 // One warp per row, persistent over rows, 16 warps per SM (8 for rows wider than 1024).  The rows a warp will work on
@@ -358,9 +357,9 @@ __global__ void __launch_bounds__(256) lnParamFoldKernel(const float *partial, i
 
 // Backward, part 2, for rows wider than 1024: dgamma[c] = sum_r dy[r,c] * xhat[r,c], dbeta[c] = sum_r dy[r,c].
 // A CTA owns 64 columns and one slice of the rows; partial sums go to
-// `partial` ([gridDim.y][2][C], fp32 scratch); the CTA that finishes a column block last folds them into dgamma / dbeta.
+// `partial` ([gridDim.y][2][C], fp32 scratch), which lnParamFoldKernel folds into dgamma / dbeta.
 __global__ void __launch_bounds__(256) lnBwdParamKernel(const bf16 *dy, const bf16 *x, const float *mean, const float *rstd, float *partial,
-                                                        int M, int C, bf16 *dgamma, bf16 *dbeta, int accumulate) {
+                                                        int M, int C) {
   __shared__ float redG[32][64 + 1], redB[32][64 + 1];
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
@@ -413,34 +412,7 @@ __global__ void __launch_bounds__(256) lnBwdParamKernel(const bf16 *dy, const bf
 #pragma unroll 8
     for (int j = 0; j < 32; j++) s += isB ? redB[j][c] : redG[j][c];
     partial[((size_t)blockIdx.y * 2 + (isB ? 1 : 0)) * C + col0 + c] = s;
-    __threadfence();
   }
-  if (dgamma == nullptr) return;  // partial sums only
-  // the CTA that finishes this 64-column block last folds them (ticket scheme of colSumFusedKernel)
-  __shared__ unsigned int ticket;
-  __syncthreads();
-  if (threadIdx.x == 0) ticket = atomicAdd(&gLnTickets[blockIdx.x], 1u);
-  __syncthreads();
-  if (ticket != gridDim.y - 1) return;
-  __threadfence();
-  {
-    // 128 outputs (64 dgamma, 64 dbeta), two halves of the partial sums per output
-    const int o = threadIdx.x & 127, half = threadIdx.x >> 7, c = o & 63;
-    const bool isB = o >= 64;
-    float s = 0.f;
-    for (int p = half; p < (int)gridDim.y; p += 2) s += __ldcg(partial + ((size_t)p * 2 + (isB ? 1 : 0)) * C + col0 + c);
-    __syncthreads();
-    float *fold = &redB[0][0];
-    fold[half * 128 + o] = s;
-    __syncthreads();
-    if (threadIdx.x < 128) {
-      s = fold[o] + fold[128 + o];
-      bf16 *dst = isB ? dbeta + col0 + c : dgamma + col0 + c;
-      if (accumulate) s += __bfloat162float(*dst);
-      *dst = __float2bfloat16_rn(s);
-    }
-  }
-  if (threadIdx.x == 0) gLnTickets[blockIdx.x] = 0;
 }
 
 // ---------------------------------------------------------------- bias + GELU (tanh form)
@@ -613,67 +585,60 @@ __global__ void colSumReduceKernel(const float *__restrict__ partial, int nparts
   out[c] = __float2bfloat16_rn(s);
 }
 
-// Both steps of the column sum in ONE launch: the CTA that finishes a 64-column block last (a ticket per block, taken
-// after the partial sums are visible) folds the block's partial sums and writes the result.  The tickets live in the
-// library image and return to zero by themselves; concurrent calls on one device would share them, so calls must be
-// stream-ordered (they are: the backward pass runs on one stream).
-__global__ void __launch_bounds__(256) colSumFusedKernel(const bf16 *a, float *partial, bf16 *out, int M, int C, int accumulate) {
+// The column sums in ONE launch.  A CTA owns 64 columns and a slice of the rows; the CTAs of a column block form a cluster
+// (up to eight), whose first CTA adds up the others' sums out of their shared memory.  Nothing outlives the launch, so calls
+// on several streams do not meet; with tickets in the library image, as this kernel had before, concurrent calls of a device
+// took each other's.  Bound by memory once there are rows enough, by latency below.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) colSumClusterKernel(const bf16 *a, bf16 *out, int M, int C, int accumulate) {
+  constexpr int ROWS = THREADS / 8, WARPS = THREADS / 32;
+  __shared__ float red[WARPS][64], sums[64];
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
-  const int col0 = blockIdx.x * 64;
-  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const int col0 = blockIdx.x * 64, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;  // 8 vector columns x ROWS row lanes
   const int rowsPer = (M + gridDim.y - 1) / gridDim.y;
-  const int r0 = blockIdx.y * rowsPer, r1 = min(M, r0 + rowsPer);
-  int r = r0 + ty;
-  for (; r + 96 < r1; r += 128) {
+  const int r1 = min(M, (int)(blockIdx.y + 1) * rowsPer);
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int r = blockIdx.y * rowsPer + ty; r < r1; r += 4 * ROWS) {  // four rows in flight per thread
     Bf8 p[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) p[u] = *(const Bf8 *)(a + (size_t)(r + 32 * u) * C + col0 + tx * 8);
+    for (int u = 0; u < 4; u++)
+      if (r + u * ROWS < r1) p[u] = *(const Bf8 *)(a + (size_t)(r + u * ROWS) * C + col0 + tx * 8);
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      float v[8];
-      unpack8(p[u], v);
+    for (int u = 0; u < 4; u++)
+      if (r + u * ROWS < r1) {
+        float v[8];
+        unpack8(p[u], v);
 #pragma unroll
-      for (int k = 0; k < 8; k++) acc[k] += v[k];
-    }
+        for (int k = 0; k < 8; k++) acc[k] += v[k];
+      }
   }
-  for (; r < r1; r += 32) {
-    float v[8];
-    unpack8(*(const Bf8 *)(a + (size_t)r * C + col0 + tx * 8), v);
 #pragma unroll
-    for (int k = 0; k < 8; k++) acc[k] += v[k];
+  for (int k = 0; k < 8; k++) {  // the four rows of a warp
+    acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 8);
+    acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
   }
-  __shared__ float red[32][64 + 1];
-  __shared__ unsigned int ticket;
+  if (lane < 8) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) red[ty][tx * 8 + k] = acc[k];
-  __syncthreads();
-  if (threadIdx.x < 64) {
-    float s = 0.f;
-#pragma unroll 8
-    for (int j = 0; j < 32; j++) s += red[j][threadIdx.x];
-    partial[(size_t)blockIdx.y * C + col0 + threadIdx.x] = s;
-    __threadfence();
+    for (int k = 0; k < 8; k++) red[warp][lane * 8 + k] = acc[k];
   }
   __syncthreads();
-  if (threadIdx.x == 0) ticket = atomicAdd(&gColTickets[blockIdx.x], 1u);
-  __syncthreads();
-  if (ticket != gridDim.y - 1) return;
-  __threadfence();
-  // last CTA of this column block: four groups of 64 threads fold a quarter of the partial sums each
-  const int c = threadIdx.x & 63, grp = threadIdx.x >> 6;
   float s = 0.f;
-  for (int p = grp; p < (int)gridDim.y; p += 4) s += __ldcg(partial + (size_t)p * C + col0 + c);
-  __syncthreads();  // red is reused
-  red[grp][c] = s;
-  __syncthreads();
   if (threadIdx.x < 64) {
-    s = red[0][c] + red[1][c] + red[2][c] + red[3][c];
-    if (accumulate) s += __bfloat162float(out[col0 + c]);
-    out[col0 + c] = __float2bfloat16_rn(s);
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) s += red[w][threadIdx.x];
+    sums[threadIdx.x] = s;
   }
-  if (threadIdx.x == 0) gColTickets[blockIdx.x] = 0;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  if (blockIdx.y == 0 && threadIdx.x < 64) {
+    for (unsigned int i = 1; i < gridDim.y; i++) s += *cluster.map_shared_rank(&sums[threadIdx.x], i);
+    bf16 *dst = out + col0 + threadIdx.x;
+    if (accumulate) s += __bfloat162float(*dst);
+    *dst = __float2bfloat16_rn(s);
+  }
+  cluster.sync();  // nobody's shared memory goes before it has been read
 }
 
 // ---------------------------------------------------------------- softmax cross-entropy
@@ -980,9 +945,10 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
   e = fcxpdl::launchPdl(kernel, std::max(1, std::min(smCount(), (M + WARPS - 1) / WARPS)), WARPS * 32, smem, s, (const bf16 *)dy,
                                     (const bf16 *)x, (const bf16 *)gamma, mean, rstd, (const bf16 *)dres, (bf16 *)dx, M, C);
   if (e != cudaSuccess) return e;
-  // C <= 2048 here, so the 64-column blocks fit the ticket array: parameter partials and their reduction in one launch
-  return fcxpdl::launchPdl(lnBwdParamKernel, dim3(C / 64, lnParts(M)), 256, 0, s, (const bf16 *)dy, (const bf16 *)x, mean, rstd, partial, M, C,
-                           (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
+  const int parts = lnParts(M);
+  e = fcxpdl::launchPdl(lnBwdParamKernel, dim3(C / 64, parts), 256, 0, s, (const bf16 *)dy, (const bf16 *)x, mean, rstd, partial, M, C);
+  if (e != cudaSuccess) return e;
+  return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, 256, 0, s, (const float *)partial, parts, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
 }
 
 cudaError_t fcxBiasGeluFwd(const void *x, const void *bias, void *y, size_t M, int C, cudaStream_t s) {
@@ -1021,16 +987,17 @@ cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void
   return fcxpdl::launchPdl(colSumFoldKernel, C / 32, 256, 0, s, (const float *)partial, parts, C, (bf16 *)dbias, accumulate);
 }
 
-// `partial` must hold fcxColSumPartials(M) * C floats.
-cudaError_t fcxColSum(const void *a, void *out, float *partial, int M, int C, int accumulate, cudaStream_t s) {
+cudaError_t fcxColSum(const void *a, void *out, int M, int C, int accumulate, cudaStream_t s) {
   if (C % 64 != 0) return cudaErrorInvalidValue;
-  int parts = fcxColSumPartials(M);
-  if (C / 64 <= 1024) {
-    return fcxpdl::launchPdl(colSumFusedKernel, dim3(C / 64, parts), 256, 0, s, (const bf16 *)a, partial, (bf16 *)out, M, C, accumulate);
-  }
-  colSumKernel<<<dim3(C / 64, parts), 256, 0, s>>>((const bf16 *)a, partial, M, C);
-  colSumReduceKernel<<<(C + 255) / 256, 256, 0, s>>>(partial, parts, C, (bf16 *)out, accumulate);
-  return cudaGetLastError();
+  // A CTA for every 256 rows, up to the eight of a portable cluster.  From 1024 rows on, CTAs of 512 threads while they all fit
+  // on the SMs at once (three each): in microseconds, 256 / 512 threads, 2328 x 2944 6.6 / 6.0, 8192 x 1024 9.9 / 7.8,
+  // 8192 x 3072 12.8 / 11.0, but 8192 x 4096 (512 CTAs) 13.8 / 18.0 and 64 x 3072 2.3 / 2.5.  (With tickets: 7.5, 7.6, 14.2, 15.8, 3.1.)
+  int parts = 1;
+  while (parts < 8 && parts * 512 <= M) parts *= 2;
+  auto run = [&](auto kernel, int threads) {
+    return fcxpdl::launchPdlCluster(kernel, dim3(C / 64, parts), threads, dim3(1, parts), s, (const bf16 *)a, (bf16 *)out, M, C, accumulate);
+  };
+  return M >= 1024 && C / 64 * parts <= 3 * smCount() ? run(colSumClusterKernel<512>, 512) : run(colSumClusterKernel<256>, 256);
 }
 
 cudaError_t fcxCrossEntropyFwdBwd(void *logits, const int64_t *targets, float *losses, int M, int V, int Vpad, float gradScale,
@@ -1109,7 +1076,7 @@ extern "C" int fcxColSumNoAlloc(const void *a, void *out, int M, int C, int accu
 extern "C" const char *fcxNoAllocErrorString(int code) {
   switch (code) {
     case 0: return "success";
-    case FCX_NOALLOC_TOO_LARGE: return "shape needs more than the built-in scratch (partials x C > 262144 floats); use fcxColSum with your own scratch";
+    case FCX_NOALLOC_TOO_LARGE: return "shape needs more than the built-in scratch (partials x C > 262144 floats); use fcxColSum";
     case FCX_NOALLOC_BAD_SHAPE: return "M and C must be positive and C a multiple of 64";
     case FCX_NOALLOC_NULL_POINTER: return "input and output pointers must not be null";
     case FCX_NOALLOC_MISALIGNED: return "input and output pointers must be 16-byte aligned";

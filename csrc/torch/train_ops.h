@@ -20,7 +20,7 @@ int fcxBiasGeluBwdPartials(int M, int C);
 cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void *dx, void *dbias, float *partial, int M, int C,
                            int accumulate, cudaStream_t s);
 int fcxColSumPartials(int M);
-cudaError_t fcxColSum(const void *a, void *out, float *partial, int M, int C, int accumulate, cudaStream_t s);
+cudaError_t fcxColSum(const void *a, void *out, int M, int C, int accumulate, cudaStream_t s);
 cudaError_t fcxCrossEntropyFwdBwd(void *logits, const int64_t *targets, float *losses, int M, int V, int Vpad, float gradScale,
                                   cudaStream_t s);
 cudaError_t fcxAdamW(float *master, void *param, void *grad, float *m, float *v, size_t n, float lr, float b1, float b2, float eps,

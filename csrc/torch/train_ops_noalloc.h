@@ -8,8 +8,10 @@
 // later cudaMalloc simply fails), a control loop that cannot afford the
 // device-wide synchronisation hidden in cudaMalloc/cudaFree, and callers
 // outside PyTorch that have no caching allocator to lean on.  The regular
-// entry point, fcxColSum (train_ops.h), wants a scratch buffer from its
-// caller; this one brings its own.
+// entry point, fcxColSum (train_ops.h), needs no scratch either: it folds its
+// partial sums inside a thread-block cluster, and calls of it may run at the
+// same time.  This one is two plain launches, checks its arguments and
+// explains what it refuses.
 //
 // How: the per-row-slice partial sums go to a fixed array that is part of the
 // library image (`static __device__`, 1 MiB).  Every GPU that loads the

@@ -146,10 +146,10 @@ def test_dispatch_and_combine_edges(nat, comm1, entries, experts, H, exchange):
         assert ep.count_mat[0].tolist() == [int((idx == e).sum().item()) for e in range(experts)]
 
 
-@pytest.mark.parametrize("M,C", [(1, 256), (1185, 1024), (1184 * 4 + 3, 768), (9, 512)])
+@pytest.mark.parametrize("M,C", [(1, 256), (1185, 1024), (1184 * 4 + 3, 768), (9, 512), (1, 1280), (4099, 2048)])
 @pytest.mark.parametrize("with_dres", [False, True])
 def test_layernorm_backward_in_one_pass(nat, M, C, with_dres):
-    """One row, one more row than warps on the GPU, and rows past the ring's depth."""
+    """One row, one more row than warps on the GPU, and rows past the ring's depth; rows wider than 1024 take a second pass."""
     torch.manual_seed(M)
     x, dy, g, b = _bf(M, C), _bf(M, C), _bf(C) + 1, _bf(C)
     dres = _bf(M, C) if with_dres else None
@@ -185,6 +185,18 @@ def test_bias_gelu_backward_sums_its_own_gradient(nat, M, C):
     before = into.clone()
     nat.bias_gelu_bwd(dy, x, b, into)
     _close(into, before.double() + dx.double().sum(0), before.double().abs() + dx.double().abs().sum(0), max(8, M // 8))
+
+
+@pytest.mark.parametrize("M,C", [(1, 64), (511, 128), (512, 64), (1025, 192), (2047, 64), (4097, 448), (9000, 3584), (8192, 64), (5, 65600)])
+def test_column_sums(nat, M, C):
+    """One CTA and clusters of two to eight, rows that divide among them and rows that do not, both CTA sizes, very wide."""
+    torch.manual_seed(M)
+    a = _bf(M, C)
+    _close(nat.col_sum(a), a.double().sum(0), a.double().abs().sum(0), max(8, M // 8))
+    into = _bf(C)
+    before = into.clone()
+    nat.col_sum(a, into)
+    _close(into, before.double() + a.double().sum(0), before.double().abs() + a.double().abs().sum(0), max(8, M // 8))
 
 
 @pytest.mark.parametrize("shape,n_out,bias", [((40, 64), 192, True), ((2, 20, 64), 128, True), ((3, 8, 72), 64, False)])

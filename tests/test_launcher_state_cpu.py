@@ -19,6 +19,15 @@ def test_no_plain_static_variable_inside_a_function(path):
     assert not bad, bad
 
 
+def test_kernels_share_no_memory_of_the_library_image():
+    """A __device__ array is one for all launches on a device: two streams that use it at a time take each other's values.  The
+    one exception is the scratch of the entry point whose contract says so (train_ops_noalloc.h)."""
+    bad = []
+    for path in TORCH.glob("*.cu*"):
+        bad += [(path.name, line) for line in re.findall(r"^(?:static )?__device__ (?:__align__\(\d+\) )?[^()\n]*;.*$", path.read_text(), re.M)]
+    assert [b for b in bad if "gNoAllocScratch" not in b[1]] == []
+
+
 PROGRAM = r"""
 #include "device_state.h"
 #include <cstdio>

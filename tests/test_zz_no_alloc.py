@@ -7,7 +7,7 @@ PyTorch's caching allocator.  For them the library carries a fixed 1 MiB
 scratch array and exposes one C symbol that uses it.  This test calls that
 symbol the way such a user would (ctypes, raw pointers, the current stream),
 twice in a row, and checks both results against the regular entry point
-(`col_sum`, which takes its scratch from the caller).  The file name sorts
+(`col_sum`, which needs no scratch).  The file name sorts
 last so that it runs after every other test; it also passes on its own.
 """
 import ctypes
