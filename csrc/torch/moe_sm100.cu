@@ -181,8 +181,9 @@ __global__ void __launch_bounds__(256) siluMulKernel(const __nv_bfloat16 *__rest
 }
 
 // out[t] = sum_k w[t,k] * ret[t,k], after every CTA of every expert's output GEMM has reported.
-// KC > 0: K is KC (1, 2, 4), 8 / KC output vectors per thread and step with every choice's row loaded before the first is
-// used, eight 16-byte loads in flight; positions in 32 bits (their 64-bit divisions cost more than the loads).
+// KC > 0: K is KC (1 to 4), 8 / KC output vectors per thread and step with every choice's row loaded before the first is
+// used, eight 16-byte loads in flight (six for three choices); positions in 32 bits (their 64-bit divisions cost more than the
+// loads).  Three choices took 70 us one vector at a time and take 51 so at 8192 x 4096; two take 36, four 55.
 // KC = 0: any K and any size, one vector at a time.
 template <int KC>
 __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, const __nv_bfloat16 *ret, const float *w, __nv_bfloat16 *out, int T,
@@ -285,7 +286,7 @@ extern "C" cudaError_t fcxMoeCombine(const FcxDevComm *dc, const void *ret, cons
   if (H % 8) return cudaErrorInvalidValue;
   // positions may run past the total by up to eight grid strides
   const bool small = (uint64_t)T * (H / 8) + 16ull * 592 * 256 < (1ull << 32);
-  auto kernel = !small ? moeCombineKernel<0> : K == 1 ? moeCombineKernel<1> : K == 2 ? moeCombineKernel<2> : K == 4 ? moeCombineKernel<4>
-                                                                                                                 : moeCombineKernel<0>;
+  auto kernel = !small ? moeCombineKernel<0> : K == 1 ? moeCombineKernel<1> : K == 2 ? moeCombineKernel<2> : K == 3 ? moeCombineKernel<3>
+                : K == 4 ? moeCombineKernel<4> : moeCombineKernel<0>;
   return fcxpdl::launchPdl(kernel, 592, 256, 0, s, *dc, (const __nv_bfloat16 *)ret, w, (__nv_bfloat16 *)out, T, H, K, doneOff, want, errFlag);
 }
