@@ -123,9 +123,28 @@ static int64_t moeDown(uint64_t comm, const at::Tensor &h, const std::vector<at:
   FcxDevComm dc = devComm(comm);
   int grid = 0;
   auto e = fcxMoeDownGrouped(&dc, h.data_ptr(), ptrs.data(), rows.data_ptr<int>(), (int)L, (int)(h.size(0) / L), (int)w[0].size(0),
-                             (int)h.size(1), ld.data(), info.data_ptr(), heapOffset(comm, combine), heapOffset(comm, doneCounter), (int)topk,
+                             (int)h.size(1), (int)h.stride(0), ld.data(), info.data_ptr(), heapOffset(comm, combine), heapOffset(comm, doneCounter), (int)topk,
                              err.data_ptr<int>(), &grid, cur());
   TORCH_CHECK(e == cudaSuccess, "grouped expert GEMM + combine launch failed: ", cudaGetErrorString(e));
+  return grid;
+}
+
+// The same for one expert: any number of rows, strided rows, and its row count m_ptr.
+static int64_t gemmRowMap(uint64_t comm, const at::Tensor &a, const at::Tensor &b, const at::Tensor &mPtr, const at::Tensor &info,
+                          at::Tensor &combine, at::Tensor &doneCounter, int64_t topk, at::Tensor &err) {
+  checkBf16Mat(a, "a");
+  checkBf16Mat(b, "b");
+  TORCH_CHECK(a.size(1) == b.size(1), "inner dimensions differ");
+  TORCH_CHECK(info.scalar_type() == at::kInt && info.numel() >= a.size(0) * 4, "info must be int32 [rows, 4]");
+  c10::cuda::CUDAGuard g(a.device());
+  FcxDevComm dc = devComm(comm);
+  const void *w = b.data_ptr();
+  const int ldw = (int)b.stride(0);
+  int grid = 0;
+  auto e = fcxMoeDownGrouped(&dc, a.data_ptr(), &w, mPtr.data_ptr<int>(), 1, (int)a.size(0), (int)b.size(0), (int)a.size(1), (int)a.stride(0),
+                             &ldw, info.data_ptr(), heapOffset(comm, combine), heapOffset(comm, doneCounter), (int)topk, err.data_ptr<int>(),
+                             &grid, cur());
+  TORCH_CHECK(e == cudaSuccess, "fused GEMM combine launch failed: ", cudaGetErrorString(e));
   return grid;
 }
 
@@ -148,6 +167,7 @@ void bindMoe(py::module &m) {
         py::arg("err"), py::arg("ctas"), py::arg("experts_per_rank") = 1, py::arg("exchange") = false);
   m.def("silu_mul", &siluMul, py::arg("gu"), py::arg("h"), py::arg("rows") = py::none());
   m.def("gemm_dyn_m", &gemmDynM);
+  m.def("gemm_rowmap", &gemmRowMap);
   m.def("moe_up", &moeUp);
   m.def("moe_down", &moeDown);
   m.def("moe_combine", &moeCombine);

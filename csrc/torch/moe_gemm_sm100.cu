@@ -330,13 +330,13 @@ extern "C" cudaError_t fcxMoeUpGrouped(const void *x, const void *const *w, void
 }
 
 extern "C" cudaError_t fcxMoeDownGrouped(const FcxDevComm *dc, const void *h, const void *const *w, const int *rows, int L, int capL, int H,
-                                         int F, const int *ldw, const void *rowInfo, size_t combineOff, size_t doneOff, int topk,
+                                         int F, int ldh, const int *ldw, const void *rowInfo, size_t combineOff, size_t doneOff, int topk,
                                          int *errFlag, int *gridOut, cudaStream_t s) {
-  if (L < 1 || L > FCX_MOE_MAX_EXPERTS || capL <= 0 || capL % 128 || H % 8 || F % 8 || H <= 0 || F <= 0) return cudaErrorInvalidValue;
+  if (L < 1 || L > FCX_MOE_MAX_EXPERTS || capL <= 0 || H % 8 || F % 8 || H <= 0 || F <= 0 || ldh % 8) return cudaErrorInvalidValue;
   if ((uintptr_t)h & 15) return cudaErrorInvalidValue;
   CUtensorMap ma;
   WeightMaps wm{};
-  if (!makeTileMap(&ma, h, (uint64_t)L * capL, F, F, BM, 2)) return cudaErrorNotSupported;
+  if (!makeTileMap(&ma, h, (uint64_t)L * capL, F, ldh, BM, 2)) return cudaErrorNotSupported;
   for (int e = 0; e < L; e++)
     if (ldw[e] % 8 || ((uintptr_t)w[e] & 15) || !makeTileMap(&wm.m[e], w[e], H, F, ldw[e], BOX, 2)) return cudaErrorInvalidValue;
   GroupParams p{};

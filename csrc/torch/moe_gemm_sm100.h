@@ -14,10 +14,10 @@ extern "C" {
 // between rows.  Rows of a segment past rows[l] may be overwritten in h up to the next multiple of 32.
 cudaError_t fcxMoeUpGrouped(const void *x, const void *const *w, void *h, const int *rows, int L, int capL, int H, int F, const int *ldw,
                             int *errFlag, cudaStream_t s);
-// y = h[r] w^T, stored at its token's place on the rank it came from: heap[info[r].x] + combineOff + (info[r].y * topk + info[r].z)
+// y = h[r] w^T (h bf16, `ldh` elements between rows), stored at its token's place on the rank it came from: heap[info[r].x] + combineOff + (info[r].y * topk + info[r].z)
 // * H elements.  w: L matrices [H, F].  Afterwards every CTA of the launch (gridOut of them) adds 1 to the u64 counter at
 // doneOff on every rank.
-cudaError_t fcxMoeDownGrouped(const FcxDevComm *dc, const void *h, const void *const *w, const int *rows, int L, int capL, int H, int F,
+cudaError_t fcxMoeDownGrouped(const FcxDevComm *dc, const void *h, const void *const *w, const int *rows, int L, int capL, int H, int F, int ldh,
                               const int *ldw, const void *rowInfo, size_t combineOff, size_t doneOff, int topk, int *errFlag, int *gridOut,
                               cudaStream_t s);
 // Accumulator columns of a tile (256 or 128) for that many 256-row blocks and columns; the kernels decide for themselves.

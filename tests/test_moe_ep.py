@@ -1,6 +1,7 @@
 """Expert-parallel MoE pieces on one GPU against fp32 PyTorch references:
-the device-row-count GEMM, SiLU-mul, and the whole fused layer on a one-rank
-communicator (dispatch kernel, ROWMAP GEMM epilogue, combine kernel)."""
+the building blocks of one expert (device-row-count GEMM, SiLU-mul, the GEMM that
+scatters its rows), and the whole fused layer on a one-rank communicator
+(dispatch kernel, grouped expert GEMMs, combine kernel)."""
 import pytest
 import torch
 
@@ -41,6 +42,30 @@ def test_gemm_with_device_row_count(nat, rows):
         e = (c[:rows].float() - ref[:rows]).abs().max() / ref.abs().max()
         assert e < 2e-2
     assert bool((c[rows:] == 7.0).all())  # rows beyond the count stay untouched
+
+
+@pytest.mark.parametrize("rows,cap,pad", [(0, 200, 0), (1, 40, 8), (129, 200, 0), (300, 300, 16)])
+def test_gemm_that_scatters_its_rows(nat, comm1, rows, cap, pad):
+    """One expert's output projection: buffers whose row count is no multiple of a tile, strided rows, top-2 places."""
+    lib, comm = comm1
+    torch.manual_seed(rows)
+    K, N, T = 136, 200, 150
+    a = (torch.randn(cap, K + pad, device="cuda") * 0.5).bfloat16()[:, :K]
+    b = (torch.randn(N, K + pad, device="cuda") * 0.5).bfloat16()[:, :K]
+    place = torch.randperm(2 * T, device="cuda")[:cap]  # (token, choice) of each row
+    info = torch.zeros(cap, 4, dtype=torch.int32, device="cuda")
+    info[:, 1], info[:, 2] = place // 2, place % 2
+    back = nat.heap_tensor(comm.value, [2 * T, N], torch.bfloat16).fill_(5.0)
+    done = nat.heap_tensor(comm.value, [2], torch.int64).zero_()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    m = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    grid = nat.gemm_rowmap(comm.value, a, b, m, info, back, done, 2, err)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and int(done[0].item()) == grid
+    want = torch.full((2 * T, N), 5.0, dtype=torch.float64, device="cuda")
+    want[place[:rows]] = a[:rows].double() @ b.double().t()
+    bound = 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * K  # one rounding; products stay below one on average
+    assert bool(((back.double() - want).abs() <= bound).all())
 
 
 def test_silu_mul(nat):
