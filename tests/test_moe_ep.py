@@ -133,3 +133,39 @@ def test_fused_layer_with_four_experts_on_one_rank(nat, comm1):
         ref = moe_reference(x, idx, wts, w1, w2)
         e = (out.float() - ref).abs().max() / ref.abs().max()
         assert e < 3e-2, (rep, float(e))
+
+
+@pytest.mark.parametrize("T,H,F,L", [(512, 1024, 2048, 4), (777, 264, 520, 3)])
+def test_fused_layer_repeats_exactly_and_rounds_gate_and_up_only_once(nat, comm1, T, H, F, L):
+    """Call after call gives the same bits, with other inputs in between; and the result is no further from 64 bits than
+    the layer whose gate and up products are rounded to bf16 before the activation, which the fused one does without."""
+    from flagcx_b200.parallel.ep import ExpertParallelContext
+    lib, comm = comm1
+    K = 2
+    ep = ExpertParallelContext(comm.value, 1, 0, T, H, F, K, experts_per_rank=L, capacity_factor=2.0)
+    torch.manual_seed(T)
+    up = [(torch.randn(2 * F, H, device="cuda") * 0.02).bfloat16() for _ in range(L)]
+    down = [(torch.randn(H, F, device="cuda") * 0.02).bfloat16() for _ in range(L)]
+    batches = []
+    for _ in range(2):
+        w, idx = torch.topk(torch.softmax(torch.randn(T, L, device="cuda"), -1), K, dim=-1)
+        batches.append((torch.randn(T, H, device="cuda").bfloat16(), idx.int().contiguous(), w.contiguous()))
+    first = [ep.forward(*b, up, down) for b in batches]
+    for _ in range(3):
+        for b, want in zip(batches, first):
+            assert torch.equal(ep.forward(*b, up, down), want)
+    ep.check()
+
+    def layer(x, idx, w, rounded):
+        r = (lambda t: t.bfloat16().double()) if rounded else (lambda t: t)
+        out = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+        for e in range(L):
+            rows, choice = (idx == e).nonzero(as_tuple=True)
+            gu = r(x[rows].double() @ up[e].double().t())
+            y = r(r(torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]) @ down[e].double().t())
+            out.index_add_(0, rows, w[rows, choice].double()[:, None] * y)
+        return r(out)
+
+    for b, got in zip(batches, first):
+        exact, rounded = layer(*b, False), layer(*b, True)
+        assert float((got.double() - exact).norm()) < 0.9 * float((rounded - exact).norm())
