@@ -113,5 +113,4 @@ def test_two_products_in_one_launch_cover_every_unit_once(ext):
             units, lens = units[::-1], lens[::-1]
         assert ext.fcxGemmUnitsCovered(74, units[0], units[1], extra.value, lens[0], lens[1], ctypes.byref(longest)) == 1
         share = (uw * kw + ux * kx) / 74
-        print(i, o, s0.value, s1.value, units, lens, extra.value, longest.value, share)
         assert longest.value <= share + 1.5 * lens[1], (i, o, longest.value, share)

@@ -1,4 +1,6 @@
 """GPU kernels at the sizes where a tile, a group or a slice ends, against float64 PyTorch."""
+import ctypes
+
 import pytest
 import torch
 
@@ -32,6 +34,46 @@ def _close(got, ref, magnitude, k, roundings=1):
     bound = roundings * 2.0 ** -8 * ref.abs() + k * 2.0 ** -23 * magnitude + 1e-30
     worst = ((got.double() - ref).abs() / bound).max()
     assert worst <= 1.0, float(worst)
+
+
+@pytest.fixture(scope="module")
+def ext(nat):
+    lib = ctypes.CDLL(nat.__file__)
+    lib.fcxGemmTileCost.restype = ctypes.c_double
+    return lib
+
+
+def _cdiv(a, b):
+    return -(-a // b)
+
+
+def _tiles(ext, m, n, k):
+    """(CTA pairs or not, tiles, pieces of K) that a launch of its own uses for an [m, n] product of k terms."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    bn = ctypes.c_int(256)
+    ext.fcxGemmTileCost(m, n, k, sms, ctypes.byref(bn))
+    pair = bool(ext.fcxGemmPairSuits(m, n, k))
+    units = _cdiv(m, 256) * _cdiv(n, 256) if pair else _cdiv(m, 128) * _cdiv(n, bn.value)
+    return pair, units, ext.fcxGemmPieces(0, m, n, k, units, sms // 2 if pair else sms, sms)
+
+
+def _close_in_pieces(got, a, b, pieces, before=None):
+    """got = a^T b (+ before) with a [k, m] and b [k, n], K cut into `pieces`.  fp32 sums; every piece p_i is rounded to bf16
+    (8 significant bits: unit roundoff 2^-8) and, where there are several or a value before, so is each of the partial
+    totals it is added to, in any order: at most 2^-8 (sum |p_i| + pieces (|before| + sum |p_i|)), with the pieces' own
+    sums taken in 64 bits."""
+    k, per = a.shape[0], _cdiv(_cdiv(a.shape[0], 64), pieces) * 64
+    assert _cdiv(k, per) == pieces
+    parts = [a[i:i + per].double().t() @ b[i:i + per].double() for i in range(0, k, per)]
+    ref, size = sum(parts), sum(p.abs() for p in parts)
+    rounding = size
+    if before is not None or pieces > 1:
+        rounding = size + pieces * (size + (before.abs() if before is not None else 0))
+    if before is not None:
+        ref = ref + before
+    bound = 1.02 * 2.0 ** -8 * rounding + k * 2.0 ** -23 * (a.double().abs().t() @ b.double().abs()) + 1e-30
+    worst = float(((got.double() - ref).abs() / bound).max())
+    assert worst <= 1.0, worst
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (64, 72, 256), (128, 192, 1024), (129, 1000, 136), (40, 3072, 1024), (384, 1000, 64)])
@@ -224,7 +266,7 @@ def test_linear_in_one_call_each_way(nat, shape, n_out, bias):
 
 
 @pytest.mark.parametrize("rows,k,n", [(128, 64, 72), (640, 512, 264), (2048, 1024, 512)])
-def test_tensor_parallel_halves_of_one_rank(nat, comm1, rows, k, n):
+def test_tensor_parallel_halves_of_one_rank(nat, comm1, ext, rows, k, n):
     from flagcx_b200.parallel.tp import TensorParallelContext, column_parallel_linear, row_parallel_linear
     torch.manual_seed(rows)
     for half in (column_parallel_linear, row_parallel_linear):
@@ -237,32 +279,34 @@ def test_tensor_parallel_halves_of_one_rank(nat, comm1, rows, k, n):
         xd, wd, dyd = x.detach().double(), w.detach().double(), dy.double()
         _close(y.detach(), xd @ wd.t(), xd.abs() @ wd.abs().t(), k)
         _close(dx, dyd @ wd, dyd.abs() @ wd.abs(), n)
-        # the weight gradient may be cut into up to eight pieces that are added in bf16
-        _close(dw, dyd.t() @ xd, 2.0 ** 23 / rows * 8 * 2.0 ** -8 * (dyd.abs().t() @ xd.abs()) / rows ** 0.5 + dyd.abs().t() @ xd.abs(), rows)
+        _close_in_pieces(dw, dy, x.detach(), _tiles(ext, n, k, rows)[2])
 
 
 @pytest.mark.parametrize("T,I,O", [(8, 64, 64), (136, 264, 520), (128, 256, 1024), (776, 72, 200), (2328, 1000, 2944), (3000, 512, 2048),
                                    (8192, 1024, 1024), (64, 1024, 3072)])
 @pytest.mark.parametrize("into", [False, True])
-def test_input_and_weight_gradients_in_one_launch(nat, T, I, O, into):
+def test_input_and_weight_gradients_in_one_launch(nat, ext, T, I, O, into):
     """Both kernels (single CTAs, CTA pairs), sizes that they leave to two launches, cut and uncut sums over the tokens,
-    and a weight gradient that is added to what is there."""
+    and a weight gradient that is added to what is there.  The bounds are those of the pieces that the launch is cut into."""
     torch.manual_seed(T + I + O)
     dy, x, w = _bf(T, O), _bf(T, I), _bf(O, I)
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     dw_into, db_into = (_bf(O, I), _bf(O)) if into and O % 64 == 0 else (None, None)
-    before = [t.double() if t is not None else 0 for t in (dw_into, db_into)]
+    before = [t.double() if t is not None else None for t in (dw_into, db_into)]
     dx, dw, db = nat.linear_bwd(dy, x, w, True, True, O % 64 == 0, err, dw_into, db_into)
     assert int(err.item()) == 0
     assert (dw is None) == (dw_into is not None)
-    dyd, xd, wd = dy.double(), x.double(), w.double()
-    # a cut sum is rounded once per piece and once per addition: up to eight pieces, each addition's rounding of the size of
-    # the partial sums, which for independent signs stay within six times abs / sqrt(n)
-    def check(got, ref, mag, k):
-        pieces = 16 * 2.0 ** -8 * 6 * mag / k ** 0.5
-        bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -23 * mag + pieces
-        assert float(((got.double() - ref).abs() / bound).max()) <= 1.0
-    check(dx, dyd @ wd, dyd.abs() @ wd.abs(), O)
-    check(dw if dw is not None else dw_into, dyd.t() @ xd + before[0], dyd.abs().t() @ xd.abs() + abs(before[0]), T)
+    pair_x, units_x, alone_x = _tiles(ext, T, I, O)
+    pair_w, units_w, alone_w = _tiles(ext, O, I, T)
+    pieces_x, pieces_w = alone_x, alone_w
+    if pair_x == pair_w:
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        cut_w, cut_x, swap, extra = (ctypes.c_int(0) for _ in range(4))
+        if ext.fcxGemmDualPlan(units_w, _cdiv(T, 64), alone_w, units_x, _cdiv(O, 64), alone_x, sms // 2 if pair_x else sms,
+                               *(ctypes.byref(v) for v in (cut_w, cut_x, swap, extra))):
+            pieces_x, pieces_w = cut_x.value, cut_w.value
+    _close_in_pieces(dx, dy.t(), w, pieces_x)
+    _close_in_pieces(dw if dw is not None else dw_into, dy, x, pieces_w, before[0])
     if O % 64 == 0:
-        _close(db if db is not None else db_into, dyd.sum(0) + before[1], dyd.abs().sum(0) + abs(before[1]), max(8, T // 8))
+        dyd, b0 = dy.double(), before[1] if before[1] is not None else torch.zeros(O, dtype=torch.float64, device="cuda")
+        _close(db if db is not None else db_into, dyd.sum(0) + b0, dyd.abs().sum(0) + b0.abs(), max(8, T // 8))
