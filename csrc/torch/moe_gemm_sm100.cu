@@ -84,7 +84,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + 4);
 
   const int nK = (p.K + BK - 1) / BK;
-  fcxpdl::pdlRelease();
   if (threadIdx.x < 64) fcxpdl::pdlWait();  // the row counts come from the kernel before
   if ((int)threadIdx.x < p.L) rowsOf[threadIdx.x] = max(0, min(p.rows[threadIdx.x], p.capL));
   if (threadIdx.x == 0) {
@@ -113,6 +112,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   clusterSync();  // the peer's barriers exist before anything arrives on them
   fenceAfter();
   const uint32_t tmemBase = *tmemBaseSlot;
+  fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
   const int nTiles = tileStart[p.L];
   const int bn = tileCols, bnh = bn / 2, COLS = UP ? bnh : bn;  // COLS: result columns per tile

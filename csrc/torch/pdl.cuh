@@ -7,6 +7,9 @@
 // The pointer parameters of such a kernel carry no __restrict__: what they point to may still be written, by the kernel
 // before, while this one is resident.  For a `const ... __restrict__` pointer the compiler may use the non-coherent load
 // path, which is for memory that nobody writes while the kernel lives, and may move a load across the wait.
+//
+// A kernel that allocates TMEM calls pdlRelease() after its allocation: a successor that allocated first would hold the
+// columns while it waits for this kernel, which waits for the columns.
 #pragma once
 #include <cuda_runtime.h>
 

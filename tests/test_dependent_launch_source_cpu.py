@@ -31,6 +31,12 @@ def test_no_load_of_a_predecessors_memory_may_take_the_read_only_path(name):
     assert "__restrict__" not in head and "__ldg" not in body and "ld.global.nc" not in body
 
 
+@pytest.mark.parametrize("name", sorted(n for n, (_, body) in KERNELS.items() if "tcgen05.alloc" in body and "pdlRelease" in body))
+def test_successors_come_up_only_after_the_tmem_allocation(name):
+    body = KERNELS[name][1]
+    assert body.index("pdlRelease") > body.index("tcgen05.alloc")
+
+
 @pytest.mark.parametrize("name", sorted(LAUNCHED & set(KERNELS)))
 def test_every_kernel_launched_that_way_waits_for_its_predecessor(name):
     assert "pdlWait()" in KERNELS[name][1]
