@@ -12,7 +12,7 @@
 // columns apart, and an epilogue thread needs nobody else's values; the [rows, 2F] intermediate never reaches memory
 // (at 16384 rows and F = 14336 that is 0.94 GB written and read again).  Where the tiles are few, a tile is 256 x 128
 // columns instead, so that the chain of K steps of a small layer is spread over more SMs; which of the two takes fewer
-// waves times the time of a K step (moeTileColumns) depends on the row counts and is decided by every CTA for itself.
+// waves times the time of a wave (moeTileColumns) depends on the row counts and is decided by every CTA for itself.
 //
 // Pipeline, barriers and bounded waits are those of the pair kernel in gemm2_sm100.cu.
 #include "../kernels/prims.cuh"
@@ -56,12 +56,16 @@ struct GroupParams {
   int topk;
 };
 
-// 256 or 128 accumulator columns per tile for `rowBlocks` 256-row blocks and `cols` columns.  A K block of the narrow tile
-// takes a little over half of the wide one's time: at 512 tokens, H 1024, F 2048 and 4 experts the gate / up product took
-// 23 us in three waves of narrow tiles and about 36 us in two waves of wide ones.
-__host__ __device__ inline int moeTileColumns(long long rowBlocks, int cols, int pairs) {
+// 256 or 128 accumulator columns per tile for `rowBlocks` 256-row blocks, `cols` columns and sums of length K.  Narrow tiles
+// where they take no more waves.  Otherwise a narrow wave costs about 0.7 to 0.85 of a wide one, which more waves (3 for 2, 5
+// for 3, up to twice as many) eat up, except for short sums of the gate / up product, whose wide tiles spend their time on
+// the activation.  Measured with cold weights, narrow / wide in us: gate / up 3:2 waves K 512 21.2 / 25.3, 768 25.6 / 25.6, 1024
+// 29.8 / 31.7, 1280 33.8 / 31.8, 2048 45.9 / 39.9, 3328 62.5 / 50.1; 5:3 waves K 512 25.6 / 27.6, 1024 37.9 / 31.5; down 3:2 waves
+// K 1024 39.9 / 35.8, 2816 (7:4) 119.8 / 82.9, 5632 97.3 / 76.8.
+__host__ __device__ inline int moeTileColumns(long long rowBlocks, int cols, int K, bool up, int pairs) {
   const long long wide = (rowBlocks * ((cols + 255) / 256) + pairs - 1) / pairs, narrow = (rowBlocks * ((cols + 127) / 128) + pairs - 1) / pairs;
-  return narrow * 10 < wide * 18 ? 128 : 256;
+  const int tenths = !up || K > 1024 ? 10 : K > 512 ? 15 : 17;  // narrow waves per ten wide ones that still pay
+  return narrow * 10 <= wide * tenths ? 128 : 256;
 }
 
 template <bool UP>
@@ -99,7 +103,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   if (threadIdx.x == 0) {
     int blocks = 0, sum = 0;
     for (int e = 0; e < p.L; e++) blocks += (rowsOf[e] + 2 * BM - 1) / (2 * BM);
-    const int bnHere = moeTileColumns(blocks, UP ? 2 * p.N : p.N, nPairs), cols = UP ? bnHere / 2 : bnHere;
+    const int bnHere = moeTileColumns(blocks, UP ? 2 * p.N : p.N, p.K, UP, nPairs), cols = UP ? bnHere / 2 : bnHere;
     for (int e = 0; e < p.L; e++) {
       tileStart[e] = sum;
       sum += (rowsOf[e] + 2 * BM - 1) / (2 * BM) * ((p.N + cols - 1) / cols);
@@ -311,7 +315,7 @@ cudaError_t launchGroup(const CUtensorMap &a, const CUtensorMap &h, const Weight
 
 }  // namespace
 
-extern "C" int fcxMoeTileColumns(int rowBlocks, int cols, int pairs) { return moeTileColumns(rowBlocks, cols, pairs); }
+extern "C" int fcxMoeTileColumns(int rowBlocks, int cols, int K, int up, int pairs) { return moeTileColumns(rowBlocks, cols, K, up != 0, pairs); }
 
 extern "C" cudaError_t fcxMoeUpGrouped(const void *x, const void *const *w, void *h, const int *rows, int L, int capL, int H, int F,
                                        const int *ldw, int *errFlag, cudaStream_t s) {

@@ -20,8 +20,9 @@ cudaError_t fcxMoeUpGrouped(const void *x, const void *const *w, void *h, const 
 cudaError_t fcxMoeDownGrouped(const FcxDevComm *dc, const void *h, const void *const *w, const int *rows, int L, int capL, int H, int F, int ldh,
                               const int *ldw, const void *rowInfo, size_t combineOff, size_t doneOff, int topk, int *errFlag, int *gridOut,
                               cudaStream_t s);
-// Accumulator columns of a tile (256 or 128) for that many 256-row blocks and columns; the kernels decide for themselves.
-int fcxMoeTileColumns(int rowBlocks, int cols, int pairs);
+// Accumulator columns of a tile (256 or 128) for that many 256-row blocks and columns and sums of length K; the kernels decide for
+// themselves.
+int fcxMoeTileColumns(int rowBlocks, int cols, int K, int up, int pairs);
 #ifdef __cplusplus
 }
 #endif

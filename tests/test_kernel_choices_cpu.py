@@ -87,11 +87,20 @@ def test_fp8_tile(ext):
 
 
 def test_moe_tile(ext):
+    """Narrow tiles only where they were measured to be faster: as many waves, or a few more for short gate / up sums."""
     for blocks in (0, 1, 5, 74, 500):
         for cols in (8, 128, 1024, 28672):
-            assert ext.fcxMoeTileColumns(blocks, cols, 74) in (128, 256)
-    assert ext.fcxMoeTileColumns(68, 28672, 74) == 256
-    assert ext.fcxMoeTileColumns(6, 1024, 74) == 128  # 24 wide tiles on 74 pairs
+            for k in (8, 512, 1024, 14336):
+                for up in (0, 1):
+                    assert ext.fcxMoeTileColumns(blocks, cols, k, up, 74) in (128, 256)
+    for up in (0, 1):
+        assert ext.fcxMoeTileColumns(68, 28672, 4096, up, 74) == 256
+        assert ext.fcxMoeTileColumns(6, 1024, 2048, up, 74) == 128  # 24 wide or 48 narrow tiles on 74 pairs: one wave
+    three_for_two = (6, 4096)  # 96 wide tiles, 192 narrow ones
+    assert [ext.fcxMoeTileColumns(*three_for_two, k, 1, 74) for k in (512, 1024, 1280, 2048, 3328)] == [128, 128, 256, 256, 256]
+    assert [ext.fcxMoeTileColumns(*three_for_two, k, 0, 74) for k in (512, 1024, 5632)] == [256] * 3
+    five_for_three = (11, 4096)  # 176 and 352
+    assert [ext.fcxMoeTileColumns(*five_for_three, k, 1, 74) for k in (512, 1024, 2560)] == [128, 256, 256]
 
 
 def test_two_products_in_one_launch_cover_every_unit_once(ext):
