@@ -6,11 +6,11 @@ Each case touches more than the 126 MB L2 but holds at most a few GB, runs a
 couple of warm-up launches and three measured ones, and prints the
 CUDA-event time with the achieved fraction of the measured HBM copy rate
 (MEASURED_PEAKS.json, else 6.65 TB/s).  Cases: adamw, cross_entropy,
-layernorm_fwd, layernorm_bwd, bias_gelu, emu_allreduce (8 emulated ranks,
+layernorm_fwd, layernorm_bwd, bias_gelu, bias_gelu_bwd, col_sum, emu_allreduce (8 emulated ranks,
 two-shot kernel, one cooperative launch on this GPU), emu_allgather, gemm / gemm_one_cta
 (tcgen05 GEMM, against the measured cuBLAS rate), gemm_fp8 (block-scaled e4m3 GEMM), moe_dispatch and moe_layer
 (expert-parallel kernels on a one-rank communicator), emu_allreduce_zc / emu_allreduce_ll / emu_sendrecv (zero-copy,
-LL and grouped send/recv kernels on emulated ranks), gemm_dgrad / gemm_wgrad (transposed-operand GEMMs), gemm_ag /
+LL and grouped send/recv kernels on emulated ranks), gemm_dgrad / gemm_wgrad (transposed-operand GEMMs), linear_bwd (both in one launch), gemm_ag /
 gemm_rs (fused all-gather / reduce-scatter GEMMs on a one-rank communicator)."""
 from __future__ import annotations
 
@@ -81,11 +81,19 @@ def main():
             dy = torch.randn_like(y)
             ms = timed(lambda: nat.layernorm_bwd(dy, res, g, mean, rstd, d))
             nbytes = M * C * 2 * 4
-    elif args.case == "bias_gelu":
+    elif args.case in ("bias_gelu", "bias_gelu_bwd", "col_sum"):
         M, C = 32768, 4096
         x, b = torch.randn(M, C, device="cuda").bfloat16(), torch.randn(C, device="cuda").bfloat16()
-        ms = timed(lambda: nat.bias_gelu_fwd(x, b))
-        nbytes = M * C * 2 * 2
+        if args.case == "bias_gelu":
+            ms = timed(lambda: nat.bias_gelu_fwd(x, b))
+            nbytes = M * C * 2 * 2
+        elif args.case == "bias_gelu_bwd":
+            dy = torch.randn_like(x)
+            ms = timed(lambda: nat.bias_gelu_bwd(dy, x, b))
+            nbytes = M * C * 2 * 3
+        else:
+            ms = timed(lambda: nat.col_sum(x))
+            nbytes = M * C * 2
     elif args.case in ("emu_allreduce", "emu_allgather"):
         from flagcx_b200.wrapper import FLAGCXLibrary
         lib = FLAGCXLibrary()
@@ -142,23 +150,27 @@ def main():
             ms = timed(lambda: lib.call("flagcxEmuCollective", emu, 6, kind, ctas, s, r, count, 7, 7, ctypes.c_float(1.0), 0, 0, None, st))
             nbytes = n * count * 4 * 2 if zc else n * count * 4 * (1 + 2 * (n - 1) * 2 + 1)  # zc: every element read once and written once per rank
         lib.call("flagcxEmuDestroy", emu)
-    elif args.case in ("gemm_dgrad", "gemm_wgrad", "gemm_ag", "gemm_rs"):
-        # the backward GEMMs of a linear layer (operands read transposed in place; the weight gradient splits K) and
+    elif args.case in ("gemm_dgrad", "gemm_wgrad", "linear_bwd", "gemm_ag", "gemm_rs"):
+        # the backward GEMMs of a linear layer (operands read transposed in place; the weight gradient splits K), both in one
+        # launch, and
         # the fused all-gather / reduce-scatter forms on a one-rank communicator: the kernels of several ranks, asked for
         # explicitly (one rank takes the plain GEMM otherwise), with this GPU as its own peer (flags, staging, tail reduction)
         err = torch.zeros(1, dtype=torch.int32, device="cuda")
         pk = ROOT / "MEASURED_PEAKS.json"
         tf_peak = json.loads(pk.read_text())["bf16_tflops"] if pk.exists() else 1590.0
-        if args.case in ("gemm_dgrad", "gemm_wgrad"):
-            T, O, I = 8192, 4096, 4096
+        if args.case in ("gemm_dgrad", "gemm_wgrad", "linear_bwd"):
+            T, O, I = 8192, 4096, 4096 if args.case != "linear_bwd" else 1024
             dy = (torch.randn(T, O, device="cuda") * 0.1).bfloat16()
             w = (torch.randn(O, I, device="cuda") * 0.1).bfloat16()
             x = (torch.randn(T, I, device="cuda") * 0.1).bfloat16()
             if args.case == "gemm_dgrad":
                 ms = timed(lambda: nat.gemm(dy, w, False, True, None, 0, err))
-            else:
+            elif args.case == "gemm_wgrad":
                 ms = timed(lambda: nat.gemm(dy, x, True, True, None, 0, err))
             flops = 2.0 * T * O * I
+            if args.case == "linear_bwd":
+                ms = timed(lambda: nat.linear_bwd(dy, x, w, True, True, False, err))
+                flops *= 2
         else:
             import os
             os.environ.setdefault("FLAGCX_HEAP_USER_BYTES", "1G")
