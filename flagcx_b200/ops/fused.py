@@ -154,9 +154,11 @@ def gemm(a, b, a_mn: bool = False, b_mn: bool = False, bias=None, split_k: int =
 
 
 class _Linear(torch.autograd.Function):
-    """For parameters whose gradients are added in place; the others take the same path in native code.  y = x w^T (+ bias) with all three GEMMs (forward, input gradient, weight gradient) on the library's own
-    tcgen05 kernel: the backward operands are read transposed in place, the weight gradient splits its long
-    reduction over the tokens across CTAs, the bias gradient is the library's column-sum kernel."""
+    """y = x w^T (+ bias) for parameters whose gradients are added in place; the others take the same path in native code.
+
+    All three GEMMs (forward, input gradient, weight gradient) run on the library's own tcgen05 kernels: the backward
+    operands are read transposed in place, the weight gradient splits its long reduction over the tokens across CTAs,
+    the bias gradient is the library's column-sum kernel."""
 
     @staticmethod
     def forward(ctx, x, w, bias):
