@@ -96,12 +96,13 @@ flagcxResult_t flagcxEmuCollective(flagcxEmu_t e, flagcxCommOp_t op, const char 
     FCX_WARN("emulation needs all %d x %d CTAs resident at once (%d SMs)", e->n, nctas, sms);
     return flagcxInvalidArgument;
   }
+  // an absent rank is one whose kernel finds no elements to send: enough for the low-latency reductions, which have no barrier
+  if (e->absent && k != FCX_K_AR_LL && k != FCX_K_RS_LL && k != FCX_K_REDUCE_LL) return flagcxNotSupported;
   const int n = e->n;
   const size_t es = dtypeSize(dt);
   FcxEmuRanks l;
   memset(&l, 0, sizeof l);
   memcpy(l.dc, e->host, sizeof(FcxDevComm) * n);
-  l.absent = e->absent;
   FcxCollArgs *as = l.args;
   uint64_t seq = ++e->seq;
   for (int r = 0; r < n; r++) {
@@ -116,7 +117,7 @@ flagcxResult_t flagcxEmuCollective(flagcxEmu_t e, flagcxCommOp_t op, const char 
     a.seq = seq;
     a.send = send ? send[r] : nullptr;
     a.recv = recv ? recv[r] : nullptr;
-    a.count = count;
+    a.count = e->absent >> r & 1u ? 0 : count;
     a.sendHeapOff = a.recvHeapOff = ~0ull;
     a.sendSeg = a.recvSeg = FCX_SEG_NONE;
     if (k == FCX_K_AR_ZC || k == FCX_K_RS_ZC || k == FCX_K_REDUCE_ZC || k == FCX_K_MOVE_ZC) {

@@ -149,8 +149,9 @@ flagcxResult_t flagcxEmuCollective(flagcxEmu_t emu, flagcxCommOp_t op, const cha
 flagcxResult_t flagcxEmuSendRecv(flagcxEmu_t emu, int nops, const int *srcRank, const int *dstRank, void *const *sendbuf,
                                  void *const *recvbuf, const size_t *bytes, int ctasPerOp, void *cudaStream);
 flagcxResult_t flagcxEmuGetError(flagcxEmu_t emu, int *code);
-/* Ranks (bit r: rank r) that take no part in the collectives from here on, like a process that never joins: the other
- * ranks' waits run out after FLAGCX_KERNEL_TIMEOUT_MS.  For tests; the group is good for nothing but destroying afterwards. */
+/* Ranks (bit r: rank r) that send nothing from here on, like a process that never joins: the other ranks' waits run out after
+ * FLAGCX_KERNEL_TIMEOUT_MS.  For tests of the low-latency reductions (other kinds are refused); the group is good for nothing
+ * but destroying afterwards. */
 flagcxResult_t flagcxEmuSetAbsent(flagcxEmu_t emu, unsigned int ranks);
 /* What flagcxCommGetDeviceError tells of a real rank. */
 flagcxResult_t flagcxEmuGetDeviceError(flagcxEmu_t emu, int rank, int *code, int *peer, int *where, unsigned long long *expected,

@@ -126,6 +126,15 @@ __device__ __forceinline__ uint4 llLoad(const char *line) {
   return v;
 }
 
+// The pair of lines of a peer's unit is looked at once more for the report: the tag of an earlier collective tells a peer that
+// is behind from one that never wrote.  Kept out of the wait itself, which it would slow down.
+static __device__ __noinline__ void giveUpOnLine(const FcxDevComm &dc, uint32_t code, int peer, size_t llOff, size_t u, int cta, uint32_t tag,
+                                                 uint64_t seq) {
+  const char *line = dc.heap[dc.rank] + llOff + (size_t)peer * FCX_LL_SLOT_BYTES + u * 32;
+  const uint32_t first = llLoad(line).y, second = llLoad(line + 16).y;
+  giveUp(dc, code, peer, FCX_WAIT_LL, cta, tag, first != tag ? first : second, seq);
+}
+
 // mode 0: all-reduce (everybody sends its whole vector to everybody and reduces);
 // mode 1: reduce-scatter (piece p goes to rank p, every rank reduces the pieces it received and its own);
 // mode 2: reduce (everybody sends its whole vector to the root, which reduces).
@@ -187,14 +196,14 @@ __device__ void arLL(const FcxDevComm &dc, const FcxCollArgs &a, uint64_t seq, i
       if (!pending) break;
       if (spins == 0) t0 = globalTimerNs();
       if ((++spins & 63u) == 0u) {
+        const int late = __ffs(pending) - 1;
         if (*(volatile unsigned int *)&localOf(dc)->abortSeen) return;
-        const bool late = globalTimerNs() - t0 > dc.timeoutNs;
-        if (late || ((spins & 1023u) == 0u && *dc.abortWord)) {
-          // looked at once more for the report: the tag of an earlier collective tells a peer that is behind from one that never wrote
-          const int p = __ffs(pending) - 1;
-          const char *line = lines + (size_t)p * FCX_LL_SLOT_BYTES + u * 32;
-          const uint32_t first = llLoad(line).y, second = llLoad(line + 16).y;
-          giveUp(dc, late ? FCX_ERR_TIMEOUT : FCX_ERR_ABORT, p, FCX_WAIT_LL, cta, tag, first != tag ? first : second, seq);
+        if (globalTimerNs() - t0 > dc.timeoutNs) {
+          giveUpOnLine(dc, FCX_ERR_TIMEOUT, late, llOff, u, cta, tag, seq);
+          return;
+        }
+        if ((spins & 1023u) == 0u && *dc.abortWord) {
+          giveUpOnLine(dc, FCX_ERR_ABORT, late, llOff, u, cta, tag, seq);
           return;
         }
       }
@@ -1067,14 +1076,12 @@ __global__ void __launch_bounds__(FCX_THREADS, 1) fcxP2pKernel(FcxDevComm dc, Fc
 // all emulated ranks are resident at once and may wait on one another.
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxCollEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
-  if (l.absent >> (blockIdx.x / ctasPerRank) & 1u) return;
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
   fcxCollBody<TIn, TOut>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxMoveEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
-  if (l.absent >> (blockIdx.x / ctasPerRank) & 1u) return;
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);

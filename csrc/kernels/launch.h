@@ -10,7 +10,6 @@
 struct FcxEmuRanks {
   FcxDevComm dc[FCX_MAX_RANKS];
   FcxCollArgs args[FCX_MAX_RANKS];
-  unsigned int absent;  // bit r: rank r takes no part (its CTAs leave at once), so that the others' waits run out
 };
 
 #ifdef __cplusplus

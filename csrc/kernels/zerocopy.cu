@@ -16,14 +16,12 @@ __global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcMoveKernel(FcxDevComm dc,
 }
 template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcReduceEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
-  if (l.absent >> (blockIdx.x / ctasPerRank) & 1u) return;
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
   fcxZcReduceBody<TIn, TOut>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxZcMoveEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
-  if (l.absent >> (blockIdx.x / ctasPerRank) & 1u) return;
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);

@@ -403,6 +403,8 @@ def test_low_latency_wait_that_runs_out_reports_the_tag_it_saw(lib, monkeypatch,
         lib.call("flagcxEmuSetAbsent", emu.h, 1 << 2)
         with pytest.raises(AssertionError, match="gave up, code 1"):
             emu.coll(op, kind, 1, send, recv, count, torch.float32)
+        with pytest.raises(Exception):  # kinds with barriers: an absent rank would still take part in those
+            emu.coll("allgather", "ag", 1, send, recv, 4, torch.float32)
         for r in range(n):
             code, peer, where = (ctypes.c_int() for _ in range(3))
             want, seen = ctypes.c_ulonglong(), ctypes.c_ulonglong()
