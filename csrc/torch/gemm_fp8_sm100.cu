@@ -333,7 +333,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
             if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
             fenceAfter();
             const uint32_t sa = smemAddr(tiles + stage * PSTAGE_BYTES), sb = sa + A_BYTES;
-  #pragma unroll
+#pragma unroll
             for (int k = 0; k < BK / 32; k++)
               mmaF8Pair(tmemBase + (uint32_t)buf * PN, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, k > 0 ? 1u : 0u);
             mmaCommitPair(&emptyBar[stage]);
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256) quantActKernel(const __nv_bfloat16 *x, __
   const int sub = threadIdx.x / LANES, l = threadIdx.x % LANES;
   const uint64_t first = (uint64_t)blockIdx.x * PER_CTA * UNROLL + sub;
   // One division for the first block, additions for the others: a 64-bit division and remainder for every block, once to
-  // load and once to store it, took longer than the loads (39 us in place of 15 at 8192 x 4096).
+  // load and once to store it, took longer than the loads (39 us in place of 23 at 8192 x 4096, 101 MB).
   uint32_t row0, kb0;
   if (total <= 0xffffffffu) {
     row0 = (uint32_t)first / nKb;
@@ -557,8 +557,10 @@ cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap 
 }  // namespace
 
 // Which tile: 0 = 256 x 256 on CTA pairs, 128 or 64 = 128 x that many columns on single CTAs.  The time is about the
-// number of waves times the time of one 128-deep slice of a tile, in nanoseconds: 7, 14 and 28 waves of 32 slices took 177,
-// 212 and 396 us at 8192 x 4096 x 4096.
+// number of waves times the time of one 128-deep slice of a tile, in nanoseconds.  Measured, us for pairs / 128 / 64 columns:
+// 8192 x 4096 x 4096 180 / 215 / 396, 8192 x 1024 x 4096 60.6 / 65.3 / 102.5, 4096 x 4096 x 1024 33.0 / 33.2 / 54.8, 3000 x 2000 x 4096
+// 54.5 / 50.1 / 87.3, 1024 x 4096 x 2048 17.4 / 19.6 / 32.1, 512 x 4096 x 4096 29.7 / 19.3 / 32.1, 1024 x 1024 x 1024 9.9 / 7.3 / 6.8,
+// 333 x 1792 x 4096 27.0 / 18.2 / 17.6: the rule takes the fastest at each.
 extern "C" int fcxGemmFp8Tile(int M, int N, int sms) {
   const int m1 = (M + 127) / 128, m2 = (M + 255) / 256;
   auto waves = [](long long tiles, int slots) { return (double)((tiles + slots - 1) / slots); };

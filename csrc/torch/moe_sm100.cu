@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, con
         if (wk == 0.f) continue;  // a choice that was not dispatched (expert id out of range, capacity overflow) has no row
         uint4 v = *(const uint4 *)(ret + ((t * K + k) * H) + c * 8);
         const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&v;
-  #pragma unroll
+#pragma unroll
         for (int j = 0; j < 4; j++) {
           float2 f = __bfloat1622float2(h2[j]);
           acc[2 * j] += wk * f.x;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, con
       }
       uint4 o;
       __nv_bfloat162 *o2 = (__nv_bfloat162 *)&o;
-  #pragma unroll
+#pragma unroll
       for (int j = 0; j < 4; j++) o2[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
       *(uint4 *)(out + t * H + c * 8) = o;
     }

@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdDxKernel(const bf16 *dy
 // read dy and x again: 33 MB at 8192 x 1024).  The three rows of a warp stream through a ring in shared memory.  A thread
 // holds 32 columns' dgamma and dbeta sums, which leaves no room for the row: it is looked at twice in shared memory, once
 // for the two means and once for the results, so that sixteen warps fit on an SM (with eight that keep the row in
-// registers the arithmetic set the pace: 19 us at 8192 x 1024).  At the end the warps fold their sums in shared memory and
+// registers the arithmetic set the pace: 19 us at 8192 x 1024 without the fold; with it 19.5 now, 21.6 with inputs beyond L2, where the
+// two kernels that each read dy and x took 26).  At the end the warps fold their sums in shared memory and
 // a CTA leaves [2][C] of them in `partial` for lnParamFoldKernel.
 template <int MAXV, int STAGES, int LN_WARPS>
 __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdFusedKernel(const bf16 *dy, const bf16 *x, const bf16 *gamma, const float *mean,
@@ -466,7 +467,8 @@ __global__ void __launch_bounds__(256) biasGeluFwdKernel(const bf16 *x, const bf
 // folded by colSumFoldKernel).  A CTA owns VX * 8 columns (all 256 threads side by side on wide rows) and every gridDim.y-th
 // group of 256 / VX rows, four rows (eight 16-byte loads) in flight per thread; a thread keeps its eight columns throughout.
 // Bound by memory (dy, x, dx: 201 MB and 30 us at 8192 x 4096) with the arithmetic close behind.  Blocks of 64 columns with a
-// fold in the last CTA, as in the plain column sum, took 55 us: their CTAs lived for eight rows per thread.
+// fold in the last CTA took 55 us: their CTAs lived for eight rows per thread.  With the fold kernel 49 us (53 while its pointers were
+// restrict-qualified).
 __global__ void __launch_bounds__(256) biasGeluBwdKernel(const bf16 *dy, const bf16 *x, const bf16 *bias, bf16 *dx, float *partial, int M, int C,
                                                          int VX) {
   __shared__ float red[2048];
