@@ -334,26 +334,43 @@ __global__ void __launch_bounds__(LN_WARPS * 32, 1) lnBwdFusedKernel(const bf16 
   }
 }
 
-// dgamma / dbeta from the `parts` partial sums of lnBwdFusedKernel: a CTA folds 32 of the 2 C columns, eight groups of
-// lanes an eighth of the parts each.
-__global__ void __launch_bounds__(256) lnParamFoldKernel(const float *partial, int parts, int C, bf16 *dgamma, bf16 *dbeta, int accumulate) {
-  __shared__ float red[8][33];
-  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // 2 C is a multiple of 32
-  fcxpdl::pdlRelease();
-  fcxpdl::pdlWait();
+// The `parts` partial sums of each of `width` columns -> one, as bf16, (+)= *target(column).  A CTA folds 32 columns with 32 warps, a
+// 32nd of the parts each and up to eight loads of them in flight: the fold is a chain of memory latencies and nothing else.
+// With eight warps of four loads in flight (148 parts: five turns, 296: ten) a fold kept the stream for 4.6 us in a GPT-2-medium
+// step at C = 1024 (LayerNorm) and 5.4 at C = 4096 (bias of the GELU), and keeps it for 3.3 and 3.4 now.
+constexpr int FOLD_WARPS = 32;
+template <typename Target>
+__device__ __forceinline__ void foldColumns(const float *partial, int parts, int width, int accumulate, Target target) {
+  __shared__ float red[FOLD_WARPS][33];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // width is a multiple of 32
   float t = 0.f;
-#pragma unroll 4
-  for (int p = grp; p < parts; p += 8) t += partial[(size_t)p * 2 * C + c];
+#pragma unroll 8
+  for (int p = grp; p < parts; p += FOLD_WARPS) t += partial[(size_t)p * width + c];
   red[grp][lane] = t;
   __syncthreads();
   if (grp == 0) {
     t = 0.f;
 #pragma unroll
-    for (int g = 0; g < 8; g++) t += red[g][lane];
-    bf16 *dst = c < C ? dgamma + c : dbeta + (c - C);
+    for (int g = 0; g < FOLD_WARPS; g++) t += red[g][lane];
+    bf16 *dst = target(c);
     if (accumulate) t += __bfloat162float(*dst);
     *dst = __float2bfloat16_rn(t);
   }
+}
+
+// dgamma / dbeta from the [2][C] partial sums of the LayerNorm backward kernels.
+__global__ void __launch_bounds__(FOLD_WARPS * 32) lnParamFoldKernel(const float *partial, int parts, int C, bf16 *dgamma, bf16 *dbeta,
+                                                                     int accumulate) {
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
+  foldColumns(partial, parts, 2 * C, accumulate, [&](int c) { return c < C ? dgamma + c : dbeta + (c - C); });
+}
+
+// A bias gradient from the [C] partial sums of biasGeluBwdKernel.
+__global__ void __launch_bounds__(FOLD_WARPS * 32) colSumFoldKernel(const float *partial, int parts, int C, bf16 *out, int accumulate) {
+  fcxpdl::pdlRelease();
+  fcxpdl::pdlWait();
+  foldColumns(partial, parts, C, accumulate, [&](int c) { return out + c; });
 }
 
 // Backward, part 2, for rows wider than 1024: dgamma[c] = sum_r dy[r,c] * xhat[r,c], dbeta[c] = sum_r dy[r,c].
@@ -515,26 +532,6 @@ __global__ void __launch_bounds__(256) biasGeluBwdKernel(const bf16 *dy, const b
     float t = 0.f;
     for (int y = 0; y < RY; y++) t += red[y * VX * 8 + c];
     partial[(size_t)blockIdx.y * C + blockIdx.x * VX * 8 + c] = t;
-  }
-}
-
-// out[c] (+)= the sum of `parts` partial column sums; a CTA folds 32 columns, eight groups of lanes an eighth of the parts each.
-__global__ void __launch_bounds__(256) colSumFoldKernel(const float *partial, int parts, int C, bf16 *out, int accumulate) {
-  __shared__ float red[8][33];
-  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;  // C is a multiple of 64
-  fcxpdl::pdlRelease();
-  fcxpdl::pdlWait();
-  float t = 0.f;
-#pragma unroll 4
-  for (int p = grp; p < parts; p += 8) t += partial[(size_t)p * C + c];
-  red[grp][lane] = t;
-  __syncthreads();
-  if (grp == 0) {
-    t = 0.f;
-#pragma unroll
-    for (int g = 0; g < 8; g++) t += red[g][lane];
-    if (accumulate) t += __bfloat162float(out[c]);
-    out[c] = __float2bfloat16_rn(t);
   }
 }
 
@@ -936,7 +933,7 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
     e = fcxpdl::launchPdl(kernel, grid, WARPS * 32, smem, s, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)gamma, mean, rstd,
                                       (const bf16 *)dres, (bf16 *)dx, partial, M, C);
     if (e != cudaSuccess) return e;
-    return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, 256, 0, s, (const float *)partial, grid, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
+    return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, FOLD_WARPS * 32, 0, s, (const float *)partial, grid, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
   }
   constexpr int WARPS = 8;
   const size_t smem = (size_t)WARPS * 3 * 2 * C * 2;  // warps x 3-deep ring x (dy, x) x row bytes <= 192 KB
@@ -950,7 +947,7 @@ cudaError_t fcxLayerNormBwd(const void *dy, const void *x, const void *gamma, co
   const int parts = lnParts(M);
   e = fcxpdl::launchPdl(lnBwdParamKernel, dim3(C / 64, parts), 256, 0, s, (const bf16 *)dy, (const bf16 *)x, mean, rstd, partial, M, C);
   if (e != cudaSuccess) return e;
-  return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, 256, 0, s, (const float *)partial, parts, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
+  return fcxpdl::launchPdl(lnParamFoldKernel, 2 * C / 32, FOLD_WARPS * 32, 0, s, (const float *)partial, parts, C, (bf16 *)dgamma, (bf16 *)dbeta, accumulate);
 }
 
 cudaError_t fcxBiasGeluFwd(const void *x, const void *bias, void *y, size_t M, int C, cudaStream_t s) {
@@ -986,7 +983,7 @@ cudaError_t fcxBiasGeluBwd(const void *dy, const void *x, const void *bias, void
   cudaError_t e = fcxpdl::launchPdl(biasGeluBwdKernel, dim3(C / 8 / vx, parts), 256, 0, s, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)bias,
                                     (bf16 *)dx, partial, M, C, vx);
   if (e != cudaSuccess) return e;
-  return fcxpdl::launchPdl(colSumFoldKernel, C / 32, 256, 0, s, (const float *)partial, parts, C, (bf16 *)dbias, accumulate);
+  return fcxpdl::launchPdl(colSumFoldKernel, C / 32, FOLD_WARPS * 32, 0, s, (const float *)partial, parts, C, (bf16 *)dbias, accumulate);
 }
 
 cudaError_t fcxColSum(const void *a, void *out, int M, int C, int accumulate, cudaStream_t s) {
