@@ -6,6 +6,7 @@
 
 #include "flagcx.h"
 #include "flagcx_ext.h"
+#include "embedding.h"
 #include "train_ops.h"
 
 namespace fcxt {
@@ -116,6 +117,44 @@ at::Tensor colSum(const at::Tensor &a, const c10::optional<at::Tensor> &intoT) {
   auto out = into ? *intoT : at::empty({C}, a.options());
   CUDA_OK(fcxColSum(a.data_ptr(), out.data_ptr(), M, C, into ? 1 : 0, cur()));
   return out;
+}
+
+// Whether the embedding kernels take these tensors (else the caller has the library's embedding).
+static bool embeddingTakes(const at::Tensor &tokens, const at::Tensor &wte, const at::Tensor &wpe) {
+  auto table = [](const at::Tensor &t) {
+    return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.is_contiguous() && ((uintptr_t)t.data_ptr() & 15) == 0;
+  };
+  return tokens.is_cuda() && tokens.scalar_type() == at::kLong && tokens.dim() == 2 && table(wte) && table(wpe) && wpe.size(0) >= tokens.size(1) &&
+         wpe.size(1) == wte.size(1) && wte.size(0) < (1ll << 31) && tokens.device() == wte.device() && wpe.device() == wte.device() &&
+         fcxEmbeddingTakes(tokens.numel(), wte.size(1));
+}
+
+// tokens [B, T] -> wte[tokens] + wpe[:T], [B, T, C]
+static at::Tensor embeddingFwd(const at::Tensor &tokens, const at::Tensor &wte, const at::Tensor &wpe) {
+  TORCH_CHECK(embeddingTakes(tokens, wte, wpe) && tokens.is_contiguous(), "embedding_fwd: tensors that embedding_takes refuses");
+  c10::cuda::CUDAGuard g(wte.device());
+  auto x = at::empty({tokens.size(0), tokens.size(1), wte.size(1)}, wte.options());
+  CUDA_OK(fcxEmbeddingFwd(tokens.data_ptr<int64_t>(), wte.data_ptr(), wpe.data_ptr(), x.data_ptr(), (int)tokens.numel(), (int)tokens.size(1),
+                          (int)wte.size(1), (int)wte.size(0), cur()));
+  return x;
+}
+
+// Adds the gradients of both tables to dwte / dwpe, as asked.
+static void embeddingBwd(const at::Tensor &dx, const at::Tensor &tokens, const c10::optional<at::Tensor> &dwte, const c10::optional<at::Tensor> &dwpe,
+                         int64_t vocab) {
+  checkBf16(dx, "dx");
+  c10::cuda::CUDAGuard g(dx.device());
+  const int64_t C = dx.size(-1), T = tokens.size(1);
+  TORCH_CHECK(tokens.is_cuda() && tokens.scalar_type() == at::kLong && tokens.is_contiguous() && dx.numel() == tokens.numel() * C,
+              "dx must be [B, T, C] for int64 tokens [B, T]");
+  auto target = [&](const c10::optional<at::Tensor> &t, int64_t rows, const char *name) -> void * {
+    if (!t.has_value() || !t->defined()) return nullptr;
+    checkBf16(*t, name);
+    TORCH_CHECK(t->dim() == 2 && t->size(0) >= rows && t->size(1) == C, name, " has the wrong shape");
+    return t->data_ptr();
+  };
+  CUDA_OK(fcxEmbeddingBwd(dx.data_ptr(), tokens.data_ptr<int64_t>(), target(dwte, vocab, "dwte"), target(dwpe, T, "dwpe"), (int)tokens.numel(), (int)T,
+                          (int)C, (int)vocab, cur()));
 }
 
 // In place: logits become d(mean loss)/d(logits) * grad_scale; returns per-row losses (fp32).
@@ -271,6 +310,9 @@ PYBIND11_MODULE(_flagcx_torch, m) {
   m.def("bias_gelu_fwd", &fcxt::biasGeluFwd);
   m.def("bias_gelu_bwd", &fcxt::biasGeluBwd, py::arg("dy"), py::arg("x"), py::arg("bias"), py::arg("dbias_into") = py::none());
   m.def("col_sum", &fcxt::colSum, py::arg("a"), py::arg("into") = py::none());
+  m.def("embedding_takes", &fcxt::embeddingTakes);
+  m.def("embedding_fwd", &fcxt::embeddingFwd);
+  m.def("embedding_bwd", &fcxt::embeddingBwd, py::arg("dx"), py::arg("tokens"), py::arg("dwte"), py::arg("dwpe"), py::arg("vocab"));
   m.def("cross_entropy_", &fcxt::crossEntropy);
   m.def("adamw_", &fcxt::adamw, py::arg("master"), py::arg("param"), py::arg("grad"), py::arg("m"), py::arg("v"), py::arg("lr"),
         py::arg("b1"), py::arg("b2"), py::arg("eps"), py::arg("wd"), py::arg("step"), py::arg("grad_scale"), py::arg("zero_grad"),

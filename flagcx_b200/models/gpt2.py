@@ -28,7 +28,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from flagcx_b200.ops import add_layernorm, bias_gelu, cross_entropy, linear, linear_bias_gelu
+from flagcx_b200.ops import add_layernorm, bias_gelu, cross_entropy, embed, linear, linear_bias_gelu
 
 
 def _linear_fn():
@@ -116,7 +116,7 @@ class GPT2(nn.Module):
     def forward(self, tokens, targets):
         """tokens, targets: int64 [B, T] on the GPU.  Returns the mean loss."""
         B, T = tokens.shape
-        x = F.embedding(tokens, self.wte) + self.wpe[:T]
+        x = embed(tokens, self.wte, self.wpe)
         delta = None
         for blk in self.blocks:
             x, delta = blk(x, delta)
@@ -131,13 +131,8 @@ class GPT2(nn.Module):
         """``(parameter, single_use)`` pairs for ``flagcx_b200.ops.enable_direct_grad``: parameters whose gradient this
         model's fused ops can add straight into ``.grad``.  ``single_use`` is False for the token embedding: it is tied
         to the output projection, whose weight gradient is added in place early in the backward pass, while the
-        embedding lookup's own gradient arrives through autograd at the very end."""
-        out = []
-        for p in self.parameters():
-            if p is self.wpe:
-                continue
-            out.append((p, p is not self.wte))
-        return out
+        embedding lookup's own gradient comes at the very end."""
+        return [(p, p is not self.wte) for p in self.parameters()]
 
 
 def flatten_parameters(model: nn.Module, dtype=torch.bfloat16, device="cuda", buffer: torch.Tensor | None = None):

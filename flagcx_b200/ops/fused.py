@@ -52,12 +52,14 @@ class _AddLayerNorm(torch.autograd.Function):
         ctx.save_for_backward(res, gamma, mean, rstd)
         ctx.has_delta = delta is not None
         ctx.params = (gamma, beta)
+        ctx.set_materialize_grads(False)  # the last layer's residual is not used: no zeros are made and read for its gradient
         return res, y
 
     @staticmethod
     def backward(ctx, dres, dy):
         res, gamma, mean, rstd = ctx.saved_tensors
         dres = dres.contiguous() if dres is not None else None
+        dy = dy if dy is not None else torch.zeros_like(res)
         pg, pb = ctx.params
         gg, gb = _direct(pg), _direct(pb)
         if gg is not None and gb is not None:
@@ -72,6 +74,45 @@ class _AddLayerNorm(torch.autograd.Function):
 def add_layernorm(x, delta, gamma, beta, eps: float = 1e-5):
     """Returns ``(x + delta, LayerNorm(x + delta))``; ``delta`` may be None."""
     return _AddLayerNorm.apply(x, delta, gamma, beta, eps)
+
+
+class _Embedding(torch.autograd.Function):
+    """wte[tokens] + wpe[:T]; both gradients are sums of a few rows, added where they belong."""
+
+    @staticmethod
+    def forward(ctx, tokens, wte, wpe):
+        tokens = tokens.contiguous()
+        ctx.save_for_backward(tokens)
+        ctx.params = (wte, wpe)
+        return _n().embedding_fwd(tokens, wte, wpe)
+
+    @staticmethod
+    def backward(ctx, dx):
+        (tokens,) = ctx.saved_tensors
+        outs, targets = [], []
+        for p, need in zip(ctx.params, ctx.needs_input_grad[1:]):
+            g = _direct(p) if need else None
+            if g is not None and g.data_ptr() % 16:
+                g = None
+            new = torch.zeros_like(p) if need and g is None else None
+            outs.append(new)
+            targets.append(g if g is not None else new)
+        dx = dx.contiguous()
+        if dx.data_ptr() % 16:
+            dx = dx.clone()
+        _n().embedding_bwd(dx, tokens, targets[0], targets[1], ctx.params[0].shape[0])
+        for p, new, target in zip(ctx.params, outs, targets):
+            if new is None and target is not None:
+                _done(p)
+        return None, outs[0], outs[1]
+
+
+def embed(tokens, wte, wpe):
+    """``wte[tokens] + wpe[:T]`` for int64 tokens ``[B, T]``.  bf16 tables whose rows are whole 256-column vectors go through
+    one kernel each way (up to 16384 tokens, see embedding.cu); everything else through the library's embedding."""
+    if _n().embedding_takes(tokens, wte, wpe):
+        return _Embedding.apply(tokens, wte, wpe)
+    return torch.nn.functional.embedding(tokens, wte) + wpe[:tokens.shape[1]]
 
 
 class _BiasGelu(torch.autograd.Function):
