@@ -102,7 +102,7 @@ template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     fcxGemmPairKernel(const __grid_constant__ PairArgs args) {
   extern __shared__ uint8_t smemRaw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   volatile int *err = args.errFlag;
   const uint32_t cr = ctaRankInCluster();  // 0 = leader
   const int pair = blockIdx.x >> 1, nPairs = gridDim.x >> 1;
@@ -151,7 +151,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 
   if (warp == 0) {
     // ---- TMA producer (both CTAs): own half of A and of B; bytes counted on the leader's barrier
-    if (lane == 0) {
+    if (electOne()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -179,8 +179,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer: one thread of the leader CTA drives the tensor cores of both SMs
-    if (lane == 0 && cr == 0) {
+    // ---- MMA issuer: one thread of the leader CTA drives the tensor cores of both SMs; the warp waits as one
+    if (cr == 0) {
       int stage = 0, buf = 0;
       uint32_t phase = 0, accPhase = 0;
       bool ok = true;
@@ -189,24 +189,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         const Where w = locate(p, unit);
         const bool aMN = p.aMN, bMN = p.bMN;
         const uint32_t idesc = instrDescPair(aMN, bMN);
-        if (!mbarWait(&accEmpty[buf], accPhase ^ 1, err)) break;
+        if (!__all_sync(0xffffffffu, mbarWait(&accEmpty[buf], accPhase ^ 1, err))) break;
         fenceAfter();
         const uint32_t dTmem = tmemBase + (uint32_t)buf * BN;
         for (int kb = w.kLo; kb < w.kHi; kb++) {
-          if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
           fenceAfter();
-          const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
+          if (electOne()) {
+            const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++) {
-            const uint64_t da = aMN ? smemDescMN(sa + k * 2048, MN_BLOCK_BYTES) : smemDesc(sa + k * 32);
-            const uint64_t db = bMN ? smemDescMN(sb + k * 2048, MN_BLOCK_BYTES) : smemDesc(sb + k * 32);
-            mmaF16Pair(dTmem, da, db, idesc, (kb > w.kLo || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / 16; k++) {
+              const uint64_t da = aMN ? smemDescMN(sa + k * 2048, MN_BLOCK_BYTES) : smemDesc(sa + k * 32);
+              const uint64_t db = bMN ? smemDescMN(sb + k * 2048, MN_BLOCK_BYTES) : smemDesc(sb + k * 32);
+              mmaF16Pair(dTmem, da, db, idesc, (kb > w.kLo || k > 0) ? 1u : 0u);
+            }
+            mmaCommitPair(&emptyBar[stage]);
+            if (kb + 1 == w.kHi) mmaCommitPair(&accFull[buf]);
           }
-          mmaCommitPair(&emptyBar[stage]);
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        mmaCommitPair(&accFull[buf]);
         if (++buf == 2) { buf = 0; accPhase ^= 1; }
       }
     }

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
                                                             const __grid_constant__ CUtensorMap tmC, const Params p) {
   constexpr int STAGES = stages(BN), STAGE_BYTES = stageBytes(BN), ACC_BUFS = 4, COLS = BN / 2;
   extern __shared__ uint8_t smemRaw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   volatile int *err = p.errFlag;
   uint8_t *tiles = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
   uint8_t *epiStage = tiles + STAGES * STAGE_BYTES;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
   fcxpdl::pdlWait();  // everything above touches only this CTA's own memories
 
   if (warp == 8) {
-    if (lane == 0) {
+    if (electOne()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -173,26 +173,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
         }
       }
     }
-  } else if (warp == 9) {
-    if (lane == 0) {
-      int stage = 0, buf = 0;
-      uint32_t phase = 0, accPhase = 0;
-      bool ok = true;
-      const uint32_t idesc = instrDescF8(BM, BN);
-      for (int t = blockIdx.x; t < nTiles && ok; t += gridDim.x) {
-        for (int kb = 0; kb < nK; kb++) {
-          if (!mbarWait(&tmemEmpty[buf], accPhase ^ 1, err)) { ok = false; break; }
-          if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
-          fenceAfter();
+  } else if (warp == 9) {  // the warp waits as one, one lane issues
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, accPhase = 0;
+    bool ok = true;
+    const uint32_t idesc = instrDescF8(BM, BN);
+    for (int t = blockIdx.x; t < nTiles && ok; t += gridDim.x) {
+      for (int kb = 0; kb < nK; kb++) {
+        if (!__all_sync(0xffffffffu, mbarWait(&tmemEmpty[buf], accPhase ^ 1, err) && mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
+        fenceAfter();
+        if (electOne()) {
           const uint32_t dTmem = tmemBase + (uint32_t)buf * BN;
           const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / 32; k++)  // 32 fp8 = 32 bytes further along K inside the 128-byte swizzle row
             mmaF8(dTmem, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, k > 0 ? 1u : 0u);
           mmaCommit(&doneBar[stage]);  // the stage may be refilled and the accumulator read
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-          if (++buf == ACC_BUFS) { buf = 0; accPhase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++buf == ACC_BUFS) { buf = 0; accPhase ^= 1; }
       }
     }
   } else {
@@ -269,7 +269,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
     gemmFp8PairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                       const Params p) {
   extern __shared__ uint8_t smemRaw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   volatile int *err = p.errFlag;
   const uint32_t cr = ctaRankInCluster();  // 0 = leader
   const int pair = blockIdx.x >> 1, nPairs = gridDim.x >> 1;
@@ -302,7 +302,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGS));
     if (warp == 8) {
       // ---- TMA producer (both CTAs): own 128 rows of A, own 128 of the 256 weight rows; bytes counted on the leader's barrier
-      if (lane == 0) {
+      if (electOne()) {
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -321,23 +321,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
         }
       }
     } else if (warp == 9) {
-      // ---- MMA issuer: one thread of the leader CTA
-      if (lane == 0 && cr == 0) {
+      // ---- MMA issuer: one thread of the leader CTA; the warp waits as one
+      if (cr == 0) {
         int stage = 0, buf = 0;
         uint32_t phase = 0, accPhase = 0;
         bool ok = true;
         const uint32_t idesc = instrDescF8(2 * BM, PN);
         for (int t = pair; t < nTiles && ok; t += nPairs) {
           for (int kb = 0; kb < nK; kb++) {
-            if (!mbarWait(&accEmpty[buf], accPhase ^ 1, err)) { ok = false; break; }
-            if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbarWait(&accEmpty[buf], accPhase ^ 1, err) && mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
             fenceAfter();
-            const uint32_t sa = smemAddr(tiles + stage * PSTAGE_BYTES), sb = sa + A_BYTES;
+            if (electOne()) {
+              const uint32_t sa = smemAddr(tiles + stage * PSTAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
-            for (int k = 0; k < BK / 32; k++)
-              mmaF8Pair(tmemBase + (uint32_t)buf * PN, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, k > 0 ? 1u : 0u);
-            mmaCommitPair(&emptyBar[stage]);
-            mmaCommitPair(&accFull[buf]);
+              for (int k = 0; k < BK / 32; k++)
+                mmaF8Pair(tmemBase + (uint32_t)buf * PN, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, k > 0 ? 1u : 0u);
+              mmaCommitPair(&emptyBar[stage]);
+              mmaCommitPair(&accFull[buf]);
+            }
+            __syncwarp();
             if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
             if (++buf == 2) { buf = 0; accPhase ^= 1; }
           }

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
                                                             const FcxDevComm dc, const __grid_constant__ SecondProduct second) {
   constexpr bool PLAIN = MODE == FCX_GEMM_PLAIN || MODE == FCX_GEMM_DUAL;
   extern __shared__ uint8_t smemRaw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   volatile int *err = p0.errFlag;
 
   // ------------------------------------------------------------ communication CTAs (AG mode only)
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
 
   if (warp == 0) {
     // ---- TMA producer
-    if (lane == 0) {
+    if (electOne()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -234,23 +234,23 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer
-    if (lane == 0) {
-      int stage = 0, buf = 0;
-      uint32_t phase = 0, accPhase = 0;
-      bool ok = true;
-      while (ok && it.next(&which, &unit)) {
-        const FcxGemmParams &p = MODE == FCX_GEMM_DUAL && which ? second.p : p0;
-        const Where w = locate(p, MODE == FCX_GEMM_DUAL ? p.M : rows0, unit);
-        const int bn = p.bn;
-        const bool aMN = PLAIN && p.aMN, bMN = PLAIN && p.bMN;
-        const uint32_t idesc = instrDesc(bn, aMN, bMN);
-        if (!mbarWait(&tmemEmpty[buf], accPhase ^ 1, err)) break;
+    // ---- MMA issuer: the warp waits as one, one lane issues
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, accPhase = 0;
+    bool ok = true;
+    while (ok && it.next(&which, &unit)) {
+      const FcxGemmParams &p = MODE == FCX_GEMM_DUAL && which ? second.p : p0;
+      const Where w = locate(p, MODE == FCX_GEMM_DUAL ? p.M : rows0, unit);
+      const int bn = p.bn;
+      const bool aMN = PLAIN && p.aMN, bMN = PLAIN && p.bMN;
+      const uint32_t idesc = instrDesc(bn, aMN, bMN);
+      if (!__all_sync(0xffffffffu, mbarWait(&tmemEmpty[buf], accPhase ^ 1, err))) break;
+      fenceAfter();
+      const uint32_t dTmem = tmemBase + (uint32_t)buf * 256;
+      for (int kb = w.kLo; kb < w.kHi; kb++) {
+        if (!__all_sync(0xffffffffu, mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
         fenceAfter();
-        const uint32_t dTmem = tmemBase + (uint32_t)buf * 256;
-        for (int kb = w.kLo; kb < w.kHi; kb++) {
-          if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
-          fenceAfter();
+        if (electOne()) {
           const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / 16; k++) {
@@ -260,13 +260,14 @@ __global__ void __launch_bounds__(THREADS, 1) fcxGemmKernel(const __grid_constan
             const uint64_t db = bMN ? smemDescMN(sb + k * 2048, MN_BLOCK_BYTES) : smemDesc(sb + k * 32);
             mmaF16(dTmem, da, db, idesc, (kb > w.kLo || k > 0) ? 1u : 0u);
           }
-          mmaCommit(&emptyBar[stage]);  // the stage may be refilled once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          mmaCommit(&emptyBar[stage]);                         // the stage may be refilled once these MMAs have read it
+          if (kb + 1 == w.kHi) mmaCommit(&tmemFull[buf]);      // accumulator complete
         }
-        if (!ok) break;
-        mmaCommit(&tmemFull[buf]);  // accumulator complete
-        if (++buf == 2) { buf = 0; accPhase ^= 1; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (++buf == 2) { buf = 0; accPhase ^= 1; }
     }
   } else if (warp >= 4) {
     // ---- epilogue: warp w owns TMEM lanes [32*(w%4), +32) = rows of the tile.

@@ -76,7 +76,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   __shared__ int tileStart[FCX_MOE_MAX_EXPERTS + 1];
   __shared__ int rowsOf[FCX_MOE_MAX_EXPERTS];
   __shared__ int tileCols;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   volatile int *err = p.errFlag;
   const uint32_t cr = ctaRankInCluster();
   const int pair = blockIdx.x >> 1, nPairs = gridDim.x >> 1;
@@ -135,7 +135,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 
   if (warp == 0) {
     // ---- TMA producer (both CTAs): own 128 rows of A, own half of the tile's weight rows
-    if (lane == 0) {
+    if (electOne()) {
       int stage = 0, e = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -156,29 +156,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer: one thread of the leader CTA
-    if (lane == 0 && cr == 0) {
+    // ---- MMA issuer: one thread of the leader CTA; the warp waits as one
+    if (cr == 0) {
       int stage = 0, buf = 0;
       uint32_t phase = 0, accPhase = 0;
       bool ok = true;
       // D fp32, A and B bf16, both K-major, M = 256 over the pair, N = bn
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
       for (int t = pair; t < nTiles && ok; t += nPairs) {
-        if (!mbarWait(&accEmpty[buf], accPhase ^ 1, err)) break;
+        if (!__all_sync(0xffffffffu, mbarWait(&accEmpty[buf], accPhase ^ 1, err))) break;
         fenceAfter();
         const uint32_t dTmem = tmemBase + (uint32_t)buf * BN_MAX;
         for (int kb = 0; kb < nK; kb++) {
-          if (!mbarWait(&fullBar[stage], phase, err)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
           fenceAfter();
-          const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
+          if (electOne()) {
+            const uint32_t sa = smemAddr(tiles + stage * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++)
-            mmaF16Pair(dTmem, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          mmaCommitPair(&emptyBar[stage]);
+            for (int k = 0; k < BK / 16; k++)
+              mmaF16Pair(dTmem, smemDesc(sa + k * 32), smemDesc(sb + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            mmaCommitPair(&emptyBar[stage]);
+            if (kb + 1 == nK) mmaCommitPair(&accFull[buf]);
+          }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        mmaCommitPair(&accFull[buf]);
         if (++buf == 2) { buf = 0; accPhase ^= 1; }
       }
     }

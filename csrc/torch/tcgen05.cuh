@@ -12,6 +12,23 @@ namespace fcxmma {
 
 constexpr uint32_t SPIN_LIMIT = 1u << 28;  // mbarrier polls before giving up (seconds of wall time)
 
+// The roles of a warp.  TMA loads, tcgen05.mma and tcgen05.commit take their operands from registers that a whole warp shares, so the
+// compiler must know that one lane issues them for the warp: the warp's index comes from a shuffle (the same in every lane by
+// construction) and the lane from elect.sync.  Behind a test of the lane's own index each of these instructions is wrapped in
+// code that looks for the active lane.  Clocks a turn of a loop, lane test / elect.sync, sizes so small that nothing else counts:
+// wait + TMA load 419 / 395, a second load 55 / 16 more; wait + commit + four MMAs 723 / 558 with elect.sync around the loop and
+// 480 with the waits in all lanes and elect.sync around what is issued (an MMA of 256 columns takes 128).
+__device__ __forceinline__ int warpIndex() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool electOne() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 __device__ __forceinline__ uint32_t smemAddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbarInit(uint64_t *bar, uint32_t count) {
