@@ -86,6 +86,31 @@ struct Scales {
   }
 };
 
+// On CTA pairs: the scales of the slices in flight, a ring in shared memory that the producer warp fills with 4-byte cp.async, so that no
+// thread ever waits for a load of its own.  A slot holds the activation scales of the CTA's 128 rows and the weight scales of
+// the tile's column blocks.  RING = stages + accumulators slots need no barrier of their own to be free: the slot of slice j is
+// filled once the stage of slice j - stages has been multiplied, which began after every epilogue warp was done with slice
+// j - stages - accumulators.  (Held in registers, a group of four slices ahead, they did not fit beside 128 sums a thread, and every
+// group stalled for 1300 clocks: 8192 x 4096 x 4096 took 142 us and takes 126, 8192 x 1024 x 4096 47.8 and 39.4.  The single-CTA
+// kernels have the room: there the ring is a wait more per slice, 333 x 1792 x 4096 12.5 us with registers and 12.9 with it.)
+struct ScaleSlot {
+  float a[BM];
+  float b[2];
+  float pad[2];
+};
+__device__ __forceinline__ void cpAsync4(void *smemDst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smemAddr(smemDst)), "l"(src) : "memory");
+}
+// All lanes of the producer warp: rows row0 .. +127 (clamped to the matrix), column blocks `block` .. + BLOCKS - 1, slice kb.
+template <int BLOCKS>
+__device__ __forceinline__ void fetchScales(ScaleSlot *slot, uint64_t *bar, const Params &p, int row0, int block, int kb, int nK, int lane) {
+  const float *a = p.sa + (size_t)kb * p.M;
+#pragma unroll
+  for (int i = 0; i < BM / 32; i++) cpAsync4(&slot->a[i * 32 + lane], a + min(row0 + i * 32 + lane, p.M - 1));
+  if (lane < BLOCKS) cpAsync4(&slot->b[lane], p.sb + (size_t)min(block + lane, (p.N - 1) / 128) * nK + kb);
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smemAddr(bar)) : "memory");
+}
+
 // COLS fp32 values per lane (one row) -> bf16 -> C, 32 columns at a time through this warp's two staging blocks (laid out
 // as the TMA unit's 64-byte swizzle wants them); the unit clips what lies beyond M and N.
 template <int COLS>
@@ -250,12 +275,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
 
 // ------------------------------------------------------------------ CTA pairs, 256 x 256 tiles
 
-constexpr int PN = 256, PNH = 128, PSTAGES = 6, PSTAGE_BYTES = A_BYTES + PNH * BK;
+constexpr int PN = 256, PNH = 128, PSTAGES = 5, PSTAGE_BYTES = A_BYTES + PNH * BK, PRING = PSTAGES + 2;
 constexpr int PTHREADS = 384;  // three warp groups: two of epilogue warps, one for the producer and the issuer
 // 128 sums per thread need more than the 168 registers that 384 threads get each: the third group gives some of its own.
 // 216 x 256 + 72 x 128 = 168 x 384.
 constexpr int EPI_REGS = 216, ROLE_REGS = 72;
-constexpr int PSMEM_BYTES = PSTAGES * PSTAGE_BYTES + EPI_BYTES + 1024 + 256;
+constexpr int PSMEM_BYTES = PSTAGES * PSTAGE_BYTES + EPI_BYTES + PRING * (int)sizeof(ScaleSlot) + 1024 + 256;
+static_assert(PSMEM_BYTES <= 232448, "shared memory of one CTA");
 
 __device__ __forceinline__ void mmaF8Pair(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -275,15 +301,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
   const int pair = blockIdx.x >> 1, nPairs = gridDim.x >> 1;
   uint8_t *tiles = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
   uint8_t *epiStage = tiles + PSTAGES * PSTAGE_BYTES;
-  uint64_t *bars = (uint64_t *)(epiStage + EPI_BYTES);
-  uint64_t *fullBar = bars, *emptyBar = bars + PSTAGES, *accFull = bars + 2 * PSTAGES, *accEmpty = bars + 2 * PSTAGES + 2;
-  uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * PSTAGES + 4);
+  ScaleSlot *scales = (ScaleSlot *)(epiStage + EPI_BYTES);
+  uint64_t *bars = (uint64_t *)(scales + PRING);
+  uint64_t *fullBar = bars, *emptyBar = bars + PSTAGES, *accFull = bars + 2 * PSTAGES, *accEmpty = accFull + 2, *scaleFull = accEmpty + 2;
+  uint32_t *tmemBaseSlot = (uint32_t *)(scaleFull + PRING);
 
   const int nN = (p.N + PN - 1) / PN, nM = (p.M + 2 * BM - 1) / (2 * BM), nTiles = nN * nM, nK = p.K / BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < PSTAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&emptyBar[s], 1); }
     for (int b = 0; b < 2; b++) { mbarInit(&accFull[b], 1); mbarInit(&accEmpty[b], 2 * EPI_WARPS); }  // the warps of both CTAs
+    for (int r = 0; r < PRING; r++) mbarInit(&scaleFull[r], 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 9) {
@@ -301,25 +329,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGS));
     if (warp == 8) {
-      // ---- TMA producer (both CTAs): own 128 rows of A, own 128 of the 256 weight rows; bytes counted on the leader's barrier
-      if (electOne()) {
-        int stage = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        for (int t = pair; t < nTiles && ok; t += nPairs) {
-          int mb, nb;
-          tileCoord(p, nM, nN, t, &mb, &nb);
-          for (int kb = 0; kb < nK; kb++) {
-            if (!mbarWait(&emptyBar[stage], phase ^ 1, err)) { ok = false; break; }
+      // ---- TMA producer (both CTAs): own 128 rows of A, own 128 of the 256 weight rows, bytes counted on the leader's barrier;
+      // and the scales of its own rows, on its own barrier
+      int stage = 0, slot = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = pair; t < nTiles && ok; t += nPairs) {
+        int mb, nb;
+        tileCoord(p, nM, nN, t, &mb, &nb);
+        const int row0 = mb * 2 * BM + (int)cr * BM;
+        for (int kb = 0; kb < nK; kb++) {
+          if (!__all_sync(0xffffffffu, mbarWait(&emptyBar[stage], phase ^ 1, err))) { ok = false; break; }
+          if (electOne()) {
             if (cr == 0) mbarExpectTx(&fullBar[stage], 2 * PSTAGE_BYTES);
             const uint32_t bar = mapToCta(smemAddr(&fullBar[stage]), 0);
             uint8_t *sa = tiles + stage * PSTAGE_BYTES, *sb = sa + A_BYTES;
-            tmaLoad2dPair(sa, &tmA, kb * BK, mb * 2 * BM + (int)cr * BM, bar);
+            tmaLoad2dPair(sa, &tmA, kb * BK, row0, bar);
             tmaLoad2dPair(sb, &tmB, kb * BK, nb * PN + (int)cr * PNH, bar);
-            if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
           }
+          __syncwarp();
+          fetchScales<2>(&scales[slot], &scaleFull[slot], p, row0, nb * 2, kb, nK, lane);
+          if (++stage == PSTAGES) { stage = 0; phase ^= 1; }
+          if (++slot == PRING) slot = 0;
         }
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == 9) {
       // ---- MMA issuer: one thread of the leader CTA; the warp waits as one
       if (cr == 0) {
@@ -329,7 +363,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
         const uint32_t idesc = instrDescF8(2 * BM, PN);
         for (int t = pair; t < nTiles && ok; t += nPairs) {
           for (int kb = 0; kb < nK; kb++) {
-            if (!__all_sync(0xffffffffu, mbarWait(&accEmpty[buf], accPhase ^ 1, err) && mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbarWait(&fullBar[stage], phase, err) && mbarWait(&accEmpty[buf], accPhase ^ 1, err))) { ok = false; break; }
             fenceAfter();
             if (electOne()) {
               const uint32_t sa = smemAddr(tiles + stage * PSTAGE_BYTES), sb = sa + A_BYTES;
@@ -350,52 +384,44 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PTHREADS, 1)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPI_REGS));
     // ---- promotion + epilogue (both CTAs): 128 fp32 sums per thread.  A warp's 128 columns are one scale block of the weight.
     const int q = warp & 3, half = warp >> 2;
-    constexpr int GROUP = 4, COLS = 128;
-    int buf = 0;
-    uint32_t accPhase = 0, blockNo = 0;
+    constexpr int COLS = 128;
+    int buf = 0, slot = 0;
+    uint32_t accPhase = 0, scalePhase = 0, blockNo = 0;
     bool live = true;
     uint8_t *stg = epiStage + (size_t)warp * 2 * STG_BYTES;
     const uint32_t emptyAddr = mapToCta(smemAddr(accEmpty), 0);
-    const int lastBlock = (p.N - 1) / 128;
+    const uint32_t lanes = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * COLS);
     for (int t = pair; t < nTiles; t += nPairs) {
       int mb, nb;
       tileCoord(p, nM, nN, t, &mb, &nb);
-      const int row0 = mb * 2 * BM + (int)cr * BM + q * 32;
-      Scales<GROUP> sc{p.sa + min(row0 + lane, p.M - 1), p.sb + (size_t)min(nb * 2 + half, lastBlock) * nK, p.M, nK};
-      sc.fetch(0);
       float acc[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; j++) acc[j] = 0.f;
-      sc.turn();
-      for (int kb0 = 0; kb0 < nK; kb0 += GROUP) {
-        sc.fetch(kb0 + GROUP);
+#pragma unroll 1
+      for (int kb = 0; kb < nK && live; kb++) {
+        live = __all_sync(0xffffffffu, mbarWait(&scaleFull[slot], scalePhase, err));
+        const float sc = scales[slot].a[q * 32 + lane] * scales[slot].b[half];
+        if (live) live = __all_sync(0xffffffffu, mbarWait(&accFull[buf], accPhase, err));
+        if (live) {
+          fenceAfter();
 #pragma unroll
-        for (int j = 0; j < GROUP; j++) {
-          if (kb0 + j < nK) {
-            if (live) live = __all_sync(0xffffffffu, mbarWait(&accFull[buf], accPhase, err));
-            if (live) {
-              fenceAfter();
-              const uint32_t taddr = tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * PN + half * COLS);
-#pragma unroll
-              for (int c = 0; c < COLS; c += 32) {
-                uint32_t r[32];
-                tmemLd32(taddr + c, r);
-                tmemLdWait();
-                if (c + 32 == COLS) {
-                  fenceBefore();
-                  __syncwarp();
-                  if (lane == 0) mbarArriveRemote(emptyAddr + buf * 8);  // all of it is in registers
-                }
-#pragma unroll
-                for (int i = 0; i < 32; i++) acc[c + i] = fmaf(sc.cur[j], __uint_as_float(r[i]), acc[c + i]);
-              }
+          for (int c = 0; c < COLS; c += 32) {
+            uint32_t r[32];
+            tmemLd32(lanes + buf * PN + c, r);
+            tmemLdWait();
+            if (c + 32 == COLS) {
+              fenceBefore();
+              __syncwarp();
+              if (lane == 0) mbarArriveRemote(emptyAddr + buf * 8);  // all of it is in registers
             }
-            if (++buf == 2) { buf = 0; accPhase ^= 1; }
+#pragma unroll
+            for (int i = 0; i < 32; i++) acc[c + i] = fmaf(sc, __uint_as_float(r[i]), acc[c + i]);
           }
         }
-        sc.turn();
+        if (++buf == 2) { buf = 0; accPhase ^= 1; }
+        if (++slot == PRING) { slot = 0; scalePhase ^= 1; }
       }
-      if (live) storeRows<COLS>(acc, &tmC, stg, row0, nb * PN + half * COLS, p.M, p.N, lane, &blockNo);
+      if (live) storeRows<COLS>(acc, &tmC, stg, mb * 2 * BM + (int)cr * BM + q * 32, nb * PN + half * COLS, p.M, p.N, lane, &blockNo);
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
