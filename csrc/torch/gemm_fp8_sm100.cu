@@ -16,13 +16,14 @@
 //   gemmFp8PairKernel  256 x 256 tiles on CTA pairs (cta_group::2), two 256-column accumulators.  A CTA fetches 32 KB per
 //                      slice for 128 x 256 results; the 128 x 128 tiles of the one-CTA kernel fetch the same for half of
 //                      them, and L2 cannot deliver that to 148 SMs at the fp8 rate.
-//   gemmFp8Kernel<BN>  128 x BN tiles on single CTAs (BN 128 or 64), four accumulators: for outputs with too few tiles.
+//   gemmFp8Kernel<BN>  128 x BN tiles on single CTAs (BN 128 or 64), four accumulators: for outputs with too few tiles; with fewer
+//                      still, the two or four CTAs of a cluster share a tile, a stretch of K each.
 // Roles: warps 0-7 promotion + epilogue (warp w reads TMEM lanes 32*(w%4).., one output row per thread, and half of the
 // tile's columns), warp 8 TMA producer (128-byte swizzle, no multicast), warp 9 MMA issuer and TMEM allocation.
-// The single-CTA kernel commits ONCE per slice, on the barrier of the slice's stage: the producer and the epilogue both wait
-// for it (8192 x 4096 x 4096 in 128-column tiles 227 -> 212 us, 333 x 1792 x 4096 18.1 -> 17.4).  It has at least as many stages
-// as accumulators, so that neither can miss a phase: the stage is not refilled before the producer has seen it done, nor its
-// successor multiplied before the epilogue has freed the accumulator.  On CTA pairs one commit was no faster (177 -> 184 us).
+// The single-CTA kernel commits ONCE per slice, on the barrier of the slice's stage: the producer and the epilogue both wait for it.
+// It has at least as many stages as accumulators, so that neither can miss a phase: the stage is not refilled before the producer
+// has seen it done, nor its successor multiplied before the epilogue has freed the accumulator.  On CTA pairs one commit was no
+// faster.
 // Every wait is bounded; a wait that gives up sets the error flag and the kernel drains and returns.
 #include <algorithm>
 #include <cstdlib>
@@ -149,7 +150,7 @@ constexpr int stageBytes(int bn) { return A_BYTES + bn * BK; }
 constexpr int stages(int bn) { return bn == 128 ? 5 : 7; }
 constexpr int smemBytes(int bn) { return stages(bn) * stageBytes(bn) + EPI_BYTES + 1024 + 256; }
 
-template <int BN>
+template <int BN, bool CUT>
 __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                                                             const __grid_constant__ CUtensorMap tmC, const Params p) {
   constexpr int STAGES = stages(BN), STAGE_BYTES = stageBytes(BN), ACC_BUFS = 4, COLS = BN / 2;
@@ -162,7 +163,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
   uint64_t *fullBar = bars, *doneBar = bars + STAGES, *tmemEmpty = bars + 2 * STAGES;
   uint32_t *tmemBaseSlot = (uint32_t *)(bars + 2 * STAGES + ACC_BUFS);
 
-  const int nN = (p.N + BN - 1) / BN, nM = (p.M + BM - 1) / BM, nTiles = nN * nM, nK = p.K / BK;
+  const int nN = (p.N + BN - 1) / BN, nM = (p.M + BM - 1) / BM, nTiles = nN * nM, nKAll = p.K / BK;
+  // CUT: the CTAs of a cluster share a tile, each with its own stretch of K; a tile per cluster
+  const int split = CUT ? (int)gridDim.x / nTiles : 1, rank = CUT ? (int)ctaRankInCluster() : 0, per = (nKAll + split - 1) / split;
+  const int kLo = rank * per, nK = min(nKAll, kLo + per), tile0 = CUT ? (int)blockIdx.x / split : (int)blockIdx.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbarInit(&fullBar[s], 1); mbarInit(&doneBar[s], 1); }
@@ -185,10 +189,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < nTiles && ok; t += gridDim.x) {
+      for (int t = tile0; t < nTiles && ok; t += gridDim.x) {
         int mb, nb;
         tileCoord(p, nM, nN, t, &mb, &nb);
-        for (int kb = 0; kb < nK; kb++) {
+        for (int kb = kLo; kb < nK; kb++) {
           if (!mbarWait(&doneBar[stage], phase ^ 1, err)) { ok = false; break; }
           mbarExpectTx(&fullBar[stage], STAGE_BYTES);
           uint8_t *sa = tiles + stage * STAGE_BYTES, *sb = sa + A_BYTES;
@@ -198,13 +202,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
         }
       }
     }
+    __syncwarp();
+    if (CUT) { clusterSync(); clusterSync(); }
   } else if (warp == 9) {  // the warp waits as one, one lane issues
     int stage = 0, buf = 0;
     uint32_t phase = 0, accPhase = 0;
     bool ok = true;
     const uint32_t idesc = instrDescF8(BM, BN);
-    for (int t = blockIdx.x; t < nTiles && ok; t += gridDim.x) {
-      for (int kb = 0; kb < nK; kb++) {
+    for (int t = tile0; t < nTiles && ok; t += gridDim.x) {
+      for (int kb = kLo; kb < nK; kb++) {
         if (!__all_sync(0xffffffffu, mbarWait(&tmemEmpty[buf], accPhase ^ 1, err) && mbarWait(&fullBar[stage], phase, err))) { ok = false; break; }
         fenceAfter();
         if (electOne()) {
@@ -220,6 +226,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
         if (++buf == ACC_BUFS) { buf = 0; accPhase ^= 1; }
       }
     }
+    if (CUT) { clusterSync(); clusterSync(); }
   } else {
     const int q = warp & 3, half = warp >> 2;  // TMEM lane quarter (fixed by warp index % 4) and column half
     constexpr int GROUP = 8;
@@ -227,17 +234,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
     uint32_t phase = 0, blockNo = 0;
     bool live = true;
     uint8_t *stg = epiStage + (size_t)warp * 2 * STG_BYTES;
-    for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
+    for (int t = tile0; t < nTiles; t += gridDim.x) {
       int mb, nb;
       tileCoord(p, nM, nN, t, &mb, &nb);
       const int row0 = mb * BM + q * 32;
-      Scales<GROUP> sc{p.sa + min(row0 + lane, p.M - 1), p.sb + (size_t)(nb * BN / 128) * nK, p.M, nK};
-      sc.fetch(0);
+      Scales<GROUP> sc{p.sa + min(row0 + lane, p.M - 1), p.sb + (size_t)(nb * BN / 128) * nKAll, p.M, nK};
+      sc.fetch(kLo);
       float acc[COLS];
 #pragma unroll
       for (int j = 0; j < COLS; j++) acc[j] = 0.f;
       sc.turn();
-      for (int kb0 = 0; kb0 < nK; kb0 += GROUP) {
+      for (int kb0 = kLo; kb0 < nK; kb0 += GROUP) {
         sc.fetch(kb0 + GROUP);
 #pragma unroll
         for (int j = 0; j < GROUP; j++) {
@@ -261,6 +268,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemmFp8Kernel(const __grid_constan
           }
         }
         sc.turn();
+      }
+      if (CUT) {
+        // Every CTA finishes an equal share of the tile's (32 rows x COLS columns) pieces, one per warp: `owner` of this warp's.  The
+        // others send it their sums, a row of 32 lanes per column, into the stages' memory, which is free once every CTA of the
+        // cluster has multiplied its last slice; they are added in the order of K.
+        const int share = EPI_WARPS / split, owner = split == 2 ? half : half + 2 * (q >> 1), mine = split == 2 ? q : q & 1;
+        auto place = [&](int from) { return (float *)tiles + ((size_t)(from - (from > owner)) * share + mine) * COLS * 32 + lane; };
+        clusterSync();
+        if (rank != owner) {
+          const uint32_t to = mapToCta(smemAddr(place(rank)), owner);
+#pragma unroll
+          for (int j = 0; j < COLS; j++) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + j * 128), "f"(acc[j]) : "memory");
+        }
+        clusterSync();
+        if (rank != owner) break;
+        for (int r = 1; r < split; r++) {
+          const float *got = place(r <= owner ? r - 1 : r);
+#pragma unroll
+          for (int j = 0; j < COLS; j++) acc[j] += got[j * 32];
+        }
       }
       if (live) storeRows<COLS>(acc, &tmC, stg, row0, nb * BN + half * COLS, p.M, p.N, lane, &blockNo);
     }
@@ -561,15 +588,16 @@ using fcxhost::smCount;
 
 namespace {
 
-template <int BN>
-cudaError_t launchOne(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
+template <int BN, bool CUT>
+cudaError_t launchOne(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, int cut, cudaStream_t s) {
   CUtensorMap mb;
   if (!makeTileMap(&mb, bq, p.N, p.K, p.K, BN, 1)) return cudaErrorNotSupported;
   static fcxhost::OncePerDevice once;
-  const cudaError_t e = once([] { return cudaFuncSetAttribute(gemmFp8Kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(BN)); });
+  const cudaError_t e = once([] { return cudaFuncSetAttribute(gemmFp8Kernel<BN, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(BN)); });
   if (e != cudaSuccess) return e;
   const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return fcxpdl::launchPdl(gemmFp8Kernel<BN>, std::min(tiles, smCount()), THREADS, smemBytes(BN), s, ma, mb, mc, p);
+  if (CUT) return fcxpdl::launchPdlAttr(gemmFp8Kernel<BN, CUT>, tiles * cut, THREADS, smemBytes(BN), dim3(cut, 1, 1), s, ma, mb, mc, p);
+  return fcxpdl::launchPdl(gemmFp8Kernel<BN, CUT>, std::min(tiles, smCount()), THREADS, smemBytes(BN), s, ma, mb, mc, p);
 }
 
 cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap &mc, const Params &p, cudaStream_t s) {
@@ -584,19 +612,43 @@ cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap 
 
 }  // namespace
 
-// Which tile: 0 = 256 x 256 on CTA pairs, 128 or 64 = 128 x that many columns on single CTAs.  The time is about the
-// number of waves times the time of one 128-deep slice of a tile, in nanoseconds.  Measured, us for pairs / 128 / 64 columns:
-// 8192 x 4096 x 4096 180 / 215 / 396, 8192 x 1024 x 4096 60.6 / 65.3 / 102.5, 4096 x 4096 x 1024 33.0 / 33.2 / 54.8, 3000 x 2000 x 4096
-// 54.5 / 50.1 / 87.3, 1024 x 4096 x 2048 17.4 / 19.6 / 32.1, 512 x 4096 x 4096 29.7 / 19.3 / 32.1, 1024 x 1024 x 1024 9.9 / 7.3 / 6.8,
-// 333 x 1792 x 4096 27.0 / 18.2 / 17.6: the rule takes the fastest at each.
-extern "C" int fcxGemmFp8Tile(int M, int N, int sms) {
+// Which tile: 0 = 256 x 256 on CTA pairs, 128 or 64 = 128 x that many columns on single CTAs; and how many CTAs of a cluster share
+// one, each with a stretch of K.  The time is about the number of waves times the time of the 128-deep slices of a tile, in
+// nanoseconds; with more than one wave the single CTAs' slices get longer (L2).  Measured, us for pairs / 128 / 64 columns, K whole:
+// 8192 x 1024 x 4096 39.0 / 47.2 / 69.1, 4096 x 4096 x 1024 25.9 / 27.5 / 39.2, 3000 x 2000 x 4096 37.5 / 36.4 / 58.9, 1024 x 4096 x 2048
+// 13.3 / 14.9 / 22.6, 512 x 4096 x 4096 20.7 / 14.3 / 22.1, 1024 x 1024 x 1024 8.5 / 6.1 / 5.5, 333 x 1792 x 4096 19.8 / 13.4 / 12.5.
+// Cut in 2 or 4 as long as all CTAs fit on the SMs at once; it costs two barriers of the cluster and the exchange of the sums.
+// 128 columns whole / 2 / 4, then 64 columns whole / 2 / 4: 16 x 512 x 4096 12.1 / 9.5 / 8.0, 11.3 / 8.0 / 6.6; 100 x 4096 x 4096 13.1 / 10.2 /
+// 8.8, 12.3 / 8.7 / -; 333 x 1792 x 4096 13.3 / 10.5 / -, 12.5 / - / -; 128 x 2048 x 2048 8.3 / 7.5 / 7.5, 7.7 / 6.3 / 6.0; but eight slices
+// are in flight at once anyway: 16 x 512 x 1024 5.1 / 6.3 / 6.6, 4.7 / 5.2 / 5.3.
+static int fp8Plan(int M, int N, int nK, int sms, bool cuts, int *cutOut) {
   const int m1 = (M + 127) / 128, m2 = (M + 255) / 256;
   auto waves = [](long long tiles, int slots) { return (double)((tiles + slots - 1) / slots); };
-  const double pair = waves((long long)m2 * ((N + 255) / 256), sms / 2) * 770;
-  const double one = waves((long long)m1 * ((N + 127) / 128), sms) * 465;
-  const double half = waves((long long)m1 * ((N + 63) / 64), sms) * 437;
-  if (pair <= one && pair <= half) return 0;
-  return one <= half ? 128 : 64;
+  double best = waves((long long)m2 * ((N + 255) / 256), sms / 2) * (nK * 562.0 + 600);
+  int tile = 0, cut = 1;
+  for (int bn : {128, 64}) {
+    const long long tiles = (long long)m1 * ((N + bn - 1) / bn);
+    for (int c = 1; c <= (cuts && nK >= 12 ? 4 : 1); c *= 2) {
+      const int per = (nK + c - 1) / c;
+      if (c > 1 && (tiles * c > sms || (c - 1) * per >= nK)) continue;
+      const double w = waves(tiles * c, sms), slice = bn == 128 ? (w > 1 ? 355 : 283) : (w > 1 ? 297 : 246);
+      const double exchange = c == 1 ? 0 : bn == 128 ? (c == 2 ? 1890 : 2700) : (c == 2 ? 660 : 1210);
+      const double time = w * per * slice + exchange;
+      if (time < best) {
+        best = time;
+        tile = bn;
+        cut = c;
+      }
+    }
+  }
+  *cutOut = cut;
+  return tile;
+}
+extern "C" int fcxGemmFp8Plan(int M, int N, int K, int sms, int *cut) { return fp8Plan(M, N, K / 128, sms, true, cut); }
+// The tile of a long sum that is not cut.
+extern "C" int fcxGemmFp8Tile(int M, int N, int sms) {
+  int cut;
+  return fp8Plan(M, N, 32, sms, false, &cut);
 }
 
 extern "C" cudaError_t fcxGemmFp8Blockwise(const void *aq, const float *sa, const void *bq, const float *sb, void *c, int M, int N, int K,
@@ -607,9 +659,12 @@ extern "C" cudaError_t fcxGemmFp8Blockwise(const void *aq, const float *sa, cons
   if (!makeTileMap(&ma, aq, M, K, K, BM, 1) || !makeStoreMap(&mc, c, M, N, ldc)) return cudaErrorNotSupported;
   Params p{};
   p.M = M; p.N = N; p.K = K; p.sa = sa; p.sb = sb; p.errFlag = errFlag;
-  const int tile = fcxGemmFp8Tile(M, N, smCount());
+  int cut = 1;
+  const int tile = fcxGemmFp8Plan(M, N, K, smCount(), &cut);
   p.group = tile == 0 ? 8 : (N + 127) / 128 >= 48 ? 16 : 8;
-  return tile == 0 ? launchPair(ma, bq, mc, p, s) : tile == 128 ? launchOne<128>(ma, bq, mc, p, s) : launchOne<64>(ma, bq, mc, p, s);
+  if (tile == 0) return launchPair(ma, bq, mc, p, s);
+  if (tile == 128) return cut > 1 ? launchOne<128, true>(ma, bq, mc, p, cut, s) : launchOne<128, false>(ma, bq, mc, p, 1, s);
+  return cut > 1 ? launchOne<64, true>(ma, bq, mc, p, cut, s) : launchOne<64, false>(ma, bq, mc, p, 1, s);
 }
 
 extern "C" cudaError_t fcxQuantFp8Act(const void *x, void *q, float *sa, int M, int K, int ldx, cudaStream_t s) {
