@@ -299,10 +299,10 @@ __device__ void fcxCollBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
   constexpr int G = 16 / (ESI < ESO ? ESI : ESO);
   constexpr int INB = G * ESI, OUTB = G * ESO;
   const int n = dc.nranks, me = dc.rank;
-  const uint64_t seq = nextSeq(dc);
+  uint64_t seq;
   const size_t gtid = (size_t)cta * blockDim.x + threadIdx.x, gstride = (size_t)nctas * blockDim.x;
 
-  if (!prologue(dc, seq, cta)) return;
+  if (!prologue(dc, cta, &seq)) return;
 
   const char *send = (const char *)a.send;
   char *recv = (char *)a.recv;
@@ -667,10 +667,10 @@ __device__ __forceinline__ bool llWaitLine(const FcxDevComm &dc, const char *lin
 // Byte-moving collectives need no element type.
 __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta, int nctas) {
   const int n = dc.nranks, me = dc.rank;
-  const uint64_t seq = nextSeq(dc);
+  uint64_t seq;
   const size_t gtid = (size_t)cta * blockDim.x + threadIdx.x, gstride = (size_t)nctas * blockDim.x;
   const size_t es = a.elemSize;
-  if (!prologue(dc, seq, cta)) return;
+  if (!prologue(dc, cta, &seq)) return;
   const char *send = (const char *)a.send;
   char *recv = (char *)a.recv;
   const size_t bytes = a.count * es;

@@ -97,36 +97,34 @@ __device__ __forceinline__ void zcFenceBeforeClose() { __threadfence_system(); }
 
 // ---------------------------------------------------------------- reducing kinds
 
-// Units [first, first + cnt) of the range for exactly P ranks.  A thread works on batches of U units whose U x P (eight)
-// loads are all issued before anything is combined, and the next batch's loads before this batch's stores: with sixteen
-// loads and then sixteen stores in turn, loads and stores waited for each other (3.5 TB/s for eight ranks on one GPU).
-template <typename TIn, typename TOut, int U, int P>
-__device__ __forceinline__ void zcReduceBulk(const FcxDevComm &dc, const FcxCollArgs &a, const char *const *src, char *const *dst, int nd,
-                                             size_t first, size_t cnt, size_t gtid, size_t gstride) {
+// `cnt` 32-byte pieces from `first` on for exactly P ranks, everything 32-byte aligned.  A thread has eight loads of 32 bytes
+// (pieces x ranks) in flight.  A GPU that stands in for all ranks at 25 MB (the loop alone, 16 CTAs per rank): 8 ranks 84 us with
+// two alternating batches of eight 16-byte loads, 72 with one of eight 32-byte loads; 4 ranks 54 and 42.
+template <typename TIn, int U, int P>
+__device__ __forceinline__ void zcReduceWide(const FcxCollArgs &a, const char *const *src, char *const *dst, int nd, size_t first, size_t cnt,
+                                             size_t gtid, size_t gstride) {
   using Acc = typename Elem<TIn>::Acc;
-  constexpr int G = 16 / (int)sizeof(TIn);
+  constexpr int G = 32 / (int)sizeof(TIn);
   const char *s[P];
 #pragma unroll
   for (int p = 0; p < P; p++) s[p] = src[p];
-  const size_t end = first + cnt, step = U * gstride;
-  uint4 buf[2][U * P];
-  auto load = [&](uint4 *raw, size_t u0) {
+  const size_t end = first + cnt;
+  for (size_t u = first + gtid; u < end; u += U * gstride) {
+    Vec32 raw[U][P];
 #pragma unroll
     for (int i = 0; i < U; i++)
-      if (u0 + i * gstride < end) {
+      if (u + i * gstride < end) {
 #pragma unroll
-        for (int p = 0; p < P; p++) raw[i * P + p] = ld16(s[p] + (u0 + i * gstride) * 16);
+        for (int p = 0; p < P; p++) raw[i][p] = ld32(s[p] + (u + i * gstride) * 32);
       }
-  };
-  auto finishAndStore = [&](const uint4 *raw, size_t u0) {
 #pragma unroll
     for (int i = 0; i < U; i++)
-      if (u0 + i * gstride < end) {
+      if (u + i * gstride < end) {
         Acc acc[G];
 #pragma unroll
         for (int p = 0; p < P; p++) {
-          union { uint4 v; TIn t[G]; } w;
-          w.v = raw[i * P + p];
+          union { Vec32 v; TIn t[G]; } w;
+          w.v = raw[i][p];
 #pragma unroll
           for (int e = 0; e < G; e++) {
             const Acc x = Elem<TIn>::up(w.t[e]);
@@ -135,19 +133,63 @@ __device__ __forceinline__ void zcReduceBulk(const FcxDevComm &dc, const FcxColl
         }
 #pragma unroll
         for (int e = 0; e < G; e++) acc[e] = finish<Acc>(acc[e], a.redop, P, a.scale);
+        union { uint4 q[2]; Vec32 v; } packed;
+        packUnit<TIn, G>(acc, packed.q);
+        for (int k = 0; k < nd; k++) st32(dst[k] + (u + i * gstride) * 32, packed.v);
+      }
+  }
+}
+
+// Units [first, first + cnt) of 16 bytes for exactly P ranks whose buffers all start `m` bytes past a 16-byte boundary, into
+// 16-byte aligned destinations.  A thread has U x P (eight) loads in flight.  A unit lies in two blocks of the source, the second
+// of which the next lane has loaded; with m > 0 the block behind the last unit's must exist.  (Element by element, as buffers that
+// were not 16-byte aligned had it before, a reduce-scatter of 4 x 1500001 fp32 took 143 us and takes 79, of 8 x 200003 bf16 42 and 38.)
+template <typename TIn, int U, int P>
+__device__ __forceinline__ void zcReduceShifted(const FcxCollArgs &a, const char *const *src, char *const *dst, int nd, size_t first, size_t cnt, int m,
+                                                size_t gtid, size_t gstride) {
+  using Acc = typename Elem<TIn>::Acc;
+  constexpr int G = 16 / (int)sizeof(TIn);
+  const size_t end = first + cnt, blocks = end + (m ? 1 : 0);
+  const int lane = threadIdx.x & 31;
+  for (size_t u0 = first + gtid; u0 - lane < end; u0 += U * gstride) {  // a whole warp goes round together
+    uint4 raw[U][P];
+#pragma unroll
+    for (int i = 0; i < U; i++)
+      if (u0 + i * gstride < blocks) {
+#pragma unroll
+        for (int p = 0; p < P; p++) raw[i][p] = ld16(src[p] - m + (u0 + i * gstride) * 16);
+      }
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      const size_t u = u0 + i * gstride;
+      Acc acc[G];
+#pragma unroll
+      for (int p = 0; p < P; p++) {
+        union { uint4 v; TIn t[G]; } w;
+        w.v = raw[i][p];
+        if (m) {
+          uint4 hi;
+          hi.x = __shfl_down_sync(0xffffffffu, w.v.x, 1);
+          hi.y = __shfl_down_sync(0xffffffffu, w.v.y, 1);
+          hi.z = __shfl_down_sync(0xffffffffu, w.v.z, 1);
+          hi.w = __shfl_down_sync(0xffffffffu, w.v.w, 1);
+          if (lane == 31 && u < end) hi = ld16(src[p] - m + (u + 1) * 16);
+          w.v = shiftBlocks(w.v, hi, m);
+        }
+#pragma unroll
+        for (int e = 0; e < G; e++) {
+          const Acc x = Elem<TIn>::up(w.t[e]);
+          acc[e] = p == 0 ? x : applyOp<Acc>(acc[e], x, a.redop);
+        }
+      }
+      if (u < end) {
+#pragma unroll
+        for (int e = 0; e < G; e++) acc[e] = finish<Acc>(acc[e], a.redop, P, a.scale);
         uint4 packed;
         packUnit<TIn, G>(acc, &packed);
-        for (int k = 0; k < nd; k++) st16(dst[k] + (u0 + i * gstride) * 16, packed);
+        for (int k = 0; k < nd; k++) st16(dst[k] + u * 16, packed);
       }
-  };
-  size_t u = first + gtid;
-  if (u < end) load(buf[0], u);
-  while (u < end) {
-    load(buf[1], u + step);
-    finishAndStore(buf[0], u);
-    load(buf[0], u + 2 * step);
-    finishAndStore(buf[1], u + step);
-    u += 2 * step;
+    }
   }
 }
 
@@ -169,21 +211,24 @@ __device__ __forceinline__ void zcReduceRange(const FcxDevComm &dc, const FcxCol
   const char *src[FCX_MAX_RANKS];
   char *dst[FCX_MAX_RANKS];
   int nd = 0;
-  bool alS = true, alD = true;
+  uintptr_t orS = 0, apart = 0, orD = 0;  // low bits: how the buffers are aligned, and whether all sources alike
   for (int p = 0; p < n; p++) {
     src[p] = z.send[p] + srcOff * ESI;
-    alS = alS && aligned16(src[p]);
+    orS |= (uintptr_t)src[p];
+    apart |= (uintptr_t)src[p] ^ (uintptr_t)src[0];
   }
   for (int k = 0; k < n; k++) {
     int p = (me + k) % n;  // own buffer first, then the peers starting with the right-hand neighbour
     if ((p == me && toSelf) || (p != me && toPeers)) {
       dst[nd] = z.recv[p] + dstOff * ESO;
-      alD = alD && aligned16(dst[nd]);
+      orD |= (uintptr_t)dst[nd];
       nd++;
     }
   }
+  const bool alS = (orS & 15u) == 0, alD = (orD & 15u) == 0;
   const size_t nunits = (nElems + G - 1) / G;
   size_t firstPlain = 0;  // units below this index are done through the switch
+  size_t edgeUnit = ~(size_t)0;  // but this one is not done yet
 
   if constexpr (ESI == ESO && Mm<TIn>::ok) {
     if (z.mcSend != nullptr && alS && alD && Mm<TIn>::opOk(a.redop)) {
@@ -215,18 +260,31 @@ __device__ __forceinline__ void zcReduceRange(const FcxDevComm &dc, const FcxCol
     }
   }
 
-  // Plain loads from peers are latency-bound (a load over NVLink takes microseconds): the aligned bulk of the
-  // range keeps eight to sixteen 16-byte loads per thread in flight (units x ranks).
+  // Plain loads from peers are latency-bound (a load over NVLink takes microseconds): the bulk of the range keeps eight
+  // loads per thread in flight (units x ranks), of 32 bytes where every buffer allows them.
   if constexpr (ESI == ESO && Mm<TIn>::ok) {  // the floating-point types of gradients and activations
-    if (alS && alD) {
-      const size_t nfull = nElems / G;
-      if (nfull > firstPlain) {
-        const size_t cnt = nfull - firstPlain;
-        if (n == 2) zcReduceBulk<TIn, TOut, 4, 2>(dc, a, src, dst, nd, firstPlain, cnt, gtid, gstride);
-        else if (n == 4) zcReduceBulk<TIn, TOut, 2, 4>(dc, a, src, dst, nd, firstPlain, cnt, gtid, gstride);
-        else if (n == 8) zcReduceBulk<TIn, TOut, 1, 8>(dc, a, src, dst, nd, firstPlain, cnt, gtid, gstride);
-        if (n == 2 || n == 4 || n == 8) firstPlain = nfull;  // at most one ragged unit is left for the path below
-      }
+    const int m = (int)((uintptr_t)src[0] & 15u);
+    const size_t nfull = nElems / G;
+    const bool ranks = n == 2 || n == 4 || n == 8;
+    // 32-byte pieces once every thread has one: below, more threads with half of the work each are sooner done (8 ranks x 20000
+    // bf16 25.4 us in units of 16 bytes, 26.6 in pieces of 32)
+    if (ranks && ((orS | orD) & 31u) == 0 && firstPlain == 0 && nfull / 2 >= gstride) {
+      const size_t cnt = nfull / 2;
+      if (n == 2) zcReduceWide<TIn, 4, 2>(a, src, dst, nd, 0, cnt, gtid, gstride);
+      else if (n == 4) zcReduceWide<TIn, 2, 4>(a, src, dst, nd, 0, cnt, gtid, gstride);
+      else zcReduceWide<TIn, 1, 8>(a, src, dst, nd, 0, cnt, gtid, gstride);
+      firstPlain = 2 * cnt;  // at most one whole and one ragged unit are left for the path below
+    } else if (ranks && alD && (apart & 15u) == 0 && nfull > firstPlain && (m == 0 || nfull >= 2 * gstride)) {
+      // With m > 0 the block before the first unit's bytes and the one behind the last unit's belong to the buffer's edges:
+      // those units are left to the path below, which is the better one for all of them while a thread has less than two
+      // (reduce-scatter, 8 ranks x 20011 bf16 25.1 us there, 28.3 here, but 200003 42.6 and 37.4).
+      const size_t lo = firstPlain, cnt = nfull - lo - (m ? 2 : 0);
+      const size_t from = lo + (m ? 1 : 0);
+      if (n == 2) zcReduceShifted<TIn, 4, 2>(a, src, dst, nd, from, cnt, m, gtid, gstride);
+      else if (n == 4) zcReduceShifted<TIn, 2, 4>(a, src, dst, nd, from, cnt, m, gtid, gstride);
+      else zcReduceShifted<TIn, 1, 8>(a, src, dst, nd, from, cnt, m, gtid, gstride);
+      firstPlain = lo + cnt + (m ? 1 : 0);
+      edgeUnit = m ? lo : ~(size_t)0;
     }
   }
 
@@ -253,7 +311,14 @@ __device__ __forceinline__ void zcReduceRange(const FcxDevComm &dc, const FcxCol
     packUnit<TOut, G>(res, packed);
     for (int k = 0; k < nd; k++) storeUnit<TOut, G>(dst[k] + u * OUTB, alD, nv, packed);
   };
-  size_t u = firstPlain + gtid;
+  // the threads that had least of the bulk take what is left of it
+  const size_t rest = firstPlain ? gstride - 1 - gtid : gtid;
+  if (edgeUnit != ~(size_t)0 && rest == 3) {  // up to three units lie behind the bulk
+    AI acc[G];
+    gather(edgeUnit, acc);
+    emit(edgeUnit, acc);
+  }
+  size_t u = firstPlain + rest;
   for (; u + gstride < nunits; u += 2 * gstride) {
     AI acc0[G], acc1[G];
     gather(u, acc0);
@@ -273,16 +338,16 @@ __device__ void fcxZcReduceBody(const FcxDevComm &dc, const FcxCollArgs &a, int 
   constexpr int ESI = (int)sizeof(TIn), ESO = (int)sizeof(TOut);
   constexpr int G = 16 / (ESI < ESO ? ESI : ESO);
   const int n = dc.nranks, me = dc.rank;
-  const uint64_t seq = nextSeq(dc);
+  uint64_t seq;
   const size_t gtid = (size_t)cta * blockDim.x + threadIdx.x, gstride = (size_t)nctas * blockDim.x;
-  if (!prologue(dc, seq, cta)) return;
+  if (!prologue(dc, cta, &seq)) return;
   ZcPeers z;
   const bool isAR = a.kind == FCX_K_AR_ZC, isRS = a.kind == FCX_K_RS_ZC;
   const size_t sendSpan = (isRS ? (size_t)(n - 1) * a.sendStride + a.count : a.count) * ESI;
   if (zcExchange(dc, a, seq, cta, true, isAR, sendSpan, a.count * ESO, nullptr, nullptr, &z)) {
     if (isAR) {
-      // slices in whole units so that every slice starts as aligned as the buffer itself
-      const size_t totalUnits = (a.count + G - 1) / G, sliceUnits = (totalUnits + n - 1) / n;
+      // slices in pairs of units so that every slice starts as aligned as the buffer itself, up to 32 bytes
+      const size_t totalUnits = (a.count + G - 1) / G, sliceUnits = ((totalUnits + n - 1) / n + 1) & ~(size_t)1;
       const size_t lo = min(a.count, (size_t)me * sliceUnits * G), hi = min(a.count, ((size_t)me + 1) * sliceUnits * G);
       zcReduceRange<TIn, TOut>(dc, a, z, lo, lo, hi - lo, true, true, gtid, gstride);
     } else if (isRS) {
@@ -290,7 +355,7 @@ __device__ void fcxZcReduceBody(const FcxDevComm &dc, const FcxCollArgs &a, int 
     } else if (me == a.root) {
       zcReduceRange<TIn, TOut>(dc, a, z, 0, 0, a.count, true, false, gtid, gstride);
     }
-    zcFenceBeforeClose();
+    if (z.mcSend || z.mcRecv) zcFenceBeforeClose();  // else the release of the closing barrier orders the CTA's stores
     ctaBarrier(dc, cta, barrierValue(seq, 2), seq);
   }
   epilogue(dc, seq, nctas);
@@ -298,35 +363,86 @@ __device__ void fcxZcReduceBody(const FcxDevComm &dc, const FcxCollArgs &a, int 
 
 // ---------------------------------------------------------------- byte-moving kinds
 
-// One read of `src`, one store into each of dst[0..nd): used where a rank sends the same bytes to several
-// peers, so that local memory is read once whatever the number of peers.
-__device__ __forceinline__ void zcCopyMulti(char *const *dst, int nd, const char *src, size_t bytes, size_t gtid, size_t gstride) {
-  if (!bytes || !nd) return;
-  bool al = aligned16(src);
-  for (int k = 0; k < nd; k++) al = al && aligned16(dst[k]);
-  if (!al) {
-    for (int k = 0; k < nd; k++) copyUnits(dst[k], src, bytes, 16, gtid, gstride);
-    return;
+// One read of `src`, one store into each of dst[0..nd), so that local memory is read once whatever the number of peers.
+// 32-byte aligned buffers move in four 32-byte accesses per thread and turn, others in four of 16 bytes at the destinations'
+// alignment, for which a source that starts elsewhere in its 16-byte blocks is shifted out of two of them (the next lane has
+// loaded the second).  Destinations of different alignments take a pass each.  Pieces of an odd number of bytes per rank, as
+// an all-gather of any count has them, went byte by byte before: 8 ranks x 200003 bf16 120 us, 29 now; 4 x 1500001 284 and 35.
+__device__ __forceinline__ void zcCopyShifted(char *const *dst, int nd, const char *src, size_t bytes, size_t gtid, size_t gstride) {
+  constexpr int U = 4;
+  const size_t head = min(bytes, (size_t)((16u - ((uintptr_t)dst[0] & 15u)) & 15u));  // bytes before the destinations' first block
+  const char *s = src + head, *blocks = (const char *)((uintptr_t)s & ~(uintptr_t)15);
+  const int m = (int)(s - blocks);
+  // destination blocks [i0, i1) whose bytes lie in whole blocks of the source
+  size_t i0 = 0, i1 = (bytes - head) / 16;
+  if (m) {
+    if (blocks < src) i0 = 1;
+    const size_t have = (size_t)(src + bytes - blocks) / 16;  // whole blocks from `blocks` on
+    i1 = min(i1, have ? have - 1 : (size_t)0);
+    i0 = min(i0, i1);
   }
-  const size_t nfull = bytes / 16;
-  size_t u = gtid;
-  for (; u + 3 * gstride < nfull; u += 4 * gstride) {
-    uint4 v[4];
+  const int lane = threadIdx.x & 31;
+  for (size_t u = i0 + gtid; u - lane < i1; u += U * gstride) {  // a whole warp goes round together
+    uint4 v[U];
 #pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = ld16(src + (u + i * gstride) * 16);
+    for (int i = 0; i < U; i++)
+      if (u + i * gstride < i1 + (m ? 1 : 0)) v[i] = ld16(blocks + (u + i * gstride) * 16);
+    if (m) {
+#pragma unroll
+      for (int i = 0; i < U; i++) {
+        uint4 hi;
+        hi.x = __shfl_down_sync(0xffffffffu, v[i].x, 1);
+        hi.y = __shfl_down_sync(0xffffffffu, v[i].y, 1);
+        hi.z = __shfl_down_sync(0xffffffffu, v[i].z, 1);
+        hi.w = __shfl_down_sync(0xffffffffu, v[i].w, 1);
+        if (lane == 31 && u + i * gstride < i1) hi = ld16(blocks + (u + i * gstride + 1) * 16);
+        v[i] = shiftBlocks(v[i], hi, m);
+      }
+    }
     for (int k = 0; k < nd; k++) {
 #pragma unroll
-      for (int i = 0; i < 4; i++) st16(dst[k] + (u + i * gstride) * 16, v[i]);
+      for (int i = 0; i < U; i++)
+        if (u + i * gstride < i1) st16(dst[k] + head + (u + i * gstride) * 16, v[i]);
     }
   }
-  for (; u < nfull; u += gstride) {
-    const uint4 v = ld16(src + u * 16);
-    for (int k = 0; k < nd; k++) st16(dst[k] + u * 16, v);
+  // the edges, byte by byte: at most 31 + 47 of them
+  const size_t before = head + i0 * 16, after = head + i1 * 16;
+  for (size_t j = gtid; j < before + (bytes - after); j += gstride) {
+    const size_t at = j < before ? j : after + (j - before);
+    const char c = src[at];
+    for (int k = 0; k < nd; k++) dst[k][at] = c;
   }
-  const size_t tail = bytes - nfull * 16;
-  if (tail && gtid == 0)
-    for (int k = 0; k < nd; k++)
-      for (size_t i = 0; i < tail; i++) dst[k][nfull * 16 + i] = src[nfull * 16 + i];
+}
+
+__device__ __forceinline__ void zcCopyMulti(char *const *dst, int nd, const char *src, size_t bytes, size_t gtid, size_t gstride) {
+  if (!bytes || !nd) return;
+  bool wide = aligned32(src), alike = true;
+  for (int k = 0; k < nd; k++) {
+    wide = wide && aligned32(dst[k]);
+    alike = alike && (((uintptr_t)dst[k] ^ (uintptr_t)dst[0]) & 15u) == 0;
+  }
+  if (wide) {
+    constexpr int U = 4;
+    const size_t nfull = bytes / 32;
+    for (size_t u = gtid; u < nfull; u += U * gstride) {
+      Vec32 v[U];
+#pragma unroll
+      for (int i = 0; i < U; i++)
+        if (u + i * gstride < nfull) v[i] = ld32(src + (u + i * gstride) * 32);
+      for (int k = 0; k < nd; k++) {
+#pragma unroll
+        for (int i = 0; i < U; i++)
+          if (u + i * gstride < nfull) st32(dst[k] + (u + i * gstride) * 32, v[i]);
+      }
+    }
+    for (size_t j = nfull * 32 + gtid; j < bytes; j += gstride) {
+      const char c = src[j];
+      for (int k = 0; k < nd; k++) dst[k][j] = c;
+    }
+    return;
+  }
+  const int together = alike ? nd : 1;
+  for (int k = 0; k < nd; k += together) zcCopyShifted(dst + k, together, src, bytes, gtid, gstride);
 }
 
 // Store the 16-byte units of `src` through the multicast alias (every rank of the communicator receives
@@ -346,13 +462,23 @@ __device__ __forceinline__ size_t zcMcPush(char *mcDst, const char *src, size_t 
   return nfull * 16;
 }
 
+// One piece per rank: piece k is copied by `copy(k, gtid, gstride)`.  Where the CTAs divide by the ranks every rank's piece has CTAs of
+// its own, so that short pieces are not one trip to memory after the other (8 ranks x 200000 bf16 41.3 us, 29.1 so).
+template <typename Copy>
+__device__ __forceinline__ void zcPieces(int n, int cta, int nctas, Copy copy) {
+  if (nctas % n == 0)
+    copy(cta % n, (size_t)(cta / n) * blockDim.x + threadIdx.x, (size_t)(nctas / n) * blockDim.x);
+  else
+    for (int k = 0; k < n; k++) copy(k, (size_t)cta * blockDim.x + threadIdx.x, (size_t)nctas * blockDim.x);
+}
+
 __device__ void fcxZcMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta, int nctas) {
   const int n = dc.nranks, me = dc.rank;
-  const uint64_t seq = nextSeq(dc);
+  uint64_t seq;
   const size_t gtid = (size_t)cta * blockDim.x + threadIdx.x, gstride = (size_t)nctas * blockDim.x;
   const size_t es = a.elemSize, bytes = a.count * es;
   const int mk = a.moveOp;
-  if (!prologue(dc, seq, cta)) return;
+  if (!prologue(dc, cta, &seq)) return;
   const bool pull = mk == FCX_K_GATHER || mk == FCX_K_A2AV;
   size_t sendSpan = 0, recvSpan = 0;
   uint64_t xTo[FCX_MAX_RANKS], yTo[FCX_MAX_RANKS];
@@ -419,31 +545,31 @@ __device__ void fcxZcMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int ct
       }
       case FCX_K_SCATTER: {
         if (me != a.root) break;
-        for (int k = 0; k < n; k++) {
+        zcPieces(n, cta, nctas, [&](int k, size_t t, size_t stride) {
           const int p = (me + k) % n;
           const char *s = send + (size_t)p * a.sendStride * es;
-          char *d = p == me ? recv : z.recv[p];
-          if (d != s) copyUnits(d, s, bytes, 16, gtid, gstride);
-        }
+          char *const d[1] = {p == me ? recv : z.recv[p]};
+          if (d[0] != s) zcCopyMulti(d, 1, s, bytes, t, stride);
+        });
         break;
       }
       case FCX_K_A2A: {
-        for (int k = 0; k < n; k++) {
+        zcPieces(n, cta, nctas, [&](int k, size_t t, size_t stride) {
           const int p = (me + k) % n;
           const char *s = send + (size_t)p * a.sendStride * es;
-          char *d = (p == me ? recv : z.recv[p]) + (size_t)me * a.recvStride * es;
-          if (d != s) copyUnits(d, s, bytes, 16, gtid, gstride);
-        }
+          char *const d[1] = {(p == me ? recv : z.recv[p]) + (size_t)me * a.recvStride * es};
+          if (d[0] != s) zcCopyMulti(d, 1, s, bytes, t, stride);
+        });
         break;
       }
       case FCX_K_GATHER: {
         if (me != a.root) break;
-        for (int k = 0; k < n; k++) {
+        zcPieces(n, cta, nctas, [&](int k, size_t t, size_t stride) {
           const int p = (me + k) % n;
           const char *s = p == me ? send : z.send[p];
-          char *d = recv + (size_t)p * a.recvStride * es;
-          if (d != s) copyUnits(d, s, bytes, 16, gtid, gstride);
-        }
+          char *const d[1] = {recv + (size_t)p * a.recvStride * es};
+          if (d[0] != s) zcCopyMulti(d, 1, s, bytes, t, stride);
+        });
         break;
       }
       case FCX_K_A2AV: {
@@ -451,14 +577,14 @@ __device__ void fcxZcMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int ct
           const int p = (me + k) % n;
           const char *s = (p == me ? send : z.send[p]) + z.x[p];
           const size_t nb = min((size_t)z.y[p], (size_t)(a.rcounts[p] * es));
-          char *d = recv + a.rdispls[p] * es;
-          if (nb && d != s) copyUnits(d, s, nb, 16, gtid, gstride);
+          char *const d[1] = {recv + a.rdispls[p] * es};
+          if (nb && d[0] != s) zcCopyMulti(d, 1, s, nb, gtid, gstride);
         }
         break;
       }
       default: break;
     }
-    zcFenceBeforeClose();
+    if (z.mcSend || z.mcRecv) zcFenceBeforeClose();  // else the release of the closing barrier orders the CTA's stores
     ctaBarrier(dc, cta, barrierValue(seq, 2), seq);
   }
   epilogue(dc, seq, nctas);
