@@ -19,7 +19,7 @@
 // same code can run as one real rank per GPU (fcxCollKernel) or as several
 // emulated ranks inside one cooperative launch on a single GPU
 // (fcxCollEmuKernel), which is how the protocol is tested without NVLink.
-#include "prims.cuh"
+#include "lowlatency.cuh"
 #include "launch.h"
 #include "dispatch.h"
 
@@ -110,129 +110,6 @@ __device__ __forceinline__ bool pipelined(const FcxDevComm &dc, int cta, uint64_
   return true;
 }
 
-// ---------------------------------------------------------------- LL one-shot all-reduce
-
-// A 16-byte LL line carries 8 payload bytes and two copies of the 32-bit
-// sequence tag: {d0, tag, d1, tag}.  Each 8-byte half is written atomically,
-// so a reader that sees the tag in a half also sees that half's payload.
-__device__ __forceinline__ void llStore(char *line, uint32_t d0, uint32_t d1, uint32_t tag) {
-  asm volatile("st.relaxed.sys.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(line), "r"(d0), "r"(tag), "r"(d1), "r"(tag)
-               : "memory");
-}
-__device__ __forceinline__ uint4 llLoad(const char *line) {
-  uint4 v;
-  asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(line) : "memory");
-  return v;
-}
-
-// The pair of lines of a peer's unit is looked at once more for the report: the tag of an earlier collective tells a peer that
-// is behind from one that never wrote.  Kept out of the wait itself, which it would slow down.
-static __device__ __noinline__ void giveUpOnLine(const FcxDevComm &dc, uint32_t code, int peer, size_t llOff, size_t u, int cta, uint32_t tag,
-                                                 uint64_t seq) {
-  const char *line = dc.heap[dc.rank] + llOff + (size_t)peer * FCX_LL_SLOT_BYTES + u * 32;
-  const uint32_t first = llLoad(line).y, second = llLoad(line + 16).y;
-  giveUp(dc, code, peer, FCX_WAIT_LL, cta, tag, first != tag ? first : second, seq);
-}
-
-// mode 0: all-reduce (everybody sends its whole vector to everybody and reduces);
-// mode 1: reduce-scatter (piece p goes to rank p, every rank reduces the pieces it received and its own);
-// mode 2: reduce (everybody sends its whole vector to the root, which reduces).
-template <typename T>
-__device__ void arLL(const FcxDevComm &dc, const FcxCollArgs &a, uint64_t seq, int cta, int nctas, int mode = 0) {
-  using Acc = typename Elem<T>::Acc;
-  constexpr int G = 16 / (int)sizeof(T);
-  const int n = dc.nranks, me = dc.rank;
-  const uint32_t tag = (uint32_t)seq;
-  const size_t gtid = (size_t)cta * blockDim.x + threadIdx.x, gstride = (size_t)nctas * blockDim.x;
-  const size_t nunits = (a.count + G - 1) / G;
-  const size_t pieceBytes = mode == 1 ? a.sendStride * sizeof(T) : 0;  // distance between the pieces of a reduce-scatter
-  const char *send = (const char *)a.send + (size_t)me * pieceBytes;    // what this rank contributes to its own result
-  const bool reduces = mode != 2 || me == a.root;
-  const bool alS = aligned16(send), alR = aligned16(a.recv);
-  const size_t llOff = FCX_OFF_LL + (size_t)(seq & 1) * FCX_MAX_RANKS * FCX_LL_SLOT_BYTES;
-  // All lines go out before any is waited for, and every peer's line of a unit is asked for before the first is used: a
-  // line at a time, the kernel spent a trip to L2 per peer and unit one after the other (7 x 0.5 us with eight ranks).
-  for (size_t u = gtid; u < nunits; u += gstride) {
-    const int nv = (int)min((size_t)G, a.count - u * G);
-    Acc mine[G];
-    uint4 raw;
-    if (mode != 1) {
-      loadUnit<T, G>(send + u * 16, alS, nv, mine);
-      packUnit<T, G>(mine, &raw);
-    }
-    for (int k = 1; k < n; k++) {
-      int p = (me + k) % n;
-      if (mode == 2 && p != a.root) continue;
-      if (mode == 1) {
-        const char *src = (const char *)a.send + (size_t)p * pieceBytes + u * 16;
-        loadUnit<T, G>(src, aligned16(src), nv, mine);
-        packUnit<T, G>(mine, &raw);
-      }
-      char *line = dc.heap[p] + llOff + (size_t)me * FCX_LL_SLOT_BYTES + u * 32;
-      llStore(line, raw.x, raw.y, tag);
-      llStore(line + 16, raw.z, raw.w, tag);
-    }
-  }
-  if (!reduces) return;
-  const char *lines = dc.heap[me] + llOff;
-  for (size_t u = gtid; u < nunits; u += gstride) {
-    const int nv = (int)min((size_t)G, a.count - u * G);
-    Acc mine[G];
-    loadUnit<T, G>(send + u * 16, alS, nv, mine);
-    uint4 lo[FCX_MAX_RANKS], hi[FCX_MAX_RANKS];
-    unsigned pending = ((1u << n) - 1u) & ~(1u << me), spins = 0;
-    uint64_t t0 = 0;
-    for (;;) {
-#pragma unroll
-      for (int p = 0; p < FCX_MAX_RANKS; p++)
-        if (pending >> p & 1u) {
-          lo[p] = llLoad(lines + (size_t)p * FCX_LL_SLOT_BYTES + u * 32);
-          hi[p] = llLoad(lines + (size_t)p * FCX_LL_SLOT_BYTES + u * 32 + 16);
-        }
-#pragma unroll
-      for (int p = 0; p < FCX_MAX_RANKS; p++)
-        if ((pending >> p & 1u) && lo[p].y == tag && lo[p].w == tag && hi[p].y == tag && hi[p].w == tag) pending &= ~(1u << p);
-      if (!pending) break;
-      if (spins == 0) t0 = globalTimerNs();
-      if ((++spins & 63u) == 0u) {
-        const int late = __ffs(pending) - 1;
-        if (*(volatile unsigned int *)&localOf(dc)->abortSeen) return;
-        if (globalTimerNs() - t0 > dc.timeoutNs) {
-          giveUpOnLine(dc, FCX_ERR_TIMEOUT, late, llOff, u, cta, tag, seq);
-          return;
-        }
-        if ((spins & 1023u) == 0u && *dc.abortWord) {
-          giveUpOnLine(dc, FCX_ERR_ABORT, late, llOff, u, cta, tag, seq);
-          return;
-        }
-      }
-    }
-    Acc acc[G];
-#pragma unroll
-    for (int p = 0; p < FCX_MAX_RANKS; p++)  // in rank order on every rank
-      if (p < n) {
-        Acc in[G];
-        if (p == me) {
-#pragma unroll
-          for (int i = 0; i < G; i++) in[i] = mine[i];
-        } else {
-          union { uint4 v; T t[G]; } w;
-          w.v = make_uint4(lo[p].x, lo[p].z, hi[p].x, hi[p].z);
-#pragma unroll
-          for (int i = 0; i < G; i++) in[i] = Elem<T>::up(w.t[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < G; i++) acc[i] = p == 0 ? in[i] : applyOp<Acc>(acc[i], in[i], a.redop);
-      }
-#pragma unroll
-    for (int i = 0; i < G; i++) acc[i] = finish<Acc>(acc[i], a.redop, n, a.scale);
-    uint4 outv;
-    packUnit<T, G>(acc, &outv);
-    storeUnit<T, G>((char *)a.recv + u * 16, alR, nv, &outv);
-  }
-}
-
 // ---------------------------------------------------------------- reductions out of staging
 
 // out[u] = finish( x_0[u] (op) x_1[u] ... x_{n-1}[u] ) over the ranks in rank
@@ -319,8 +196,6 @@ __device__ void fcxCollBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
       case FCX_K_REDUCE: need = (size_t)n * sliceUnits * (INB + OUTB); break;
       case FCX_K_AR_NVLS: need = (size_t)n * sliceUnits * 16; break;
       case FCX_K_RS_NVLS: need = (size_t)n * ((a.count * ESI + 15) / 16 * 16); break;
-      case FCX_K_AR_LL: case FCX_K_REDUCE_LL: need = a.count * ESI > FCX_LL_MAX_PAYLOAD ? ~(size_t)0 : 0; break;
-      case FCX_K_RS_LL: need = a.count * ESI > FCX_LL_MAX_PAYLOAD ? ~(size_t)0 : 0; break;
       default: break;
     }
     if (need > dc.stageBytes) {
@@ -333,19 +208,6 @@ __device__ void fcxCollBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
   switch (a.kind) {
     case FCX_K_BARRIER: {
       if (cta == 0) ctaBarrier(dc, 0, barrierValue(seq, 1), seq);
-      break;
-    }
-
-    case FCX_K_AR_LL: {
-      if constexpr (ESI == ESO) arLL<TIn>(dc, a, seq, cta, nctas);
-      break;
-    }
-    case FCX_K_RS_LL: {
-      if constexpr (ESI == ESO) arLL<TIn>(dc, a, seq, cta, nctas, 1);
-      break;
-    }
-    case FCX_K_REDUCE_LL: {
-      if constexpr (ESI == ESO) arLL<TIn>(dc, a, seq, cta, nctas, 2);
       break;
     }
 
@@ -1128,6 +990,7 @@ cudaError_t launchTypedEmu(const FcxEmuRanks &l, int nranks, int nctas, cudaStre
 static bool isMoveKind(int k) {
   return (k >= FCX_K_AG && k <= FCX_K_MOVE_LL && k != FCX_K_REDUCE) || k == FCX_K_MOVE_ZC;
 }
+static bool isLlReduceKind(int k) { return k == FCX_K_AR_LL || k == FCX_K_RS_LL || k == FCX_K_REDUCE_LL; }
 static bool isZcReduceKind(int k) { return k == FCX_K_AR_ZC || k == FCX_K_RS_ZC || k == FCX_K_REDUCE_ZC; }
 
 // A kind that cannot serve the call's element types or reduction must never be launched: its body would
@@ -1153,6 +1016,7 @@ extern "C" cudaError_t fcxLaunchColl(const FcxDevComm *dc, const FcxCollArgs *a,
     fcxMoveKernel<<<nctas, FCX_THREADS, 0, s>>>(*dc, *a);
     return cudaGetLastError();
   }
+  if (isLlReduceKind(a->kind)) return fcxLaunchLl(dc, a, nctas, s);
   if (a->kind == FCX_K_BARRIER) return launchTyped<uint8_t, uint8_t>(*dc, *a, 1, s);
 #define CALL(TI, TO) launchTyped<TI, TO>(*dc, *a, nctas, s)
   FCX_DISPATCH_ALL(a, CALL);
@@ -1176,6 +1040,7 @@ extern "C" cudaError_t fcxLaunchCollEmu(const FcxEmuRanks *l, int nranks, int nc
   if (a->kind == FCX_K_MOVE_ZC || isZcReduceKind(a->kind)) return fcxLaunchZcEmu(l, nranks, nctas, s);
   if (isMoveKind(a->kind))
     return cudaLaunchCooperativeKernel((const void *)fcxMoveEmuKernel, dim3(nranks * nctas), dim3(FCX_THREADS), params, 0, s);
+  if (isLlReduceKind(a->kind)) return fcxLaunchLlEmu(l, nranks, nctas, s);
   if (a->kind == FCX_K_BARRIER) return launchTypedEmu<uint8_t, uint8_t>(*l, nranks, nctas, s);
 #define CALL(TI, TO) launchTypedEmu<TI, TO>(*l, nranks, nctas, s)
   FCX_DISPATCH_ALL(a, CALL);

@@ -19,6 +19,9 @@ cudaError_t fcxLaunchColl(const FcxDevComm *dc, const FcxCollArgs *a, int nctas,
 // zero-copy kinds (zerocopy.cu); fcxLaunchColl forwards to these
 cudaError_t fcxLaunchZc(const FcxDevComm *dc, const FcxCollArgs *a, int nctas, cudaStream_t s);
 cudaError_t fcxLaunchZcEmu(const FcxEmuRanks *l, int nranks, int nctas, cudaStream_t s);
+// low-latency reductions (lowlatency.cu); fcxLaunchColl forwards to these, too
+cudaError_t fcxLaunchLl(const FcxDevComm *dc, const FcxCollArgs *a, int nctas, cudaStream_t s);
+cudaError_t fcxLaunchLlEmu(const FcxEmuRanks *l, int nranks, int nctas, cudaStream_t s);
 cudaError_t fcxLaunchP2p(const FcxDevComm *dc, const FcxP2pArgs *g, cudaStream_t s);
 cudaError_t fcxLaunchWaitTest(const FcxDevComm *dc, uint64_t want, cudaStream_t s);
 // Single-GPU emulation of `nranks` ranks in one cooperative launch.  The ranks' descriptors and arguments travel in the
