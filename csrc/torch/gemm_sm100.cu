@@ -559,8 +559,8 @@ static double waveCost(int M, int N, int K, int units, int slots, int sms, int c
 // for 256, 128 and 64 columns.  Narrow tiles re-read A and never pay once 256-column tiles fill the SMs, but with few
 // tiles they put more SMs to work on the same K steps.  `cut` is the launch's own: a sum that stays whole (1) keeps as many
 // SMs busy as it has tiles, one that may be cut (0) fills them whatever its tiles are.  Uncut, measured: 512 x 1024 x 4096
-// 25.4 / 26.0 / 28.6 us in 64 / 128 / 256 columns and 27.2 on CTA pairs; 640 x 3584 x 4096 46.7 / 27.1 / 29.3 and 29.0;
-// 4096 x 1024 x 1792 42.3 / 24.4 / 16.6 and 15.8.
+// 20.2 / 21.9 / 24.9 us in 64 / 128 / 256 columns and 23.1 on CTA pairs; 640 x 3584 x 4096 38.2 / 24.4 / 28.6 and 25.3;
+// 4096 x 1024 x 1792 33.2 / 20.6 / 15.0 and 13.9; 512 x 4096 x 1024 12.4 / 9.2 / 10.9 and 10.1.
 extern "C" double fcxGemmTileCostCut(int M, int N, int K, int sms, int cut, int *bnOut) {
   const int nM = (M + BM - 1) / BM;
   const int widths[3] = {256, 128, 64};

@@ -59,9 +59,10 @@ struct GroupParams {
 // 256 or 128 accumulator columns per tile for `rowBlocks` 256-row blocks, `cols` columns and sums of length K.  Narrow tiles
 // where they take no more waves.  Otherwise a narrow wave costs about 0.7 to 0.85 of a wide one, which more waves (3 for 2, 5
 // for 3, up to twice as many) eat up, except for short sums of the gate / up product, whose wide tiles spend their time on
-// the activation.  Measured with cold weights, narrow / wide in us: gate / up 3:2 waves K 512 21.2 / 25.3, 768 25.6 / 25.6, 1024
-// 29.8 / 31.7, 1280 33.8 / 31.8, 2048 45.9 / 39.9, 3328 62.5 / 50.1; 5:3 waves K 512 25.6 / 27.6, 1024 37.9 / 31.5; down 3:2 waves
-// K 1024 39.9 / 35.8, 2816 (7:4) 119.8 / 82.9, 5632 97.3 / 76.8.
+// the activation.  Measured with cold weights, narrow / wide in us: gate / up
+// 512 tokens of 1024 columns (4 experts, F 2048) 28.4 / 37.2, 256 of 768 (4, 1024) 11.4 / 14.2, 1000 of 1536 (8, 1536) 36.7 / 38.0, 470 of 2048
+// (8, 2304) 52.0 / 48.9, 700 of 1024 (2, 4096) 32.7 / 27.5, 900 of 3072 (4, 3072) 84.6 / 63.5; down, in the same order, 26.4 / 29.1, 20.2 /
+// 19.9, 32.1 / 29.1, 39.0 / 34.1, 34.3 / 38.0, 55.7 / 50.8.
 __host__ __device__ inline int moeTileColumns(long long rowBlocks, int cols, int K, bool up, int pairs) {
   const long long wide = (rowBlocks * ((cols + 255) / 256) + pairs - 1) / pairs, narrow = (rowBlocks * ((cols + 127) / 128) + pairs - 1) / pairs;
   const int tenths = !up || K > 1024 ? 10 : K > 512 ? 15 : 17;  // narrow waves per ten wide ones that still pay
