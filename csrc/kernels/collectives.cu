@@ -481,25 +481,40 @@ __device__ void fcxCollBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
 // has the payload.  The tag is the collective's sequence number; the slots are parity double-buffered
 // like the staging area.  One line slot per source rank on every receiver (FCX_LL_SLOT_BYTES each).
 __device__ __forceinline__ void ld8(const char *p, size_t valid, uint32_t *lo, uint32_t *hi) {
-  if (valid >= 8 && ((uintptr_t)p & 7u) == 0) {
-    uint2 v = *(const uint2 *)p;
-    *lo = v.x;
-    *hi = v.y;
+  const unsigned off = (unsigned)(uintptr_t)p & 7u;
+  union { uint2 v; uint16_t h[4]; char c[8]; } w;
+  w.v = make_uint2(0, 0);
+  if (valid >= 8 && off == 0) {
+    w.v = *(const uint2 *)p;
+  } else if (valid >= 8 && off == 4) {
+    w.v = make_uint2(((const uint32_t *)p)[0], ((const uint32_t *)p)[1]);
+  } else if (valid >= 8 && (off & 1u) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) w.h[i] = ((const uint16_t *)p)[i];
   } else {
-    union { uint2 v; char c[8]; } w;
-    w.v = make_uint2(0, 0);
-    for (size_t i = 0; i < valid && i < 8; i++) w.c[i] = p[i];
-    *lo = w.v.x;
-    *hi = w.v.y;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (i < (int)valid) w.c[i] = p[i];
   }
+  *lo = w.v.x;
+  *hi = w.v.y;
 }
 __device__ __forceinline__ void st8(char *p, size_t valid, uint32_t lo, uint32_t hi) {
-  if (valid >= 8 && ((uintptr_t)p & 7u) == 0) {
-    *(uint2 *)p = make_uint2(lo, hi);
+  const unsigned off = (unsigned)(uintptr_t)p & 7u;
+  union { uint2 v; uint16_t h[4]; char c[8]; } w;
+  w.v = make_uint2(lo, hi);
+  if (valid >= 8 && off == 0) {
+    *(uint2 *)p = w.v;
+  } else if (valid >= 8 && off == 4) {
+    ((uint32_t *)p)[0] = lo;
+    ((uint32_t *)p)[1] = hi;
+  } else if (valid >= 8 && (off & 1u) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) ((uint16_t *)p)[i] = w.h[i];
   } else {
-    union { uint2 v; char c[8]; } w;
-    w.v = make_uint2(lo, hi);
-    for (size_t i = 0; i < valid && i < 8; i++) p[i] = w.c[i];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (i < (int)valid) p[i] = w.c[i];
   }
 }
 // Bounded wait for one line carrying `tag`; false = gave up.
@@ -526,7 +541,11 @@ __device__ __forceinline__ bool llWaitLine(const FcxDevComm &dc, const char *lin
   }
 }
 
-// Byte-moving collectives need no element type.
+// Byte-moving collectives need no element type.  LL: FCX_K_MOVE_LL alone, for a kernel of its own as lowlatency.cu has the
+// reductions.  Kernel time in us before that, the opening in one trip (prims.cuh) and pieces of any alignment in more than single
+// bytes, and with them: all-gather of 500 fp32 among 8 emulated ranks 13.2 -> 10.8, of 5001 35.0 -> 25.2; all-to-all of 5001 bf16
+// among 4 18.7 -> 12.4.
+template <bool LL>
 __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta, int nctas) {
   const int n = dc.nranks, me = dc.rank;
   uint64_t seq;
@@ -540,8 +559,8 @@ __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
 
   {  // the pieces of one launch must fit the staging half (or the LL slots) they travel through
     size_t need = 0;
-    const int mk0 = a.kind == FCX_K_MOVE_LL ? a.moveOp : a.kind;
-    if (a.kind == FCX_K_MOVE_LL) need = bytes > FCX_LL_MAX_PAYLOAD ? ~(size_t)0 : 0;
+    const int mk0 = LL ? a.moveOp : a.kind;
+    if (LL) need = bytes > FCX_LL_MAX_PAYLOAD ? ~(size_t)0 : 0;
     else if (mk0 == FCX_K_BCAST || mk0 == FCX_K_SCATTER) need = slot;
     else if (a.kind != FCX_K_A2AV) need = (size_t)n * slot;
     if (need > dc.stageBytes) {
@@ -551,8 +570,8 @@ __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
     }
   }
 
-  if (a.kind != FCX_K_A2AV) {
-    const int mk = a.kind == FCX_K_MOVE_LL ? a.moveOp : a.kind;  // the LL form moves the same pieces
+  if (LL || a.kind != FCX_K_A2AV) {
+    const int mk = LL ? a.moveOp : a.kind;  // the LL form moves the same pieces
     // Every fixed-size byte mover is one exchange: piece out[p] goes into a slot of rank p's staging area,
     // piece in[p] arrives in a slot of this rank's staging area and is copied to its place, and the piece a
     // rank keeps for itself is copied locally.  With the multicast alias one store reaches every rank.
@@ -624,7 +643,7 @@ __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
         break;
       default: break;
     }
-    if (a.kind == FCX_K_MOVE_LL) {
+    if constexpr (LL) {
       const uint32_t tag = (uint32_t)seq;
       const size_t llOff = FCX_OFF_LL + (size_t)(seq & 1) * FCX_MAX_RANKS * FCX_LL_SLOT_BYTES;
       const size_t nwords = (bytes + 7) / 8;
@@ -639,7 +658,18 @@ __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
           llStore(dc.heap[p] + llOff + (size_t)me * FCX_LL_SLOT_BYTES + w * 16, lo, hi, tag);
         }
       }
-      if (selfSrc && selfSrc != selfDst) copyUnits(selfDst, selfSrc, bytes, 16, gtid, gstride);
+      if (selfSrc && selfSrc != selfDst) {
+        if (aligned16(selfSrc) && aligned16(selfDst)) {
+          copyUnits(selfDst, selfSrc, bytes, 16, gtid, gstride);
+        } else {  // byte by byte, every load waits for the one before it
+          for (size_t w = gtid; w < nwords; w += gstride) {
+            const size_t valid = min((size_t)8, bytes - w * 8);
+            uint32_t lo, hi;
+            ld8(selfSrc + w * 8, valid, &lo, &hi);
+            st8(selfDst + w * 8, valid, lo, hi);
+          }
+        }
+      }
       bool ok = true;
       for (size_t w = gtid; w < nwords && ok; w += gstride) {
         const size_t valid = min((size_t)8, bytes - w * 8);
@@ -657,7 +687,7 @@ __device__ void fcxMoveBody(const FcxDevComm &dc, const FcxCollArgs &a, int cta,
           }
       }
       epilogue(dc, seq, nctas);
-      return;
+      return;  // what follows is not compiled into the kernel of this kind
     }
     const size_t sub = max((size_t)16384, (pipeBytesOf(dc) / (size_t)max(1, n - 1)) & ~(size_t)15);
     const int chunks = (int)max((size_t)1, (bytes + sub - 1) / sub);
@@ -927,8 +957,9 @@ template <typename TIn, typename TOut>
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxCollKernel(FcxDevComm dc, FcxCollArgs a) {
   fcxCollBody<TIn, TOut>(dc, a, blockIdx.x, gridDim.x);
 }
+template <bool LL>
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxMoveKernel(FcxDevComm dc, FcxCollArgs a) {
-  fcxMoveBody(dc, a, blockIdx.x, gridDim.x);
+  fcxMoveBody<LL>(dc, a, blockIdx.x, gridDim.x);
 }
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxP2pKernel(FcxDevComm dc, FcxP2pArgs g) {
   fcxP2pBody(dc, g, blockIdx.x);
@@ -943,11 +974,12 @@ __global__ void __launch_bounds__(FCX_THREADS, 1) fcxCollEmuKernel(const __grid_
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
   fcxCollBody<TIn, TOut>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
+template <bool LL>
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxMoveEmuKernel(const __grid_constant__ FcxEmuRanks l, int ctasPerRank) {
   __shared__ FcxDevComm dc;
   __shared__ FcxCollArgs a;
   emuRank(l, blockIdx.x / ctasPerRank, &dc, &a);
-  fcxMoveBody(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
+  fcxMoveBody<LL>(dc, a, blockIdx.x % ctasPerRank, ctasPerRank);
 }
 __global__ void __launch_bounds__(FCX_THREADS, 1) fcxP2pEmuKernel(const FcxDevComm *dcs, const FcxP2pArgs *gs, int ctasPerRank) {
   int r = blockIdx.x / ctasPerRank;
@@ -1013,7 +1045,8 @@ extern "C" cudaError_t fcxLaunchColl(const FcxDevComm *dc, const FcxCollArgs *a,
   if (a->kind < 0 || a->kind >= FCX_K_NUM || !kindServes(a)) return cudaErrorInvalidValue;
   if (a->kind == FCX_K_MOVE_ZC || isZcReduceKind(a->kind)) return fcxLaunchZc(dc, a, nctas, s);
   if (isMoveKind(a->kind)) {
-    fcxMoveKernel<<<nctas, FCX_THREADS, 0, s>>>(*dc, *a);
+    if (a->kind == FCX_K_MOVE_LL) fcxMoveKernel<true><<<nctas, FCX_THREADS, 0, s>>>(*dc, *a);
+    else fcxMoveKernel<false><<<nctas, FCX_THREADS, 0, s>>>(*dc, *a);
     return cudaGetLastError();
   }
   if (isLlReduceKind(a->kind)) return fcxLaunchLl(dc, a, nctas, s);
@@ -1039,7 +1072,7 @@ extern "C" cudaError_t fcxLaunchCollEmu(const FcxEmuRanks *l, int nranks, int nc
   void *params[] = {(void *)l, (void *)&nctas};
   if (a->kind == FCX_K_MOVE_ZC || isZcReduceKind(a->kind)) return fcxLaunchZcEmu(l, nranks, nctas, s);
   if (isMoveKind(a->kind))
-    return cudaLaunchCooperativeKernel((const void *)fcxMoveEmuKernel, dim3(nranks * nctas), dim3(FCX_THREADS), params, 0, s);
+    return cudaLaunchCooperativeKernel(a->kind == FCX_K_MOVE_LL ? (const void *)fcxMoveEmuKernel<true> : (const void *)fcxMoveEmuKernel<false>, dim3(nranks * nctas), dim3(FCX_THREADS), params, 0, s);
   if (isLlReduceKind(a->kind)) return fcxLaunchLlEmu(l, nranks, nctas, s);
   if (a->kind == FCX_K_BARRIER) return launchTypedEmu<uint8_t, uint8_t>(*l, nranks, nctas, s);
 #define CALL(TI, TO) launchTypedEmu<TI, TO>(*l, nranks, nctas, s)
