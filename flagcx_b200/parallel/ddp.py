@@ -126,8 +126,9 @@ class DataParallelTrainer:
         self.done_event = torch.cuda.Event()
         self.pre_tail_event = torch.cuda.Event()
         self.split_tail = os.environ.get("FLAGCX_DDP_SPLIT_TAIL", "1") != "0"
-        # Measured on one B200: the per-bucket optimizer beside the backward pass gains nothing (26.7 against
-        # 26.5 ms per step; the AdamW blocks and the GEMMs compete for the same SMs), so it is off by default.
+        # Measured on one B200: the per-bucket optimizer beside the backward pass gains nothing (24.8 to 25.4 against
+        # 24.45 ms per step, with the optimizer on 148, 296 or 1184 CTAs, although registers and shared memory leave
+        # room for both on an SM: the chip is at its power limit), so it is off by default.
         self.overlap_optimizer = os.environ.get("FLAGCX_DDP_OVERLAP_OPT", "0") != "0"
         # the bucket that closes last has nothing left to overlap with: it may take more of the GPU
         self.tail_ctas = int(os.environ.get("FLAGCX_DDP_TAIL_CTAS", "64"))
@@ -306,12 +307,12 @@ class DataParallelTrainer:
         fused LayerNorm forward, 2 x 2 backward (dx; parameter gradients),
         bias-GELU forward + 2 backward (dx; bias gradient); the tcgen05 GEMMs
         of the projections and the LM head (input and weight gradients in one
-        launch, so this is a lower bound where they take two); the final
-        LayerNorm (1 + 2), the loss kernel, and per bucket one all-reduce
+        launch, so this is a lower bound where they take two); the embedding
+        (one kernel each way), the final LayerNorm (1 + 2), the loss kernel, and per bucket one all-reduce
         kernel (more than one rank) and one AdamW kernel (one AdamW kernel in
         all when the optimizer is not overlapped)."""
         L = len(getattr(self.model, "blocks", []))
-        own = L * (2 + 4 + 1 + 2) + (1 + 2) + 1
+        own = L * (2 + 4 + 1 + 2) + 2 + (1 + 2) + 1
         if os.environ.get("FLAGCX_MODEL_GEMM", "own") != "library" and os.environ.get("FLAGCX_MODEL_FUSED_GELU", "1") != "0":
             own -= L  # the GELU of the forward pass runs in the epilogue of the up-projection GEMM
         if os.environ.get("FLAGCX_MODEL_GEMM", "own") != "library":
