@@ -26,6 +26,7 @@
 // faster.
 // Every wait is bounded; a wait that gives up sets the error flag and the kernel drains and returns.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -617,20 +618,23 @@ cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap 
 // nanoseconds; with more than one wave the single CTAs' slices get longer (L2).  Measured, us for pairs / 128 / 64 columns, K whole:
 // 8192 x 1024 x 4096 39.0 / 47.2 / 69.1, 4096 x 4096 x 1024 25.9 / 27.5 / 39.2, 3000 x 2000 x 4096 37.5 / 36.4 / 58.9, 1024 x 4096 x 2048
 // 13.3 / 14.9 / 22.6, 512 x 4096 x 4096 20.7 / 14.3 / 22.1, 1024 x 1024 x 1024 8.5 / 6.1 / 5.5, 333 x 1792 x 4096 19.8 / 13.4 / 12.5.
-// Cut in 2 or 4 as long as all CTAs fit on the SMs at once; it costs two barriers of the cluster and the exchange of the sums.
+// Cut in 2 or 4 as long as all clusters fit on the chip at once; it costs two barriers of the cluster and the exchange of the sums.
+// A cluster's SMs are of one GPC, so 148 SMs hold 74 clusters of two CTAs but not 37 of four (33 on the B200 that was timed): the
+// caller gives both numbers.  One cluster too many is a second wave: 100 rows x K 4096 in 33 / 34 tiles of 64 columns, cut in four
+// 6.8 / 12.1, in two 8.0 / 8.0; of 128 columns 8.5 / 15.1 and 9.6 / 9.6; 74 tiles cut in two 8.5 and 10.5, whole 11.7 and 12.9.
 // 128 columns whole / 2 / 4, then 64 columns whole / 2 / 4: 16 x 512 x 4096 12.1 / 9.5 / 8.0, 11.3 / 8.0 / 6.6; 100 x 4096 x 4096 13.1 / 10.2 /
 // 8.8, 12.3 / 8.7 / -; 333 x 1792 x 4096 13.3 / 10.5 / -, 12.5 / - / -; 128 x 2048 x 2048 8.3 / 7.5 / 7.5, 7.7 / 6.3 / 6.0; but eight slices
 // are in flight at once anyway: 16 x 512 x 1024 5.1 / 6.3 / 6.6, 4.7 / 5.2 / 5.3.
-static int fp8Plan(int M, int N, int nK, int sms, bool cuts, int *cutOut) {
+static int fp8Plan(int M, int N, int nK, int sms, int pairs, int quads, int *cutOut) {
   const int m1 = (M + 127) / 128, m2 = (M + 255) / 256;
   auto waves = [](long long tiles, int slots) { return (double)((tiles + slots - 1) / slots); };
   double best = waves((long long)m2 * ((N + 255) / 256), sms / 2) * (nK * 562.0 + 600);
   int tile = 0, cut = 1;
   for (int bn : {128, 64}) {
     const long long tiles = (long long)m1 * ((N + bn - 1) / bn);
-    for (int c = 1; c <= (cuts && nK >= 12 ? 4 : 1); c *= 2) {
+    for (int c = 1; c <= (nK >= 12 ? 4 : 1); c *= 2) {
       const int per = (nK + c - 1) / c;
-      if (c > 1 && (tiles * c > sms || (c - 1) * per >= nK)) continue;
+      if (c > 1 && (tiles > (c == 2 ? pairs : quads) || (c - 1) * per >= nK)) continue;
       const double w = waves(tiles * c, sms), slice = bn == 128 ? (w > 1 ? 355 : 283) : (w > 1 ? 297 : 246);
       const double exchange = c == 1 ? 0 : bn == 128 ? (c == 2 ? 1890 : 2700) : (c == 2 ? 660 : 1210);
       const double time = w * per * slice + exchange;
@@ -644,11 +648,49 @@ static int fp8Plan(int M, int N, int nK, int sms, bool cuts, int *cutOut) {
   *cutOut = cut;
   return tile;
 }
-extern "C" int fcxGemmFp8Plan(int M, int N, int K, int sms, int *cut) { return fp8Plan(M, N, K / 128, sms, true, cut); }
-// The tile of a long sum that is not cut.
+// The rule by itself: `pairs` clusters of two CTAs or `quads` of four are on the chip at once (0: not cut that way).
+extern "C" int fcxGemmFp8PlanFor(int M, int N, int K, int sms, int pairs, int quads, int *cut) { return fp8Plan(M, N, K / 128, sms, pairs, quads, cut); }
+
+namespace {
+
+// How many clusters of `cut` CTAs the current device holds at once.  Both widths' kernels fill an SM, so one is asked for both.
+// Without a device: eight GPCs of whole pairs of SMs, each of which may leave a pair over.
+int clustersAtOnce(int cut) {
+  static std::atomic<int> known[2][fcxhost::MAX_DEVICES];
+  const int dev = fcxhost::currentDevice(), which = cut == 2 ? 0 : 1;
+  int n = dev < fcxhost::MAX_DEVICES ? known[which][dev].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n - 1;
+  const auto kernel = gemmFp8Kernel<128, true>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cut);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smemBytes(128);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cut;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  n = -1;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes(128)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 0) {
+    cudaGetLastError();
+    return cut == 2 ? smCount() / 2 : std::max(0, smCount() - 16) / 4;
+  }
+  if (dev < fcxhost::MAX_DEVICES) known[which][dev].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+}  // namespace
+
+// The plan of a launch on the current device.
+extern "C" int fcxGemmFp8Plan(int M, int N, int K, int sms, int *cut) {
+  return fcxGemmFp8PlanFor(M, N, K, sms, std::min(clustersAtOnce(2), sms / 2), std::min(clustersAtOnce(4), sms / 4), cut);
+}
+// The tile of a long sum that is not cut, as the tables of timings above have it; launches ask fcxGemmFp8Plan.
 extern "C" int fcxGemmFp8Tile(int M, int N, int sms) {
   int cut;
-  return fp8Plan(M, N, 32, sms, false, &cut);
+  return fp8Plan(M, N, 32, sms, 0, 0, &cut);
 }
 
 extern "C" cudaError_t fcxGemmFp8Blockwise(const void *aq, const float *sa, const void *bq, const float *sb, void *c, int M, int N, int K,
