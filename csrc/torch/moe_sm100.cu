@@ -40,6 +40,7 @@ constexpr int THREADS = 512;
 __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm dc, const FcxMoeParams p) {
   cg::grid_group grid = cg::this_grid();
   const int n = dc.nranks, me = dc.rank, L = p.L, E = n * L, capL = p.cap / L;
+  const bool talk = n > 1 || p.exchange;
   const int entries = p.T * p.K;
   __shared__ int warpTotals[THREADS / 32];
   volatile int *err = p.errFlag;
@@ -77,8 +78,9 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
   __threadfence();
   grid.sync();
 
-  // ---- phase 2: every rank learns the whole count matrix [source][expert]
-  if (blockIdx.x == 0 && (int)threadIdx.x < n) {
+  // ---- phase 2: every rank learns the whole count matrix [source][expert].  One rank alone has it already: no message, no
+  // flag to wait for, and at the end nobody to tell, unless the caller asks for it all the same.
+  if (talk && blockIdx.x == 0 && (int)threadIdx.x < n) {
     const int r = threadIdx.x;
     int *mat = (int *)(dc.heap[r] + p.countMatOff) + me * E;
     for (int e = 0; e < E; e++) mat[e] = p.localCounts[e];
@@ -88,11 +90,11 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
   __shared__ int baseOf[64];  // where this rank's tokens start in expert e's segment
   {
     bool ok = true;
-    if ((int)threadIdx.x < n)
+    if (talk && (int)threadIdx.x < n)
       ok = fcxdev::waitGe(dc, (const uint64_t *)(dc.heap[me] + p.countFlagOff) + threadIdx.x, p.epoch, threadIdx.x, FCX_WAIT_DEVAPI,
                           blockIdx.x, p.epoch);
     if (!__syncthreads_and(ok)) { if (threadIdx.x == 0) *err = 1; }
-    const int *mat = (const int *)(dc.heap[me] + p.countMatOff);
+    const int *mat = talk ? (const int *)(dc.heap[me] + p.countMatOff) : p.localCounts;
     if ((int)threadIdx.x < E) {
       int b = 0, tot = 0;
       for (int r = 0; r < n; r++) {
@@ -102,6 +104,7 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
       }
       baseOf[threadIdx.x] = b;
       if (tot > capL && blockIdx.x == 0) *err = 2;  // an expert's segment would overflow: tokens beyond the capacity are dropped
+      if (!talk && blockIdx.x == 0) p.recvTotal[threadIdx.x] = min(tot, capL);
     }
     __syncthreads();
   }
@@ -136,6 +139,7 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
       if (lane == 0) ((int4 *)(dc.heap[dstRank] + p.infoOff))[pos] = make_int4(me, t, k, 0);
     }
   }
+  if (!talk) return;
   __threadfence_system();
   grid.sync();
 
@@ -159,14 +163,15 @@ __global__ void __launch_bounds__(THREADS, 1) moeDispatchKernel(const FcxDevComm
 // wait for.  Every CTA numbers its own stretch of the entries after counting, by itself, the entries before it per expert
 // (in registers, eight experts to a 64-bit word), so the only order between CTAs is that of the launches around it.  The
 // first row of every warp is already on its way while it counts.  The numbers are those of the cooperative kernel (token
-// order within an expert).  Bound by latency on small batches and by memory on large ones: two CTAs per SM keep 128 KB of
-// rows in flight where the cooperative kernel's 64 CTAs left the copy to 64 SMs.  In us, before and now: 512
-// tokens x 1024, two choices 8.4 / 4.6, 8192 x 4096 68 / 39.
+// order within an expert).  Bound by latency on small batches and by memory on large ones, where 32 warps per SM keep 128 KB of
+// rows in flight.  On 64 SMs, cooperative kernel / this one, us: 512 tokens x 1024 with two choices of 4 experts 7.6 / 3.7, 2048 x
+// 2048 (8 experts) 13.9 / 9.6, 8192 x 4096 64.5 / 51.2; on 148 SMs 7.8 / 3.7, 10.8 / 7.1, 45.1 / 37.8.
 constexpr int LOCAL_CHUNK = 1024;  // most entries of one CTA
-__global__ void __launch_bounds__(THREADS, 2) moeDispatchLocalKernel(const FcxDevComm dc, const FcxMoeParams p) {
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) moeDispatchLocalKernel(const FcxDevComm dc, const FcxMoeParams p) {
   const int E = p.L, capL = p.cap / p.L, entries = p.T * p.K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int WARPS = THREADS / 32;
+  constexpr int WARPS = NT / 32;
   __shared__ int count[64], slotOf[LOCAL_CHUNK], expertOf[LOCAL_CHUNK];
   const int per = (entries + gridDim.x - 1) / gridDim.x;
   const int lo = (int)min((long long)entries, (long long)blockIdx.x * per), hi = min(entries, lo + per);
@@ -182,15 +187,15 @@ __global__ void __launch_bounds__(THREADS, 2) moeDispatchLocalKernel(const FcxDe
     for (int j = 0; j < 8; j++)
       if (lane + 32 * j < vecs) head[j] = src[lane + 32 * j];
   }
-  for (int i = lo + threadIdx.x; i < hi; i += THREADS) expertOf[i - lo] = p.topkIdx[i];
+  for (int i = lo + threadIdx.x; i < hi; i += NT) expertOf[i - lo] = p.topkIdx[i];
   __syncthreads();
   for (int e0 = 0; e0 < E; e0 += 8) {
     // at most 128 entries of a thread between two turns of the outer loop: a byte per expert holds them
-    for (int from = 0; from < lo; from += 128 * THREADS) {
-      const int to = min(lo, from + 128 * THREADS);
+    for (int from = 0; from < lo; from += 128 * NT) {
+      const int to = min(lo, from + 128 * NT);
       uint64_t c = 0;
 #pragma unroll 8
-      for (int i = from + (int)threadIdx.x; i < to; i += THREADS) {
+      for (int i = from + (int)threadIdx.x; i < to; i += NT) {
         const uint32_t d = (uint32_t)(p.topkIdx[i] - e0);
         c += d < 8u ? 1ull << (8 * d) : 0ull;
       }
@@ -350,14 +355,26 @@ __global__ void __launch_bounds__(256) moeCombineKernel(const FcxDevComm dc, con
 
 }  // namespace
 
+// The launch of a dispatch that exchanges nothing: CTAs of moeDispatchLocalKernel (and `threads` of each), or 0 for the cooperative
+// kernel.  `ctas` is the number of SMs that the caller lets the dispatch have, so no more CTAs than that are launched; where their
+// shared memory does not hold the entries, the cooperative kernel has as many CTAs.  A CTA has 16 warps up to eight entries for
+// each (less set-up), 32 beyond (more rows in flight).  16 / 32 warps, us: 4096 entries x 2048 on 148 SMs (1.7 entries per warp of 16)
+// 7.1 / 7.4, on 64 (4) 9.6 / 9.9, 16384 x 4096 on 148 (7) 37.8 / 40.1, on 64 (16) 56.1 / 51.2, 32768 x 1024 on 148 (14) 23.7 / 20.3.
+extern "C" int fcxMoeDispatchPlan(int64_t entries, int ctas, int sms, int *threads) {
+  const int64_t most = std::max(1, std::min(ctas, sms));
+  *threads = entries <= 8 * 16 * most ? 512 : 1024;
+  const int64_t warps = *threads / 32, grid = std::max<int64_t>(1, std::min(most, (entries + warps - 1) / warps));
+  if ((entries + grid - 1) / grid > LOCAL_CHUNK) return 0;
+  return (int)grid;
+}
+
 extern "C" cudaError_t fcxMoeDispatch(const FcxDevComm *dc, const FcxMoeParams *p, int ctas, cudaStream_t s) {
   if (p->H % 8 || p->K < 1 || dc->nranks > FCX_MAX_RANKS || p->L < 1 || dc->nranks * p->L > 64 || p->cap % p->L) return cudaErrorInvalidValue;
   const int sms = fcxhost::smCount();
   if (dc->nranks == 1 && !p->exchange) {
-    // a warp per entry as long as two CTAs per SM hold them; `ctas` is the number of SMs that an exchange may keep busy
-    const int entries = p->T * p->K;
-    const int grid = std::max(std::max(1, (entries + LOCAL_CHUNK - 1) / LOCAL_CHUNK), std::min(2 * sms, (entries + THREADS / 32 - 1) / (THREADS / 32)));
-    return fcxpdl::launchPdl(moeDispatchLocalKernel, grid, THREADS, 0, s, *dc, *p);
+    int threads = 0;
+    const int grid = fcxMoeDispatchPlan((int64_t)p->T * p->K, ctas, sms, &threads);
+    if (grid) return fcxpdl::launchPdl(threads == 512 ? moeDispatchLocalKernel<512> : moeDispatchLocalKernel<1024>, grid, threads, 0, s, *dc, *p);
   }
   ctas = std::max(dc->nranks * p->L, std::min(ctas, sms));  // one CTA per expert at least; all resident: the kernel synchronises the grid
   void *args[] = {(void *)dc, (void *)p};

@@ -55,6 +55,7 @@ class ExpertParallelContext:
     def __init__(self, comm: int, nranks: int, rank: int, tokens: int, hidden: int, ffn: int, topk: int = 2,
                  capacity_factor: float = 1.25, dispatch_ctas: int = 64, device=None, experts_per_rank: int = 1):
         """``tokens``: tokens per rank; ``capacity_factor`` x the balanced load bounds the rows an expert accepts;
+        ``dispatch_ctas``: the dispatch kernel takes at most that many CTAs, one to an SM (one per expert at least where it exchanges);
         ``experts_per_rank``: expert e lives on rank ``e // experts_per_rank`` (at most 64 experts in all)."""
         self.nat = flagcx_b200.native()
         self.comm, self.n, self.rank = comm, nranks, rank
