@@ -21,6 +21,12 @@ def test_plan_keeps_to_the_callers_bound():
             assert grid == 0 or grid * 1024 >= entries  # what a CTA's shared memory holds
 
 
+def test_counting_does_not_grow_with_the_square_of_the_entries():
+    """Every CTA reads all entries before its own stretch: more of them than were timed go to the cooperative kernel."""
+    assert _plan(148 * 1024, 148)[0] == 148 and _plan(148 * 1024 + 1, 148)[0] == 0
+    assert _plan(1 << 20, 1000)[0] == 0 and _plan(65537, 64)[0] == 0 and _plan(8193, 8)[0] == 0
+
+
 def test_timed_choices():
     assert _plan(1024, 64) == (64, 512) and _plan(4096, 64) == (64, 512) and _plan(16384, 148) == (148, 512)
     assert _plan(16384, 64) == (64, 1024) and _plan(32768, 148) == (148, 1024)
