@@ -89,6 +89,11 @@ class _Embedding(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dx):
         (tokens,) = ctx.saved_tensors
+        if torch.is_grad_enabled() and dx.requires_grad:  # create_graph: the same sums as operations with a derivative of their own
+            wte, wpe = ctx.params
+            dwte = torch.ops.aten.embedding_dense_backward(dx, tokens, wte.shape[0], -1, False) if ctx.needs_input_grad[1] else None
+            dwpe = torch.nn.functional.pad(dx.sum(0), (0, 0, 0, wpe.shape[0] - dx.shape[1])) if ctx.needs_input_grad[2] else None
+            return None, dwte, dwpe
         outs, targets = [], []
         for p, need in zip(ctx.params, ctx.needs_input_grad[1:]):
             g = _direct(p) if need else None
@@ -109,8 +114,10 @@ class _Embedding(torch.autograd.Function):
 
 def embed(tokens, wte, wpe):
     """``wte[tokens] + wpe[:T]`` for int64 tokens ``[B, T]``.  bf16 tables whose rows are whole 256-column vectors go through
-    one kernel each way (up to 16384 tokens, see embedding.cu); everything else through the library's embedding."""
-    if _n().embedding_takes(tokens, wte, wpe):
+    one kernel each way (up to 16384 tokens, see embedding.cu); everything else, and whatever is transformed (vmap and the other
+    functional transforms, forward-mode derivatives, tracing), through the library's embedding."""
+    transformed = torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing()
+    if not transformed and _n().embedding_takes(tokens, wte, wpe):
         return _Embedding.apply(tokens, wte, wpe)
     return torch.nn.functional.embedding(tokens, wte) + wpe[:tokens.shape[1]]
 
