@@ -8,8 +8,8 @@ CUDA-event time with the achieved fraction of the measured HBM copy rate
 (MEASURED_PEAKS.json, else 6.65 TB/s).  Cases: adamw, cross_entropy,
 layernorm_fwd, layernorm_bwd, bias_gelu, bias_gelu_bwd, col_sum, emu_allreduce (8 emulated ranks,
 two-shot kernel, one cooperative launch on this GPU), emu_allgather, gemm / gemm_one_cta
-(tcgen05 GEMM, against the measured cuBLAS rate), gemm_fp8 (block-scaled e4m3 GEMM), moe_dispatch and moe_layer
-(expert-parallel kernels on a one-rank communicator), emu_allreduce_zc / emu_allreduce_ll / emu_sendrecv (zero-copy,
+(tcgen05 GEMM, against the measured cuBLAS rate), gemm_fp8 (block-scaled e4m3 GEMM), moe_dispatch, moe_dispatch_local and
+moe_layer (expert-parallel kernels on a one-rank communicator), emu_allreduce_zc / emu_allreduce_ll / emu_sendrecv (zero-copy,
 LL and grouped send/recv kernels on emulated ranks), gemm_dgrad / gemm_wgrad (transposed-operand GEMMs), linear_bwd (both in one launch), gemm_ag /
 gemm_rs (fused all-gather / reduce-scatter GEMMs on a one-rank communicator)."""
 from __future__ import annotations
@@ -119,7 +119,7 @@ def main():
         ms = timed(lambda: lib.call("flagcxEmuCollective", emu, op, kind, 16, s, r, count, 7, 7, ctypes.c_float(1.0), 0, 0, None, st))
         lib.call("flagcxEmuDestroy", emu)
     elif args.case in ("emu_allreduce_zc", "emu_allreduce_ll", "emu_sendrecv"):
-        # the zero-copy all-reduce (plain peer loads, 16 in flight per thread: one GPU has no switch to reduce in),
+        # the zero-copy all-reduce (plain peer loads, eight of 32 bytes in flight per thread: one GPU has no switch to reduce in),
         # the LL all-reduce at 4 KiB, and the grouped send/recv kernel, each as 8 (2) emulated ranks in one launch
         from flagcx_b200.wrapper import FLAGCXLibrary
         lib = FLAGCXLibrary()
@@ -219,9 +219,9 @@ def main():
         print(json.dumps({"case": args.case, "shape": [M, N, K], "ms": round(ms, 4), "tflops": round(tf, 1),
                           "fraction_of_gemm_peak": round(tf / tf_peak, 3), "peak": label, "err": int(err.item())}))
         return
-    elif args.case in ("moe_dispatch", "moe_layer"):
+    elif args.case in ("moe_dispatch", "moe_dispatch_local", "moe_layer"):
         # one-rank communicator: dispatch, grouped expert GEMMs with the row-scattering epilogue, combine; the dispatch
-        # exchanges counts and arrivals as several ranks do (one rank skips that otherwise), with this GPU as its own peer
+        # exchanges counts and arrivals as several ranks do, with this GPU as its own peer; moe_dispatch_local is one rank's own
         import os
         os.environ.setdefault("FLAGCX_HEAP_USER_BYTES", "1G")
         from flagcx_b200.parallel.ep import ExpertParallelContext
@@ -230,20 +230,20 @@ def main():
         comm = lib.flagcxCommInitRank(1, lib.flagcxGetUniqueId(), 0)
         T, H, F, K = 8192, 4096, 2048, 2
         ep = ExpertParallelContext(comm.value, 1, 0, T, H, F, K)
-        ep.exchange = True
+        ep.exchange = args.case != "moe_dispatch_local"
         x = torch.randn(T, H, device="cuda").bfloat16()
         idx = torch.zeros(T, K, dtype=torch.int32, device="cuda")
         wts = torch.rand(T, K, device="cuda")
         w1 = (torch.randn(2 * F, H, device="cuda") * 0.02).bfloat16()
         w2 = (torch.randn(H, F, device="cuda") * 0.02).bfloat16()
-        if args.case == "moe_dispatch":
+        if args.case in ("moe_dispatch", "moe_dispatch_local"):
             state = {"calls": 0}
 
             def disp():
                 par, epoch = state["calls"] & 1, (state["calls"] >> 1) + 1
                 state["calls"] += 1
                 nat.moe_dispatch(comm.value, x, idx, ep.count_mat[par], ep.count_flags[par], ep.recv[par], ep.info[par], ep.disp_done[par],
-                                 epoch, ep.slot, ep.local_counts, ep.recv_total, ep.err, ep.dispatch_ctas, 1, True)
+                                 epoch, ep.slot, ep.local_counts, ep.recv_total, ep.err, ep.dispatch_ctas, 1, ep.exchange)
             ms = timed(disp)
             nbytes = T * K * H * 2 * 2  # every (token, choice) row read once and written once
         else:
