@@ -615,9 +615,11 @@ cudaError_t launchPair(const CUtensorMap &ma, const void *bq, const CUtensorMap 
 
 // Which tile: 0 = 256 x 256 on CTA pairs, 128 or 64 = 128 x that many columns on single CTAs; and how many CTAs of a cluster share
 // one, each with a stretch of K.  The time is about the number of waves times the time of the 128-deep slices of a tile, in
-// nanoseconds; with more than one wave the single CTAs' slices get longer (L2).  Measured, us for pairs / 128 / 64 columns, K whole:
+// nanoseconds; with more than one wave the single CTAs' slices get longer (L2), and the tiles follow one another with a gap, which is what
+// short sums consist of.  Measured, us for pairs / 128 / 64 columns, K whole:
 // 8192 x 1024 x 4096 39.0 / 47.2 / 69.1, 4096 x 4096 x 1024 25.9 / 27.5 / 39.2, 3000 x 2000 x 4096 37.5 / 36.4 / 58.9, 1024 x 4096 x 2048
 // 13.3 / 14.9 / 22.6, 512 x 4096 x 4096 20.7 / 14.3 / 22.1, 1024 x 1024 x 1024 8.5 / 6.1 / 5.5, 333 x 1792 x 4096 19.8 / 13.4 / 12.5.
+// 8192 x 4096 x 128 15.7 / 24.2 / 36.1, x 512 27.0 / 33.5 / 49.6, x 1024 39.9 / 47.8 / 73.0, 2048 x 2048 x 128 5.5 / 5.1 / 6.9.
 // Cut in 2 or 4 as long as all clusters fit on the chip at once; it costs two barriers of the cluster and the exchange of the sums.
 // A cluster's SMs are of one GPC, so 148 SMs hold 74 clusters of two CTAs but not 37 of four (33 on the B200 that was timed): the
 // caller gives both numbers.  One cluster too many is a second wave: 100 rows x K 4096 in 33 / 34 tiles of 64 columns, cut in four
@@ -635,9 +637,9 @@ static int fp8Plan(int M, int N, int nK, int sms, int pairs, int quads, int *cut
     for (int c = 1; c <= (nK >= 12 ? 4 : 1); c *= 2) {
       const int per = (nK + c - 1) / c;
       if (c > 1 && (tiles > (c == 2 ? pairs : quads) || (c - 1) * per >= nK)) continue;
-      const double w = waves(tiles * c, sms), slice = bn == 128 ? (w > 1 ? 355 : 283) : (w > 1 ? 297 : 246);
+      const double w = waves(tiles * c, sms), slice = bn == 128 ? (w > 1 ? 320 : 283) : (w > 1 ? 260 : 246), turn = bn == 128 ? 800 : 600;
       const double exchange = c == 1 ? 0 : bn == 128 ? (c == 2 ? 1890 : 2700) : (c == 2 ? 660 : 1210);
-      const double time = w * per * slice + exchange;
+      const double time = w * per * slice + (w - 1) * turn + exchange;
       if (time < best) {
         best = time;
         tile = bn;

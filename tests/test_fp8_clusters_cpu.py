@@ -58,3 +58,12 @@ def test_timed_choices(lib, m, n, k, want):
 
 def test_short_sums_stay_whole(lib):
     assert _plan(lib, 16, 512, 11 * 128)[1] == 1 and _plan(lib, 16, 512, 16 * 128)[1] > 1
+
+
+# us on CTA pairs / in 128 columns: many waves of a short sum are the gaps between tiles
+@pytest.mark.parametrize("m,n,k", [(8192, 4096, 128),   # 15.7 / 24.2
+                                   (5612, 3904, 256),   # 14.5 / 20.0
+                                   (3589, 3384, 512),   # 14.4 / 16.0
+                                   (8192, 1024, 128)])  # 7.1 / 8.2
+def test_many_short_sums_run_on_pairs(lib, m, n, k):
+    assert _plan(lib, m, n, k) == (0, 1)
