@@ -11,12 +11,16 @@
 //
 // Duplicates are found by looking at all M tokens, which lie in shared memory as 32-bit numbers, 128 at a time: a position
 // whose token occurred before is skipped, the first one collects all of its rows.  That is M^2 / 128 steps of a warp, little
-// beside the rows themselves up to the EMB_MAX_TOKENS positions that the caller keeps to.  A token with many rows (padding,
-// punctuation) is left to the whole CTA, whose warps take a stretch of the positions each.
+// beside the rows themselves up to the EMB_MAX_TOKENS positions that the caller keeps to.  A token with many rows (punctuation) is
+// left to the whole CTA, whose warps take a stretch of the positions each, and one that holds a good part of all positions
+// (padding) to a pair of CTAs, whose warps take every 32nd position each: one SM alone reads about 100 GB/s.
+// Forward and backward, library / one CTA for every token / so, us: 16 x 1024 positions of one token, 2048 columns 570 / 790 / 389; 8
+// x 1024 x 1024, half of the positions one token, 328 / 177 / 78 (256 tokens in the table 165 / 188 / 69).
 //
 // The reference has no model code; this serves the data-parallel benchmark's decoder.
 #include <algorithm>
 #include <cassert>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,6 +29,8 @@
 #include "embedding.h"
 #include "pdl.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace {
 
 using bf16 = __nv_bfloat16;
@@ -32,6 +38,9 @@ using bf16 = __nv_bfloat16;
 constexpr int WARPS = 16;
 constexpr int HEAVY = 8;         // more rows than this are the whole CTA's work
 constexpr int HEAVY_LIST = 128;  // heavy tokens of one CTA; one that finds the list full is worked on by its warp alone
+// More rows than this, and than a quarter of all, are the work of a pair of CTAs.  Fewer, or more of such tokens, are as soon done by
+// one CTA each (8 tokens of 1024 rows of 1024: 49 us, 69 by pairs; 1164 rows 50 and 56).
+constexpr int PAIRED = 2048;
 
 __device__ __forceinline__ void addRow(float *acc, const uint4 &u) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -75,12 +84,12 @@ template <int MAXV>
 __global__ void __launch_bounds__(WARPS * 32, 1) embBwdKernel(const bf16 *dx, const int64_t *tokens, bf16 *dwte, bf16 *dwpe, int M, int T, int C,
                                                               int V) {
   extern __shared__ __align__(16) uint8_t embSmem[];
-  __shared__ int heavy[HEAVY_LIST], nHeavy;
+  __shared__ int heavy[HEAVY_LIST], nHeavy, paired[3], nPaired;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = C / 256;
   float *partial = (float *)embSmem;                // [WARPS][C]
   int *tok = (int *)(partial + (size_t)WARPS * C);  // [M, rounded up to 128]
   const int padded = (M + 127) / 128 * 128;
-  if (threadIdx.x == 0) nHeavy = 0;
+  if (threadIdx.x == 0) nHeavy = nPaired = 0;
   fcxpdl::pdlRelease();
   fcxpdl::pdlWait();
   if (dwte)
@@ -149,6 +158,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) embBwdKernel(const bf16 *dx, co
       int n = 0;
       for (int base = i & ~127; base < M; base += 128) n += __popc(matches(base, t, i, M));
       n = __reduce_add_sync(0xffffffffu, n);
+      if (n > PAIRED && n > M / 4) {
+        if (lane == 0) paired[atomicAdd(&nPaired, 1)] = i;
+        continue;
+      }
       if (n > HEAVY) {
         int at = 0;
         if (lane == 0) at = atomicAdd(&nHeavy, 1);
@@ -172,14 +185,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) embBwdKernel(const bf16 *dx, co
       addInto(dwpe, r);
     }
   }
-  __syncthreads();
-  const int todo = min(nHeavy, HEAVY_LIST);
-  for (int h = 0; h < todo; h++) {
-    const int i = heavy[h], t = tok[i];
-    const int per = (M - i + WARPS - 1) / WARPS, from = min(M, i + warp * per), to = min(M, from + per);
-    clear();
-    collect(t, from, to);
-    float *mine = partial + (size_t)warp * C;
+  auto leave = [&](int w) {
+    float *mine = partial + (size_t)w * C;
 #pragma unroll
     for (int v = 0; v < MAXV; v++)
       if (v < nv) {
@@ -187,6 +194,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1) embBwdKernel(const bf16 *dx, co
         d[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
         d[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
       }
+  };
+  __syncthreads();
+  const int todo = min(nHeavy, HEAVY_LIST);
+  for (int h = 0; h < todo; h++) {
+    const int i = heavy[h], t = tok[i];
+    const int per = (M - i + WARPS - 1) / WARPS, from = min(M, i + warp * per), to = min(M, from + per);
+    clear();
+    collect(t, from, to);
+    leave(warp);
     __syncthreads();
     for (int c = threadIdx.x; c < C; c += WARPS * 32) {
       float s = 0.f;
@@ -197,6 +213,36 @@ __global__ void __launch_bounds__(WARPS * 32, 1) embBwdKernel(const bf16 *dx, co
     }
     __syncthreads();
   }
+  if (M <= PAIRED) return;  // launched without clusters
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  const int rank = (int)cluster.block_rank();
+  for (int r = 0; r < 2; r++) {
+    const int many = *cluster.map_shared_rank(&nPaired, r);
+    for (int h = 0; h < many; h++) {
+      const int i = *cluster.map_shared_rank(&paired[h], r), t = tok[i];
+      clear();
+      const int turn = rank * WARPS + warp;  // of 32 warps
+      for (int base = i & ~31; base < M; base += 1024) {
+        const int j = base + turn + 32 * lane;
+        for (unsigned any = __ballot_sync(0xffffffffu, j >= i && j < M && tok[j] == t); any; any &= any - 1) take(base + turn + 32 * (__ffs(any) - 1));
+      }
+      leave(warp);
+      cluster.sync();
+      for (int c = rank * (C / 2) + threadIdx.x; c < (rank + 1) * (C / 2); c += WARPS * 32) {  // half of the columns each
+        float s = 0.f;
+        for (int q = 0; q < 2; q++) {
+          const float *part = cluster.map_shared_rank(partial, q) + c;
+#pragma unroll
+          for (int w = 0; w < WARPS; w++) s += part[(size_t)w * C];
+        }
+        bf16 *dst = dwte + (size_t)t * C + c;
+        *dst = __float2bfloat16_rn(__bfloat162float(*dst) + s);
+      }
+      cluster.sync();
+    }
+  }
+  cluster.sync();  // nobody's shared memory goes before it has been read
 }
 
 }  // namespace
@@ -216,12 +262,13 @@ cudaError_t fcxEmbeddingBwd(const void *dx, const int64_t *tokens, void *dwte, v
   if (!fcxEmbeddingTakes(M, C) || T <= 0 || M % T) return cudaErrorInvalidValue;
   if (((uintptr_t)dx | (uintptr_t)dwte | (uintptr_t)dwpe) & 15) return cudaErrorInvalidValue;
   const size_t smem = (size_t)WARPS * C * 4 + (size_t)(M + 127) / 128 * 128 * 4;  // at most 128 + 64 KB
-  const int grid = std::max(1, std::min(fcxhost::smCount(), (std::max(M, T) + WARPS - 1) / WARPS));
+  int grid = std::min(fcxhost::smCount(), (M + WARPS - 1) / WARPS);  // M >= T
+  if (M > PAIRED) grid &= ~1;
   auto run = [&](auto kernel, int which) {
     static fcxhost::OncePerDevice once[2];
     const cudaError_t e = once[which]([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
     if (e != cudaSuccess) return e;
-    return fcxpdl::launchPdl(kernel, grid, WARPS * 32, smem, s, (const bf16 *)dx, tokens, (bf16 *)dwte, (bf16 *)dwpe, M, T, C, V);
+    return fcxpdl::launchPdlAttr(kernel, grid, WARPS * 32, smem, dim3(M > PAIRED ? 2 : 0, 1, 1), s, (const bf16 *)dx, tokens, (bf16 *)dwte, (bf16 *)dwpe, M, T, C, V);
   };
   return C <= 1024 ? run(embBwdKernel<4>, 0) : run(embBwdKernel<8>, 1);
 }
