@@ -97,10 +97,11 @@ __device__ __forceinline__ void zcFenceBeforeClose() { __threadfence_system(); }
 
 // ---------------------------------------------------------------- reducing kinds
 
-// `cnt` 32-byte pieces from `first` on for exactly P ranks, everything 32-byte aligned.  A thread has eight loads of 32 bytes
-// (pieces x ranks) in flight.  A GPU that stands in for all ranks at 25 MB (the loop alone, 16 CTAs per rank): 8 ranks 84 us with
-// two alternating batches of eight 16-byte loads, 72 with one of eight 32-byte loads; 4 ranks 54 and 42.
-template <typename TIn, int U, int P>
+// `cnt` 32-byte pieces from `first` on for exactly P ranks, everything 32-byte aligned, or (not WIDE) 16-byte aligned and
+// each piece in two accesses.  A thread has eight loads of 32 bytes (pieces x ranks) in flight.  A GPU that stands in for all ranks at 25 MB (the loop alone, 16 CTAs per rank): 8 ranks 84 us with
+// two alternating batches of eight 16-byte loads, 72 with one of eight 32-byte loads; 4 ranks 54 and 42.  Not 32-byte aligned, the
+// whole all-reduce of 8 ranks: 112 us so, 126 in one batch of eight 16-byte loads, 92 in pieces of two.
+template <typename TIn, int U, int P, bool WIDE>
 __device__ __forceinline__ void zcReduceWide(const FcxCollArgs &a, const char *const *src, char *const *dst, int nd, size_t first, size_t cnt,
                                              size_t gtid, size_t gstride) {
   using Acc = typename Elem<TIn>::Acc;
@@ -115,7 +116,17 @@ __device__ __forceinline__ void zcReduceWide(const FcxCollArgs &a, const char *c
     for (int i = 0; i < U; i++)
       if (u + i * gstride < end) {
 #pragma unroll
-        for (int p = 0; p < P; p++) raw[i][p] = ld32(s[p] + (u + i * gstride) * 32);
+        for (int p = 0; p < P; p++) {
+          const char *at = s[p] + (u + i * gstride) * 32;
+          if constexpr (WIDE) {
+            raw[i][p] = ld32(at);
+          } else {
+            union { uint4 q[2]; Vec32 v; } w;
+            w.q[0] = ld16(at);
+            w.q[1] = ld16(at + 16);
+            raw[i][p] = w.v;
+          }
+        }
       }
 #pragma unroll
     for (int i = 0; i < U; i++)
@@ -135,33 +146,44 @@ __device__ __forceinline__ void zcReduceWide(const FcxCollArgs &a, const char *c
         for (int e = 0; e < G; e++) acc[e] = finish<Acc>(acc[e], a.redop, P, a.scale);
         union { uint4 q[2]; Vec32 v; } packed;
         packUnit<TIn, G>(acc, packed.q);
-        for (int k = 0; k < nd; k++) st32(dst[k] + (u + i * gstride) * 32, packed.v);
+        for (int k = 0; k < nd; k++) {
+          char *at = dst[k] + (u + i * gstride) * 32;
+          if constexpr (WIDE) {
+            st32(at, packed.v);
+          } else {
+            st16(at, packed.q[0]);
+            st16(at + 16, packed.q[1]);
+          }
+        }
       }
   }
 }
 
 // Units [first, first + cnt) of 16 bytes for exactly P ranks whose buffers all start `m` bytes past a 16-byte boundary, into
-// 16-byte aligned destinations.  A thread has U x P (eight) loads in flight.  A unit lies in two blocks of the source, the second
-// of which the next lane has loaded; with m > 0 the block behind the last unit's must exist.  (Element by element, as buffers that
-// were not 16-byte aligned had it before, a reduce-scatter of 4 x 1500001 fp32 took 143 us and takes 79, of 8 x 200003 bf16 42 and 38.)
+// 16-byte aligned destinations.  A thread has U x P (eight) loads in flight.  With m > 0 a unit lies in two blocks of the source, the
+// second of which the next lane has loaded: a warp takes 31 units and its last lane loads a block only (were it to load the 32nd unit's
+// second block itself, that load would be waited for in the middle of the sums).  The block behind the last unit's must exist.
+// Reduce-scatter, element by element (as all buffers that were not 16-byte aligned once were) / with that load in the middle / so, us:
+// 4 x 1500001 fp32 on 16 CTAs 144 / 81 / 71, 4 x 113463 on 3 38 / 44 / 33, 8 x 158030 on 4 70 / 76 / 52, 8 x 200003 bf16 on 16 40 / 36 / 33.
 template <typename TIn, int U, int P>
 __device__ __forceinline__ void zcReduceShifted(const FcxCollArgs &a, const char *const *src, char *const *dst, int nd, size_t first, size_t cnt, int m,
                                                 size_t gtid, size_t gstride) {
   using Acc = typename Elem<TIn>::Acc;
   constexpr int G = 16 / (int)sizeof(TIn);
   const size_t end = first + cnt, blocks = end + (m ? 1 : 0);
-  const int lane = threadIdx.x & 31;
-  for (size_t u0 = first + gtid; u0 - lane < end; u0 += U * gstride) {  // a whole warp goes round together
+  const int lane = threadIdx.x & 31, lanes = m ? 31 : 32;
+  const size_t mine = gtid / 32 * lanes + lane, stride = gstride / 32 * lanes;
+  for (size_t u0 = first + mine; u0 - lane < end; u0 += U * stride) {  // a whole warp goes round together
     uint4 raw[U][P];
 #pragma unroll
     for (int i = 0; i < U; i++)
-      if (u0 + i * gstride < blocks) {
+      if (u0 + i * stride < blocks) {
 #pragma unroll
-        for (int p = 0; p < P; p++) raw[i][p] = ld16(src[p] - m + (u0 + i * gstride) * 16);
+        for (int p = 0; p < P; p++) raw[i][p] = ld16(src[p] - m + (u0 + i * stride) * 16);
       }
 #pragma unroll
     for (int i = 0; i < U; i++) {
-      const size_t u = u0 + i * gstride;
+      const size_t u = u0 + i * stride;
       Acc acc[G];
 #pragma unroll
       for (int p = 0; p < P; p++) {
@@ -173,7 +195,6 @@ __device__ __forceinline__ void zcReduceShifted(const FcxCollArgs &a, const char
           hi.y = __shfl_down_sync(0xffffffffu, w.v.y, 1);
           hi.z = __shfl_down_sync(0xffffffffu, w.v.z, 1);
           hi.w = __shfl_down_sync(0xffffffffu, w.v.w, 1);
-          if (lane == 31 && u < end) hi = ld16(src[p] - m + (u + 1) * 16);
           w.v = shiftBlocks(w.v, hi, m);
         }
 #pragma unroll
@@ -182,7 +203,7 @@ __device__ __forceinline__ void zcReduceShifted(const FcxCollArgs &a, const char
           acc[e] = p == 0 ? x : applyOp<Acc>(acc[e], x, a.redop);
         }
       }
-      if (u < end) {
+      if (lane < lanes && u < end) {
 #pragma unroll
         for (int e = 0; e < G; e++) acc[e] = finish<Acc>(acc[e], a.redop, P, a.scale);
         uint4 packed;
@@ -268,16 +289,18 @@ __device__ __forceinline__ void zcReduceRange(const FcxDevComm &dc, const FcxCol
     const bool ranks = n == 2 || n == 4 || n == 8;
     // 32-byte pieces once every thread has one: below, more threads with half of the work each are sooner done (8 ranks x 20000
     // bf16 25.4 us in units of 16 bytes, 26.6 in pieces of 32)
-    if (ranks && ((orS | orD) & 31u) == 0 && firstPlain == 0 && nfull / 2 >= gstride) {
+    if (ranks && alS && alD && firstPlain == 0 && nfull / 2 >= gstride) {
       const size_t cnt = nfull / 2;
-      if (n == 2) zcReduceWide<TIn, 4, 2>(a, src, dst, nd, 0, cnt, gtid, gstride);
-      else if (n == 4) zcReduceWide<TIn, 2, 4>(a, src, dst, nd, 0, cnt, gtid, gstride);
-      else zcReduceWide<TIn, 1, 8>(a, src, dst, nd, 0, cnt, gtid, gstride);
+      const bool wide = ((orS | orD) & 31u) == 0;
+      if (n == 2) wide ? zcReduceWide<TIn, 4, 2, true>(a, src, dst, nd, 0, cnt, gtid, gstride) : zcReduceWide<TIn, 4, 2, false>(a, src, dst, nd, 0, cnt, gtid, gstride);
+      else if (n == 4) wide ? zcReduceWide<TIn, 2, 4, true>(a, src, dst, nd, 0, cnt, gtid, gstride) : zcReduceWide<TIn, 2, 4, false>(a, src, dst, nd, 0, cnt, gtid, gstride);
+      else wide ? zcReduceWide<TIn, 1, 8, true>(a, src, dst, nd, 0, cnt, gtid, gstride) : zcReduceWide<TIn, 1, 8, false>(a, src, dst, nd, 0, cnt, gtid, gstride);
       firstPlain = 2 * cnt;  // at most one whole and one ragged unit are left for the path below
-    } else if (ranks && alD && (apart & 15u) == 0 && nfull > firstPlain && (m == 0 || nfull >= 2 * gstride)) {
+    } else if (ranks && alD && (apart & 15u) == 0 && nfull > firstPlain && (m == 0 || nfull >= 3 * gstride)) {
       // With m > 0 the block before the first unit's bytes and the one behind the last unit's belong to the buffer's edges:
-      // those units are left to the path below, which is the better one for all of them while a thread has less than two
-      // (reduce-scatter, 8 ranks x 20011 bf16 25.1 us there, 28.3 here, but 200003 42.6 and 37.4).
+      // those units are left to the path below, which is the better one for all of them while a thread has less than three
+      // (reduce of 27752 fp16 on 2 ranks, 2.3 units each, 15.7 us there, 16.7 here; reduce-scatter of 200003 bf16 on 8, 3.1 each, 40.4
+      // and 32.5).
       const size_t lo = firstPlain, cnt = nfull - lo - (m ? 2 : 0);
       const size_t from = lo + (m ? 1 : 0);
       if (n == 2) zcReduceShifted<TIn, 4, 2>(a, src, dst, nd, from, cnt, m, gtid, gstride);
@@ -313,11 +336,6 @@ __device__ __forceinline__ void zcReduceRange(const FcxDevComm &dc, const FcxCol
   };
   // the threads that had least of the bulk take what is left of it
   const size_t rest = firstPlain ? gstride - 1 - gtid : gtid;
-  if (edgeUnit != ~(size_t)0 && rest == 3) {  // up to three units lie behind the bulk
-    AI acc[G];
-    gather(edgeUnit, acc);
-    emit(edgeUnit, acc);
-  }
   size_t u = firstPlain + rest;
   for (; u + gstride < nunits; u += 2 * gstride) {
     AI acc0[G], acc1[G];
@@ -326,10 +344,14 @@ __device__ __forceinline__ void zcReduceRange(const FcxDevComm &dc, const FcxCol
     emit(u, acc0);
     emit(u + gstride, acc1);
   }
-  for (; u < nunits; u += gstride) {
+  bool edge = edgeUnit != ~(size_t)0 && rest == 3;  // up to three units lie behind the bulk
+  while (u < nunits || edge) {
+    const size_t v = u < nunits ? u : edgeUnit;
+    edge = edge && u < nunits;
+    u += gstride;
     AI acc[G];
-    gather(u, acc);
-    emit(u, acc);
+    gather(v, acc);
+    emit(v, acc);
   }
 }
 
