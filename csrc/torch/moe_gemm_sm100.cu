@@ -57,12 +57,13 @@ struct GroupParams {
 };
 
 // 256 or 128 accumulator columns per tile for `rowBlocks` 256-row blocks, `cols` columns and sums of length K.  Narrow tiles
-// where they take no more waves.  Otherwise a narrow wave costs about 0.7 to 0.85 of a wide one, which more waves (3 for 2, 5
+// where they take no more waves.  Otherwise a narrow wave costs about 0.6 to 0.75 of a wide one, which more waves (3 for 2, 5
 // for 3, up to twice as many) eat up, except for short sums of the gate / up product, whose wide tiles spend their time on
-// the activation.  Measured with cold weights, narrow / wide in us: gate / up
-// 512 tokens of 1024 columns (4 experts, F 2048) 28.4 / 37.2, 256 of 768 (4, 1024) 11.4 / 14.2, 1000 of 1536 (8, 1536) 36.7 / 38.0, 470 of 2048
-// (8, 2304) 52.0 / 48.9, 700 of 1024 (2, 4096) 32.7 / 27.5, 900 of 3072 (4, 3072) 84.6 / 63.5; down, in the same order, 26.4 / 29.1, 20.2 /
-// 19.9, 32.1 / 29.1, 39.0 / 34.1, 34.3 / 38.0, 55.7 / 50.8.
+// the activation.  Measured with cold weights, 8 row blocks, narrow / wide in us.  Gate / up, 3:2 waves: K 256 14.0 / 16.2, 512 15.4 /
+// 17.9, 768 17.5 / 19.5, 1024 20.2 / 21.2, 1088 21.1 / 21.6, 1280 23.5 / 23.7, 1536 26.2 / 26.2, 2048 32.9 / 31.7, 3328 47.9 / 44.0; 5:3
+// waves: K 256 19.3 / 21.0, 512 21.2 / 22.8, 576 21.7 / 23.2, 768 23.7 / 24.6, 1024 28.4 / 26.6; 2:1 K 1024 15.8 / 15.8, 3328 34.2 / 28.0.
+// Down, 3:2: K 512 23.7 / 22.2, 1024 29.8 / 27.4, 2816 52.2 / 45.3, 5632 85.0 / 75.2; 1:1 K 512 18.2 / 18.8, 1024 20.3 / 20.4, 2816 27.1 /
+// 29.8.  Both lines could lie a little higher (5:3 up to K 768, 3:2 up to 1280); what that would win is 2 to 6 %.
 __host__ __device__ inline int moeTileColumns(long long rowBlocks, int cols, int K, bool up, int pairs) {
   const long long wide = (rowBlocks * ((cols + 255) / 256) + pairs - 1) / pairs, narrow = (rowBlocks * ((cols + 127) / 128) + pairs - 1) / pairs;
   const int tenths = !up || K > 1024 ? 10 : K > 512 ? 15 : 17;  // narrow waves per ten wide ones that still pay
